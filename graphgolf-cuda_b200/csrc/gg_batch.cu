@@ -10,22 +10,29 @@
 // folded into per-thread popcounts and one __syncthreads_or per level.  The grid
 // barrier of the single-graph path is not needed: a task never leaves its CTA.
 //
-// Affected sources (default): per base, one pass of the same kernel also writes
-// the base's distance matrix as 4 bit-planes, from which every source's distance
-// sum and eccentricity follow.  A candidate then searches only from the sources
-// its 2-opt can affect (the test of gg_inc.cu: a removed edge between
-// consecutive BFS levels whose deeper end has no other parent, or an added edge
-// between vertices whose distances differ by 2 or more); its result is the base's
-// total minus those sources' old sums plus their new sums, and the larger of their
-// new eccentricities and the others' old ones.  Bases that are not symmetric,
-// not connected or of diameter above 15 (and the histogram pass) search every
-// source.  GG_BATCH_FULL=1 searches every source for every candidate.
+// Near sources (default): per base, one pass of the single-graph engine also writes the
+// base's distance matrix as 4 bit-planes, from which every source's distance sum and
+// eccentricity follow.  A candidate then searches only from the set T of sources that
+//   * its 2-opt can affect (the test of gg_inc.cu: a removed edge between consecutive
+//     BFS levels whose deeper end has no other parent, or an added edge between vertices
+//     whose distances differ by 2 or more), and that
+//   * lie within floor((diameter - 1) / 2) of one of its four endpoints.
+// A pair whose distance changes has a shortest path, old or new, no longer than the old
+// diameter through a changed edge, so one of the two lies that near to an endpoint of it
+// (in the base graph) -- and both are affected.  The distance matrices are symmetric, so
+// with w = 1 for v in T and 2 for the others
+//   new total = old total + sum over s in T, every v, of w(v) (new - old distance),
+// and every changed pair is seen.  T is 116 of 1024 sources (d = 6), 442 of 3000 (d = 4),
+// 221 of 4096 (d = 8) on average, against 406, 1859 and 1116 affected ones.
+// The diameter is the larger of the largest new distance from T and the largest old
+// distance between vertices outside T.  Bases that are not symmetric, not connected or of
+// diameter above 15, candidates whose removed edges the base does not hold (or not
+// equally often at both ends) and the histogram pass search every source;
+// GG_BATCH_FULL=1 makes every candidate do so.
 //
-// Task order: t -> chunk = maxchunks-1 - t / n_cand, cand = t % n_cand, so the
-// extra chunks of the largest bases come first and the common chunks fill the
-// tail (largest-first scheduling with no task list on the host).  Both n_cand and
-// maxchunks are read from device memory, so one captured CUDA graph serves every
-// batch size up to the capacity it was captured for.
+// batch_select finds each candidate's sources and cuts them into work units; the units
+// come off one counter, and the candidate and base counts are read from device memory, so
+// one captured CUDA graph serves every batch size up to the capacity it was captured for.
 #include "gg.h"
 #include "gg_internal.h"
 #include "gg_planes.cuh"
@@ -53,29 +60,45 @@ struct BatchBase {
     int n, d;
     int log_nc;           // chunks (of 128 sources) per task row = 1 << log_nc
     int chunks;           // tasks per candidate = ceil(n / (128 << log_nc))
-    // affected-source mode (valid != 0)
+    // near-source mode (valid != 0)
     const uint4 *planes;  // [kPlanes][n][cols]: bit k of dist(source, vertex)
-    unsigned cols;        // chunks << log_nc
+    unsigned cols;        // plane columns of 128 sources
     const unsigned *rowsum;  // [n]: distance sum of each source
     const unsigned *ecc;     // [n]: eccentricity of each source
+    const unsigned *top;     // [n]: vertices at distance `levels` from each source
     unsigned long long total, reached;  // the base's own counts
+    unsigned long long at_top;          // ordered pairs at distance `levels`
     int levels;
+    int radius;           // floor((levels - 1) / 2)
     int valid;            // symmetric, connected, diameter <= 15
 };
 
-// Per candidate, from the affected-source test.
-struct IncCand {
-    unsigned long long old_sum;   // base distance sums of the affected sources
-    unsigned count;               // affected sources (the candidate's search list)
-    unsigned max_other;           // largest eccentricity among the other sources
-    int full;                     // search every source instead
-    int pad;
+// How a candidate is scored.
+enum { kNear = 0, kFull = 1, kBase = 2 };
+
+// A candidate's state between the launches of one evaluation.
+struct CandState {
+    unsigned long long old_sum;   // base distance sums of T
+    unsigned long long tt_sum;    // base distances within T
+    unsigned count;               // |T|
+    unsigned tops;                // pairs (T, any) at distance `levels` of the base
+    unsigned groups_done;         // blocks of batch_select that finished the candidate
+    int mode;
+};
+
+// A work unit: `ns` sources of a candidate from `first` on (entries of its list, or
+// vertices for a full search), rows of 1 << log_nc chunks.
+struct Unit {
+    int cand;
+    int first;
+    int ns;
+    int log_nc;
 };
 
 struct BatchCtl {
-    unsigned task_ctr;
+    unsigned unit_ctr;    // work units taken
     int n_cand;
-    int max_chunks;
+    int n_units;          // work units
     int bad;              // set by batch_reset when a candidate is outside the domain
     int n_bases;          // registered bases
     int bad_index;        // lowest index of such a candidate (INT_MAX: none)
@@ -90,9 +113,13 @@ struct BatchArgs {
     BatchCtl *ctl;
     unsigned *hist;       // nullptr, or [n][hist_k]: per-vertex new pairs at levels 1..hist_k
     int hist_k;           // (only meaningful for a launch of one candidate)
-    IncCand *inc;         // nullptr: every candidate searches every source
-    uint16_t *lists;      // [cand][list_stride]: affected sources
+    CandState *cs;        // [cand]
+    uint16_t *lists;      // [cand][list_stride]: the sources of T
     int list_stride;
+    uint32_t *tbits;      // [cand][tbits_stride]: bit v: v in T
+    int tbits_stride;
+    Unit *units;
+    int force_full;       // every candidate searches every source
 };
 
 __device__ __forceinline__ uint4 z4() { return make_uint4(0u, 0u, 0u, 0u); }
@@ -123,16 +150,113 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, unsigned phase) {
 
 constexpr long long kCopyWaitNs = 2000000000ll;   // 2 s: a copy of at most 128 KB never takes that
 
+// The four pull entries a 2-opt replaces: row r[i] lists t[i] in place of f[i].
+struct SwapRows {
+    int r[4], f[4], t[4];
+    __device__ __forceinline__ explicit SwapRows(const gg_swap &s) {
+        r[0] = s.a; r[1] = s.b; r[2] = s.c; r[3] = s.d;
+        f[0] = s.b; f[1] = s.a; f[2] = s.d; f[3] = s.c;
+        t[0] = s.mode ? s.d : s.c; t[1] = s.mode ? s.c : s.d;
+        t[2] = s.mode ? s.b : s.a; t[3] = s.mode ? s.a : s.b;
+    }
+};
+
+// The d neighbour ids of a row in shared memory, in the widest loads its alignment
+// allows (rows start at multiples of 2 d bytes).
+template <int D>
+__device__ __forceinline__ void row_ids(const uint16_t *ar, unsigned (&id)[D]) {
+    if constexpr (D % 8 == 0) {
+#pragma unroll
+        for (int k = 0; k < D / 8; ++k) {
+            const uint4 q = reinterpret_cast<const uint4 *>(ar)[k];
+            id[8 * k] = q.x & 0xffffu; id[8 * k + 1] = q.x >> 16;
+            id[8 * k + 2] = q.y & 0xffffu; id[8 * k + 3] = q.y >> 16;
+            id[8 * k + 4] = q.z & 0xffffu; id[8 * k + 5] = q.z >> 16;
+            id[8 * k + 6] = q.w & 0xffffu; id[8 * k + 7] = q.w >> 16;
+        }
+    } else if constexpr (D % 4 == 0) {
+#pragma unroll
+        for (int k = 0; k < D / 4; ++k) {
+            const uint2 q = reinterpret_cast<const uint2 *>(ar)[k];
+            id[4 * k] = q.x & 0xffffu; id[4 * k + 1] = q.x >> 16;
+            id[4 * k + 2] = q.y & 0xffffu; id[4 * k + 3] = q.y >> 16;
+        }
+    } else if constexpr (D % 2 == 0) {
+#pragma unroll
+        for (int k = 0; k < D / 2; ++k) {
+            const unsigned q = reinterpret_cast<const unsigned *>(ar)[k];
+            id[2 * k] = q & 0xffffu; id[2 * k + 1] = q >> 16;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < D; ++k) id[k] = ar[k];
+    }
+}
+
+// One level of a unit: nxt = cur | OR of the neighbours' cur, every row.  Bound by the
+// shared-memory gathers: random 16-byte rows put 8 lanes on 2.6 of 8 bank groups.  cnt: new pairs
+// of the thread, wcnt: the same weighted (1 where bit v of tb is set, else 2).
+// D > 0: the degree at compile time, a row's gathers all in flight together.
+template <int D>
+static __device__ __forceinline__ void level_pass(const uint4 *cur, uint4 *nxt, const uint16_t *adj, const int d,
+                                               const int items, const int lnc, const uint32_t *tb, unsigned *hist,
+                                               const int hist_k, const int L, unsigned &cnt_out, unsigned &wcnt_out) {
+    const int nC = 1 << lnc;
+    unsigned cnt = 0u, wcnt = 0u;
+    for (int t = threadIdx.x; t < items; t += kBatchBlock) {
+        const int v = t >> lnc, c = t & (nC - 1);
+        const uint4 own = cur[t];
+        uint4 out = own;
+        if ((own.x & own.y & own.z & own.w) != 0xffffffffu) {
+            uint4 acc = z4();
+            const uint16_t *ar = adj + v * d;
+            if constexpr (D > 0) {
+                unsigned id[D];
+                row_ids<D>(ar, id);
+#pragma unroll
+                for (int i = 0; i < D; ++i) {
+                    const uint4 x = cur[(id[i] << lnc) + c];
+                    acc.x |= x.x; acc.y |= x.y; acc.z |= x.z; acc.w |= x.w;
+                }
+            } else {
+                for (int i = 0; i < d; ++i) {
+                    const uint4 x = cur[((int)ar[i] << lnc) + c];
+                    acc.x |= x.x; acc.y |= x.y; acc.z |= x.z; acc.w |= x.w;
+                }
+            }
+            out = make_uint4(own.x | acc.x, own.y | acc.y, own.z | acc.z, own.w | acc.w);
+            const unsigned pc = __popc(acc.x & ~own.x) + __popc(acc.y & ~own.y) + __popc(acc.z & ~own.z) +
+                                __popc(acc.w & ~own.w);
+            cnt += pc;
+            wcnt += pc << (((tb[v >> 5] >> (v & 31)) & 1u) ^ 1u);
+            if (hist && L <= hist_k && pc) atomicAdd(hist + (size_t)v * hist_k + (L - 1), pc);
+        }
+        nxt[t] = out;
+    }
+    cnt_out = cnt;
+    wcnt_out = wcnt;
+}
+
+// The first levels of a unit of few sources from the other side: source j's walk ends of
+// length L (d^L of them) get bit j, the ones not set before are its new pairs.  A pass
+// reads d + 2 rows of 16 bytes per vertex whatever is new; a walk end costs one atomic and
+// L dependent id loads, so the walk takes the levels with at most kWalkItems ends a row.
+//
+// batch_kernel and its three small launches, 2048 x (n=1024, d=6) + 512 x (n=3000, d=4)
+// candidates: 2243 us a call with every affected source searched (2020 us of it here), 720
+// (632) with T; 32 x (n=4096, d=8): 215 (162) and 90 us (45).
+constexpr int kWalkItems = 5;   // walk ends of all sources, at most this many times the rows
+
 __global__ void __launch_bounds__(kBatchBlock, 1) batch_kernel(const BatchArgs a) {
     extern __shared__ uint4 sm[];
-    __shared__ unsigned s_task;
+    __shared__ unsigned s_unit;
     __shared__ unsigned long long s_tot[kBatchBlock / 32], s_reach[kBatchBlock / 32];
+    __shared__ unsigned s_cnt[3];
     __shared__ __align__(8) uint64_t s_bar;   // completion of the adjacency copy
     __shared__ int s_late;
     if (a.ctl->bad) return;   // batch_reset rejected a candidate: index nothing
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n_cand = a.ctl->n_cand, max_chunks = a.ctl->max_chunks;
-    const unsigned n_tasks = (unsigned)n_cand * (unsigned)max_chunks;
+    const unsigned n_units = (unsigned)a.ctl->n_units;
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_addr(&s_bar)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -141,38 +265,55 @@ __global__ void __launch_bounds__(kBatchBlock, 1) batch_kernel(const BatchArgs a
     unsigned phase = 0;
 
     for (;;) {
-        if (tid == 0) s_task = atomicAdd(&a.ctl->task_ctr, 1u);
+        if (tid == 0) s_unit = atomicAdd(&a.ctl->unit_ctr, 1u);
         __syncthreads();
-        const unsigned task = s_task;
-        if (task >= n_tasks) return;
-        const int cand = (int)(task % (unsigned)n_cand);
-        const int chunk = max_chunks - 1 - (int)(task / (unsigned)n_cand);
+        const unsigned u = s_unit;
+        if (u >= n_units) return;
+        const Unit un = a.units[u];
+        const int cand = un.cand, lnc = un.log_nc, ns = un.ns;
         const gg_swap sw = a.cands[cand];
-        const BatchBase B = a.bases[sw.base];
-        const int n = B.n, d = B.d, lnc = B.log_nc, nC = 1 << lnc;
-        const int S = 128 << lnc;
-        // sources of this candidate: every vertex, or its affected-source list
-        const bool full = a.inc == nullptr || a.inc[cand].full;
-        const int count = full ? n : (int)a.inc[cand].count;
-        if (chunk * S >= count) {  // this candidate has fewer chunks
-            __syncthreads();
-            continue;
-        }
-        const int s0 = chunk * S;
-        const int ns = min(S, count - s0);
-        const int items = n << lnc;
+        const BatchBase &B = a.bases[sw.base];
+        const int n = B.n, d = B.d, nC = 1 << lnc;
+        const bool full = a.cs[cand].mode != kNear;
+        const int items = n << lnc, twords = (n + 31) / 32;
+        const uint16_t *lst = a.lists + (size_t)cand * a.list_stride + un.first;   // (not full)
 
-        // shared memory: adjacency (uint16, padded to 16 bytes), then two bitsets.
-        // The base's packed rows arrive by one bulk copy; every thread waits on the
-        // mbarrier (bounded: past kCopyWaitNs the CTA flags a timeout and stops).
+        // shared memory: adjacency (uint16, padded to 16 bytes), T's bits (padded too),
+        // then two bitsets.  The base's packed rows arrive by one bulk copy; every thread
+        // waits on the mbarrier (bounded: past kCopyWaitNs the CTA flags a timeout and stops).
         uint16_t *adj = reinterpret_cast<uint16_t *>(sm);
-        uint4 *cur = sm + (((size_t)n * d * 2 + 15) / 16);
+        uint32_t *tb = reinterpret_cast<uint32_t *>(sm + ((size_t)n * d * 2 + 15) / 16);
+        uint4 *cur = reinterpret_cast<uint4 *>(tb) + (twords + 3) / 4;
         uint4 *nxt = cur + items;
         if (tid == 0) {
-            // the previous task's generic-proxy accesses to this memory come first
+            // the previous unit's generic-proxy accesses to this memory come first
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             bulk_to_smem(adj, B.adj16, B.adj16_bytes, &s_bar);
             s_late = 0;
+        }
+        if (tid < 3) s_cnt[tid] = 0u;
+        for (int k = tid; k < twords; k += kBatchBlock)
+            tb[k] = full ? 0xffffffffu : __ldcg(a.tbits + (size_t)cand * a.tbits_stride + k);
+        // visited after level 0: the padding sources and (below) the diagonal
+        for (int t = tid; t < items; t += kBatchBlock) {
+            const int b = (t & (nC - 1)) * 128;
+            cur[t] = make_uint4(padw(b, ns), padw(b + 32, ns), padw(b + 64, ns), padw(b + 96, ns));
+        }
+        if (!full) {
+            // base distances within T, from these sources' plane rows (their loads and the
+            // adjacency copy are in flight together)
+            const uint32_t *pw = reinterpret_cast<const uint32_t *>(B.planes);
+            const size_t ps = (size_t)n * B.cols * 4, cw = (size_t)B.cols * 4;
+            const uint32_t *tg = a.tbits + (size_t)cand * a.tbits_stride;
+            unsigned sum = 0u;
+            for (int j = warp; j < ns; j += kBatchBlock / 32) {
+                const size_t row = (size_t)__ldcg(lst + j) * cw;
+#pragma unroll 4
+                for (int k = lane; k < twords; k += 32)
+                    sum += dist4_sum(dist4_load(pw, ps, row + k), __ldcg(tg + k));
+            }
+            sum = __reduce_add_sync(0xffffffffu, sum);
+            if (lane == 0 && sum) atomicAdd(&a.cs[cand].tt_sum, (unsigned long long)sum);
         }
         {
             bool done = mbar_try_wait(&s_bar, phase);
@@ -194,78 +335,86 @@ __global__ void __launch_bounds__(kBatchBlock, 1) batch_kernel(const BatchArgs a
         __syncthreads();
         if (s_late) {
             // the copy did not complete: report it and leave (the host sees
-            // GG_TIMEOUT); only this CTA's tail of tasks is left unscored
+            // GG_TIMEOUT); only this CTA's tail of units is left unscored
             if (tid == 0) atomicExch(&a.ctl->timeout, 1);
             return;
         }
         if (sw.a >= 0 && tid < 4) {
             // 2-opt: (a,b),(c,d) -> (a,c),(b,d) [mode 0] or (a,d),(b,c) [mode 1]
-            const int x[4] = {sw.a, sw.b, sw.c, sw.d};
-            const int from[4] = {sw.b, sw.a, sw.d, sw.c};
-            const int to0[4] = {sw.c, sw.d, sw.a, sw.b};
-            const int to1[4] = {sw.d, sw.c, sw.b, sw.a};
-            const int row = x[tid], f = from[tid], t = sw.mode ? to1[tid] : to0[tid];
+            const SwapRows sr(sw);
+            const int row = tid == 0 ? sr.r[0] : tid == 1 ? sr.r[1] : tid == 2 ? sr.r[2] : sr.r[3];
+            const int f = tid == 0 ? sr.f[0] : tid == 1 ? sr.f[1] : tid == 2 ? sr.f[2] : sr.f[3];
+            const int t = tid == 0 ? sr.t[0] : tid == 1 ? sr.t[1] : tid == 2 ? sr.t[2] : sr.t[3];
             for (int j = 0; j < d; ++j)
                 if (adj[row * d + j] == (uint16_t)f) { adj[row * d + j] = (uint16_t)t; break; }
         }
-        // visited after level 0: the diagonal plus the padding sources
-        for (int t = tid; t < items; t += kBatchBlock) {
-            const int v = t >> lnc, c = t & (nC - 1);
-            const int b = c * 128;
-            uint4 w = make_uint4(padw(b, ns), padw(b + 32, ns), padw(b + 64, ns), padw(b + 96, ns));
-            const int i = v - s0;
-            if (full && i >= b && i < b + 128 && i < ns) {
-                const unsigned bit = 1u << (i & 31);
-                switch ((i - b) >> 5) {
-                    case 0: w.x |= bit; break;
-                    case 1: w.y |= bit; break;
-                    case 2: w.z |= bit; break;
-                    default: w.w |= bit; break;
-                }
-            }
-            cur[t] = w;
-        }
+        // source j of the unit: vertex un.first + j, or entry j of the list
+        auto set_bit = [&](const int v, const int j) -> bool {
+            const unsigned bit = 1u << (j & 31);
+            return !(atomicOr(reinterpret_cast<unsigned *>(cur + ((v << lnc) + (j >> 7))) + ((j >> 5) & 3), bit) & bit);
+        };
+        for (int j = tid; j < ns; j += kBatchBlock) set_bit(full ? un.first + j : (int)__ldcg(lst + j), j);
         __syncthreads();
-        if (!full) {
-            // source j of the chunk is vertex lists[s0 + j]
-            const uint16_t *lst = a.lists + (size_t)cand * a.list_stride + s0;
-            for (int j = tid; j < ns; j += kBatchBlock) {
-                const int v = lst[j];
-                atomicOr(reinterpret_cast<unsigned *>(cur + ((v << lnc) + (j >> 7))) + ((j >> 5) & 3),
-                         1u << (j & 31));
-            }
-            __syncthreads();
-        }
 
-        unsigned long long tot = 0, reach = 0;
-        int L = 1;
-        for (;; ++L) {
-            unsigned cnt = 0;
-            for (int t = tid; t < items; t += kBatchBlock) {
-                const int v = t >> lnc, c = t & (nC - 1);
-                const uint4 own = cur[t];
-                uint4 out = own;
-                if ((own.x & own.y & own.z & own.w) != 0xffffffffu) {
-                    uint4 acc = z4();
-                    const uint16_t *ar = adj + v * d;
-                    for (int i = 0; i < d; ++i) {
-                        const uint4 x = cur[((int)ar[i] << lnc) + c];
-                        acc.x |= x.x; acc.y |= x.y; acc.z |= x.z; acc.w |= x.w;
+        unsigned long long tot = 0, reach = 0;   // weighted, this thread's
+        const unsigned all = (unsigned)ns * (unsigned)n;
+        unsigned seen = (unsigned)ns;            // pairs reached, the same in every thread
+        int L = 1, last = 0;
+        bool done = seen == all;
+        // walk ends: levels 1, 2, .. while they are few (a pass visits every row)
+        if (!a.hist) {
+            for (unsigned ends = (unsigned)d; !done; ends *= (unsigned)d, ++L) {
+                if ((unsigned long long)ends * (unsigned)ns > (unsigned long long)kWalkItems * (unsigned)n) break;
+                unsigned cnt = 0u, wcnt = 0u;
+                for (unsigned k = (unsigned)tid; k < ends * (unsigned)ns; k += kBatchBlock) {
+                    const int j = (int)(k / ends);
+                    unsigned w = k - (unsigned)j * ends;
+                    int v = full ? un.first + j : (int)__ldcg(lst + j);
+                    for (int l = 0; l < L; ++l) {
+                        const unsigned q = w / (unsigned)d;
+                        v = adj[v * d + (int)(w - q * (unsigned)d)];
+                        w = q;
                     }
-                    out = make_uint4(own.x | acc.x, own.y | acc.y, own.z | acc.z, own.w | acc.w);
-                    const unsigned pc = __popc(acc.x & ~own.x) + __popc(acc.y & ~own.y) +
-                                        __popc(acc.z & ~own.z) + __popc(acc.w & ~own.w);
-                    cnt += pc;
-                    if (a.hist && L <= a.hist_k && pc) atomicAdd(a.hist + (size_t)v * a.hist_k + (L - 1), pc);
+                    if (set_bit(v, j)) {
+                        cnt += 1u;
+                        wcnt += 2u - ((tb[v >> 5] >> (v & 31)) & 1u);
+                    }
                 }
-                nxt[t] = out;
+                tot += (unsigned long long)L * wcnt;
+                reach += wcnt;
+                const unsigned wsum = __reduce_add_sync(0xffffffffu, cnt);
+                if (lane == 0 && wsum) atomicAdd(&s_cnt[L % 3], wsum);
+                __syncthreads();
+                const unsigned c = s_cnt[L % 3];
+                if (tid == 0) s_cnt[(L + 2) % 3] = 0u;
+                seen += c;
+                if (c) last = L;
+                done = c == 0u || seen == all;
             }
-            tot += (unsigned long long)L * cnt;
-            reach += cnt;
-            if (!__syncthreads_or(cnt != 0)) break;
+        }
+        for (; !done; ++L) {
+            unsigned cnt = 0u, wcnt = 0u;
+            switch (d) {
+                case 3: level_pass<3>(cur, nxt, adj, d, items, lnc, tb, a.hist, a.hist_k, L, cnt, wcnt); break;
+                case 4: level_pass<4>(cur, nxt, adj, d, items, lnc, tb, a.hist, a.hist_k, L, cnt, wcnt); break;
+                case 5: level_pass<5>(cur, nxt, adj, d, items, lnc, tb, a.hist, a.hist_k, L, cnt, wcnt); break;
+                case 6: level_pass<6>(cur, nxt, adj, d, items, lnc, tb, a.hist, a.hist_k, L, cnt, wcnt); break;
+                case 7: level_pass<7>(cur, nxt, adj, d, items, lnc, tb, a.hist, a.hist_k, L, cnt, wcnt); break;
+                case 8: level_pass<8>(cur, nxt, adj, d, items, lnc, tb, a.hist, a.hist_k, L, cnt, wcnt); break;
+                default: level_pass<0>(cur, nxt, adj, d, items, lnc, tb, a.hist, a.hist_k, L, cnt, wcnt); break;
+            }
+            tot += (unsigned long long)L * wcnt;
+            reach += wcnt;
+            const unsigned wsum = __reduce_add_sync(0xffffffffu, cnt);
+            if (lane == 0 && wsum) atomicAdd(&s_cnt[L % 3], wsum);
+            __syncthreads();
+            const unsigned c = s_cnt[L % 3];
+            if (tid == 0) s_cnt[(L + 2) % 3] = 0u;
+            seen += c;
+            if (c) last = L;
+            done = c == 0u || seen == all;
             uint4 *sw2 = cur; cur = nxt; nxt = sw2;
         }
-        // L is the first level without new pairs
         unsigned long long wt = tot, wr = reach;
         for (int o = 16; o; o >>= 1) {
             wt += __shfl_down_sync(0xffffffffu, wt, o);
@@ -278,32 +427,63 @@ __global__ void __launch_bounds__(kBatchBlock, 1) batch_kernel(const BatchArgs a
             for (int w = 0; w < kBatchBlock / 32; ++w) { bt += s_tot[w]; br += s_reach[w]; }
             atomicAdd(reinterpret_cast<unsigned long long *>(&a.out[cand].total), bt);
             atomicAdd(reinterpret_cast<unsigned long long *>(&a.out[cand].reached), br);
-            atomicMax(&a.out[cand].levels, L - 1);
+            atomicMax(&a.out[cand].levels, last);
         }
-        __syncthreads();  // the next task overwrites shared memory
+        __syncthreads();  // the next unit overwrites shared memory
     }
 }
 
-__global__ void batch_finalize(const BatchArgs a) {
+// One warp per candidate: the result from the searched sources' counts.
+__global__ void __launch_bounds__(128) batch_finalize(const BatchArgs a) {
     const int n_cand = a.ctl->n_cand;
-    if (a.ctl->bad || a.ctl->timeout) {
-        // a rejected or timed-out launch scores nothing: every result says so
-        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_cand; i += gridDim.x * blockDim.x)
-            a.out[i] = gg_cand_result{0ull, 0ull, -1, 0};
-        return;
-    }
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_cand; i += gridDim.x * blockDim.x) {
-        const BatchBase B = a.bases[a.cands[i].base];
-        gg_cand_result r = a.out[i];
-        if (a.inc && !a.inc[i].full) {
-            // the other sources keep the base's distances
-            const IncCand &ic = a.inc[i];
-            r.total = B.total - ic.old_sum + r.total;
-            r.reached = B.reached - (unsigned long long)ic.count * B.n + r.reached;
-            r.levels = max(r.levels, (int)ic.max_other);
+    const int lane = threadIdx.x & 31;
+    const int w0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), nw = (int)((gridDim.x * blockDim.x) >> 5);
+    const bool dead = a.ctl->bad || a.ctl->timeout;
+    for (int i = w0; i < n_cand; i += nw) {
+        if (dead) {
+            // a rejected or timed-out launch scores nothing: every result says so
+            if (lane == 0) a.out[i] = gg_cand_result{0ull, 0ull, -1, 0};
+            continue;
         }
-        r.connected = r.reached == (unsigned long long)B.n * (unsigned long long)B.n;
-        a.out[i] = r;
+        const BatchBase &B = a.bases[a.cands[i].base];
+        const CandState cs = a.cs[i];
+        gg_cand_result r = a.out[i];
+        const unsigned long long nn = (unsigned long long)B.n * (unsigned long long)B.n;
+        if (cs.mode != kFull) {
+            const unsigned long long T = cs.count;
+            r.total = B.total - (2ull * cs.old_sum - cs.tt_sum) + r.total;
+            r.reached = B.reached - (2ull * T * B.n - T * T) + r.reached;
+            // The largest distance between vertices outside T stays the base's diameter when
+            // the pairs that T touches cannot be all there are at it.  Otherwise look for it:
+            // from the diameter down, a source outside T with another such vertex there.
+            int top = B.levels;
+            if (B.at_top <= 2ull * cs.tops) {
+                const uint32_t *tb = a.tbits + (size_t)i * a.tbits_stride;
+                const uint32_t *pw = reinterpret_cast<const uint32_t *>(B.planes);
+                const size_t ps = (size_t)B.n * B.cols * 4, cw = (size_t)B.cols * 4;
+                const int words = (B.n + 31) / 32;
+                for (bool found = false; top > r.levels; --top) {
+                    for (int s0 = 0; s0 < B.n && !found; s0 += 32) {
+                        const int s = s0 + lane;
+                        const bool in = s < B.n && !((__ldcg(tb + (s0 >> 5)) >> lane) & 1u) && (int)__ldg(B.ecc + s) >= top;
+                        for (unsigned m = __ballot_sync(0xffffffffu, in); m && !found; m &= m - 1u) {
+                            const int v = s0 + __ffs((int)m) - 1;
+                            bool hit = false;
+                            for (int k = lane; k < words; k += 32) {
+                                uint32_t live = ~__ldcg(tb + k);
+                                if (k == words - 1 && (B.n & 31)) live &= (1u << (B.n & 31)) - 1u;
+                                hit |= (dist4_eq(dist4_load(pw, ps, (size_t)v * cw + k), dist4_const((unsigned)top)) & live) != 0u;
+                            }
+                            found = __any_sync(0xffffffffu, hit);
+                        }
+                    }
+                    if (found) break;
+                }
+            }
+            r.levels = max(r.levels, top);
+        }
+        r.connected = r.reached == nn;
+        if (lane == 0) a.out[i] = r;
     }
 }
 
@@ -315,7 +495,7 @@ __global__ void batch_reset(const BatchArgs a) {
     const int n_cand = a.ctl->n_cand;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_cand; i += gridDim.x * blockDim.x) {
         a.out[i] = gg_cand_result{0ull, 0ull, 0, 0};
-        if (a.inc) a.inc[i] = IncCand{0ull, 0u, 0u, 0, 0};
+        a.cs[i] = CandState{0ull, 0ull, 0u, 0u, 0u, kNear};
         const gg_swap sw = a.cands[i];
         bool ok = sw.base >= 0 && sw.base < a.ctl->n_bases;
         if (ok && sw.a >= 0) {
@@ -329,84 +509,141 @@ __global__ void batch_reset(const BatchArgs a) {
             atomicMin(&a.ctl->bad_index, i);
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.ctl->task_ctr = 0u;
 }
 
-__device__ __forceinline__ unsigned plane_dist(const uint32_t *pw, size_t pstride_w, unsigned cols4,
-                                               unsigned x, unsigned s) {
-    const size_t base = (size_t)x * cols4 + (s >> 5);
-    unsigned dv = 0;
-#pragma unroll
-    for (int k = 0; k < kPlanes; ++k) dv |= ((__ldg(pw + (size_t)k * pstride_w + base) >> (s & 31u)) & 1u) << k;
-    return dv;
-}
-
-// One thread per (candidate, source): the affected-source test (see the file
-// comment).  Affected sources join the candidate's list with their base
-// distance sums; the others give the largest eccentricity that stays.
-__global__ void batch_affected(const BatchArgs a, int max_n, int force_full) {
+// T of every candidate, and the work units.  A block of four warps takes a candidate and
+// 1024 sources (32 a lane), a warp per endpoint: the distances of the endpoint's
+// neighbours come as 4 plane words each (coalesced; a base's planes sit in the L2), four
+// neighbours' loads in flight together, and every test is a few logic operations on 32
+// sources at once.  The block that finishes a candidate cuts its list into units.  Bound
+// by the dependent round trips (row ids, then planes) of a group of four neighbours.
+// (One thread per (candidate, source), the plane bits gathered one by one, took 187 us
+// for 2048 x 1024 + 512 x 3000 sources.)
+__global__ void __launch_bounds__(128) batch_select(const BatchArgs a, const int max_n) {
+    __shared__ uint32_t s_aff[4][32], s_near[4][32];
     if (a.ctl->bad) return;   // batch_reset rejected a candidate
-    const int n_cand = a.ctl->n_cand;
-    const unsigned long long total = (unsigned long long)n_cand * (unsigned long long)max_n;
+    const unsigned n_cand = (unsigned)a.ctl->n_cand;
+    const unsigned groups = ((unsigned)max_n + 1023u) / 1024u;
     const unsigned lane = threadIdx.x & 31u;
-    for (unsigned long long g0 = (unsigned long long)blockIdx.x * blockDim.x; g0 < total;
-         g0 += (unsigned long long)gridDim.x * blockDim.x) {
-        const unsigned long long g = g0 + threadIdx.x;
-        const bool in = g < total;
-        const int cand = in ? (int)(g / (unsigned)max_n) : 0;
-        const int s = in ? (int)(g % (unsigned)max_n) : 0;
+    const int i = (int)(threadIdx.x >> 5);   // the warp's endpoint
+    const unsigned long long total = (unsigned long long)n_cand * groups;
+    for (unsigned long long q = blockIdx.x; q < total; q += gridDim.x) {
+        const unsigned cand = (unsigned)(q / groups), grp = (unsigned)(q % groups);
         const gg_swap sw = a.cands[cand];
         const BatchBase &B = a.bases[sw.base];
-        const bool live = in && s < B.n;
-        bool aff = false, other = false;
-        if (live && (force_full || !B.valid)) {
-            if (s == 0) a.inc[cand].full = 1;
-        } else if (live) {
-            other = true;
-            if (sw.a >= 0) {
-                const uint32_t *pw = reinterpret_cast<const uint32_t *>(B.planes);
-                const size_t psw = (size_t)B.n * B.cols * 4;
-                const unsigned c4 = B.cols * 4;
-                const int ends[2][2] = {{sw.a, sw.b}, {sw.c, sw.d}};
-                for (int e = 0; e < 2 && !aff; ++e) {
-                    const int x = ends[e][0], y = ends[e][1];
-                    const unsigned dx = plane_dist(pw, psw, c4, x, s), dy = plane_dist(pw, psw, c4, y, s);
-                    if (dx == dy) continue;
-                    const int lo = dx < dy ? x : y, hi = dx < dy ? y : x;
-                    const unsigned l = min(dx, dy);
-                    bool par = false, skipped = false;
-                    for (int i = 0; i < B.d && !par; ++i) {
-                        const int z = __ldg(B.adj + (size_t)hi * B.d + i);
-                        if (z == lo && !skipped) { skipped = true; continue; }
-                        par = plane_dist(pw, psw, c4, (unsigned)z, s) == l;
-                    }
-                    aff = !par;
+        const int n = B.n, d = B.d;
+        if ((int)(grp * 1024u) >= n) continue;
+        const SwapRows sr(sw);
+        const int r = i == 0 ? sr.r[0] : i == 1 ? sr.r[1] : i == 2 ? sr.r[2] : sr.r[3];
+        const int f = i == 0 ? sr.f[0] : i == 1 ? sr.f[1] : i == 2 ? sr.f[2] : sr.f[3];
+        const int t = i == 0 ? sr.t[0] : i == 1 ? sr.t[1] : i == 2 ? sr.t[2] : sr.t[3];
+        int mode = a.force_full || !B.valid ? kFull : (sw.a < 0 ? kBase : kNear);
+        if (mode == kNear) {
+            // both ends list each removed edge equally often (the edited graph is symmetric)
+            int c[4] = {0, 0, 0, 0};
+            for (int j0 = 0; j0 < d; j0 += 32)
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    c[k] += __popc(__ballot_sync(0xffffffffu, j0 + (int)lane < d &&
+                                                 __ldg(B.adj + (size_t)sr.r[k] * d + j0 + lane) == sr.f[k]));
+            if (c[0] < 1 || c[0] != c[1] || c[2] < 1 || c[2] != c[3]) mode = kFull;
+        }
+        if (mode != kNear) {   // uniform over the block
+            if (grp == 0u && threadIdx.x == 0u) a.cs[cand].mode = mode;
+            if (grp == 0u && i == 0 && mode == kFull) {
+                const int S = 128 << B.log_nc;
+                unsigned u0 = 0u;
+                if (lane == 0u) u0 = (unsigned)atomicAdd(&a.ctl->n_units, B.chunks);
+                u0 = __shfl_sync(0xffffffffu, u0, 0);
+                for (int k = (int)lane; k < B.chunks; k += 32)
+                    a.units[u0 + k] = Unit{(int)cand, k * S, min(S, n - k * S), B.log_nc};
+            }
+            continue;
+        }
+        const unsigned w = grp * 32u + lane, words = ((unsigned)n + 31u) / 32u;
+        const bool in = w < words;
+        const uint32_t *pw = reinterpret_cast<const uint32_t *>(B.planes);
+        const size_t ps = (size_t)n * B.cols * 4, cw = (size_t)B.cols * 4;
+        const unsigned wl = in ? w : 0u;
+        const Dist4 er = dist4_load(pw, ps, (size_t)r * cw + wl);
+        const Dist4 ef = dist4_load(pw, ps, (size_t)f * cw + wl);
+        const Dist4 et = dist4_load(pw, ps, (size_t)t * cw + wl);
+        uint32_t lost = dist4_eq(dist4_inc(ef), er);
+        bool skipped = false;   // the first slot that lists f is the one that goes
+        for (int j = 0; j < d; j += 4) {
+            int u[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                u[k] = __ldg(B.adj + (size_t)r * d + min(j + k, d - 1));
+                if (j + k < d && !skipped && u[k] == f) { u[k] = r; skipped = true; }   // (r itself is no parent)
+                if (j + k >= d) u[k] = r;
+            }
+            Dist4 x[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) x[k] = dist4_load(pw, ps, (size_t)u[k] * cw + wl);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) lost &= ~dist4_eq(x[k], ef);
+        }
+        s_aff[i][lane] = lost | dist4_lt(dist4_inc(et), er);
+        s_near[i][lane] = ~dist4_lt(dist4_const((unsigned)B.radius), er);
+        __syncthreads();
+        if (i == 0) {
+            uint32_t go = (s_near[0][lane] | s_near[1][lane] | s_near[2][lane] | s_near[3][lane]) &
+                          (s_aff[0][lane] | s_aff[1][lane] | s_aff[2][lane] | s_aff[3][lane]);
+            if (!in) go = 0u;
+            else if (w == words - 1u && (n & 31)) go &= (1u << (n & 31)) - 1u;
+            if (in) a.tbits[(size_t)cand * a.tbits_stride + w] = go;
+            // these sources into the candidate's list
+            const unsigned mine = __popc(go);
+            unsigned incl = mine;
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+                if ((int)lane >= o) incl += y;
+            }
+            const unsigned cnt = __shfl_sync(0xffffffffu, incl, 31);
+            unsigned first = 0u;
+            if (lane == 0u && cnt) first = atomicAdd(&a.cs[cand].count, cnt);
+            unsigned at = __shfl_sync(0xffffffffu, first, 0) + incl - mine;
+            unsigned sum = 0u, tops = 0u;
+            uint16_t *lst = a.lists + (size_t)cand * a.list_stride;
+            for (uint32_t m = go; m; m &= m - 1u) {
+                const unsigned s = w * 32u + (unsigned)__ffs((int)m) - 1u;
+                lst[at++] = (uint16_t)s;
+                sum += __ldg(B.rowsum + s);
+                tops += __ldg(B.top + s);
+            }
+            // (32 lanes x 32 sources x a sum below 16 n: below 2^32 for n < 2^18)
+            sum = __reduce_add_sync(0xffffffffu, sum);
+            tops = __reduce_add_sync(0xffffffffu, tops);
+            unsigned prev = 0u;
+            if (lane == 0u) {
+                if (cnt) {
+                    atomicAdd(&a.cs[cand].old_sum, (unsigned long long)sum);
+                    atomicAdd(&a.cs[cand].tops, tops);
                 }
-                if (!aff) {
-                    const int p = sw.mode ? sw.d : sw.c, q = sw.mode ? sw.c : sw.d;
-                    const unsigned da = plane_dist(pw, psw, c4, sw.a, s), dp = plane_dist(pw, psw, c4, p, s);
-                    const unsigned db = plane_dist(pw, psw, c4, sw.b, s), dq = plane_dist(pw, psw, c4, q, s);
-                    aff = (da > dp ? da - dp : dp - da) >= 2u || (db > dq ? db - dq : dq - db) >= 2u;
+                __threadfence();
+                prev = atomicAdd(&a.cs[cand].groups_done, 1u);
+            }
+            prev = __shfl_sync(0xffffffffu, prev, 0);
+            if (prev + 1u == ((unsigned)n + 1023u) / 1024u) {
+                // every group of the candidate is in: equal units of at most 128 << l sources,
+                // l the least that takes them at once within the base's chunk width
+                unsigned T = 0u, u0 = 0u;
+                if (lane == 0u) T = atomicAdd(&a.cs[cand].count, 0u);
+                T = __shfl_sync(0xffffffffu, T, 0);
+                int l = 0;
+                while (l < B.log_nc && (128u << l) < T) ++l;
+                const unsigned nu = (T + (128u << l) - 1u) >> (7 + l);
+                if (nu) {
+                    const unsigned per = (T + nu - 1u) / nu;
+                    if (lane == 0u) u0 = (unsigned)atomicAdd(&a.ctl->n_units, (int)nu);
+                    u0 = __shfl_sync(0xffffffffu, u0, 0);
+                    for (unsigned k = lane; k < nu; k += 32u)
+                        a.units[u0 + k] = Unit{(int)cand, (int)(k * per), (int)min(per, T - k * per), l};
                 }
             }
-            other = !aff;
         }
-        // one set of atomics per candidate present in the warp
-        const unsigned peers = __match_any_sync(0xffffffffu, live ? cand : -1);
-        const unsigned am = __ballot_sync(0xffffffffu, aff) & peers;
-        const int leader = __ffs((int)peers) - 1;
-        const unsigned rs = __reduce_add_sync(peers, aff ? __ldg(B.rowsum + s) : 0u);
-        const unsigned mx = __reduce_max_sync(peers, other ? __ldg(B.ecc + s) : 0u);
-        unsigned first = 0;
-        if ((int)lane == leader && live) {
-            if (am) {
-                first = atomicAdd(&a.inc[cand].count, (unsigned)__popc(am));
-                atomicAdd(&a.inc[cand].old_sum, (unsigned long long)rs);
-            }
-            atomicMax(&a.inc[cand].max_other, mx);
-        }
-        first = __shfl_sync(0xffffffffu, first, leader);
-        if (aff) a.lists[(size_t)cand * a.list_stride + first + __popc(am & ((1u << lane) - 1u))] = (uint16_t)s;
+        __syncthreads();
     }
 }
 
@@ -448,15 +685,20 @@ struct gg_batch {
     unsigned *d_hist = nullptr;            // vertex histogram output
     size_t hist_cap = 0;
     double last_ms = 0.0;
-    // affected-source mode
+    // near-source mode
     bool full_only = false;                // GG_BATCH_FULL=1: every candidate searches every source
     std::vector<uint4 *> base_planes;      // per base: [kPlanes][n][cols]
-    std::vector<unsigned *> base_stats;    // per base: rowsum[n] then ecc[n]
+    std::vector<unsigned *> base_stats;    // per base: rowsum[n], ecc[n], top[n]
     std::vector<std::pair<std::pair<int, int>, gg_engine *>> engines;  // per (n, degree): base passes
     int *d_flag = nullptr, *h_flag = nullptr;
-    IncCand *d_inc = nullptr;              // [cap]
+    CandState *d_cs = nullptr;             // [cap]
     uint16_t *d_lists = nullptr;           // [cap][list_stride]
     int list_stride = 0;                   // largest base n
+    uint32_t *d_tbits = nullptr;           // [cap][tbits_stride]
+    int tbits_stride = 0;
+    Unit *d_units = nullptr;               // [cap * max_chunks]
+    int units_per_cand = 0;
+    int max_chunks = 1;                    // most units a candidate can take
 };
 
 namespace {
@@ -468,9 +710,14 @@ void drop_graph(gg_batch *b) {
     b->graph = nullptr;
 }
 
+// Shared memory of a unit with rows of 1 << l chunks: adjacency, T's bits, two bitsets.
+size_t unit_smem(int n, int d, int l) {
+    const size_t adj = ((size_t)n * d * 2 + 15) / 16 * 16, tb = ((size_t)(n + 31) / 32 * 4 + 15) / 16 * 16;
+    return adj + tb + 2 * (size_t)n * (16u << l);
+}
+// (T's bits, at most 4 KB, come on top of the budget that decides which bases fit)
 bool log_nc_fits(int n, int d, int l) {
-    const size_t adj = ((size_t)n * d * 2 + 15) / 16 * 16;
-    return adj + 2 * (size_t)n * (16u << l) <= kSmemBudget;
+    return unit_smem(n, d, l) - ((size_t)(n + 31) / 32 * 4 + 15) / 16 * 16 <= kSmemBudget;
 }
 
 std::string batch_tune_key(int device, int n, int d) { return gg::tune_key(device, "batch", {n, d}); }
@@ -495,18 +742,17 @@ gg_status refresh_plan(gg_batch *b) {
     size_t smem = 0;
     int max_chunks = 1;
     for (auto &B : b->bases) {
-        const size_t need = ((size_t)B.n * B.d * 2 + 15) / 16 * 16 + 2 * (size_t)B.n * (16u << B.log_nc);
-        smem = std::max(smem, need);
+        smem = std::max(smem, unit_smem(B.n, B.d, B.log_nc));
         max_chunks = std::max(max_chunks, B.chunks);
     }
     b->smem = smem;
+    b->max_chunks = max_chunks;
     GB_CK(cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0, sms = 0;
     GB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel, kBatchBlock, smem));
     GB_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device));
     if (per_sm < 1) return bfail(GG_BAD_ARG, "batch task does not fit in shared memory");
     b->grid = per_sm * sms;
-    b->h_ctl->max_chunks = max_chunks;
     GB_CK(cudaMemcpy(b->d_bases, b->bases.data(), b->bases.size() * sizeof(BatchBase),
                      cudaMemcpyHostToDevice));
     drop_graph(b);
@@ -516,48 +762,54 @@ gg_status refresh_plan(gg_batch *b) {
 gg_status ensure_cap(gg_batch *b, int n) {
     int max_n = 0;
     for (auto &B : b->bases) max_n = std::max(max_n, B.n);
-    if (n <= b->cap && max_n <= b->list_stride) return GG_OK;
-    const int cap = std::max({n, 2 * b->cap, 1});
-    cudaFree(b->d_cands); cudaFree(b->d_out); cudaFree(b->d_inc); cudaFree(b->d_lists);
+    if (n <= b->cap && max_n <= b->list_stride && b->max_chunks <= b->units_per_cand) return GG_OK;
+    const int cap = std::max({n, n > b->cap ? 2 * b->cap : b->cap, 1});
+    cudaFree(b->d_cands); cudaFree(b->d_out); cudaFree(b->d_cs); cudaFree(b->d_lists);
+    cudaFree(b->d_tbits); cudaFree(b->d_units);
     cudaFreeHost(b->h_cands); cudaFreeHost(b->h_out);
     b->d_cands = nullptr; b->d_out = nullptr; b->h_cands = nullptr; b->h_out = nullptr;
-    b->d_inc = nullptr; b->d_lists = nullptr;
+    b->d_cs = nullptr; b->d_lists = nullptr; b->d_tbits = nullptr; b->d_units = nullptr;
     b->cap = 0;
+    b->list_stride = std::max(max_n, 1);
+    b->tbits_stride = (b->list_stride + 31) / 32;
+    b->units_per_cand = b->max_chunks;
     GB_CK(cudaMalloc(&b->d_cands, (size_t)cap * sizeof(gg_swap)));
     GB_CK(cudaMalloc(&b->d_out, (size_t)cap * sizeof(gg_cand_result)));
     GB_CK(cudaMallocHost(&b->h_cands, (size_t)cap * sizeof(gg_swap)));
     GB_CK(cudaMallocHost(&b->h_out, (size_t)cap * sizeof(gg_cand_result)));
-    GB_CK(cudaMalloc(&b->d_inc, (size_t)cap * sizeof(IncCand)));
-    b->list_stride = std::max(max_n, 1);
+    GB_CK(cudaMalloc(&b->d_cs, (size_t)cap * sizeof(CandState)));
     GB_CK(cudaMalloc(&b->d_lists, (size_t)cap * b->list_stride * sizeof(uint16_t)));
+    GB_CK(cudaMalloc(&b->d_tbits, (size_t)cap * b->tbits_stride * sizeof(uint32_t)));
+    GB_CK(cudaMalloc(&b->d_units, (size_t)cap * b->units_per_cand * sizeof(Unit)));
     b->cap = cap;
     drop_graph(b);
     return GG_OK;
 }
 
-// Enqueue reset -> batch kernel -> finalize on `st` for candidates `cands`,
-// results `out`; the candidate count and task geometry come from d_ctl.
+// Enqueue reset -> select -> batch kernel -> finalize on `st` for candidates `cands`,
+// results `out`; the candidate count comes from d_ctl.
 gg_status enqueue(gg_batch *b, const gg_swap *cands, gg_cand_result *out, cudaStream_t st,
                   unsigned *hist = nullptr, int hist_k = 0) {
-    // the histogram pass searches every source of its one candidate
-    const bool inc = !hist;
-    BatchArgs a{b->d_bases, cands, out, b->d_ctl, hist, hist_k, inc ? b->d_inc : nullptr,
-                b->d_lists, b->list_stride};
+    BatchArgs a{};
+    a.bases = b->d_bases; a.cands = cands; a.out = out; a.ctl = b->d_ctl;
+    a.hist = hist; a.hist_k = hist_k;
+    a.cs = b->d_cs;
+    a.lists = b->d_lists; a.list_stride = b->list_stride;
+    a.tbits = b->d_tbits; a.tbits_stride = b->tbits_stride;
+    a.units = b->d_units;
+    a.force_full = b->full_only || hist;   // the histogram pass searches every source of its one candidate
     batch_reset<<<64, 256, 0, st>>>(a);
-    if (inc) {
-        const unsigned long long pairs = (unsigned long long)b->cap * b->list_stride;
-        const int g = (int)std::min<unsigned long long>((pairs + 255) / 256, 148ull * 16);
-        batch_affected<<<g, 256, 0, st>>>(a, b->list_stride, b->full_only ? 1 : 0);
-    }
+    const unsigned long long blocks = (unsigned long long)b->cap * ((b->list_stride + 1023) / 1024);
+    batch_select<<<(int)std::min<unsigned long long>(blocks, 148ull * 16), 128, 0, st>>>(a, b->list_stride);
     batch_kernel<<<b->grid, kBatchBlock, b->smem, st>>>(a);
-    batch_finalize<<<64, 256, 0, st>>>(a);
+    batch_finalize<<<(int)std::min((b->cap + 3) / 4, 148 * 8), 128, 0, st>>>(a);
     GB_CK(cudaGetLastError());
     return GG_OK;
 }
 
 constexpr int kIncMaxN = 16384;   // larger bases search every source (planes of 4 n^2/8 bytes)
 
-// The base pass of base `id` (affected-source mode): the single-graph engine
+// The base pass of base `id` (near-source mode): the single-graph engine
 // evaluates the base with its distance planes (at most 16 levels), then every
 // source's distance sum and eccentricity follow from the planes.  valid = 0
 // (every candidate of the base searches every source) unless the base is
@@ -579,7 +831,7 @@ gg_status base_pass(gg_batch *b, int id) {
         if (!b->base_planes[id]) {
             B.cols = (unsigned)gg::engine_plane_cols(eng);
             GB_CK(cudaMalloc(&b->base_planes[id], (size_t)kPlanes * B.n * B.cols * sizeof(uint4)));
-            GB_CK(cudaMalloc(&b->base_stats[id], 2 * (size_t)B.n * sizeof(unsigned)));
+            GB_CK(cudaMalloc(&b->base_stats[id], 3 * (size_t)B.n * sizeof(unsigned)));
         }
         GB_CK(cudaMemsetAsync(b->d_flag, 0, sizeof(int), st));
         const long long ent = (long long)B.n * B.d;
@@ -587,6 +839,8 @@ gg_status base_pass(gg_batch *b, int id) {
         GB_CK(cudaGetLastError());
         gg_eval_opts o{};
         o.max_levels = 1 << kPlanes;      // a base that needs more levels searches every source
+        uint64_t counts[(1 << kPlanes) + 1] = {};
+        o.level_counts = counts;
         gg::EvalExtra x;
         x.planes = b->base_planes[id];
         x.nplanes = kPlanes;
@@ -600,7 +854,7 @@ gg_status base_pass(gg_batch *b, int id) {
         // `valid` below requires
         plane_row_stats<kPlanes><<<plane_row_stats_grid(B.n, sms), 256, 0, st>>>(
             b->base_planes[id], (unsigned long long)B.n * B.cols, B.cols, B.n, b->base_stats[id],
-            b->base_stats[id] + B.n);
+            b->base_stats[id] + B.n, b->base_stats[id] + 2 * B.n, (unsigned)r.levels);
         GB_CK(cudaGetLastError());
         GB_CK(cudaMemcpyAsync(b->h_flag, b->d_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
         GB_CK(cudaStreamSynchronize(st));
@@ -609,6 +863,9 @@ gg_status base_pass(gg_batch *b, int id) {
             B.total = r.total;
             B.reached = r.reached;
             B.levels = r.levels;
+            B.at_top = counts[r.levels];
+            B.radius = (std::max(r.levels, 1) - 1) / 2;
+            B.top = b->base_stats[id] + 2 * B.n;
             B.planes = b->base_planes[id];
             B.rowsum = b->base_stats[id];
             B.ecc = b->base_stats[id] + B.n;
@@ -631,6 +888,8 @@ unsigned adj16_bytes(int n, int d) { return (unsigned)((((size_t)n * d * 2) + 15
 
 // The device-side candidate check starts clean for every launch.
 void arm_check(gg_batch *b) {
+    b->h_ctl->unit_ctr = 0;
+    b->h_ctl->n_units = 0;
     b->h_ctl->bad = 0;
     b->h_ctl->timeout = 0;
     b->h_ctl->bad_index = 0x7fffffff;
@@ -738,8 +997,7 @@ gg_status gg_batch_set_chunk(gg_batch *b, int base_id, int sources) {
     while ((128 << l) < sources) ++l;
     if ((128 << l) != sources) return bfail(GG_BAD_ARG, "chunk width must be 128 * 2^k");
     BatchBase &B = b->bases[base_id];
-    const size_t need = ((size_t)B.n * B.d * 2 + 15) / 16 * 16 + 2 * (size_t)B.n * (16u << l);
-    if (need > kSmemBudget) return bfail(GG_BAD_ARG, "chunk does not fit in shared memory");
+    if (!log_nc_fits(B.n, B.d, l)) return bfail(GG_BAD_ARG, "chunk does not fit in shared memory");
     B.log_nc = l;
     B.chunks = (B.n + (128 << l) - 1) / (128 << l);
     GB_CK(cudaSetDevice(b->device));
@@ -807,7 +1065,6 @@ gg_status gg_batch_eval(gg_batch *b, int n_cand, const gg_swap *cands, gg_cand_r
     if (s != GG_OK) return s;
     std::memcpy(b->h_cands, cands, (size_t)n_cand * sizeof(gg_swap));
     b->h_ctl->n_cand = n_cand;
-    b->h_ctl->task_ctr = 0;
     arm_check(b);
     GB_CK(cudaMemcpyAsync(b->d_cands, b->h_cands, (size_t)n_cand * sizeof(gg_swap),
                           cudaMemcpyHostToDevice, b->stream));
@@ -842,10 +1099,9 @@ gg_status gg_batch_eval_device(gg_batch *b, int n_cand, const gg_swap *d_cands,
     if (n_cand == 0) return GG_OK;
     GB_CK(cudaSetDevice(b->device));
     cudaStream_t st = stream ? (cudaStream_t)stream : b->stream;
-    gg_status cs = ensure_cap(b, n_cand);   // per-candidate lists of the affected-source mode
+    gg_status cs = ensure_cap(b, n_cand);   // per-candidate lists of the near-source mode
     if (cs != GG_OK) return cs;
     b->h_ctl->n_cand = n_cand;
-    b->h_ctl->task_ctr = 0;
     arm_check(b);
     // the control block goes by value as a kernel argument: this call returns
     // before the GPU runs it, and the next call may change the host copy
@@ -892,7 +1148,6 @@ gg_status gg_batch_vertex_hist(gg_batch *b, int base_id, int K, uint32_t *hist) 
     const gg_swap self{base_id, -1, -1, -1, -1, 0};
     b->h_cands[0] = self;
     b->h_ctl->n_cand = 1;
-    b->h_ctl->task_ctr = 0;
     arm_check(b);
     cudaError_t e = cudaMemsetAsync(d_hist, 0, (size_t)n * K * sizeof(unsigned), b->stream);
     if (e == cudaSuccess)
@@ -927,7 +1182,7 @@ gg_status gg_batch_destroy(gg_batch *b) {
     for (auto p : b->base_planes) cudaFree(p);
     for (auto p : b->base_stats) cudaFree(p);
     for (auto &pe : b->engines) gg_destroy(pe.second);
-    cudaFree(b->d_inc); cudaFree(b->d_lists);
+    cudaFree(b->d_cs); cudaFree(b->d_lists); cudaFree(b->d_tbits); cudaFree(b->d_units);
     cudaFree(b->d_flag); cudaFreeHost(b->h_flag);
     cudaFree(b->d_bases); cudaFree(b->d_ctl); cudaFreeHost(b->h_ctl);
     cudaFree(b->d_cands); cudaFree(b->d_out); cudaFreeHost(b->h_cands); cudaFreeHost(b->h_out);

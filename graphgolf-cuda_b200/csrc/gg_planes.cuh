@@ -15,15 +15,61 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+// ---- bit-sliced distances: four plane words hold 32 sources' distances ------------
+struct Dist4 {
+    uint32_t p[4];
+};
+__device__ __forceinline__ Dist4 dist4_load(const uint32_t *planes, const size_t stride, const size_t at) {
+    Dist4 d;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) d.p[k] = __ldg(planes + (size_t)k * stride + at);
+    return d;
+}
+__device__ __forceinline__ Dist4 dist4_const(const unsigned v) {
+    Dist4 d;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) d.p[k] = (v >> k) & 1u ? 0xffffffffu : 0u;
+    return d;
+}
+__device__ __forceinline__ Dist4 dist4_inc(const Dist4 a) {
+    Dist4 r;
+    uint32_t c = 0xffffffffu;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        r.p[k] = a.p[k] ^ c;
+        c &= a.p[k];
+    }
+    return r;
+}
+// a == b, a < b, per source
+__device__ __forceinline__ uint32_t dist4_eq(const Dist4 a, const Dist4 b) {
+    uint32_t x = 0u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) x |= a.p[k] ^ b.p[k];
+    return ~x;
+}
+__device__ __forceinline__ uint32_t dist4_lt(const Dist4 a, const Dist4 b) {
+    uint32_t lt = 0u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) lt = (~a.p[k] & b.p[k]) | (~(a.p[k] ^ b.p[k]) & lt);
+    return lt;
+}
+// the sum of the distances of the sources in `mask`
+__device__ __forceinline__ unsigned dist4_sum(const Dist4 a, const uint32_t mask) {
+    return __popc(a.p[0] & mask) + 2u * __popc(a.p[1] & mask) + 4u * __popc(a.p[2] & mask) + 8u * __popc(a.p[3] & mask);
+}
+
+// Distance sum and eccentricity of every source; with `top`, also the number of its
+// vertices at distance `diam`.
 template <int NP>
 static __global__ void plane_row_stats(const uint4 *planes, unsigned long long stride, unsigned cols, int n,
-                                       unsigned *rowsum, unsigned *ecc) {
+                                       unsigned *rowsum, unsigned *ecc, unsigned *top = nullptr, unsigned diam = 0u) {
     const unsigned lane = threadIdx.x & 31u;
     const unsigned long long nwarps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
     for (unsigned long long v = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < (unsigned)n;
          v += nwarps) {
         const uint4 *row = planes + v * cols;
-        unsigned sum = 0, mx = 0;
+        unsigned sum = 0, mx = 0, tops = 0;
 #pragma unroll 2
         for (unsigned c = lane; c < cols; c += 32) {
             uint4 w[NP];
@@ -43,11 +89,22 @@ static __global__ void plane_row_stats(const uint4 *planes, unsigned long long s
                     }
                 }
                 mx = max(mx, val);
+                if (top) {
+                    unsigned at = 0xffffffffu;   // (planes past the last source are 0: diam >= 1)
+#pragma unroll
+                    for (int p = 0; p < NP; ++p) {
+                        const unsigned x = k == 0 ? w[p].x : k == 1 ? w[p].y : k == 2 ? w[p].z : w[p].w;
+                        at &= (diam >> p) & 1u ? x : ~x;
+                    }
+                    tops += (unsigned)__popc(at);
+                }
             }
         }
         sum = __reduce_add_sync(0xffffffffu, sum);
         mx = __reduce_max_sync(0xffffffffu, mx);
+        if (top) tops = __reduce_add_sync(0xffffffffu, tops);
         if (lane == 0) {
+            if (top) top[v] = tops;
             rowsum[v] = sum;
             ecc[v] = mx;
         }

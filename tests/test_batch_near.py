@@ -1,0 +1,119 @@
+"""Batched 2-opt candidates scored from the sources near their edit (csrc/gg_batch.cu).
+
+CPU: the set of sources and the weights, restated in numpy, give every candidate's exact
+total, reach and diameter.  GPU: candidates of bases at the edges of the kernel's groups
+(32-source words, 1024-source groups, 128-source units), degrees with and without an
+unrolled pass, small and large diameters, disconnecting moves and moves whose removed
+edge the two ends do not list equally often, against the oracle."""
+import numpy as np
+import pytest
+
+import graphgolf as G
+import instances as I
+import oracle as O
+
+
+def dist(adj):
+    """All-pairs distances (99: not reached), row s = source s, by the pull rule."""
+    n = len(adj)
+    D = np.full((n, n), 99, dtype=np.int64)
+    np.fill_diagonal(D, 0)
+    for L in range(1, n + 1):
+        reach = (D[:, adj] == L - 1).any(axis=2) & (D == 99)
+        if not reach.any():
+            break
+        D[reach] = L
+    return D
+
+
+def near_total(adj, D, s):
+    """(total, reached, diameter) of the candidate from the rows of T alone."""
+    n = len(adj)
+    a, b, c, d = (int(s[k]) for k in "abcd")
+    p, q = (d, c) if s["mode"] else (c, d)
+    new = G.apply_swap(adj, s)
+    aff = np.zeros(n, dtype=bool)
+    for r, f, t in ((a, b, p), (b, a, q), (c, d, a if p == c else b), (d, c, b if p == c else a)):
+        row = list(adj[r])
+        row.remove(f)
+        aff |= (D[:, f] + 1 == D[:, r]) & ~(D[:, row] == D[:, [f]]).any(axis=1)
+        aff |= D[:, t] + 1 < D[:, r]
+    radius = (max(int(D.max()), 1) - 1) // 2
+    T = aff & (D[:, [a, b, c, d]].min(axis=1) <= radius)
+    w = np.where(T, 1, 2)
+    Dn = dist(new)[T]
+    total = int(D.sum()) + int(((np.where(Dn == 99, 0, Dn) - D[T]) * w).sum())
+    reached = n * n - int(((Dn == 99) * w).sum())
+    rest = D[np.ix_(~T, ~T)]
+    return total, reached, max(int(np.where(Dn == 99, 0, Dn).max(initial=0)), int(rest.max(initial=0)))
+
+
+@pytest.mark.parametrize("adj", [G.random_regular(60, 3, 1), G.random_regular(90, 4, 2), G.random_regular(64, 7, 3),
+                                 I.cycle(20), I.hypercube(4), I.complete(8)[:, :7]], ids=range(6))
+def test_near_sources_see_every_change(adj):
+    adj = np.asarray(adj, dtype=np.int32)
+    D = dist(adj)
+    rng = np.random.default_rng(7)
+    sw = []
+    while len(sw) < 40:   # any two disjoint edges: repeated edges may come out
+        a, c = rng.integers(len(adj), size=2)
+        b, d = adj[a, rng.integers(adj.shape[1])], adj[c, rng.integers(adj.shape[1])]
+        if len({int(a), int(b), int(c), int(d)}) == 4:
+            sw.append((0, a, b, c, d, rng.integers(2)))
+    for s in np.array(sw, dtype=G.SWAP_DTYPE):
+        Dn = dist(G.apply_swap(adj, s))
+        ok = Dn != 99
+        assert near_total(adj, D, s) == (int(Dn[ok].sum()), int(ok.sum()), int(Dn[ok].max()))
+
+
+def bases():
+    two = np.concatenate([I.complete(6), I.complete(6) + 6]).astype(np.int32)   # two cliques ...
+    two[0, 0], two[6, 0] = 6, 0                                                  # ... and one pair of links
+    two[1, 0], two[7, 0] = 7, 1
+    return {
+        "n31_d4": G.random_regular(31, 4, 1), "n33_d3": G.random_regular(34, 3, 2), "n129_d5": G.random_regular(130, 5, 3),
+        "n1023_d6": G.random_regular(1023, 6, 4), "n1025_d6": G.random_regular(1025, 6, 5),
+        "n700_d7": G.random_regular(700, 7, 6), "n513_d16": G.random_regular(513, 16, 7),
+        "n900_d3": G.random_regular(900, 3, 8), "n2100_d8": G.random_regular(2100, 8, 9),
+        "cycle28": I.cycle(28), "hypercube": I.hypercube(6), "two_cliques": two,
+        "multi": I.random_regular_np(90, 4, 11),   # repeated edges and loops
+    }
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", list(bases()))
+def test_near_candidates_equal_the_oracle(name):
+    adj = np.asarray(bases()[name], dtype=np.int32)
+    n, deg = adj.shape
+    rng = np.random.default_rng(5)
+    sw = []
+    while len(sw) < 24:
+        a, c = rng.integers(n, size=2)
+        b, d = adj[a, rng.integers(deg)], adj[c, rng.integers(deg)]
+        if len({int(a), int(b), int(c), int(d)}) == 4:
+            sw.append((0, a, b, c, d, rng.integers(2)))
+    v = rng.choice(n, 4, replace=False)
+    sw.append((0, v[0], v[1], v[2], v[3], 0))     # most likely no edges of the base
+    sw.append((0, -1, -1, -1, -1, 0))
+    sw = np.array(sw, dtype=G.SWAP_DTYPE)
+
+    def apply(s):   # each row whose removed neighbour it lists, as the header says
+        t = adj.copy()
+        if s["a"] < 0:
+            return t
+        a, b, c, d = (int(s[k]) for k in "abcd")
+        to = (c, d, a, b) if s["mode"] == 0 else (d, c, b, a)
+        for row, frm, u in zip((a, b, c, d), (b, a, d, c), to):
+            j = np.nonzero(t[row] == frm)[0]
+            if len(j):
+                t[row, j[0]] = u
+        return t
+
+    b = G.Batch(0)
+    b.add_base(adj)
+    for part in (sw, sw[:1]):
+        res = b.eval(part)
+        for s, got in zip(part, res):
+            r = O.bfs_pull(apply(s), np.arange(n))
+            assert (int(got["total"]), int(got["reached"]), int(got["levels"]), bool(got["connected"])) == \
+                (r.total(), int(r.reached.sum()), r.levels, bool(r.connected)), (name, s)
