@@ -565,27 +565,7 @@ __global__ void __launch_bounds__(128) batch_select(const BatchArgs a, const int
         const uint32_t *pw = reinterpret_cast<const uint32_t *>(B.planes);
         const size_t ps = (size_t)n * B.cols * 4, cw = (size_t)B.cols * 4;
         const unsigned wl = in ? w : 0u;
-        const Dist4 er = dist4_load(pw, ps, (size_t)r * cw + wl);
-        const Dist4 ef = dist4_load(pw, ps, (size_t)f * cw + wl);
-        const Dist4 et = dist4_load(pw, ps, (size_t)t * cw + wl);
-        uint32_t lost = dist4_eq(dist4_inc(ef), er);
-        bool skipped = false;   // the first slot that lists f is the one that goes
-        for (int j = 0; j < d; j += 4) {
-            int u[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                u[k] = __ldg(B.adj + (size_t)r * d + min(j + k, d - 1));
-                if (j + k < d && !skipped && u[k] == f) { u[k] = r; skipped = true; }   // (r itself is no parent)
-                if (j + k >= d) u[k] = r;
-            }
-            Dist4 x[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) x[k] = dist4_load(pw, ps, (size_t)u[k] * cw + wl);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) lost &= ~dist4_eq(x[k], ef);
-        }
-        s_aff[i][lane] = lost | dist4_lt(dist4_inc(et), er);
-        s_near[i][lane] = ~dist4_lt(dist4_const((unsigned)B.radius), er);
+        edit_masks(pw, ps, cw, B.adj, d, r, f, t, wl, (unsigned)B.radius, s_aff[i][lane], s_near[i][lane]);
         __syncthreads();
         if (i == 0) {
             uint32_t go = (s_near[0][lane] | s_near[1][lane] | s_near[2][lane] | s_near[3][lane]) &

@@ -156,6 +156,8 @@ struct gg_engine {
     bool p_dirty = true;                 // push buffers must be zeroed before the next launch
     unsigned long long *d_counts = nullptr;
     unsigned *d_masks = nullptr;
+    unsigned long long *d_wcounts = nullptr, *h_wcounts = nullptr;   // pairs within the sources (on first use)
+    size_t wcounts_n = 0;
     unsigned long long *d_level_ns = nullptr, *h_level_ns = nullptr;
     int *d_levels_run = nullptr, *h_levels_run = nullptr;                 // [nb_alloc]
     unsigned long long *d_batch_ns = nullptr, *h_batch_ns = nullptr;     // [2 * nb_alloc]
@@ -202,6 +204,9 @@ void free_counters(gg_engine *e) {
     cudaFree(e->d_status); cudaFree(e->d_masks); cudaFree(e->d_level_ns); cudaFree(e->d_vtot);
     cudaFreeHost(e->h_status); cudaFreeHost(e->h_masks);
     cudaFreeHost(e->h_level_ns);
+    cudaFree(e->d_wcounts); cudaFreeHost(e->h_wcounts);
+    e->d_wcounts = e->h_wcounts = nullptr;
+    e->wcounts_n = 0;
     e->d_status = e->h_status = nullptr;
     e->d_bad = e->d_asym = e->d_wasym = e->h_bad = nullptr;
     e->d_vtot = nullptr;
@@ -245,23 +250,23 @@ int kernel_degree_slot(int d) {
     }
 }
 
-template <bool PL>
+template <int MODE>
 void *kernel_for_t(int d) {
     switch (kernel_degree_slot(d)) {
-        case 3: return (void *)gg::bfs_batch_kernel<3, PL>;
-        case 4: return (void *)gg::bfs_batch_kernel<4, PL>;
-        case 6: return (void *)gg::bfs_batch_kernel<6, PL>;
-        case 8: return (void *)gg::bfs_batch_kernel<8, PL>;
-        case 12: return (void *)gg::bfs_batch_kernel<12, PL>;
-        case 16: return (void *)gg::bfs_batch_kernel<16, PL>;
-        default: return (void *)gg::bfs_batch_kernel<0, PL>;
+        case 3: return (void *)gg::bfs_batch_kernel<3, MODE>;
+        case 4: return (void *)gg::bfs_batch_kernel<4, MODE>;
+        case 6: return (void *)gg::bfs_batch_kernel<6, MODE>;
+        case 8: return (void *)gg::bfs_batch_kernel<8, MODE>;
+        case 12: return (void *)gg::bfs_batch_kernel<12, MODE>;
+        case 16: return (void *)gg::bfs_batch_kernel<16, MODE>;
+        default: return (void *)gg::bfs_batch_kernel<0, MODE>;
     }
 }
 
-// The BFS kernel for degree d; `planes`: the variant that also writes the
-// distance planes.
-void *kernel_for(int d, bool planes = false) {
-    return planes ? kernel_for_t<true>(d) : kernel_for_t<false>(d);
+// The BFS kernel for degree d; mode: see gg::kPlain.
+void *kernel_for(int d, int mode = gg::kPlain) {
+    return mode == gg::kPlanes ? kernel_for_t<gg::kPlanes>(d)
+                               : mode == gg::kWithin ? kernel_for_t<gg::kWithin>(d) : kernel_for_t<gg::kPlain>(d);
 }
 
 // Walk ends per row up to depth K: d + d^2 + ... + d^K.
@@ -599,8 +604,22 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
     const bool want_ns = o && o->level_ns;
     const int ns_all = s1 - s0;
     const int nb = (ns_all + e->batch_bits - 1) / e->batch_bits;
+    const bool within = x && x->within;
+    if (within && (!x->inv || wvc || x->planes || e->form != FORM_GRAPH)) return fail(GG_BAD_ARG, "pairs within the sources need a source list");
+    // Row width.  A short source list fills one batch of narrower rows (1600 of 65536
+    // sources: 13 chunks instead of 32).
+    const int nC = within && nb == 1 ? (ns_all + 127) / 128 : e->nC;
+    const uint32_t items = (uint32_t)((long long)e->rows * nC);
     gg_status s = ensure_counters(e, cap_req, nb);
     if (s != GG_OK) return s;
+    if (within && (size_t)nb * (cap_req + 1) > e->wcounts_n) {
+        cudaFree(e->d_wcounts); cudaFreeHost(e->h_wcounts);
+        e->d_wcounts = e->h_wcounts = nullptr;
+        e->wcounts_n = 0;
+        GG_CK(cudaMalloc(&e->d_wcounts, (size_t)nb * (cap_req + 1) * sizeof(unsigned long long)));
+        GG_CK(cudaMallocHost(&e->h_wcounts, (size_t)nb * (cap_req + 1) * sizeof(unsigned long long)));
+        e->wcounts_n = (size_t)nb * (cap_req + 1);
+    }
     const int stride = cap_req + 1;      // counts of batch b at [b * stride, (b + 1) * stride)
 
     (void)cudaGetLastError();  // launch checks below must not see an earlier, unrelated error
@@ -622,7 +641,7 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
     if (want_ns) d2h += lv * sizeof(unsigned long long);
     // Walk pass for this evaluation: not with the WVC masks or the distance planes
     // (their per-level bookkeeping lives in the level loop), at most the level cap.
-    const int walk_K = (wvc || (x && x->planes)) ? 0 : std::min(e->walk_K, cap_req);
+    const int walk_K = (wvc || (x && (x->planes || within))) ? 0 : std::min(e->walk_K, cap_req);
     const int launches = 1 + ((long long)e->rows * e->d > 0 ? 1 : 0) + (walk_K > 0 ? 1 : 0) + (walk_K >= 3 ? 1 : 0);
     void *wall = walk_K > 0 ? walk_all_for(e, walk_K, nb) : nullptr;
 
@@ -636,7 +655,9 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
         // control block, range-check and symmetry words
         GG_CK(cudaMemsetAsync(e->d_status, 0, sizeof(Ctl) + 3 * sizeof(int), q));   // ctl, bad, asym, wasym
         const long long n = (long long)e->rows * e->d;
-        if (e->form == FORM_GRAPH) {
+        if (e->form == FORM_GRAPH && within) {
+            // read in place
+        } else if (e->form == FORM_GRAPH) {
             if (d_table_in != e->d_table)
                 GG_CK(cudaMemcpyAsync(e->d_table, d_table_in, e->table_elems * 4, cudaMemcpyDeviceToDevice, q));
             if (n > 0) {
@@ -720,7 +741,7 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
             GG_CK(cudaLaunchKernel(wk, dim3(wgrid), dim3(gg::kIndexBlock), wargs, wsmem, q));
         }
         BfsArgs a{};
-        a.adj = e->d_adj;
+        a.adj = within ? d_table_in : e->d_adj;
         a.inv = x && x->inv ? x->inv : e->d_inv;
         a.src_first = x && x->inv ? 0 : e->src_first;
         if (x && x->planes) {
@@ -736,7 +757,7 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
         a.fl0 = e->d_fl0; a.fl1 = e->d_fl1;
         a.P0 = e->d_P0; a.P1 = e->d_P1; a.pf0 = e->d_pf0; a.pf1 = e->d_pf1;
         // Below ~1M chunks a pull level costs about one grid barrier anyway.
-        a.push_ppm = (long long)e->items >= (long long)e->push_min_items ? e->push_ppm : 0;
+        a.push_ppm = (long long)items >= (long long)e->push_min_items ? e->push_ppm : 0;
         a.nf = e->d_nf;
         a.nf2 = e->d_nf2;
         a.asym = e->d_asym;
@@ -747,8 +768,9 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
         a.level_ns = want_ns ? e->d_level_ns : nullptr;
         a.batch_ns = e->d_batch_ns;
         a.ctl = e->d_ctl;
-        a.rows = e->rows; a.d = e->d; a.nC = e->nC; a.items = e->items;
-        a.div_nc = FastDiv((uint32_t)e->nC);
+        a.rows = e->rows; a.d = e->d; a.nC = nC; a.items = items;
+        a.div_nc = FastDiv((uint32_t)nC);
+        a.wcounts = within ? e->d_wcounts : nullptr;
         a.max_levels = cap_req;
         a.dense_w_ppm = e->dense_w_ppm;
         a.dense_r_ppm = e->dense_r_ppm;
@@ -772,7 +794,8 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
         a.vall_fl = wall ? e->d_vall_fl : nullptr;
         a.third = wall && e->walk_third ? e->d_F0 : nullptr;
         void *args[] = {&a};
-        GG_CK(cudaLaunchCooperativeKernel(kernel_for(e->d, a.planes != nullptr), dim3(e->grid), dim3(gg::kBlock), args,
+        const int mode = a.planes ? gg::kPlanes : within ? gg::kWithin : gg::kPlain;
+        GG_CK(cudaLaunchCooperativeKernel(kernel_for(e->d, mode), dim3(e->grid), dim3(gg::kBlock), args,
                                           wall ? (size_t)e->walk_smem_off : e->smem_bytes, q));
         if (timed) GG_CK(cudaEventRecord(e->ev1, q));
         // One copy back: control block, status words, per-batch levels and
@@ -781,6 +804,9 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
                               cudaMemcpyDeviceToHost, q));
         if (wvc)
             GG_CK(cudaMemcpyAsync(e->h_masks, e->d_masks, (size_t)nb * stride * sizeof(unsigned),
+                                  cudaMemcpyDeviceToHost, q));
+        if (within)
+            GG_CK(cudaMemcpyAsync(e->h_wcounts, e->d_wcounts, (size_t)nb * stride * sizeof(unsigned long long),
                                   cudaMemcpyDeviceToHost, q));
         if (want_ns)
             GG_CK(cudaMemcpyAsync(e->h_level_ns, e->d_level_ns, lv * sizeof(unsigned long long),
@@ -834,7 +860,7 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
     e->last_launches = launches;
     e->last_batches = nb;
 
-    if (e->form == FORM_GRAPH && *e->h_bad)
+    if (e->form == FORM_GRAPH && !within && *e->h_bad)
         return fail(GG_BAD_ARG, "adjacency entry outside [0, N)");
     if (e->h_ctl->err)
         return fail(GG_TIMEOUT, "grid barrier wait exceeded its limit at level " +
@@ -866,6 +892,15 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
         if (run >= cap_req && c[cap_req]) R.capped = 1;
     }
     R.connected = (!R.capped && R.reached == R.pairs) ? 1 : 0;
+    if (within) {
+        x->within[0] = x->within[1] = 0;
+        for (int b = 0; b < nb; ++b)
+            for (int L = 0; L <= e->h_levels_run[b] && L <= cap_req; ++L) {
+                const unsigned long long c = e->h_wcounts[(size_t)b * stride + L];
+                x->within[0] += (uint64_t)L * c;
+                x->within[1] += c;
+            }
+    }
     if (wvc) {
         // Lane-aggregated completion masks across batches: a batch's mask stays
         // at its final value after its last level.

@@ -17,6 +17,9 @@ struct EvalExtra {
     uint4 *planes = nullptr;       // distance bit-planes to write (every source, in order)
     int nplanes = 0;
     bool no_graph = false;         // launch directly, neither capture nor replay
+    uint64_t *within = nullptr;    // host [2]: total distance and number of the pairs whose vertex is a
+                                   // source of the list too (diagonal included); needs `inv`, and a
+                                   // plain-graph table that is range-checked already (read in place)
 };
 
 __attribute__((visibility("hidden"))) void set_last_error(const char *msg);

@@ -158,7 +158,13 @@ struct BfsArgs {
     uint4 *vall;
     const uint32_t *vall_fl;
     uint4 *third;
+    // kWithin only, [nb][stride]: the pairs of counts[] whose vertex is a source itself
+    // (inv[v] >= 0)
+    unsigned long long *wcounts;
 };
+
+// What bfs_batch_kernel does besides counting pairs.
+enum { kPlain = 0, kPlanes = 1, kWithin = 2 };   // nothing; distance planes; pairs within the sources
 
 // Where a level's new pairs go in the distance planes.
 struct PlaneOut {
@@ -344,14 +350,15 @@ constexpr int kGrab = GG_GRAB;  // tiles a warp takes (and keeps in flight) at o
 // One level's work on tiles [tile0, tile0 + U) of the calling warp (a tile is 32
 // consecutive uint4 chunks, one per lane).  Every load of the U tiles is issued
 // before any result is used, so each warp keeps U*(d+1) 16-byte loads in flight.
-template <int D, int U, bool PL>
+template <int D, int U, int MODE>
 __device__ __forceinline__ void level_tiles(const BfsArgs &a, const int d, const int32_t *adj,
                                             const unsigned v_base, const unsigned tile0,
                                             const unsigned t_hi, const uint4 *Fc, uint4 *Fn,
                                             const uint32_t *fc, uint32_t *fn, const bool dense,
                                             const bool write_all, const bool skip_full,
                                             const bool split, const unsigned lane, unsigned &cnt, unsigned &and_pre,
-                                            unsigned &and_post) {
+                                            unsigned &and_post, unsigned &wcnt) {
+    constexpr bool PL = MODE == kPlanes;
     unsigned t[U], c[U];
     bool ok[U], have[U];
     uint4 own[U], acc[U], nw[U];
@@ -442,6 +449,9 @@ __device__ __forceinline__ void level_tiles(const BfsArgs &a, const int d, const
                 and_post &= u4and(u4or(own[u], nw[u]));
             }
             cnt += u4popc(nw[u]);
+            if constexpr (MODE == kWithin) {
+                if (u4any(nw[u]) && __ldg(a.inv + a.div_nc.div(t[u])) >= 0) wcnt += u4popc(nw[u]);
+            }
         }
         const unsigned b = __ballot_sync(0xffffffffu, u4any(nw[u]));
         if (lane == 0 && (tile0 + u) < t_hi) fn[tile0 + u] = b;
@@ -585,29 +595,41 @@ __device__ __forceinline__ void vpull_tiles(const BfsArgs &a, const int d, const
     }
 }
 
+// Tiles a warp takes at once in the skip-full stage (their not-full words in one load).
+// It works through the ones that still miss a source one after the other, so while many
+// do (a missing pair or more for every four tiles) a block's range is cut into at least
+// four groups a warp: 32 at a time left half of a block's warps idle and the others with
+// up to 32 tiles in a row (n = 16000, d = 6: the last level took 44 us, 24 so).  When
+// nearly all tiles are full, 32 at a time (n = 65536, d = 8: 5.7 against 8.1 us).
+__device__ __forceinline__ unsigned skip_group(const unsigned tiles, const bool many) {
+    return many ? min(32u, max(1u, tiles / (kBlock / 32 * 4))) : 32u;
+}
+
 // One visited-set pull level over the block's tiles [s_next, t_hi) (s_next set by the
 // caller); returns this thread's count of new pairs (no_own: of the pairs in the
 // rows it wrote, padding included; every chunk is then written).  nf_use (the skip-full stage,
-// with nfc written whole by the level before): a warp takes 32 tiles, passes over
+// with nfc written whole by the level before): a warp takes a group of tiles, passes over
 // those whose chunks are all full, and runs the others LAZY.
 template <int D>
 static __device__ __noinline__ unsigned vpull_level(const BfsArgs &a, const int d, const int32_t *adj,
-                                                    const unsigned v_base, const unsigned t_hi, const uint4 *X,
-                                                    uint4 *Y, const uint32_t *fc, uint32_t *fn, const uint32_t *nfc,
-                                                    uint32_t *nfn, const bool dense, const bool wr_all,
+                                                    const unsigned v_base, const unsigned t_lo, const unsigned t_hi,
+                                                    const uint4 *X, uint4 *Y, const uint32_t *fc, uint32_t *fn,
+                                                    const uint32_t *nfc, uint32_t *nfn, const bool dense, const bool wr_all,
                                                     const bool skip_full, const bool split, const bool nf_use,
-                                                    const bool no_own, unsigned *s_next) {
+                                                    const bool nf_many, const bool no_own, unsigned *s_next) {
     const unsigned lane = threadIdx.x & 31u;
     unsigned cnt = 0u;
     if (nf_use) {
+        const unsigned group = skip_group(t_hi - t_lo, nf_many);
         for (;;) {
             unsigned tile0 = 0;
-            if (lane == 0) tile0 = atomicAdd(s_next, 32u);
+            if (lane == 0) tile0 = atomicAdd(s_next, group);
             tile0 = __shfl_sync(0xffffffffu, tile0, 0);
             if (tile0 >= t_hi) break;
             const unsigned my = tile0 + lane;
-            const unsigned w = my < t_hi ? __ldcg(nfc + my) : 0u;
-            if (my < t_hi && w == 0u) {
+            const bool in = lane < group && my < t_hi;
+            const unsigned w = in ? __ldcg(nfc + my) : 0u;
+            if (in && w == 0u) {
                 fn[my] = 0u;
                 nfn[my] = 0u;
             }
@@ -1802,8 +1824,9 @@ static __device__ __noinline__ unsigned walk_batch(const BfsArgs &a, const int b
 // the diagonal set, level-1 frontier and its flags written) -> grid barrier ->
 // levels, each ended by a grid barrier.  One launch instead of one per batch
 // saves the launch gap and the shared-memory adjacency reload per batch.
-template <int D, bool PL>
+template <int D, int MODE>
 __global__ void __launch_bounds__(kBlock, min_blocks_for(D)) bfs_batch_kernel(const __grid_constant__ BfsArgs a) {
+    constexpr bool PL = MODE == kPlanes;
     const int d = D > 0 ? D : a.d;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned gtid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1842,7 +1865,7 @@ __global__ void __launch_bounds__(kBlock, min_blocks_for(D)) bfs_batch_kernel(co
     if (threadIdx.x == 0) {
         S.sym = a.walk_asym != nullptr && a.vtot != nullptr && ld_acquire_i(a.walk_asym) == 0;
         S.push_on = D > 0 && 32 % D == 0 && a.push_ppm > 0 && a.P0 != nullptr && a.asym != nullptr &&
-                    a.masks == nullptr && (PL || a.walk_K == 0);
+                    a.masks == nullptr && MODE != kWithin && (PL || a.walk_K == 0);
         S.dirty_p = -1;
     }
     __syncthreads();
@@ -1860,7 +1883,7 @@ __global__ void __launch_bounds__(kBlock, min_blocks_for(D)) bfs_batch_kernel(co
         __syncthreads();
     }
 
-    const bool walk = !PL && a.walk_K > 0;
+    const bool walk = MODE == kPlain && a.walk_K > 0;
     const bool vp = walk && vpull_on(a);   // visited-set pull after the walk
     for (int b = 0; b < a.nb; ++b) {
         const int ns = min(128 * a.nC, a.ns_total - b * 128 * a.nC);
@@ -1879,6 +1902,8 @@ __global__ void __launch_bounds__(kBlock, min_blocks_for(D)) bfs_batch_kernel(co
             if (blockIdx.x == 0)
                 for (int i = threadIdx.x; i <= a.max_levels; i += blockDim.x) {
                     counts[i] = i == 0 ? (unsigned long long)ns : 0ull;
+                    if constexpr (MODE == kWithin)
+                        a.wcounts[(size_t)b * (size_t)a.stride + i] = counts[i];   // (a source's own pair)
                     if (masks) masks[i] = 0xffffffffu;
                 }
             const int dirty = S.dirty_p, clean = dirty == 0 ? 1 : 0;
@@ -1934,13 +1959,14 @@ __global__ void __launch_bounds__(kBlock, min_blocks_for(D)) bfs_batch_kernel(co
                                c_prev * 1000000ull >= pairs * (unsigned long long)a.dense_r_ppm;
             const bool skip_full = S.reached * 1000000ull >= pairs * (unsigned long long)a.full_skip_ppm;
             const bool nf_use = !push && skip_full && S.nf_valid;
+            const bool nf_many = (pairs - S.reached) * 4ull > ntiles;
             const bool split = dense && S.reached * 1000000ull >= pairs * (unsigned long long)a.split_ppm;
             const bool write_all =
                 !nf_use && c_prev * 1000000ull >= pairs * (unsigned long long)a.dense_w_ppm;
             // dense visited-set pull on a table without one-way entries: no own chunks
             const bool no_own = vp && S.sym && dense && !nf_use;
             const bool odd = (L & 1) != 0;
-            unsigned cnt = 0u, and_pre = 0xffffffffu, and_post = 0xffffffffu;
+            unsigned cnt = 0u, wcnt = 0u, and_pre = 0xffffffffu, and_post = 0xffffffffu;
             if (push) {
                 uint4 *Pc = in_p ? a.P1 : a.P0;
                 uint4 *Pn = in_p ? a.P0 : a.P1;
@@ -1973,10 +1999,10 @@ __global__ void __launch_bounds__(kBlock, min_blocks_for(D)) bfs_batch_kernel(co
                     cnt = dense_rows32<(D > 0 ? D : 1)>(X, Y, adj, v_base, t_hi, odd ? a.fl1 : a.fl0,
                                                         odd ? a.nf2 : a.nf, split, &s_next);
                 else
-                    cnt = vpull_level<D>(a, d, adj, v_base, t_hi, X, Y,
+                    cnt = vpull_level<D>(a, d, adj, v_base, t_lo, t_hi, X, Y,
                                          first ? S.fl_walk : (odd ? a.fl0 : a.fl1), odd ? a.fl1 : a.fl0,
                                          odd ? a.nf : a.nf2, odd ? a.nf2 : a.nf, dense,
-                                         first || (L == a.walk_K + 2 && r_on), skip_full, split, nf_use, no_own,
+                                         first || (L == a.walk_K + 2 && r_on), skip_full, split, nf_use, nf_many, no_own,
                                          &s_next);
             } else {
                 const uint4 *Fc = in_p >= 0 ? (in_p ? a.P1 : a.P0) : (odd ? a.F0 : a.F1);
@@ -1988,21 +2014,23 @@ __global__ void __launch_bounds__(kBlock, min_blocks_for(D)) bfs_batch_kernel(co
                 if (threadIdx.x == 0) s_next = t_lo;
                 __syncthreads();
                 if (nf_use) {
-                    // Skip-full stage: a warp takes 32 tiles, reads their not-full
+                    // Skip-full stage: a warp takes a group of tiles, reads their not-full
                     // words in one load, clears the frontier flags of the full ones
                     // and works only on the others.
+                    const unsigned group = skip_group(t_hi - t_lo, nf_many);
                     for (;;) {
                         unsigned tile0 = 0;
-                        if (lane == 0) tile0 = atomicAdd(&s_next, 32u);
+                        if (lane == 0) tile0 = atomicAdd(&s_next, group);
                         tile0 = __shfl_sync(0xffffffffu, tile0, 0);
                         if (tile0 >= t_hi) break;
                         const unsigned my = tile0 + lane;
-                        const unsigned w = my < t_hi ? __ldcg(a.nf + my) : 0u;
-                        if (my < t_hi && w == 0u) fn[my] = 0u;
+                        const bool in = lane < group && my < t_hi;
+                        const unsigned w = in ? __ldcg(a.nf + my) : 0u;
+                        if (in && w == 0u) fn[my] = 0u;
                         for (unsigned todo = __ballot_sync(0xffffffffu, w != 0u); todo; todo &= todo - 1u) {
                             const unsigned tj = tile0 + (unsigned)(__ffs((int)todo) - 1);
-                            level_tiles<D, 1, PL>(a, d, adj, v_base, tj, t_hi, Fc, Fn, fc, fn, dense, write_all,
-                                              skip_full, split, lane, cnt, and_pre, and_post);
+                            level_tiles<D, 1, MODE>(a, d, adj, v_base, tj, t_hi, Fc, Fn, fc, fn, dense, write_all,
+                                                skip_full, split, lane, cnt, and_pre, and_post, wcnt);
                         }
                     }
                 } else {
@@ -2011,9 +2039,9 @@ __global__ void __launch_bounds__(kBlock, min_blocks_for(D)) bfs_batch_kernel(co
                         if (lane == 0) tile0 = atomicAdd(&s_next, (unsigned)kGrab);
                         tile0 = __shfl_sync(0xffffffffu, tile0, 0);
                         if (tile0 >= t_hi) break;
-                        level_tiles<D, kGrab, PL>(a, d, adj, v_base, tile0, t_hi, Fc, Fn, fc, fn, dense,
-                                              write_all, skip_full, split, lane, cnt, and_pre,
-                                              and_post);
+                        level_tiles<D, kGrab, MODE>(a, d, adj, v_base, tile0, t_hi, Fc, Fn, fc, fn, dense,
+                                                write_all, skip_full, split, lane, cnt, and_pre,
+                                                and_post, wcnt);
                     }
                 }
             }
@@ -2023,6 +2051,10 @@ __global__ void __launch_bounds__(kBlock, min_blocks_for(D)) bfs_batch_kernel(co
             unsigned *masks = a.masks ? a.masks + (size_t)b * (size_t)a.stride : nullptr;
             const unsigned wsum = __reduce_add_sync(0xffffffffu, cnt);
             if (lane == 0) s_sum[threadIdx.x >> 5] = wsum;
+            if constexpr (MODE == kWithin) {
+                const unsigned w = __reduce_add_sync(0xffffffffu, wcnt);
+                if (lane == 0 && w) atomicAdd(a.wcounts + (size_t)b * (size_t)a.stride + L, (unsigned long long)w);
+            }
             if (masks) {
                 const unsigned w0 = __reduce_and_sync(0xffffffffu, and_pre);
                 const unsigned w1 = __reduce_and_sync(0xffffffffu, and_post);

@@ -59,6 +59,36 @@ __device__ __forceinline__ unsigned dist4_sum(const Dist4 a, const uint32_t mask
     return __popc(a.p[0] & mask) + 2u * __popc(a.p[1] & mask) + 4u * __popc(a.p[2] & mask) + 8u * __popc(a.p[3] & mask);
 }
 
+// What one replaced pull entry of a 2-opt (row r lists t in place of f) does to 32 sources
+// (word w of the planes): `aff` -- the row loses its last parent, or the added edge
+// shortens it; `near` -- the source lies within `radius` of r.  The rows' plane words are
+// coalesced over the lanes' words, four neighbours' loads in flight together.
+__device__ __forceinline__ void edit_masks(const uint32_t *pw, const size_t ps, const size_t cw, const int32_t *adj,
+                                           const int d, const int r, const int f, const int t, const unsigned w,
+                                           const unsigned radius, uint32_t &aff, uint32_t &near) {
+    const Dist4 er = dist4_load(pw, ps, (size_t)r * cw + w);
+    const Dist4 ef = dist4_load(pw, ps, (size_t)f * cw + w);
+    const Dist4 et = dist4_load(pw, ps, (size_t)t * cw + w);
+    uint32_t lost = dist4_eq(dist4_inc(ef), er);
+    bool skipped = false;   // the first slot that lists f is the one that goes
+    for (int j = 0; j < d; j += 4) {
+        int u[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            u[k] = __ldg(adj + (size_t)r * d + min(j + k, d - 1));
+            if (j + k < d && !skipped && u[k] == f) { u[k] = r; skipped = true; }   // (r itself is no parent)
+            if (j + k >= d) u[k] = r;
+        }
+        Dist4 x[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = dist4_load(pw, ps, (size_t)u[k] * cw + w);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) lost &= ~dist4_eq(x[k], ef);
+    }
+    aff = lost | dist4_lt(dist4_inc(et), er);
+    near = ~dist4_lt(dist4_const(radius), er);
+}
+
 // Distance sum and eccentricity of every source; with `top`, also the number of its
 // vertices at distance `diam`.
 template <int NP>
