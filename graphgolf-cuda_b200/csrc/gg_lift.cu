@@ -33,7 +33,16 @@
 // and group into counts[L][k]); after the grid barrier every block reads the
 // round's counts, and the round ends when no candidate found a pair or every
 // candidate reached all M*N pairs.
+//
+// Moves by change (default, within the limits of delta_limits): the base's distance rows
+// are kept (one search of the base that also writes bit-planes, when the first
+// population after gg_lift_set_base comes), and a candidate is scored by following what
+// its edit changes in the rows near it (gg_delta.cuh): lift_select lists the rows,
+// lift_delta follows them.  Edits that leave the lift asymmetric, changes that outgrow
+// the lists or reach distances past kDeltaMax, bases that are asymmetric, disconnected or
+// of diameter above 15, and handles with an explicit group run the search above.
 #include "gg.h"
+#include "gg_delta.cuh"
 #include "gg_internal.h"
 #include "gg_kernels.cuh"
 
@@ -65,7 +74,20 @@ struct LiftArgs {
     gg::Ctl *ctl;
     unsigned expected;
     long long wait_ns;
+    // Distance bit-planes of a single candidate (the base), all zero before: bit s % 128 of
+    // planes[(p * N + v) * cpc + s / 128] is bit p of the distance of (source s, vertex v);
+    // distances up to 15.  nullptr: none.
+    uint4 *planes;
 };
+
+// New pairs of chunk t at level L into the planes (one writer a chunk).
+__device__ __forceinline__ void put_planes(const LiftArgs &a, const size_t t, const int L, const uint4 nw) {
+    for (int p = 0; p < 4; ++p)
+        if ((L >> p) & 1) {
+            uint4 *q = a.planes + (size_t)p * a.N * a.cpc + t;
+            *q = gg::u4or(*q, nw);
+        }
+}
 
 // Candidate tables ([K][M][d][comps], comps = axes of the lift): slot (k, r, i)
 // is the base slot unless candidate k's edit names slot (r, i).
@@ -244,6 +266,7 @@ __device__ __forceinline__ unsigned level1_pass(const LiftArgs &a, const int32_t
             n1 = gg::andnot(make_uint4(nb[0], nb[1], nb[2], nb[3]), vis);
             gg::or_into(vis, n1);
             cnt += gg::u4popc(n1);
+            if (a.planes && gg::u4any(n1)) put_planes(a, (size_t)v * W + w, 1, n1);
         }
         a.V[(size_t)v * W + w] = vis;
         Fn[(size_t)v * W + w] = n1;
@@ -324,6 +347,7 @@ __global__ void __launch_bounds__(kLiftBlock, 4) lift_kernel(const LiftArgs a) {
                         if (gg::u4any(nw)) {
                             a.V[t] = gg::u4or(own, nw);
                             cnt += gg::u4popc(nw);
+                            if (a.planes) put_planes(a, t, L, nw);
                         }
                     }
                     Fn[t] = nw;
@@ -361,6 +385,459 @@ __global__ void __launch_bounds__(kLiftBlock, 4) lift_kernel(const LiftArgs a) {
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) a.ctl->levels_run = levels_run;
+}
+
+// ---- moves by change ---------------------------------------------------------------
+
+// The lift's axes: n lifted and m orbit sizes; a part has one axis.
+struct LiftAxes {
+    int axes;
+    int n[3], m[3];
+    // vertex of copy c of orbit o
+    __device__ __forceinline__ int vertex(int o, int c) const {
+        int v = 0, mul = 1;
+        for (int j = axes - 1; j >= 0; --j) {
+            const int k = n[j] / m[j], x = o % m[j] + m[j] * (c % k);
+            o /= m[j];
+            c /= k;
+            v += x * mul;
+            mul *= n[j];
+        }
+        return v;
+    }
+    // orbit and copy of vertex v
+    __device__ __forceinline__ void place(int v, int &o, int &c) const {
+        int mo = 1, mc = 1;
+        o = c = 0;
+        for (int j = axes - 1; j >= 0; --j) {
+            const int x = v % n[j];
+            v /= n[j];
+            o += x % m[j] * mo;
+            c += x / m[j] * mc;
+            mo *= m[j];
+            mc *= n[j] / m[j];
+        }
+    }
+    // v moved by the diff df (components in [0, n))
+    __device__ __forceinline__ int move(int v, const int32_t *df) const {
+        int r = 0, mul = 1;
+        for (int j = axes - 1; j >= 0; --j) {
+            int x = v % n[j] + df[j];
+            v /= n[j];
+            x -= x >= n[j] ? n[j] : 0;
+            r += x * mul;
+            mul *= n[j];
+        }
+        return r;
+    }
+    // orbit that the diff df leads to from orbit o, and the reverse diff
+    __device__ __forceinline__ int orbit_at(int o, const int32_t *df) const {
+        int r = 0, mul = 1;
+        for (int j = axes - 1; j >= 0; --j) {
+            r += (o % m[j] + df[j]) % m[j] * mul;
+            o /= m[j];
+            mul *= m[j];
+        }
+        return r;
+    }
+    __device__ __forceinline__ bool reverse(const int32_t *a, const int32_t *b) const {
+        for (int j = 0; j < axes; ++j)
+            if ((a[j] + b[j]) % n[j] != 0) return false;
+        return true;
+    }
+    __device__ __forceinline__ bool same(const int32_t *a, const int32_t *b) const {
+        for (int j = 0; j < axes; ++j)
+            if (a[j] != b[j]) return false;
+        return true;
+    }
+};
+
+// A row of the base adjacency: rw 16-bit words -- the d neighbours, padding with the vertex
+// itself, then its orbit and its copy in the last two.
+__global__ void delta_rows_kernel(const int32_t *table, const LiftAxes ax, int N, int d, int rw, uint16_t *rows) {
+    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < N; v += gridDim.x * blockDim.x) {
+        int o, c;
+        ax.place(v, o, c);
+        uint16_t *out = rows + (size_t)v * rw;
+        for (int i = 0; i < rw - 2; ++i)
+            out[i] = (uint16_t)(i < d ? ax.move(v, table + ((size_t)o * d + i) * ax.axes) : v);
+        out[rw - 2] = (uint16_t)o;
+        out[rw - 1] = (uint16_t)c;
+    }
+}
+
+// A part's diffs as 16-bit words, dp a row, padded with 0.
+__global__ void delta_diffs_kernel(const int32_t *table, int M, int d, int dp, uint16_t *diffs) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < M * dp; k += gridDim.x * blockDim.x) {
+        const int o = k / dp, i = k % dp;
+        diffs[k] = (uint16_t)(i < d ? table[(size_t)o * d + i] : 0);
+    }
+}
+
+// 1 into *asym when some entry of the table and its reverse entry are not listed equally
+// often by their rows.
+__global__ void delta_symmetry(const int32_t *table, const LiftAxes ax, int M, int d, int *asym) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < M * d; k += gridDim.x * blockDim.x) {
+        const int o = k / d;
+        const int32_t *df = table + (size_t)k * ax.axes;
+        const int q = ax.orbit_at(o, df);
+        int here = 0, back = 0;
+        for (int j = 0; j < d; ++j) {
+            here += ax.same(table + ((size_t)o * d + j) * ax.axes, df);
+            back += ax.reverse(table + ((size_t)q * d + j) * ax.axes, df);
+        }
+        if (here != back) *asym = 1;
+    }
+}
+
+// Distance planes -> byte rows dist[s][v] (pitch bytes a row).  A block takes 128 vertices
+// and 128 sources: a thread holds its vertex's four plane words, and each source's bytes go
+// out 32 a warp.
+__global__ void __launch_bounds__(128) delta_bytes(const uint4 *planes, int N, int M, int cpc, uint8_t *dist, int pitch) {
+    const int v = blockIdx.x * 128 + (int)threadIdx.x, c = blockIdx.y;
+    uint4 x[4];
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+        x[p] = v < N ? __ldg(planes + ((size_t)p * N + v) * cpc + c) : gg::u4zero();
+    if (v >= pitch) return;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        unsigned w[4];
+#pragma unroll
+        for (int p = 0; p < 4; ++p) w[p] = gg::comp_of(x[p], k);
+        const int s0 = c * 128 + k * 32;
+#pragma unroll 8
+        for (int i = 0; i < 32; ++i) {
+            if (s0 + i >= M) break;
+            dist[(size_t)(s0 + i) * pitch + v] =
+                (uint8_t)(((w[0] >> i) & 1u) | (((w[1] >> i) & 1u) << 1) | (((w[2] >> i) & 1u) << 2) | (((w[3] >> i) & 1u) << 3));
+        }
+    }
+}
+
+// ball[o]: the orbits with a vertex within `radius` of representative o, one bit each.
+__global__ void __launch_bounds__(256) delta_balls(const uint8_t *dist, int pitch, int N, const uint16_t *rows, int rw,
+                                                   int words, unsigned radius, uint32_t *ball) {
+    extern __shared__ uint32_t s_ball[];
+    const int o = blockIdx.x;
+    for (int k = threadIdx.x; k < words; k += blockDim.x) s_ball[k] = 0u;
+    __syncthreads();
+    const uint4 *row = reinterpret_cast<const uint4 *>(dist + (size_t)o * pitch);
+    const unsigned r4 = radius * 0x01010101u;
+    for (int k = threadIdx.x; k < pitch / 16; k += blockDim.x) {
+        const uint4 q = __ldg(row + k);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            for (unsigned m = __vcmpleu4(gg::comp_of(q, j), r4) & 0x01010101u; m; m &= m - 1u) {
+                const int v = k * 16 + j * 4 + (__ffs((int)m) - 1) / 8;
+                if (v >= N) continue;
+                const unsigned b = __ldg(rows + (size_t)v * rw + rw - 2);
+                atomicOr(s_ball + (b >> 5), 1u << (b & 31u));
+            }
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < words; k += blockDim.x) ball[(size_t)o * words + k] = s_ball[k];
+}
+
+// A candidate's state: how it is scored, and the change of its number of pairs at each
+// distance (kDeltaInf: unreached).
+enum { kByChange = 0, kSearch = 1 };
+struct DeltaCand {
+    int mode;
+    int count;                     // rows followed
+    int edited;                    // distinct edited orbits
+    int orbit[4];                  // they, or -1
+    int hist[gg::kDeltaLevels];
+};
+
+// `rows` sources of a candidate's list, from `first` on.
+struct DeltaUnit {
+    int cand, first, rows;
+};
+
+struct DeltaArgs {
+    LiftAxes ax;
+    int N, M, d, g, K;
+    const int32_t *table;          // base table, diffs in [0, n)
+    const gg_lift_edit *ed;
+    const uint16_t *rows;          // base adjacency rows
+    int rw;
+    const uint16_t *diffs;         // part: base diffs, dp a row
+    int dp;
+    gg::FastDiv div_m;             // division by M
+    const uint8_t *dist;
+    int pitch;
+    const uint32_t *ball;
+    int words;                     // words of a bit per orbit
+    DeltaCand *cand;
+    uint32_t *near;                // [K][words]: P
+    uint16_t *lists;               // [K][M]
+    uint3 *changes;                // [K][4 g]
+    uint16_t *patch;               // part: [K][4][dp] diff rows of the edited orbits; else [K][4][g][rw]
+    DeltaUnit *units;
+    int *ctr;                      // [0] units made, [1] units taken
+    int unit_rows;
+    uint32_t *spill;               // [blocks of lift_delta][3][kDeltaSpill]
+};
+
+// One block a candidate: whether its edit keeps the lift symmetric, P from the edited
+// orbits' balls, the work units, the changed pull entries and the edited rows.
+__global__ void __launch_bounds__(128) lift_select(const DeltaArgs a) {
+    __shared__ int s_mode, s_ne, s_orb[4], s_cnt, s_u0;
+    const int k = blockIdx.x, tid = threadIdx.x;
+    const gg_lift_edit &e = a.ed[k];
+    const int ne_max = e.count;
+    if (tid == 0) {
+        int mode = kByChange, ne = 0;
+        const int32_t *old[4], *add[4];
+        for (int j = 0; j < ne_max; ++j) {
+            old[j] = a.table + ((size_t)e.row[j] * a.d + e.slot[j]) * a.ax.axes;
+            add[j] = e.diff[j];
+            for (int i = 0; i < j; ++i)
+                if (e.row[i] == e.row[j] && e.slot[i] == e.slot[j]) mode = kSearch;   // a slot edited twice
+            bool seen = false;
+            for (int i = 0; i < ne; ++i) seen |= s_orb[i] == e.row[j];
+            if (!seen) s_orb[ne++] = e.row[j];
+        }
+        // the removed entries, and the added ones, hold each entry as often as its reverse
+        for (int t = 0; t < 2; ++t)
+            for (int j = 0; j < ne_max; ++j) {
+                const int32_t *const *df = t ? add : old;
+                const int q = a.ax.orbit_at(e.row[j], df[j]);
+                int here = 0, back = 0;
+                for (int i = 0; i < ne_max; ++i) {
+                    here += e.row[i] == e.row[j] && a.ax.same(df[i], df[j]);
+                    back += e.row[i] == q && a.ax.reverse(df[i], df[j]);
+                }
+                if (here != back) mode = kSearch;
+            }
+        s_mode = mode;
+        s_ne = ne;
+        s_cnt = 0;
+        DeltaCand &c = a.cand[k];
+        c.mode = mode;
+        c.edited = ne;
+        for (int i = 0; i < 4; ++i) c.orbit[i] = i < ne ? s_orb[i] : -1;
+    }
+    if (tid < gg::kDeltaLevels) a.cand[k].hist[tid] = 0;
+    __syncthreads();
+    if (s_mode != kByChange) {
+        if (tid == 0) a.cand[k].count = 0;
+        return;
+    }
+    const int ne = s_ne;
+    uint16_t *lst = a.lists + (size_t)k * a.M;
+    for (int w = tid; w < a.words; w += blockDim.x) {
+        uint32_t p = 0u;
+        for (int i = 0; i < ne; ++i) p |= __ldg(a.ball + (size_t)s_orb[i] * a.words + w);
+        a.near[(size_t)k * a.words + w] = p;
+        if (p) {
+            int at = atomicAdd(&s_cnt, __popc(p));
+            for (; p; p &= p - 1u) lst[at++] = (uint16_t)(w * 32 + __ffs((int)p) - 1);
+        }
+    }
+    for (int q = tid; q < ne_max * a.g; q += blockDim.x) {
+        const int j = q / a.g, c = q % a.g;
+        const int r = a.ax.vertex(e.row[j], c);
+        a.changes[(size_t)k * 4 * a.g + q] = make_uint3((unsigned)r, __ldg(a.rows + (size_t)r * a.rw + e.slot[j]),
+                                                        (unsigned)a.ax.move(r, e.diff[j]));
+    }
+    if (a.ax.axes == 1) {
+        for (int q = tid; q < ne * a.dp; q += blockDim.x) {
+            const int i = q / a.dp, x = q % a.dp;
+            int v = __ldg(a.diffs + (size_t)s_orb[i] * a.dp + x);
+            for (int j = 0; j < ne_max; ++j)
+                if (e.row[j] == s_orb[i] && e.slot[j] == x) v = e.diff[j][0];
+            a.patch[(size_t)k * 4 * a.dp + q] = (uint16_t)v;
+        }
+    } else {
+        for (int q = tid; q < ne * a.g; q += blockDim.x) {
+            const int i = q / a.g, c = q % a.g;
+            const int v = a.ax.vertex(s_orb[i], c);
+            uint16_t *out = a.patch + ((size_t)(k * 4 + i) * a.g + c) * a.rw;
+            for (int x = 0; x < a.rw; ++x) out[x] = __ldg(a.rows + (size_t)v * a.rw + x);
+            for (int j = 0; j < ne_max; ++j)
+                if (e.row[j] == s_orb[i]) out[e.slot[j]] = (uint16_t)a.ax.move(v, e.diff[j]);
+        }
+    }
+    __syncthreads();
+    const int cnt = s_cnt, nu = (cnt + a.unit_rows - 1) / a.unit_rows;
+    if (tid == 0) {
+        a.cand[k].count = cnt;
+        s_u0 = nu ? atomicAdd(a.ctr, nu) : 0;
+    }
+    __syncthreads();
+    for (int u = tid; u < nu; u += blockDim.x)
+        a.units[s_u0 + u] = DeltaUnit{k, u * a.unit_rows, min(a.unit_rows, cnt - u * a.unit_rows)};
+}
+
+// A candidate's graph: base rows of RW words, the edited orbits' rows from its patch.
+template <int RW>
+struct LiftGraph {
+    const uint16_t *rows, *patch;
+    unsigned o0, o1, o2, o3, g, rw;
+    __device__ __forceinline__ unsigned width() const { return RW > 0 ? (unsigned)RW : rw; }
+    __device__ __forceinline__ unsigned slots() const { return width() - 2u; }
+    __device__ __forceinline__ const uint16_t *row(const unsigned v, const unsigned place) const {
+        const unsigned o = place & 0xffffu, c = place >> 16;
+        if (o == o0 || o == o1 || o == o2 || o == o3)
+            return patch + ((o == o0 ? 0u : o == o1 ? 1u : o == o2 ? 2u : 3u) * g + c) * width();
+        return rows + (size_t)v * width();
+    }
+    __device__ __forceinline__ unsigned place(const unsigned v) const {   // orbit | copy << 16
+        return __ldg(reinterpret_cast<const unsigned *>(rows + (size_t)v * width()) + width() / 2u - 1u);
+    }
+    __device__ __forceinline__ unsigned orbit(const unsigned v) const { return place(v) & 0xffffu; }
+    // (the base row and the vertex's place are loaded together, the patch only if need be)
+    __device__ __forceinline__ unsigned at(const unsigned v, const unsigned i) const {
+        const uint16_t *own = rows + (size_t)v * width();
+        unsigned u = __ldg(own + i);
+        const uint16_t *r = row(v, place(v));
+        if (r != own) u = __ldg(r + i);
+        return u;
+    }
+    template <class F>
+    __device__ __forceinline__ void each(const unsigned v, F f) const {
+        const uint16_t *own = rows + (size_t)v * width();
+        const unsigned nq = width() / 8u;
+        constexpr unsigned Q = RW > 0 ? RW / 8u : 1u;
+        uint4 q[Q];
+#pragma unroll
+        for (unsigned k = 0; k < Q; ++k) q[k] = __ldg(reinterpret_cast<const uint4 *>(own) + k);
+        const uint16_t *r = row(v, RW > 0 ? q[Q - 1u].w : place(v));
+        if (RW == 0 || r != own) {
+#pragma unroll
+            for (unsigned k = 0; k < Q; ++k) q[k] = __ldg(reinterpret_cast<const uint4 *>(r) + k);
+        }
+        for (unsigned k0 = 0;; k0 += Q) {
+#pragma unroll
+            for (unsigned k = 0; k < Q; ++k) {
+                f(q[k].x & 0xffffu); f(q[k].x >> 16); f(q[k].y & 0xffffu); f(q[k].y >> 16);
+                f(q[k].z & 0xffffu); f(q[k].z >> 16);
+                if (k0 + k + 1u < nq) { f(q[k].w & 0xffffu); f(q[k].w >> 16); }
+            }
+            if (RW > 0 || k0 + 1u >= nq) break;
+            q[0] = __ldg(reinterpret_cast<const uint4 *>(r) + k0 + 1u);
+        }
+    }
+};
+
+// The same for a part, from its diffs: vertex v of orbit v mod M has the neighbours
+// v + diff mod N.  The table (24 KB at m = 1024, d = 12) stays in the L1, where the
+// expanded rows (1 MB at N = 32768) do not: a row costs 40 cycles instead of 300, and the
+// steps of lift_delta are chains of a few such loads.  DP diffs a row, padded with 0 (0: a
+// run-time multiple of 4).
+template <int DP>
+struct PartGraph {
+    const uint16_t *diffs, *patch;
+    unsigned o0, o1, o2, o3, N, dp;
+    gg::FastDiv div_m;
+    __device__ __forceinline__ unsigned slots() const { return DP > 0 ? (unsigned)DP : dp; }
+    __device__ __forceinline__ unsigned orbit(const unsigned v) const { return v - div_m.div(v) * div_m.d; }
+    __device__ __forceinline__ const uint16_t *row(const unsigned o) const {
+        if (o == o0 || o == o1 || o == o2 || o == o3)
+            return patch + (o == o0 ? 0u : o == o1 ? 1u : o == o2 ? 2u : 3u) * slots();
+        return diffs + o * slots();
+    }
+    __device__ __forceinline__ unsigned step(const unsigned v, const unsigned df) const {
+        const unsigned u = v + df;
+        return u - (u >= N ? N : 0u);
+    }
+    __device__ __forceinline__ unsigned at(const unsigned v, const unsigned i) const {
+        return step(v, __ldg(row(orbit(v)) + i));
+    }
+    template <class F>
+    __device__ __forceinline__ void each(const unsigned v, F f) const {
+        const uint2 *p = reinterpret_cast<const uint2 *>(row(orbit(v)));
+#pragma unroll
+        for (unsigned k = 0; k < (DP > 0 ? DP / 4u : dp / 4u); ++k) {
+            const uint2 q = __ldg(p + k);
+            f(step(v, q.x & 0xffffu)); f(step(v, q.x >> 16)); f(step(v, q.y & 0xffffu)); f(step(v, q.y >> 16));
+        }
+    }
+};
+
+constexpr int kDeltaBlock = 128;
+
+// Follows every listed row of every candidate, a work unit (as many rows as the block's
+// shared memory holds) a block at a time: the lookups are random bytes of those rows and
+// never leave the SM.  Bound by the latency of the steps (waves and sweeps of a handful of
+// entries a row, a block barrier each); blocks a SM hide some of it.
+// make_graph(a, cand): the candidate's graph.
+template <class Make>
+__device__ __forceinline__ void lift_delta_run(const DeltaArgs &a, Make make_graph) {
+    extern __shared__ uint4 sm_rows[];
+    __shared__ gg::DeltaShared s;
+    __shared__ int s_unit;
+    const int n_units = a.ctr[0];
+    const gg::DeltaBlock b{&s, a.spill + (size_t)blockIdx.x * 3 * gg::kDeltaSpill,
+                           (unsigned)__cvta_generic_to_shared(sm_rows), (unsigned)a.pitch};
+    const unsigned q = (unsigned)a.pitch / 16u;
+    int taken = 0;
+    if (threadIdx.x == 0u) taken = atomicAdd(a.ctr + 1, 1);
+    for (;;) {
+        if (threadIdx.x == 0u) s_unit = taken;
+        __syncthreads();
+        const int u = s_unit;
+        if (u >= n_units) break;
+        if (threadIdx.x == 0u) taken = atomicAdd(a.ctr + 1, 1);   // the next one, on the way meanwhile
+        const DeltaUnit un = a.units[u];
+        const DeltaCand &c = a.cand[un.cand];
+        const uint16_t *lst = a.lists + (size_t)un.cand * a.M + un.first;
+        for (int slot = 0; slot < un.rows; ++slot) {
+            const uint8_t *src = a.dist + (size_t)__ldg(lst + slot) * a.pitch;
+            const unsigned dst = b.row((unsigned)slot);
+            for (unsigned k = threadIdx.x; k < q; k += kDeltaBlock) gg::delta_cp16(dst + k * 16u, src + k * 16u);
+        }
+        const auto G = make_graph(c, un.cand);
+        const uint3 *ch = a.changes + (size_t)un.cand * 4 * a.g;
+        gg::delta_cp_wait();
+        gg::delta_rows(G, b, (unsigned)un.rows, (unsigned)(a.ed[un.cand].count * a.g),
+                       [&](const unsigned j) { return ch[j]; });
+        if (s.overflow) {
+            if (threadIdx.x == 0u) a.cand[un.cand].mode = kSearch;
+        } else {
+            int h = 0;
+            const uint32_t *near = a.near + (size_t)un.cand * a.words;
+            gg::delta_count(b, [&](const unsigned v) {
+                const unsigned o = G.orbit(v);
+                return 2u - ((__ldg(near + (o >> 5)) >> (o & 31u)) & 1u);
+            }, h);
+            if (h) atomicAdd(&a.cand[un.cand].hist[threadIdx.x & 31u], h);
+        }
+        __syncthreads();   // the next unit overwrites the rows and the list
+    }
+}
+
+template <int RW>
+__global__ void __launch_bounds__(kDeltaBlock) lift_delta(const DeltaArgs a) {
+    lift_delta_run(a, [&](const DeltaCand &c, const int k) {
+        return LiftGraph<RW>{a.rows, a.patch + (size_t)k * 4 * a.g * a.rw, (unsigned)c.orbit[0], (unsigned)c.orbit[1],
+                             (unsigned)c.orbit[2], (unsigned)c.orbit[3], (unsigned)a.g, (unsigned)a.rw};
+    });
+}
+
+template <int DP>
+__global__ void __launch_bounds__(kDeltaBlock) part_delta(const DeltaArgs a) {
+    lift_delta_run(a, [&](const DeltaCand &c, const int k) {
+        return PartGraph<DP>{a.diffs, a.patch + (size_t)k * 4 * a.dp, (unsigned)c.orbit[0], (unsigned)c.orbit[1],
+                             (unsigned)c.orbit[2], (unsigned)c.orbit[3], (unsigned)a.N, (unsigned)a.dp, a.div_m};
+    });
+}
+
+void *lift_delta_for(int axes, int dp, int rw) {
+    if (axes == 1) switch (dp) {
+        case 4: return (void *)part_delta<4>;
+        case 8: return (void *)part_delta<8>;
+        case 12: return (void *)part_delta<12>;
+        case 16: return (void *)part_delta<16>;
+        default: return (void *)part_delta<0>;
+    }
+    switch (rw) {
+        case 8: return (void *)lift_delta<8>;
+        case 16: return (void *)lift_delta<16>;
+        default: return (void *)lift_delta<0>;
+    }
 }
 
 template <bool EXPL>
@@ -419,6 +896,24 @@ struct gg_lift {
     long long wait_ns = 10ll * 1000 * 1000 * 1000;
     bool base_set = false;
     float last_ms = 0.f;
+    // moves by change
+    bool delta_on = false;                           // the lift is within the limits and the buffers are there
+    int base_state = 0;                              // distances of the base: 0 not computed, 1 usable, -1 not usable
+    int rw = 0, pitch = 0, words = 0, unit_rows = 1, delta_grid = 0;
+    uint4 *d_planes = nullptr;                       // [4][N][cpc]
+    uint8_t *d_dist = nullptr;                       // [M][pitch]
+    uint16_t *d_rows = nullptr;                      // [N][rw]
+    uint16_t *d_diffs = nullptr;                     // part: [M][dp]
+    int dp = 0;
+    uint32_t *d_ball = nullptr, *d_spill = nullptr;
+    int *d_ctr = nullptr;                            // [3]: units made, taken; asymmetric base
+    int delta_cap = 0;                               // candidates the next buffers hold
+    DeltaCand *d_cand = nullptr, *h_cand = nullptr;
+    uint32_t *d_near = nullptr;
+    uint16_t *d_lists = nullptr, *d_patch = nullptr;
+    uint3 *d_changes = nullptr;
+    DeltaUnit *d_units = nullptr;
+    unsigned long long base_hist[gg::kDeltaLevels] = {};
 };
 
 namespace {
@@ -433,6 +928,9 @@ void lift_free(gg_lift *h) {
     cudaFree(h->d_counts); cudaFreeHost(h->h_counts);
     cudaFree(h->d_level_ns); cudaFreeHost(h->h_level_ns);
     cudaFree(h->d_ctl); cudaFreeHost(h->h_ctl);
+    cudaFree(h->d_planes); cudaFree(h->d_dist); cudaFree(h->d_rows); cudaFree(h->d_diffs); cudaFree(h->d_ball); cudaFree(h->d_spill);
+    cudaFree(h->d_ctr); cudaFree(h->d_cand); cudaFreeHost(h->h_cand); cudaFree(h->d_near); cudaFree(h->d_lists);
+    cudaFree(h->d_patch); cudaFree(h->d_changes); cudaFree(h->d_units);
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
     if (h->stream) cudaStreamDestroy(h->stream);
@@ -486,6 +984,70 @@ extern "C" {
 }  // extern "C"
 
 namespace {
+
+// Buffers of the moves by change, where the lift is within their limits: 16-bit vertex
+// and orbit ids, a distance row within a block's shared memory (at 64 KB three blocks a
+// SM), and 1 GiB of distance rows.  Without them (or the memory) candidates are searched.
+constexpr size_t kDeltaRowBytes = 24 * 1024;   // rows of a block, when one is smaller
+void delta_open(gg_lift *h) {
+    const char *off = std::getenv("GG_LIFT_SEARCH");   // 1: search every candidate
+    const size_t pitch = ((size_t)h->N + 15) / 16 * 16;
+    if ((off && std::atoi(off) != 0) || h->N > 65536 || h->M > 65535 || h->N / h->M > 65535 ||
+        pitch * h->M > (1ull << 30))
+        return;
+    h->pitch = (int)pitch;
+    h->rw = (h->d + 2 + 7) / 8 * 8;
+    h->dp = (h->d + 3) / 4 * 4;
+    h->words = (h->M + 31) / 32;
+    const size_t smem = std::max(kDeltaRowBytes, pitch);
+    h->unit_rows = (int)std::min<size_t>(gg::kDeltaRows, smem / pitch);
+    int per_sm = 0;
+    void *k = lift_delta_for(h->axes, h->dp, h->rw);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kDeltaBlock, smem);
+    h->delta_grid = per_sm * h->sms;
+    if (e == cudaSuccess && per_sm < 1) e = cudaErrorInvalidConfiguration;
+    if (e == cudaSuccess) e = cudaMalloc(&h->d_planes, 4 * (size_t)h->N * h->cpc * sizeof(uint4));
+    if (e == cudaSuccess) e = cudaMalloc(&h->d_dist, pitch * h->M);
+    if (e == cudaSuccess) e = cudaMalloc(&h->d_rows, (size_t)h->N * h->rw * sizeof(uint16_t));
+    if (e == cudaSuccess) e = cudaMalloc(&h->d_diffs, (size_t)h->M * h->dp * sizeof(uint16_t));
+    if (e == cudaSuccess) e = cudaMalloc(&h->d_ball, (size_t)h->M * h->words * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&h->d_spill, (size_t)h->delta_grid * 3 * gg::kDeltaSpill * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&h->d_ctr, 3 * sizeof(int));
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        return;
+    }
+    h->delta_on = true;
+}
+
+// Per-candidate buffers of the moves by change; false: not enough memory.
+bool delta_ensure(gg_lift *h, int n) {
+    if (n <= h->delta_cap) return true;
+    const size_t cap = (size_t)std::max(n, 2 * h->delta_cap), g = (size_t)h->N / h->M;
+    cudaFree(h->d_cand); cudaFreeHost(h->h_cand); cudaFree(h->d_near); cudaFree(h->d_lists);
+    cudaFree(h->d_patch); cudaFree(h->d_changes); cudaFree(h->d_units);
+    h->d_cand = h->h_cand = nullptr;
+    h->d_near = nullptr;
+    h->d_lists = h->d_patch = nullptr;
+    h->d_changes = nullptr;
+    h->d_units = nullptr;
+    h->delta_cap = 0;
+    const size_t units = (size_t)(h->M + h->unit_rows - 1) / h->unit_rows;
+    cudaError_t e = cudaMalloc(&h->d_cand, cap * sizeof(DeltaCand));
+    if (e == cudaSuccess) e = cudaMallocHost(&h->h_cand, cap * sizeof(DeltaCand));
+    if (e == cudaSuccess) e = cudaMalloc(&h->d_near, cap * h->words * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&h->d_lists, cap * h->M * sizeof(uint16_t));
+    if (e == cudaSuccess) e = cudaMalloc(&h->d_patch, cap * 4 * (h->axes == 1 ? h->dp : g * h->rw) * sizeof(uint16_t));
+    if (e == cudaSuccess) e = cudaMalloc(&h->d_changes, cap * 4 * g * sizeof(uint3));
+    if (e == cudaSuccess) e = cudaMalloc(&h->d_units, cap * units * sizeof(DeltaUnit));
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    h->delta_cap = (int)cap;
+    return true;
+}
 
 // A handle for a lift of `axes` axes: lifted sizes n, orbit sizes m.
 gg_status lift_open(int axes, const int n_in[3], const int m_in[3], int degree, int device, gg_lift **out) {
@@ -558,7 +1120,188 @@ gg_status lift_open(int axes, const int n_in[3], const int m_in[3], int degree, 
     // bitsets for the automatic group (a larger group set later reallocates)
     const gg_status s = alloc_group(h, h->g_auto);
     if (s != GG_OK) return fail(s);
+    delta_open(h);
     *out = h;
+    return GG_OK;
+}
+
+// Searches the candidates whose edits are in h->h_ed[0 .. n_cand); with `planes`, n_cand is
+// 1 and the distance planes are written too.
+gg_status lift_search(gg_lift *h, int n_cand, int max_levels, gg_cand_result *out, uint4 *planes = nullptr) {
+    gg_status s;
+    // Count rows for the first kFirstLevels levels; a population where some candidate
+    // still finds pairs there (a lift of very large diameter) runs again with rows
+    // for the full cap, so the buffers stay small for the usual diameters.
+    const int ml_full = max_levels > 0 ? std::min(max_levels, h->N) : h->N;
+    for (int ml = std::min(ml_full, kFirstLevels);; ml = ml_full) {
+        s = ensure_counts(h, (size_t)(ml + 1) * n_cand);
+        if (s != GG_OK) return s;
+        if (ml + 1 > h->level_ns_n) {
+            cudaFree(h->d_level_ns); cudaFreeHost(h->h_level_ns);
+            h->d_level_ns = nullptr; h->h_level_ns = nullptr; h->level_ns_n = 0;
+            GL_CK(cudaMalloc(&h->d_level_ns, (size_t)(ml + 1) * sizeof(unsigned long long)));
+            GL_CK(cudaMallocHost(&h->h_level_ns, (size_t)(ml + 1) * sizeof(unsigned long long)));
+            h->level_ns_n = ml + 1;
+        }
+        const int G = std::min(h->group ? h->group : h->g_auto, n_cand);
+        const cudaStream_t st = h->stream;
+        GL_CK(cudaMemcpyAsync(h->d_ed, h->h_ed, (size_t)n_cand * sizeof(gg_lift_edit), cudaMemcpyHostToDevice, st));
+        GL_CK(cudaMemsetAsync(h->d_ctl, 0, sizeof(gg::Ctl), st));
+        GL_CK(cudaMemsetAsync(h->d_counts, 0, (size_t)std::min(ml + 1, 2) * n_cand * sizeof(unsigned long long), st));
+        GL_CK(cudaEventRecord(h->ev0, st));
+        const long long tab_n = (long long)n_cand * h->M * h->d;
+        lift_tables<<<(int)std::min<long long>((tab_n + 255) / 256, (long long)h->sms * 16), 256, 0, st>>>(
+            h->d_base, h->d_ed, n_cand, h->M, h->d, h->axes, h->d_tab);
+        GL_CK(cudaGetLastError());
+        if (h->axes > 1) {
+            const long long rows_n = (long long)n_cand * h->N;
+            lift_expand<<<(int)std::min<long long>((rows_n + 255) / 256, (long long)h->sms * 16), 256, 0, st>>>(
+                h->d_tab, n_cand, h->M, h->d, h->axes, h->n[0], h->n[1], h->n[2], h->m[0], h->m[1], h->m[2], h->d_adj);
+            GL_CK(cudaGetLastError());
+        }
+        LiftArgs a{};
+        a.tab = h->d_tab;
+        a.adj = h->d_adj;
+        a.inv = h->d_inv;
+        a.N = h->N; a.M = h->M; a.d = h->d; a.K = n_cand; a.G = G; a.cpc = h->cpc; a.W = G * h->cpc;
+        a.V = h->V; a.F0 = h->F0; a.F1 = h->F1;
+        a.counts = h->d_counts;
+        a.max_levels = ml;
+        const unsigned threads = (unsigned)h->grid * kLiftBlock;
+        if ((unsigned)a.W > threads) return lfail(GG_BAD_ARG, "more chunk columns than threads: lower the group");
+        a.cols_threads = threads / (unsigned)a.W * (unsigned)a.W;
+        a.vstep = a.cols_threads / (unsigned)a.W;
+        a.half_ppm = h->half_ppm;
+        a.level_ns = h->d_level_ns;
+        a.ctl = h->d_ctl;
+        a.wait_ns = h->wait_ns;
+        a.planes = planes;
+        a.expected = (unsigned)h->grid;
+        GL_CK(cudaMemsetAsync(h->d_level_ns, 0, (size_t)(ml + 1) * sizeof(unsigned long long), st));
+        void *args[] = {&a};
+        GL_CK(cudaLaunchCooperativeKernel(lift_kernel_for(h->d, h->axes > 1), dim3(h->grid), dim3(kLiftBlock), args, 0,
+                                          st));
+        GL_CK(cudaEventRecord(h->ev1, st));
+        GL_CK(cudaMemcpyAsync(h->h_ctl, h->d_ctl, sizeof(gg::Ctl), cudaMemcpyDeviceToHost, st));
+        GL_CK(cudaStreamSynchronize(st));
+        if (h->h_ctl->err) return lfail(GG_TIMEOUT, "grid barrier wait exceeded the limit");
+        const int lr = std::min(h->h_ctl->levels_run, ml);
+        GL_CK(cudaMemcpyAsync(h->h_counts, h->d_counts, (size_t)(lr + 1) * n_cand * sizeof(unsigned long long),
+                              cudaMemcpyDeviceToHost, st));
+        GL_CK(cudaMemcpyAsync(h->h_level_ns, h->d_level_ns, (size_t)(lr + 1) * sizeof(unsigned long long),
+                              cudaMemcpyDeviceToHost, st));
+        GL_CK(cudaStreamSynchronize(st));
+        GL_CK(cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1));
+        const unsigned long long all = (unsigned long long)h->M * (unsigned long long)h->N;
+        for (int k = 0; k < n_cand; ++k) {
+            unsigned long long tot = 0, reach = (unsigned long long)h->M;
+            int lev = 0;
+            for (int L = 1; L <= lr; ++L) {
+                const unsigned long long c = h->h_counts[(size_t)L * n_cand + k];
+                if (!c) continue;
+                tot += (unsigned long long)L * c;
+                reach += c;
+                lev = L;
+            }
+            const bool capped = lev == ml && reach < all;
+            out[k] = gg_cand_result{tot, reach, lev, (!capped && reach == all) ? 1 : 0};
+        }
+        bool again = false;
+        for (int k = 0; k < n_cand && ml < ml_full; ++k)
+            again |= out[k].levels == ml && out[k].reached < all;
+        if (!again) break;
+    }
+    return GG_OK;
+}
+
+
+// The base's distances, rows and balls.  base_state = 1 when candidates can be scored by
+// change: a symmetric, connected base of diameter at most 15.
+gg_status delta_base(gg_lift *h) {
+    h->base_state = -1;
+    const cudaStream_t st = h->stream;
+    LiftAxes ax{h->axes, {h->n[0], h->n[1], h->n[2]}, {h->m[0], h->m[1], h->m[2]}};
+    const int blocks = h->sms * 8;
+    GL_CK(cudaMemsetAsync(h->d_planes, 0, 4 * (size_t)h->N * h->cpc * sizeof(uint4), st));
+    GL_CK(cudaMemsetAsync(h->d_ctr, 0, 3 * sizeof(int), st));
+    delta_symmetry<<<std::min(blocks, (h->M * h->d + 255) / 256), 256, 0, st>>>(h->d_base, ax, h->M, h->d, h->d_ctr + 2);
+    delta_rows_kernel<<<std::min(blocks, (h->N + 127) / 128), 128, 0, st>>>(h->d_base, ax, h->N, h->d, h->rw, h->d_rows);
+    if (h->axes == 1)
+        delta_diffs_kernel<<<std::min(blocks, (h->M * h->dp + 255) / 256), 256, 0, st>>>(h->d_base, h->M, h->d, h->dp, h->d_diffs);
+    GL_CK(cudaGetLastError());
+    h->h_ed[0] = gg_lift_edit{};   // the base itself
+    gg_cand_result r{};
+    gg_status s = lift_search(h, 1, 16, &r, h->d_planes);
+    if (s != GG_OK) return s;
+    int asym = 0;
+    GL_CK(cudaMemcpyAsync(&asym, h->d_ctr + 2, sizeof(int), cudaMemcpyDeviceToHost, st));
+    GL_CK(cudaStreamSynchronize(st));
+    if (asym || !r.connected || r.levels > 15 || r.levels < 1) return GG_OK;
+    for (int L = 0; L < gg::kDeltaLevels; ++L)
+        h->base_hist[L] = L == 0 ? (unsigned long long)h->M : L <= r.levels ? h->h_counts[L] : 0ull;
+    delta_bytes<<<dim3((unsigned)((h->N + 127) / 128), (unsigned)h->cpc), 128, 0, st>>>(h->d_planes, h->N, h->M, h->cpc,
+                                                                                h->d_dist, h->pitch);
+    delta_balls<<<h->M, 256, (size_t)h->words * 4, st>>>(h->d_dist, h->pitch, h->N, h->d_rows, h->rw, h->words,
+                                                         (unsigned)(r.levels - 1) / 2u, h->d_ball);
+    GL_CK(cudaGetLastError());
+    h->base_state = 1;
+    return GG_OK;
+}
+
+// Scores the candidates in h->h_ed[0 .. n_cand) by change; `left` gets the ones that have
+// to be searched.
+gg_status delta_eval(gg_lift *h, int n_cand, int max_levels, gg_cand_result *out, std::vector<int> &left) {
+    const cudaStream_t st = h->stream;
+    DeltaArgs a{};
+    a.ax = LiftAxes{h->axes, {h->n[0], h->n[1], h->n[2]}, {h->m[0], h->m[1], h->m[2]}};
+    a.N = h->N; a.M = h->M; a.d = h->d; a.g = h->N / h->M; a.K = n_cand;
+    a.table = h->d_base;
+    a.ed = h->d_ed;
+    a.rows = h->d_rows; a.rw = h->rw;
+    a.diffs = h->d_diffs; a.dp = h->dp;
+    a.div_m = gg::FastDiv((uint32_t)h->M);
+    a.dist = h->d_dist; a.pitch = h->pitch;
+    a.ball = h->d_ball; a.words = h->words;
+    a.cand = h->d_cand;
+    a.near = h->d_near;
+    a.lists = h->d_lists;
+    a.changes = h->d_changes;
+    a.patch = h->d_patch;
+    a.units = h->d_units;
+    a.ctr = h->d_ctr;
+    a.unit_rows = h->unit_rows;
+    a.spill = h->d_spill;
+    GL_CK(cudaMemcpyAsync(h->d_ed, h->h_ed, (size_t)n_cand * sizeof(gg_lift_edit), cudaMemcpyHostToDevice, st));
+    GL_CK(cudaMemsetAsync(h->d_ctr, 0, 2 * sizeof(int), st));
+    GL_CK(cudaEventRecord(h->ev0, st));
+    lift_select<<<n_cand, 128, 0, st>>>(a);
+    GL_CK(cudaGetLastError());
+    void *args[] = {&a};
+    GL_CK(cudaLaunchKernel(lift_delta_for(h->axes, h->dp, h->rw), dim3(h->delta_grid), dim3(kDeltaBlock), args,
+                           std::max(kDeltaRowBytes, (size_t)h->pitch), st));
+    GL_CK(cudaEventRecord(h->ev1, st));
+    GL_CK(cudaMemcpyAsync(h->h_cand, h->d_cand, (size_t)n_cand * sizeof(DeltaCand), cudaMemcpyDeviceToHost, st));
+    GL_CK(cudaStreamSynchronize(st));
+    GL_CK(cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1));
+    if (h->h_ctl) h->h_ctl->levels_run = 0;   // no level times of this evaluation
+    const unsigned long long all = (unsigned long long)h->M * (unsigned long long)h->N;
+    const int cap = max_levels > 0 ? max_levels : h->N;
+    for (int k = 0; k < n_cand; ++k) {
+        const DeltaCand &c = h->h_cand[k];
+        if (c.mode != kByChange) {
+            left.push_back(k);
+            continue;
+        }
+        unsigned long long tot = 0, reach = 0;
+        int lev = 0;
+        for (int L = 0; L < (int)gg::kDeltaInf && L <= cap; ++L) {
+            const unsigned long long n = h->base_hist[L] + (unsigned long long)(long long)c.hist[L];
+            tot += (unsigned long long)L * n;
+            reach += n;
+            if (n) lev = L;
+        }
+        out[k] = gg_cand_result{tot, reach, lev, reach == all ? 1 : 0};
+    }
     return GG_OK;
 }
 
@@ -593,6 +1336,7 @@ gg_status gg_lift_set_base(gg_lift *h, const int32_t *table) {
     GL_CK(cudaMemcpyAsync(h->d_base, nd.data(), nd.size() * sizeof(int32_t), cudaMemcpyHostToDevice, h->stream));
     GL_CK(cudaStreamSynchronize(h->stream));
     h->base_set = true;
+    h->base_state = 0;
     return GG_OK;
 }
 
@@ -682,88 +1426,32 @@ gg_status gg_lift_eval(gg_lift *h, int n_cand, const gg_lift_edit *edits, int ma
             }
         }
     }
-    // Count rows for the first kFirstLevels levels; a population where some candidate
-    // still finds pairs there (a lift of very large diameter) runs again with rows
-    // for the full cap, so the buffers stay small for the usual diameters.
-    const int ml_full = max_levels > 0 ? std::min(max_levels, h->N) : h->N;
-    for (int ml = std::min(ml_full, kFirstLevels);; ml = ml_full) {
-        s = ensure_counts(h, (size_t)(ml + 1) * n_cand);
-        if (s != GG_OK) return s;
-        if (ml + 1 > h->level_ns_n) {
-            cudaFree(h->d_level_ns); cudaFreeHost(h->h_level_ns);
-            h->d_level_ns = nullptr; h->h_level_ns = nullptr; h->level_ns_n = 0;
-            GL_CK(cudaMalloc(&h->d_level_ns, (size_t)(ml + 1) * sizeof(unsigned long long)));
-            GL_CK(cudaMallocHost(&h->h_level_ns, (size_t)(ml + 1) * sizeof(unsigned long long)));
-            h->level_ns_n = ml + 1;
+    // By change, once the base's distances are there; a first population of a few
+    // candidates is not worth computing them (a search of the base, about one candidate's).
+    std::vector<int> left;
+    const bool delta = h->delta_on && h->group == 0 && h->base_state >= 0 && (h->base_state == 1 || n_cand >= 4);
+    if (delta && delta_ensure(h, n_cand)) {
+        if (h->base_state == 0) {
+            const gg_lift_edit first = h->h_ed[0];
+            s = delta_base(h);
+            if (s != GG_OK) return s;
+            h->h_ed[0] = first;
         }
-        const int G = std::min(h->group ? h->group : h->g_auto, n_cand);
-        const cudaStream_t st = h->stream;
-        GL_CK(cudaMemcpyAsync(h->d_ed, h->h_ed, (size_t)n_cand * sizeof(gg_lift_edit), cudaMemcpyHostToDevice, st));
-        GL_CK(cudaMemsetAsync(h->d_ctl, 0, sizeof(gg::Ctl), st));
-        GL_CK(cudaMemsetAsync(h->d_counts, 0, (size_t)std::min(ml + 1, 2) * n_cand * sizeof(unsigned long long), st));
-        GL_CK(cudaEventRecord(h->ev0, st));
-        const long long tab_n = (long long)n_cand * h->M * h->d;
-        lift_tables<<<(int)std::min<long long>((tab_n + 255) / 256, (long long)h->sms * 16), 256, 0, st>>>(
-            h->d_base, h->d_ed, n_cand, h->M, h->d, h->axes, h->d_tab);
-        GL_CK(cudaGetLastError());
-        if (h->axes > 1) {
-            const long long rows_n = (long long)n_cand * h->N;
-            lift_expand<<<(int)std::min<long long>((rows_n + 255) / 256, (long long)h->sms * 16), 256, 0, st>>>(
-                h->d_tab, n_cand, h->M, h->d, h->axes, h->n[0], h->n[1], h->n[2], h->m[0], h->m[1], h->m[2], h->d_adj);
-            GL_CK(cudaGetLastError());
+        if (h->base_state == 1) {
+            s = delta_eval(h, n_cand, max_levels, out, left);
+            if (s != GG_OK || left.empty()) return s;
+            // the rest is searched
+            for (size_t i = 0; i < left.size(); ++i) h->h_ed[i] = h->h_ed[left[i]];
+            std::vector<gg_cand_result> res(left.size());
+            const float ms = h->last_ms;
+            s = lift_search(h, (int)left.size(), max_levels, res.data());
+            if (s != GG_OK) return s;
+            h->last_ms += ms;
+            for (size_t i = 0; i < left.size(); ++i) out[left[i]] = res[i];
+            return GG_OK;
         }
-        LiftArgs a{};
-        a.tab = h->d_tab;
-        a.adj = h->d_adj;
-        a.inv = h->d_inv;
-        a.N = h->N; a.M = h->M; a.d = h->d; a.K = n_cand; a.G = G; a.cpc = h->cpc; a.W = G * h->cpc;
-        a.V = h->V; a.F0 = h->F0; a.F1 = h->F1;
-        a.counts = h->d_counts;
-        a.max_levels = ml;
-        const unsigned threads = (unsigned)h->grid * kLiftBlock;
-        if ((unsigned)a.W > threads) return lfail(GG_BAD_ARG, "more chunk columns than threads: lower the group");
-        a.cols_threads = threads / (unsigned)a.W * (unsigned)a.W;
-        a.vstep = a.cols_threads / (unsigned)a.W;
-        a.half_ppm = h->half_ppm;
-        a.level_ns = h->d_level_ns;
-        a.ctl = h->d_ctl;
-        a.wait_ns = h->wait_ns;
-        a.expected = (unsigned)h->grid;
-        GL_CK(cudaMemsetAsync(h->d_level_ns, 0, (size_t)(ml + 1) * sizeof(unsigned long long), st));
-        void *args[] = {&a};
-        GL_CK(cudaLaunchCooperativeKernel(lift_kernel_for(h->d, h->axes > 1), dim3(h->grid), dim3(kLiftBlock), args, 0,
-                                          st));
-        GL_CK(cudaEventRecord(h->ev1, st));
-        GL_CK(cudaMemcpyAsync(h->h_ctl, h->d_ctl, sizeof(gg::Ctl), cudaMemcpyDeviceToHost, st));
-        GL_CK(cudaStreamSynchronize(st));
-        if (h->h_ctl->err) return lfail(GG_TIMEOUT, "grid barrier wait exceeded the limit");
-        const int lr = std::min(h->h_ctl->levels_run, ml);
-        GL_CK(cudaMemcpyAsync(h->h_counts, h->d_counts, (size_t)(lr + 1) * n_cand * sizeof(unsigned long long),
-                              cudaMemcpyDeviceToHost, st));
-        GL_CK(cudaMemcpyAsync(h->h_level_ns, h->d_level_ns, (size_t)(lr + 1) * sizeof(unsigned long long),
-                              cudaMemcpyDeviceToHost, st));
-        GL_CK(cudaStreamSynchronize(st));
-        GL_CK(cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1));
-        const unsigned long long all = (unsigned long long)h->M * (unsigned long long)h->N;
-        for (int k = 0; k < n_cand; ++k) {
-            unsigned long long tot = 0, reach = (unsigned long long)h->M;
-            int lev = 0;
-            for (int L = 1; L <= lr; ++L) {
-                const unsigned long long c = h->h_counts[(size_t)L * n_cand + k];
-                if (!c) continue;
-                tot += (unsigned long long)L * c;
-                reach += c;
-                lev = L;
-            }
-            const bool capped = lev == ml && reach < all;
-            out[k] = gg_cand_result{tot, reach, lev, (!capped && reach == all) ? 1 : 0};
-        }
-        bool again = false;
-        for (int k = 0; k < n_cand && ml < ml_full; ++k)
-            again |= out[k].levels == ml && out[k].reached < all;
-        if (!again) break;
     }
-    return GG_OK;
+    return lift_search(h, n_cand, max_levels, out);
 }
 
 gg_status gg_lift_set_half_ppm(gg_lift *h, int half_ppm) {
