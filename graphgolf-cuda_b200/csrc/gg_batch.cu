@@ -245,7 +245,7 @@ static __device__ __forceinline__ void level_pass(const uint4 *cur, uint4 *nxt, 
 // batch_kernel and its three small launches, 2048 x (n=1024, d=6) + 512 x (n=3000, d=4)
 // candidates: 2243 us a call with every affected source searched (2020 us of it here), 720
 // (632) with T; 32 x (n=4096, d=8): 215 (162) and 90 us (45).
-constexpr int kWalkItems = 5;   // walk ends of all sources, at most this many times the rows
+constexpr int kWalkItems = 2;   // walk ends of all sources, at most this many times the rows
 
 __global__ void __launch_bounds__(kBatchBlock, 1) batch_kernel(const BatchArgs a) {
     extern __shared__ uint4 sm[];
@@ -365,19 +365,24 @@ __global__ void __launch_bounds__(kBatchBlock, 1) batch_kernel(const BatchArgs a
         if (!a.hist) {
             for (unsigned ends = (unsigned)d; !done; ends *= (unsigned)d, ++L) {
                 if ((unsigned long long)ends * (unsigned)ns > (unsigned long long)kWalkItems * (unsigned)n) break;
+                // a thread takes a walk of L - 1 steps and its d ends (the ids of one row)
                 unsigned cnt = 0u, wcnt = 0u;
-                for (unsigned k = (unsigned)tid; k < ends * (unsigned)ns; k += kBatchBlock) {
-                    const int j = (int)(k / ends);
-                    unsigned w = k - (unsigned)j * ends;
+                const unsigned pre = ends / (unsigned)d;
+                for (unsigned k = (unsigned)tid; k < pre * (unsigned)ns; k += kBatchBlock) {
+                    const int j = (int)(k / pre);
+                    unsigned w = k - (unsigned)j * pre;
                     int v = full ? un.first + j : (int)__ldcg(lst + j);
-                    for (int l = 0; l < L; ++l) {
+                    for (int l = 1; l < L; ++l) {
                         const unsigned q = w / (unsigned)d;
                         v = adj[v * d + (int)(w - q * (unsigned)d)];
                         w = q;
                     }
-                    if (set_bit(v, j)) {
-                        cnt += 1u;
-                        wcnt += 2u - ((tb[v >> 5] >> (v & 31)) & 1u);
+                    for (int i = 0; i < d; ++i) {
+                        const int e = adj[v * d + i];
+                        if (set_bit(e, j)) {
+                            cnt += 1u;
+                            wcnt += 2u - ((tb[e >> 5] >> (e & 31)) & 1u);
+                        }
                     }
                 }
                 tot += (unsigned long long)L * wcnt;

@@ -44,7 +44,7 @@ constexpr unsigned kDeltaTouched = 0x80u;        // row byte: the vertex is in t
 constexpr int kDeltaRows = 32;                   // most rows a block follows together
 constexpr int kDeltaList = 768;                  // list entries kept in shared memory; the rest spill
 constexpr int kDeltaQueue = 256;                 // queue entries kept in shared memory; the rest spill
-constexpr int kDeltaSpill = 4096;                // spilled entries of each
+constexpr int kDeltaSpill = 2048;                // spilled entries of each
 
 // A list or queue entry: vertex (22 bits), row slot (5 bits), old distance (5 bits).
 constexpr unsigned kDeltaMaxVertex = 1u << 22;

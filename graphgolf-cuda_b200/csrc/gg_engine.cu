@@ -11,9 +11,13 @@
 // and the connectivity test live on the device.
 #include "gg.h"
 #include "gg_kernels.cuh"
+#include "gg_direct.cuh"
 #include "gg_internal.h"
 
 #include <algorithm>
+#include <atomic>
+#include <chrono>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -175,6 +179,17 @@ struct gg_engine {
     cudaGraphExec_t graph_exec = nullptr;
     EvalKey graph_key{};
 
+    // small graphs (direct_kernel)
+    bool direct_allowed = false;         // no launch shape or level mode was asked for by the environment
+    bool direct = false;                 // ... nor by a call
+    int sms = 0, smem_optin = 0;
+    int32_t *d_src = nullptr;            // the source list, when not consecutive
+    unsigned char *d_dir = nullptr, *h_dir = nullptr;   // DirectCtl | counts[cap + 1] | masks[cap + 1]
+    int dir_cap = 0;
+    unsigned dir_seq = 0;                // launches of direct_kernel
+    uint16_t *d_pack = nullptr, *h_pack = nullptr;      // plain-graph table as 16-bit ids (on first use)
+    bool table_stale = false;            // the last call's table went to h_pack, d_table is older
+
     double last_ms = 0.0;
     int last_launches = 0;
     int last_batches = 0;                // batches of the last evaluation
@@ -234,7 +249,8 @@ void destroy_all(gg_engine *e) {
     cudaFree(e->d_h2);
     cudaFree(e->d_went);
     cudaFree(e->d_woff);
-    cudaFree(e->d_table); cudaFree(e->d_inv);
+    cudaFree(e->d_table); cudaFree(e->d_inv); cudaFree(e->d_src);
+    cudaFree(e->d_dir); cudaFreeHost(e->h_dir); cudaFree(e->d_pack); cudaFreeHost(e->h_pack);
     cudaFreeHost(e->h_table);
     if (e->ev0) cudaEventDestroy(e->ev0);
     if (e->ev1) cudaEventDestroy(e->ev1);
@@ -520,6 +536,10 @@ gg_status ensure_counters(gg_engine *e, int cap, int nb) {
     return GG_OK;
 }
 
+void *direct_for(int W) {
+    return W == 1 ? (void *)gg::direct_kernel<1> : W == 2 ? (void *)gg::direct_kernel<2> : (void *)gg::direct_kernel<4>;
+}
+
 gg_status create_common(gg_engine *e) {
     if (fault("alloc")) return fail(GG_OUT_OF_MEMORY, "injected allocation failure");
     int ndev = 0;
@@ -554,6 +574,8 @@ gg_status create_common(gg_engine *e) {
                 return fail(GG_BAD_ARG, "sources must be distinct vertices");
             inv[(size_t)v] = (int32_t)i;
         }
+        GG_CK(cudaMalloc(&e->d_src, e->reps.size() * sizeof(int32_t)));
+        GG_CK(cudaMemcpy(e->d_src, e->reps.data(), e->reps.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
         GG_CK(cudaMalloc(&e->d_inv, inv.size() * sizeof(int32_t)));
         GG_CK(cudaMemcpy(e->d_inv, inv.data(), inv.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
     }
@@ -568,6 +590,18 @@ gg_status create_common(gg_engine *e) {
     e->push_ppm = env_int("GG_PUSH_PPM", e->push_ppm);
     e->push_min_items = env_int("GG_PUSH_MIN_ITEMS", e->push_min_items);
     e->use_graph = env_int("GG_NO_GRAPH", 0) == 0;
+    // direct_kernel unless a launch shape or level mode is asked for
+    e->direct = true;
+    for (const char *name : {"GG_BATCH_SOURCES", "GG_BLOCKS_PER_SM", "GG_WALK_LEVELS", "GG_DENSE_W_PPM", "GG_DENSE_R_PPM",
+                             "GG_FULL_SKIP_PPM", "GG_SPLIT_PPM", "GG_VPULL", "GG_OWN_SKIP", "GG_WALK_THIRD",
+                             "GG_WALK_ALL_MB", "GG_PUSH_PPM", "GG_PUSH_MIN_ITEMS", "GG_NO_GRAPH", "GG_ADJ_SMEM"})
+        if (std::getenv(name)) e->direct = false;
+    if (env_int("GG_DIRECT", 1) == 0) e->direct = false;
+    e->direct_allowed = e->direct;
+    GG_CK(cudaDeviceGetAttribute(&e->sms, cudaDevAttrMultiProcessorCount, e->device));
+    GG_CK(cudaDeviceGetAttribute(&e->smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, e->device));
+    for (int W : {1, 2, 4})
+        GG_CK(cudaFuncSetAttribute(direct_for(W), cudaFuncAttributeMaxDynamicSharedMemorySize, e->smem_optin - 1024));
     const int wait_ms = env_int("GG_WAIT_LIMIT_MS", 10000);
     e->wait_ns = (long long)std::max(wait_ms, 1) * 1000000ll;
     gg_status s = plan(e, 0);
@@ -583,6 +617,179 @@ gg_status finish_create(gg_engine *e, gg_engine **out) {
         return s;
     }
     *out = e;
+    return GG_OK;
+}
+
+// A lifted form's table (device memory) -> the pull adjacency d_adj.
+void launch_expand(gg_engine *e, const int32_t *d_table, cudaStream_t st) {
+    const long long n = (long long)e->rows * e->d;
+    ExpandArgs x{};
+    x.table = d_table;
+    x.adj = e->d_adj;
+    x.form = (e->form == FORM_PART) ? 1 : (e->form == FORM_PIECE ? 2 : 3);
+    x.rows = e->rows; x.d = e->d; x.N = e->N; x.M = e->M;
+    x.Nx = e->dims[0]; x.Ny = e->dims[1]; x.Nz = e->dims[2];
+    x.Mx = e->dims[3]; x.My = e->dims[4]; x.Mz = e->dims[5];
+    gg::expand_kernel<<<(int)std::min<long long>((n + 255) / 256, 8192), 256, 0, st>>>(x);
+}
+
+// ---- small graphs: direct_kernel -------------------------------------------------
+
+struct DirectPlan {
+    int W = 0;            // 32-source words a vertex (0: not for this evaluation)
+    bool adj_smem = false;
+    size_t smem = 0;
+    int grid = 0, block = 0;
+};
+
+// The word width that makes the fewest rounds of blocks cheapest, or none: the visited
+// sets of every width must fit a block's shared memory.  A random row of 4, 8 or 16 bytes
+// per lane costs about 3.5, 6.2 and 10.4 shared-memory cycles a warp.
+DirectPlan direct_plan(const gg_engine *e, int ns, bool wvc) {
+    DirectPlan best;
+    if (!e->direct || e->rows < 1 || e->rows > 65535 || ns < 1) return best;
+    const size_t budget = (size_t)e->smem_optin - 1024;
+    double cost = 1e300;
+    for (int W : {1, 2, 4}) {
+        const size_t set = ((size_t)e->rows * W + 3) / 4 * 16, adj = ((size_t)e->rows * e->d * 2 + 15) / 16 * 16;
+        if (2 * set > budget) continue;
+        const int grid = (ns + 32 * W - 1) / (32 * W);
+        const bool in_smem = 2 * set + adj <= budget;
+        const size_t smem = 2 * set + (in_smem ? adj : 0);
+        const int block = e->rows >= 1024 ? gg::kDirectBlock : std::max(128, (e->rows + 31) / 32 * 32);
+        const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(1024 / block, budget / std::max<size_t>(smem + 1024, 1)));
+        const double rounds = std::ceil((double)grid / (e->sms * per_sm));
+        const double c = rounds * (W == 1 ? 3.5 : W == 2 ? 6.2 : 10.4) * per_sm;
+        if (c < cost && (rounds == 1 || e->rows <= 20480)) {
+            cost = c;
+            best = DirectPlan{W, in_smem, smem, grid, block};
+        }
+    }
+    // Against bfs_batch_kernel: microseconds of the two (fits of both sides over n = 64 to
+    // 27000 and lifts of 20 to 4000 orbits).  A round of one-word groups takes 3.2 + 0.1 d
+    // ns a row (a tenth more with the WVC masks), less certain for a single round; the level
+    // loop 50 us and 0.12 ns a chunk of 128 sources.  Device times: n = 4096, d = 16: 25
+    // against 67 us; 16000, 6: 239 / 372; 20000, 8: 337 / 499; 24000, 6: 552 / 448; lifts of
+    // 6000 vertices, 500 orbits: 29 / 59, of 20000, 1000: 85 / 82, of 20000, 2000: 96 / 90.
+    if (best.W) {
+        const bool one = best.grid <= e->sms;
+        const double direct_us = cost / 3.5 * e->rows * (3.2 + 0.1 * e->d) * 1e-3 * (wvc ? 1.1 : 1.0) * (one ? 1.12 : 1.0);
+        const double chunks = (double)e->rows * ((ns + 127) / 128);
+        if (direct_us > 50.0 + 0.12e-3 * chunks) best.W = 0;
+    }
+    return best;
+}
+
+gg_status ensure_direct(gg_engine *e, int cap) {
+    if (e->d_dir && cap <= e->dir_cap) return GG_OK;
+    cap = std::max(cap, 256);
+    cudaFree(e->d_dir); cudaFreeHost(e->h_dir);
+    e->d_dir = e->h_dir = nullptr;
+    e->dir_cap = 0;
+    const size_t n = (size_t)cap + 1, bytes = 64 + n * 12;
+    GG_CK(cudaMalloc(&e->d_dir, bytes));
+    GG_CK(cudaMallocHost(&e->h_dir, bytes));
+    std::memset(e->h_dir, 0, 64);
+    GG_CK(cudaMemset(e->d_dir, 0, 64 + n * 8));
+    GG_CK(cudaMemset(e->d_dir + 64 + n * 8, 0xff, n * 4));
+    e->dir_cap = cap;
+    return GG_OK;
+}
+
+// One evaluation by direct_kernel.  `table`: the calculator table in device memory, or
+// adj16: a plain graph's checked 16-bit ids (device or pinned host memory).
+gg_status direct_eval(gg_engine *e, const DirectPlan &p, const int32_t *table, const uint16_t *adj16,
+                      const gg_eval_opts *o, int s0, int ns, int cap, gg_result *r, cudaStream_t st) {
+    gg_status s = ensure_direct(e, cap);
+    if (s != GG_OK) return s;
+    (void)cudaGetLastError();
+    if (fault("launch")) return fail(GG_CUDA_ERROR, "injected launch failure");
+    const bool wvc = o && o->want_wvc;
+    const long long n = (long long)e->rows * e->d;
+    int launches = 1;
+    gg::DirectArgs a{};
+    a.adj = e->d_adj;
+    a.adj16 = adj16;
+    if (adj16) {
+        // read as it is
+    } else if (e->form == FORM_GRAPH) {
+        a.adj = table;
+        if ((reinterpret_cast<uintptr_t>(table) & 15u) && n > 0) {   // 16-byte loads
+            GG_CK(cudaMemcpyAsync(e->d_table, table, (size_t)n * 4, cudaMemcpyDeviceToDevice, st));
+            a.adj = e->d_table;
+        }
+        if (!p.adj_smem && n > 0) {
+            GG_CK(cudaMemsetAsync(e->d_bad, 0, sizeof(int), st));
+            gg::check_table_kernel<<<(int)std::min<long long>((n + 255) / 256, 4096), 256, 0, st>>>(a.adj, n, e->rows,
+                                                                                                 e->d_bad);
+            GG_CK(cudaGetLastError());
+            a.bad_table = e->d_bad;
+            ++launches;
+        }
+    } else if (n > 0) {
+        launch_expand(e, table, st);
+        GG_CK(cudaGetLastError());
+        ++launches;
+    }
+    a.src = e->d_src;
+    a.src_first = e->src_first;
+    a.src_begin = s0;
+    a.ns_total = ns;
+    a.rows = e->rows; a.d = e->d;
+    a.max_levels = cap;
+    a.adj_smem = p.adj_smem ? 1 : 0;
+    const size_t off = 64 + ((size_t)e->dir_cap + 1) * 8;
+    a.ctl = reinterpret_cast<gg::DirectCtl *>(e->d_dir);
+    a.h_ctl = reinterpret_cast<gg::DirectCtl *>(e->h_dir);
+    a.counts = reinterpret_cast<unsigned long long *>(e->d_dir + 64);
+    a.h_counts = reinterpret_cast<unsigned long long *>(e->h_dir + 64);
+    a.masks = wvc ? reinterpret_cast<unsigned *>(e->d_dir + off) : nullptr;
+    a.h_masks = reinterpret_cast<unsigned *>(e->h_dir + off);
+    a.batch_ns = e->h_batch_ns;
+    a.seq = ++e->dir_seq;
+    if (a.seq == 0) a.seq = ++e->dir_seq;   // 0: none yet
+    void *k = direct_for(p.W);
+    void *args[] = {&a};
+    GG_CK(cudaLaunchKernel(k, dim3((unsigned)p.grid), dim3((unsigned)p.block), args, p.smem, st));
+    // The kernel's last block stores its number after the counters; a wait for the stream
+    // takes a few microseconds longer to come back.  Not there within a few milliseconds:
+    // wait for the stream (a long evaluation, or an error to report).
+    {
+        const volatile unsigned *seq = &a.h_ctl->seq;
+        const auto t0 = std::chrono::steady_clock::now();
+        unsigned it = 0;
+        while (*seq != a.seq) {
+            if ((++it & 1023u) == 0u && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(5)) {
+                GG_CK(cudaStreamSynchronize(st));
+                break;
+            }
+        }
+        std::atomic_thread_fence(std::memory_order_acquire);
+    }
+    e->last_ms = (double)(e->h_batch_ns[1] - e->h_batch_ns[0]) * 1e-6;
+    e->last_launches = launches;
+    e->last_batches = 1;
+    e->last_d2h = sizeof(gg::DirectCtl) + ((size_t)a.h_ctl->levels_run + 1) * (wvc ? 12 : 8);
+    if (a.h_ctl->bad) return fail(GG_BAD_ARG, "adjacency entry outside [0, N)");
+    const int run = a.h_ctl->levels_run;
+    gg_result R{};
+    R.scale = e->scale;
+    R.pairs = (uint64_t)ns * (uint64_t)e->rows;
+    R.n_sources = ns;
+    R.batches = 1;
+    R.wvc = -1;
+    for (int L = 0; L <= run; ++L) {
+        R.reached += a.h_counts[L];
+        R.total += (uint64_t)L * a.h_counts[L];
+        if (L > 0 && a.h_counts[L]) R.levels = L;
+    }
+    R.level_steps = run;
+    R.capped = run >= cap && a.h_counts[cap] ? 1 : 0;
+    R.connected = (!R.capped && R.reached == R.pairs) ? 1 : 0;
+    if (wvc) R.wvc = R.levels > 0 ? __builtin_popcount(a.h_masks[R.levels - 1] ^ a.h_masks[R.levels]) : 0;
+    if (o && o->level_counts)
+        for (int L = 0; L <= cap; ++L) o->level_counts[L] = L <= run ? a.h_counts[L] : 0ull;
+    *r = R;
     return GG_OK;
 }
 
@@ -603,6 +810,10 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
     const bool wvc = o && o->want_wvc;
     const bool want_ns = o && o->level_ns;
     const int ns_all = s1 - s0;
+    if (!x && !want_ns && !fault("barrier")) {
+        const DirectPlan p = direct_plan(e, ns_all, wvc);
+        if (p.W) return direct_eval(e, p, d_table_in, nullptr, o, s0, ns_all, cap_req, r, st);
+    }
     const int nb = (ns_all + e->batch_bits - 1) / e->batch_bits;
     const bool within = x && x->within;
     if (within && (!x->inv || wvc || x->planes || e->form != FORM_GRAPH)) return fail(GG_BAD_ARG, "pairs within the sources need a source list");
@@ -666,14 +877,7 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
                 GG_CK(cudaGetLastError());
             }
         } else if (n > 0) {
-            ExpandArgs x{};
-            x.table = d_table_in;
-            x.adj = e->d_adj;
-            x.form = (e->form == FORM_PART) ? 1 : (e->form == FORM_PIECE ? 2 : 3);
-            x.rows = e->rows; x.d = e->d; x.N = e->N; x.M = e->M;
-            x.Nx = e->dims[0]; x.Ny = e->dims[1]; x.Nz = e->dims[2];
-            x.Mx = e->dims[3]; x.My = e->dims[4]; x.Mz = e->dims[5];
-            gg::expand_kernel<<<(int)std::min<long long>((n + 255) / 256, 8192), 256, 0, q>>>(x);
+            launch_expand(e, d_table_in, q);
             GG_CK(cudaGetLastError());
         }
         if (want_ns)
@@ -937,10 +1141,62 @@ void copy_to_pinned(void *dst, const void *src, size_t bytes) {
     }
 }
 
+// A plain graph's table as checked 16-bit ids in pinned memory, by a few threads when it is
+// large; false: an entry outside [0, rows).
+bool pack16(uint16_t *dst, const int32_t *src, size_t n, int rows) {
+    constexpr size_t kPart = 16u << 10;
+    const int parts = (int)std::min<size_t>(8, std::max<size_t>(1, n / kPart));
+    unsigned bad = 0u;
+    auto range = [&](size_t lo, size_t hi) {
+        unsigned b = 0u;
+        for (size_t k = lo; k < hi; ++k) {
+            const unsigned x = (unsigned)src[k];
+            b |= x >= (unsigned)rows ? 1u : 0u;
+            dst[k] = (uint16_t)x;
+        }
+        return b;
+    };
+    if (parts <= 1) return range(0, n) == 0u;
+#pragma omp parallel for num_threads(parts) schedule(static) reduction(| : bad)
+    for (int i = 0; i < parts; ++i) bad |= range(n * (size_t)i / (size_t)parts, n * (size_t)(i + 1) / (size_t)parts);
+    return bad == 0u;
+}
+
+// Host table of a plain graph small enough for direct_kernel with its rows in shared
+// memory: half the bytes to copy, and none where the few blocks of a small graph read
+// them over the bus at less than a copy command costs (n = 256, d = 4: 2 KB, 8 blocks).
+constexpr size_t kZeroCopyTotal = 128u << 10;
+
+gg_status direct_host(gg_engine *e, const DirectPlan &p, const int32_t *table, const gg_eval_opts *o, gg_result *r) {
+    const size_t n = e->table_elems, bytes = (n * 2 + 15) / 16 * 16;
+    if (!e->h_pack) {
+        GG_CK(cudaMallocHost(&e->h_pack, std::max<size_t>(bytes, 16)));
+        GG_CK(cudaMalloc(&e->d_pack, std::max<size_t>(bytes, 16)));
+        std::memset(e->h_pack, 0, std::max<size_t>(bytes, 16));
+    }
+    e->table_stale = true;
+    if (!pack16(e->h_pack, table, n, e->rows)) return fail(GG_BAD_ARG, "adjacency entry outside [0, N)");
+    const uint16_t *from = e->h_pack;
+    if (bytes * (size_t)p.grid > kZeroCopyTotal) {
+        GG_CK(cudaMemcpyAsync(e->d_pack, e->h_pack, bytes, cudaMemcpyHostToDevice, e->stream));
+        from = e->d_pack;
+    }
+    const int cap = (o && o->max_levels > 0) ? o->max_levels : std::max(e->rows, 1);
+    gg_status s = direct_eval(e, p, nullptr, from, o, 0, (int)e->reps.size(), cap, r, e->stream);
+    e->last_h2d = n * 2;
+    return s;
+}
+
 gg_status eval_host(gg_engine *e, const int32_t *table, const gg_eval_opts *o, gg_result *r) {
     if (!e || !r) return fail(GG_BAD_ARG, "null engine or result");
     if (e->table_elems && !table) return fail(GG_BAD_ARG, "null table");
     GG_CK(cudaSetDevice(e->device));
+    e->table_stale = false;
+    if (e->form == FORM_GRAPH && e->table_elems && !(o && (o->level_ns || o->src_begin || o->src_end || o->want_wvc)) &&
+        !fault("barrier")) {
+        const DirectPlan p = direct_plan(e, (int)e->reps.size(), false);
+        if (p.W && p.adj_smem) return direct_host(e, p, table, o, r);
+    }
     if (e->table_elems) {
         copy_to_pinned(e->h_table, table, e->table_elems * sizeof(int32_t));
         GG_CK(cudaMemcpyAsync(e->d_table, e->h_table, e->table_elems * sizeof(int32_t),
@@ -1144,6 +1400,7 @@ gg_status gg_set_batch_sources(gg_engine *e, int sources) {
     if (!e || sources < 0) return fail(GG_BAD_ARG, "bad batch width");
     GG_CK(cudaSetDevice(e->device));
     GG_CK(cudaStreamSynchronize(e->stream));
+    e->direct = sources == 0 && e->direct_allowed;   // an explicit width runs the batches it asks for
     return plan(e, sources);
 }
 
@@ -1152,6 +1409,12 @@ gg_status gg_autotune(gg_engine *e, const int32_t *table, int trials, int *best_
     GG_CK(cudaSetDevice(e->device));
     GG_CK(cudaStreamSynchronize(e->stream));
     const int n_src = (int)e->reps.size();
+    struct Planned {   // the shapes timed here are bfs_batch_kernel's
+        gg_engine *e;
+        bool was;
+        ~Planned() { e->direct = was; }
+    } planned{e, e->direct};
+    e->direct = false;
     // the L2-resident width the default plan picks, and its neighbours
     int base = 0, max_bps = 0;
     {
@@ -1257,6 +1520,11 @@ gg_status gg_graph_calc(gg_engine *e, const int32_t *adj, int *diameter, int64_t
         *diameter = r.levels;
         *total = (int64_t)r.total;
         return GG_OK;
+    }
+    if (e->table_stale) {
+        copy_to_pinned(e->h_table, adj, e->table_elems * sizeof(int32_t));
+        GG_CK(cudaMemcpyAsync(e->d_table, e->h_table, e->table_elems * sizeof(int32_t), cudaMemcpyHostToDevice, e->stream));
+        e->table_stale = false;
     }
     // Some source hits the 199-step limit or misses a vertex: the reference
     // answers for the first 1024-source chunk (in source order) that does

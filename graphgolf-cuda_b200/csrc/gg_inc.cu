@@ -226,7 +226,7 @@ void inc_free(gg_inc *h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     if (h->eng) gg_destroy(h->eng);
     cudaFree(h->d_adj); cudaFree(h->d_cand); cudaFree(h->d_inv); cudaFree(h->d_stats);
-    cudaFree(h->d_list); cudaFree(h->d_tbits);
+    // (d_list and d_tbits lie behind d_inv)
     cudaFree(h->d_planes); cudaFree(h->d_st); cudaFreeHost(h->h_st);
     cudaFree(h->d_asym); cudaFreeHost(h->h_asym);
     if (h->stream) cudaStreamDestroy(h->stream);
@@ -317,10 +317,14 @@ gg_status gg_inc_create(int n, int degree, int device, gg_inc **out) {
     cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&h->d_adj, adj_b);
     if (e == cudaSuccess) e = cudaMalloc(&h->d_cand, adj_b);
-    if (e == cudaSuccess) e = cudaMalloc(&h->d_inv, (size_t)n * sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&h->d_list, (size_t)n * sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&h->d_tbits, (size_t)h->cols * sizeof(uint4));
-    if (e == cudaSuccess) e = cudaMemset(h->d_tbits, 0, (size_t)h->cols * sizeof(uint4));
+    // inv, list and T's bits in one allocation
+    const size_t ids = ((size_t)n * sizeof(int32_t) + 255) / 256 * 256;
+    if (e == cudaSuccess) e = cudaMalloc(&h->d_inv, 2 * ids + (size_t)h->cols * sizeof(uint4));
+    if (e == cudaSuccess) {
+        h->d_list = h->d_inv + ids / sizeof(int32_t);
+        h->d_tbits = reinterpret_cast<uint32_t *>(h->d_inv + 2 * (ids / sizeof(int32_t)));
+        e = cudaMemsetAsync(h->d_tbits, 0, (size_t)h->cols * sizeof(uint4), h->stream);
+    }
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = cudaMalloc(&h->d_stats, 3 * (size_t)n * sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMalloc(&h->d_asym, sizeof(int));

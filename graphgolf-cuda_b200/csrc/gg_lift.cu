@@ -900,6 +900,7 @@ struct gg_lift {
     bool delta_on = false;                           // the lift is within the limits and the buffers are there
     int base_state = 0;                              // distances of the base: 0 not computed, 1 usable, -1 not usable
     int rw = 0, pitch = 0, words = 0, unit_rows = 1, delta_grid = 0;
+    unsigned char *d_arena = nullptr, *d_each = nullptr;   // what the pointers below lie in (d_each: per candidate)
     uint4 *d_planes = nullptr;                       // [4][N][cpc]
     uint8_t *d_dist = nullptr;                       // [M][pitch]
     uint16_t *d_rows = nullptr;                      // [N][rw]
@@ -928,9 +929,7 @@ void lift_free(gg_lift *h) {
     cudaFree(h->d_counts); cudaFreeHost(h->h_counts);
     cudaFree(h->d_level_ns); cudaFreeHost(h->h_level_ns);
     cudaFree(h->d_ctl); cudaFreeHost(h->h_ctl);
-    cudaFree(h->d_planes); cudaFree(h->d_dist); cudaFree(h->d_rows); cudaFree(h->d_diffs); cudaFree(h->d_ball); cudaFree(h->d_spill);
-    cudaFree(h->d_ctr); cudaFree(h->d_cand); cudaFreeHost(h->h_cand); cudaFree(h->d_near); cudaFree(h->d_lists);
-    cudaFree(h->d_patch); cudaFree(h->d_changes); cudaFree(h->d_units);
+    cudaFree(h->d_arena); cudaFree(h->d_each); cudaFreeHost(h->h_cand);
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
     if (h->stream) cudaStreamDestroy(h->stream);
@@ -1007,17 +1006,30 @@ void delta_open(gg_lift *h) {
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kDeltaBlock, smem);
     h->delta_grid = per_sm * h->sms;
     if (e == cudaSuccess && per_sm < 1) e = cudaErrorInvalidConfiguration;
-    if (e == cudaSuccess) e = cudaMalloc(&h->d_planes, 4 * (size_t)h->N * h->cpc * sizeof(uint4));
-    if (e == cudaSuccess) e = cudaMalloc(&h->d_dist, pitch * h->M);
-    if (e == cudaSuccess) e = cudaMalloc(&h->d_rows, (size_t)h->N * h->rw * sizeof(uint16_t));
-    if (e == cudaSuccess) e = cudaMalloc(&h->d_diffs, (size_t)h->M * h->dp * sizeof(uint16_t));
-    if (e == cudaSuccess) e = cudaMalloc(&h->d_ball, (size_t)h->M * h->words * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&h->d_spill, (size_t)h->delta_grid * 3 * gg::kDeltaSpill * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&h->d_ctr, 3 * sizeof(int));
+    // one allocation for all of them
+    size_t at = 0;
+    auto part = [&](size_t bytes) {
+        const size_t o = at;
+        at += (bytes + 255) / 256 * 256;
+        return o;
+    };
+    const size_t o_planes = part(4 * (size_t)h->N * h->cpc * sizeof(uint4)), o_dist = part(pitch * h->M),
+                 o_rows = part((size_t)h->N * h->rw * sizeof(uint16_t)),
+                 o_diffs = part((size_t)h->M * h->dp * sizeof(uint16_t)),
+                 o_ball = part((size_t)h->M * h->words * sizeof(uint32_t)),
+                 o_spill = part((size_t)h->delta_grid * 3 * gg::kDeltaSpill * sizeof(uint32_t)), o_ctr = part(3 * sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc(&h->d_arena, at);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         return;
     }
+    h->d_planes = reinterpret_cast<uint4 *>(h->d_arena + o_planes);
+    h->d_dist = h->d_arena + o_dist;
+    h->d_rows = reinterpret_cast<uint16_t *>(h->d_arena + o_rows);
+    h->d_diffs = reinterpret_cast<uint16_t *>(h->d_arena + o_diffs);
+    h->d_ball = reinterpret_cast<uint32_t *>(h->d_arena + o_ball);
+    h->d_spill = reinterpret_cast<uint32_t *>(h->d_arena + o_spill);
+    h->d_ctr = reinterpret_cast<int *>(h->d_arena + o_ctr);
     h->delta_on = true;
 }
 
@@ -1025,26 +1037,33 @@ void delta_open(gg_lift *h) {
 bool delta_ensure(gg_lift *h, int n) {
     if (n <= h->delta_cap) return true;
     const size_t cap = (size_t)std::max(n, 2 * h->delta_cap), g = (size_t)h->N / h->M;
-    cudaFree(h->d_cand); cudaFreeHost(h->h_cand); cudaFree(h->d_near); cudaFree(h->d_lists);
-    cudaFree(h->d_patch); cudaFree(h->d_changes); cudaFree(h->d_units);
-    h->d_cand = h->h_cand = nullptr;
-    h->d_near = nullptr;
-    h->d_lists = h->d_patch = nullptr;
-    h->d_changes = nullptr;
-    h->d_units = nullptr;
-    h->delta_cap = 0;
     const size_t units = (size_t)(h->M + h->unit_rows - 1) / h->unit_rows;
-    cudaError_t e = cudaMalloc(&h->d_cand, cap * sizeof(DeltaCand));
+    cudaFree(h->d_each); cudaFreeHost(h->h_cand);
+    h->d_each = nullptr;
+    h->h_cand = nullptr;
+    h->delta_cap = 0;
+    size_t at = 0;
+    auto part = [&](size_t bytes) {
+        const size_t o = at;
+        at += (bytes + 255) / 256 * 256;
+        return o;
+    };
+    const size_t o_cand = part(cap * sizeof(DeltaCand)), o_near = part(cap * h->words * sizeof(uint32_t)),
+                 o_lists = part(cap * h->M * sizeof(uint16_t)),
+                 o_patch = part(cap * 4 * (h->axes == 1 ? h->dp : g * h->rw) * sizeof(uint16_t)),
+                 o_changes = part(cap * 4 * g * sizeof(uint3)), o_units = part(cap * units * sizeof(DeltaUnit));
+    cudaError_t e = cudaMalloc(&h->d_each, at);
     if (e == cudaSuccess) e = cudaMallocHost(&h->h_cand, cap * sizeof(DeltaCand));
-    if (e == cudaSuccess) e = cudaMalloc(&h->d_near, cap * h->words * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&h->d_lists, cap * h->M * sizeof(uint16_t));
-    if (e == cudaSuccess) e = cudaMalloc(&h->d_patch, cap * 4 * (h->axes == 1 ? h->dp : g * h->rw) * sizeof(uint16_t));
-    if (e == cudaSuccess) e = cudaMalloc(&h->d_changes, cap * 4 * g * sizeof(uint3));
-    if (e == cudaSuccess) e = cudaMalloc(&h->d_units, cap * units * sizeof(DeltaUnit));
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         return false;
     }
+    h->d_cand = reinterpret_cast<DeltaCand *>(h->d_each + o_cand);
+    h->d_near = reinterpret_cast<uint32_t *>(h->d_each + o_near);
+    h->d_lists = reinterpret_cast<uint16_t *>(h->d_each + o_lists);
+    h->d_patch = reinterpret_cast<uint16_t *>(h->d_each + o_patch);
+    h->d_changes = reinterpret_cast<uint3 *>(h->d_each + o_changes);
+    h->d_units = reinterpret_cast<DeltaUnit *>(h->d_each + o_units);
     h->delta_cap = (int)cap;
     return true;
 }

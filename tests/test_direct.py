@@ -1,0 +1,105 @@
+"""Small graphs scored without a grid barrier (csrc/gg_direct.cuh): every result field
+against the oracle and against the level loop (GG_DIRECT=0), at the edges of the groups
+(32, 64 and 128 sources), of the row tables (16-bit ids in shared memory or the table
+itself), of the table's way to the device, and for ranges, caps and rejected tables."""
+import numpy as np
+import pytest
+
+import graphgolf as G
+import instances as I
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def both(monkeypatch, make, call):
+    monkeypatch.setenv("GG_DIRECT", "0")
+    e = make()
+    want = call(e)
+    e.close()
+    monkeypatch.delenv("GG_DIRECT")
+    e = make()
+    got = call(e)
+    again = call(e)     # the counters of the first call were cleared
+    e.close()
+    return want, got, again
+
+
+KEYS = ("total", "reached", "pairs", "levels", "capped", "connected", "n_sources")
+
+
+@pytest.mark.parametrize("n,d", [(2, 1), (5, 2), (31, 4), (32, 3), (33, 4), (64, 5), (129, 6), (1000, 7), (1023, 8), (1025, 12),
+                                 (700, 16), (600, 17), (3001, 4), (4740, 6), (5001, 8), (7001, 16), (9473, 4), (12001, 6)])
+def test_direct_counts_equal_the_level_loop(n, d, monkeypatch):
+    adj = G.random_regular(n if n * d % 2 == 0 else n + 1, d, 3) if n > 2 else np.array([[1], [0]], np.int32)
+    n = len(adj)
+    cap = 40
+    want, got, again = both(monkeypatch, lambda: G.cudaASPLgraph(n, d),
+                            lambda e: e.eval(adj, max_levels=cap, level_counts=True))
+    for r in (got, again):
+        assert all(r[k] == want[k] for k in KEYS)
+        assert np.array_equal(r["level_counts"], want["level_counts"])
+    o = O.bfs_pull(adj, np.arange(n))
+    assert (got["total"], got["reached"], got["levels"]) == (o.total(), int(o.reached.sum()), o.levels)
+
+
+@pytest.mark.parametrize("form", ["part", "part_m3", "piece", "box", "wvc", "wvc_bits"])
+def test_direct_lifted_forms(form, monkeypatch):
+    if form in ("part", "part_m3", "wvc", "wvc_bits"):
+        N, M, T = G.cyclic_lift(*{"part": (150, 9, 5, 1), "part_m3": (64, 3, 4, 2), "wvc": (500, 12, 6, 3),
+                                  "wvc_bits": (37, 40, 4, 4)}[form])
+        make = lambda: G.cudaASPLconv(N, M, T.shape[1])
+        call = (lambda e: e.WVCdiameterASPL(T)) if form.startswith("wvc") else (lambda e: e.diameterASPL(T))
+    elif form == "piece":
+        a = G.piece_lift(5, 7, 4, 3, 6, 1)
+        make, call = (lambda: G.cudaASPLpiece(*a[:4], 6)), (lambda e: e.diameterASPL(a[4]))
+    else:
+        a = I.random_box(3, 2, 4, 2, 3, 2, 6, 1)
+        make, call = (lambda: G.cudaASPLbox(*a[:6], 6)), (lambda e: e.diameterASPL(a[6]))
+    want, got, again = both(monkeypatch, make, call)
+    assert got == want and again == want
+
+
+def test_direct_ranges_caps_disconnected_and_bad_tables(monkeypatch):
+    adj = G.random_regular(1500, 4, 5)
+    make = lambda: G.cudaASPLgraph(1500, 4)
+    for call in (lambda e: e.eval(adj, src_range=(3, 700)), lambda e: e.eval(adj, max_levels=3),
+                 lambda e: e.eval(adj, src_range=(1499, 1500), max_levels=2)):
+        want, got, again = both(monkeypatch, make, call)
+        assert all(got[k] == want[k] and again[k] == want[k] for k in KEYS)
+    two = np.concatenate([I.cycle(40), I.cycle(40) + 40]).astype(np.int32)    # disconnected
+    long = np.asarray(I.cycle(500), dtype=np.int32)                              # past calc's 199 levels
+    for t in (two, long, I.path_graph(70)):
+        want, got, again = both(monkeypatch, lambda: G.cudaASPLgraph(len(t), t.shape[1]), lambda e: e.calc(t))
+        assert got == want and again == want
+    wvc = np.array([[2, -2]] * 8, np.int32)                                      # two cycles, with masks
+    o = lambda e: e.eval(wvc, max_levels=50, want_wvc=True)
+    want, got, again = both(monkeypatch, lambda: G.cudaASPLconv(64, 8, 2), o)
+    assert all(got[k] == want[k] and again[k] == want[k] for k in KEYS + ("wvc",))
+    for n, d in ((100, 4), (9000, 16)):      # read over the bus; ids from the table itself
+        e = G.cudaASPLgraph(n, d)
+        good = G.random_regular(n, d, 6)
+        first = e.calc(good)
+        for v in (n, -1, 1 << 20):
+            bad = good.copy()
+            bad[n // 2, 1] = v
+            with pytest.raises(G.GGError) as err:
+                e.calc(bad)
+            assert err.value.status == G.GG_BAD_ARG
+            assert e.calc(good) == first
+        e.close()
+
+
+def test_direct_device_tables_of_any_alignment():
+    import torch
+    for n, d in ((200, 5), (3000, 8), (9000, 16)):
+        adj = G.random_regular(n, d, 7)
+        e = G.cudaASPLgraph(n, d)
+        want = e.eval(adj)
+        buf = torch.zeros(n * d + 8, dtype=torch.int32, device="cuda")
+        for shift in (0, 1, 2, 3):
+            buf[shift:shift + n * d] = torch.from_numpy(adj.ravel()).cuda()
+            torch.cuda.synchronize()
+            got = e.eval_device(buf.data_ptr() + 4 * shift)
+            assert all(got[k] == want[k] for k in KEYS)
+        e.close()
