@@ -12,6 +12,7 @@
 #include "gg.h"
 #include "gg_kernels.cuh"
 #include "gg_direct.cuh"
+#include "gg_sweep.cuh"
 #include "gg_internal.h"
 
 #include <algorithm>
@@ -84,11 +85,11 @@ __attribute__((visibility("hidden"))) void set_last_error(const char *msg) { g_e
 struct EvalKey {
     const void *table, *status, *bitsets, *inv, *planes;
     int s0, ns, cap;
-    bool wvc, want_ns;
+    bool wvc, want_ns, sweep;
     bool operator==(const EvalKey &o) const {
         return table == o.table && status == o.status && bitsets == o.bitsets && inv == o.inv &&
                planes == o.planes && s0 == o.s0 && ns == o.ns && cap == o.cap && wvc == o.wvc &&
-               want_ns == o.want_ns;
+               want_ns == o.want_ns && sweep == o.sweep;
     }
 };
 
@@ -117,6 +118,7 @@ struct gg_engine {
     int bps_cap = 0;                     // resident blocks per SM (0: as many as fit)
     int walk_pref = -1;                  // walk depth: -1 automatic, 0 off, K > 0 forced
     int walk_K = 0;                      // levels computed by the walk pass (0: off)
+    bool walk_auto = true;               // ... chosen by walk_levels, not asked for
     int walk_vpull = 1;                  // levels after the walk pull visited sets (GG_VPULL=0: frontiers)
     int walk_own_skip = 1;               // dense ones skip own chunks on tables without one-way entries (GG_OWN_SKIP)
     int walk_third = 1;                  // after the walk of all batches, levels alternate V and F0 (GG_WALK_THIRD)
@@ -150,6 +152,9 @@ struct gg_engine {
     uint32_t *d_pf0 = nullptr, *d_pf1 = nullptr;
     uint32_t *d_nf = nullptr;            // not-full bit per visited chunk
     uint32_t *d_nf2 = nullptr;           // its second copy (visited-set pull levels alternate)
+    int *d_redo = nullptr, *h_redo = nullptr;   // sweep_kernel gave up: bfs_batch_kernel instead
+    bool sweep = true;                   // sweep_kernel where it applies (GG_SWEEP, and no level mode asked for)
+    int sweep_wait = 0;                  // evaluations until it is tried again
     int *d_wasym = nullptr;              // one-way flag of the table (walk_index_kernel)
     unsigned long long *d_vtot = nullptr;   // [nb][3] level totals (dense visited-set pull without own chunks)
     // walk_all_kernel output: the level-K rows of every batch and their flag words
@@ -299,8 +304,9 @@ long long walk_cap_for(int d, int K) {
 // 64 MiB and the index (rows * (ends + buckets) uint16) within 1 GiB; off for
 // evaluations of a single source batch.  GG_WALK_LEVELS overrides the depth (0 = off;
 // still within the size limits).
-int walk_levels(const gg_engine *e) {
+int walk_levels(gg_engine *e) {
     const int env = env_int("GG_WALK_LEVELS", e->walk_pref);
+    e->walk_auto = env < 0;
     const int d = e->d;
     if (d <= 0 || e->nC > gg::kWalkMaxNC || env == 0) return 0;
     int K = 0;
@@ -321,12 +327,21 @@ int walk_levels(const gg_engine *e) {
     return K;
 }
 
+template <int D, bool ONE>
+void *walk_all_of(int K) {
+    return K == 1 ? (void *)gg::walk_all_kernel<D, 1, ONE> : K == 2 ? (void *)gg::walk_all_kernel<D, 2, ONE>
+                                                                    : (void *)gg::walk_all_kernel<D, 3, ONE>;
+}
+
 // walk_all_kernel for an evaluation of nb batches, or nullptr (a walk pass per
-// batch): visited-set pull levels, 4096-source batches, degree 4 or 8, K <= 3, and
-// the level-K rows of all nb batches within the GG_WALK_ALL_MB budget.  Grows
-// d_vall as needed (a failed allocation falls back to the per-batch pass).
+// batch): visited-set pull levels, batches of a multiple of 4096 sources, degree 3, 4, 6
+// or 8, K <= 3 (with the level-2 table, or 16-byte rows), and the level-K rows of all nb
+// batches within the GG_WALK_ALL_MB budget.  Grows d_vall as needed (a failed allocation
+// falls back to the per-batch pass).
 void *walk_all_for(gg_engine *e, int K, int nb) {
-    if (!e->walk_vpull || e->nC != 32 || K < 1 || K > 3 || (e->d != 4 && e->d != 8)) return nullptr;
+    if (!e->walk_vpull || e->nC % 32 != 0 || K < 1 || K > 3 || nb * (e->nC / 32) * K > gg::kIndexMaxKeys) return nullptr;
+    if (e->d != 3 && e->d != 4 && e->d != 6 && e->d != 8) return nullptr;
+    if (K < 3 && e->d % 4 != 0) return nullptr;
     const size_t bytes = (size_t)nb * e->items * sizeof(uint4);
     const size_t fbytes = (size_t)nb * ((e->items + 31) / 32) * sizeof(uint32_t);
     if ((long long)(bytes >> 20) > e->walk_all_mb) return nullptr;
@@ -346,14 +361,31 @@ void *walk_all_for(gg_engine *e, int K, int nb) {
         e->vall_batches = (size_t)nb;
     }
     void *k = nullptr;
-    if (e->d == 8) k = K == 1 ? (void *)gg::walk_all_kernel<8, 1> : K == 2 ? (void *)gg::walk_all_kernel<8, 2> : (void *)gg::walk_all_kernel<8, 3>;
-    else k = K == 1 ? (void *)gg::walk_all_kernel<4, 1> : K == 2 ? (void *)gg::walk_all_kernel<4, 2> : (void *)gg::walk_all_kernel<4, 3>;
+    if (e->nC == 32)
+        k = e->d == 8 ? walk_all_of<8, true>(K) : e->d == 4 ? walk_all_of<4, true>(K)
+          : e->d == 6 ? (void *)gg::walk_all_kernel<6, 3, true> : (void *)gg::walk_all_kernel<3, 3, true>;
+    else
+        k = e->d == 8 ? walk_all_of<8, false>(K) : e->d == 4 ? walk_all_of<4, false>(K)
+          : e->d == 6 ? (void *)gg::walk_all_kernel<6, 3, false> : (void *)gg::walk_all_kernel<3, 3, false>;
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, gg::walk_all_smem(K)) != cudaSuccess) {
         (void)cudaGetLastError();
         return nullptr;
     }
     return k;
 }
+
+// Share of the pairs (ppm) below which a level's feeding frontier is left to the flag words.
+constexpr int kSweepThinPpm = 2000;
+
+void *sweep_for(int d) {
+    return d == 8 ? (void *)gg::sweep_kernel<8> : d == 6 ? (void *)gg::sweep_kernel<6>
+         : d == 4 ? (void *)gg::sweep_kernel<4> : (void *)gg::sweep_kernel<3>;
+}
+
+// Pairs left (ppm) below which last_rows takes a level.  A share u of the pairs left
+// becomes about u^(d-1) with the level, and a row's 4096 pairs must then rarely (one row
+// in twenty) hold one that is still missing: those cost d^2 gathers, one after the other.
+int sweep_last_ppm(int d) { return d == 8 ? 190000 : d == 6 ? 100000 : d == 4 ? 22000 : 3400; }
 
 void *index_kernel_for(int d) {
     switch (kernel_degree_slot(d)) {
@@ -520,6 +552,8 @@ gg_status ensure_counters(gg_engine *e, int cap, int nb) {
     e->h_bad = reinterpret_cast<int *>(e->h_status + sizeof(Ctl));
     e->d_asym = e->d_bad + 1;
     e->d_wasym = e->d_bad + 2;
+    e->d_redo = e->d_bad + 3;
+    e->h_redo = e->h_bad + 3;
     GG_CK(cudaMalloc(&e->d_vtot, (size_t)nb * 3 * sizeof(unsigned long long)));
     e->d_levels_run = reinterpret_cast<int *>(e->d_status + e->off_levels_run);
     e->h_levels_run = reinterpret_cast<int *>(e->h_status + e->off_levels_run);
@@ -596,6 +630,7 @@ gg_status create_common(gg_engine *e) {
                              "GG_FULL_SKIP_PPM", "GG_SPLIT_PPM", "GG_VPULL", "GG_OWN_SKIP", "GG_WALK_THIRD",
                              "GG_WALK_ALL_MB", "GG_PUSH_PPM", "GG_PUSH_MIN_ITEMS", "GG_NO_GRAPH", "GG_ADJ_SMEM"})
         if (std::getenv(name)) e->direct = false;
+    e->sweep = e->direct && env_int("GG_SWEEP", 1) != 0;
     if (env_int("GG_DIRECT", 1) == 0) e->direct = false;
     e->direct_allowed = e->direct;
     GG_CK(cudaDeviceGetAttribute(&e->sms, cudaDevAttrMultiProcessorCount, e->device));
@@ -852,9 +887,22 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
     if (want_ns) d2h += lv * sizeof(unsigned long long);
     // Walk pass for this evaluation: not with the WVC masks or the distance planes
     // (their per-level bookkeeping lives in the level loop), at most the level cap.
-    const int walk_K = (wvc || (x && (x->planes || within))) ? 0 : std::min(e->walk_K, cap_req);
+    int walk_K = (wvc || (x && (x->planes || within))) ? 0 : std::min(e->walk_K, cap_req);
+    // (one level less where the walk of all batches then covers them: a level costs less
+    // than a walk pass per batch)
+    if (walk_K == 4 && e->walk_auto && walk_all_for(e, 3, nb)) walk_K = 3;
     const int launches = 1 + ((long long)e->rows * e->d > 0 ? 1 : 0) + (walk_K > 0 ? 1 : 0) + (walk_K >= 3 ? 1 : 0);
     void *wall = walk_K > 0 ? walk_all_for(e, walk_K, nb) : nullptr;
+    // sweep_kernel: every vertex a source, in order, and the walk's last level not thin on
+    // a graph whose walks rarely meet (others find out at batch 0 and pay for the attempt,
+    // so one that gave up keeps to bfs_batch_kernel for a while)
+    bool sweep = e->sweep && wall && walk_K == 3 && !x && !want_ns && !extra && e->walk_third && e->walk_own_skip &&
+                 !e->d_inv && e->src_first == 0 && s0 == 0 && ns_all == e->rows &&
+                 (long long)e->d * (e->d - 1) * (e->d - 1) * 1000000ll >= (long long)e->rows * kSweepThinPpm;
+    if (sweep && e->sweep_wait > 0) {
+        --e->sweep_wait;
+        sweep = false;
+    }
 
     // Everything the GPU does for one evaluation, on `q`: status words zeroed,
     // table -> adjacency (checked), one cooperative launch for every source
@@ -864,7 +912,10 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
     auto enqueue = [&](cudaStream_t q, bool timed) -> gg_status {
         if (timed) GG_CK(cudaEventRecord(e->ev0, q));
         // control block, range-check and symmetry words
-        GG_CK(cudaMemsetAsync(e->d_status, 0, sizeof(Ctl) + 3 * sizeof(int), q));   // ctl, bad, asym, wasym
+        // (and, when a walk adds into them before any grid barrier, the levels run and the counts)
+        GG_CK(cudaMemsetAsync(e->d_status, 0,
+                              walk_K > 0 ? e->off_counts + (size_t)nb * stride * sizeof(unsigned long long)
+                                         : sizeof(Ctl) + 4 * sizeof(int), q));   // ctl, bad, asym, wasym, redo
         const long long n = (long long)e->rows * e->d;
         if (e->form == FORM_GRAPH && within) {
             // read in place
@@ -883,8 +934,6 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
         if (want_ns)
             GG_CK(cudaMemsetAsync(e->d_level_ns, 0, lv * sizeof(unsigned long long), q));
         if (walk_K > 0) {
-            // blocks add the walk's level counts before any grid barrier
-            GG_CK(cudaMemsetAsync(e->d_counts, 0, (size_t)nb * stride * sizeof(unsigned long long), q));
             GG_CK(cudaMemsetAsync(e->d_vtot, 0, (size_t)nb * 3 * sizeof(unsigned long long), q));
             // the walk of all batches needs the table's one-way flag first; h2_kernel
             // takes the check along when its warps see whole neighbour rows
@@ -905,9 +954,11 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
             wi.src_first = x && x->inv ? 0 : e->src_first;
             wi.src_begin = s0;
             wi.ns_total = ns_all;
-            wi.S = 128 * e->nC;
+            const int sub = wall ? e->nC / 32 : 1;
+            wi.S = wall ? 4096 : 128 * e->nC;
+            wi.sub = sub;
             wi.div_S = FastDiv((uint32_t)wi.S);
-            wi.nb = nb;
+            wi.nb = nb * sub;
             wi.K = walk_K;
             wi.rows = e->rows;
             wi.d = e->d;
@@ -943,6 +994,38 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
                                                                               (long long)sms * std::max(per_sm, 1)));
             void *wargs[] = {&wi};
             GG_CK(cudaLaunchKernel(wk, dim3(wgrid), dim3(gg::kIndexBlock), wargs, wsmem, q));
+        }
+        if (sweep) {
+            gg::SweepArgs sa{};
+            sa.adj = e->d_adj;
+            sa.bad = e->form == FORM_GRAPH ? e->d_bad : nullptr;
+            sa.oneway = e->d_wasym;
+            sa.vall = e->d_vall;
+            sa.A = e->d_V;
+            sa.B = e->d_F0;
+            sa.ctl = e->d_ctl;
+            sa.expected = (unsigned)e->sms;
+            sa.wait_ns = e->wait_ns;
+            sa.counts = e->d_counts;
+            sa.vtot = e->d_vtot;
+            sa.stride = stride;
+            sa.levels_run = e->d_levels_run;
+            sa.batch_ns = e->d_batch_ns;
+            sa.redo = e->d_redo;
+            sa.rows = e->rows; sa.nC = e->nC; sa.nb = nb; sa.K = walk_K;
+            sa.max_levels = cap_req;
+            sa.thin_ppm = kSweepThinPpm;
+            sa.last_ppm = sweep_last_ppm(e->d);
+            const int per = (e->rows + e->sms - 1) / e->sms;
+            const size_t ssmem = (size_t)per * e->d * sizeof(int32_t);
+            sa.adj_smem_rows = ssmem <= 32u << 10 ? per : 0;   // (no opt-in needed; 65536 rows of 8 take 14 KB)
+            void *sargs[] = {&sa};
+            GG_CK(cudaLaunchCooperativeKernel(sweep_for(e->d), dim3(e->sms), dim3(gg::kSweepBlock), sargs,
+                                              sa.adj_smem_rows ? ssmem : 0, q));
+            if (timed) GG_CK(cudaEventRecord(e->ev1, q));
+            GG_CK(cudaMemcpyAsync(e->h_status, e->d_status, e->off_counts + (size_t)nb * stride * 8,
+                                  cudaMemcpyDeviceToHost, q));
+            return GG_OK;
         }
         BfsArgs a{};
         a.adj = within ? d_table_in : e->d_adj;
@@ -1023,7 +1106,7 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
     // changes the work -- the table pointer, the source range, the level cap,
     // the outputs asked for, reallocated buffers -- captures a new graph.
     const EvalKey key{d_table_in, e->d_status, e->d_V, x ? (const void *)x->inv : nullptr,
-                      x ? (const void *)x->planes : nullptr, s0, ns_all, cap_req, wvc, want_ns};
+                      x ? (const void *)x->planes : nullptr, s0, ns_all, cap_req, wvc, want_ns, sweep};
     e->p_dirty = true;  // until the launch is known to have finished cleanly
     bool replayed = false;
     if (e->use_graph && !extra && !(x && x->no_graph)) {
@@ -1062,6 +1145,16 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
     GG_CK(cudaEventElapsedTime(&ms, e->ev0, e->ev1));
     e->last_ms = ms;
     e->last_launches = launches;
+    if (sweep && *e->h_redo && !*e->h_bad && !e->h_ctl->err) {
+        sweep = false;
+        e->sweep_wait = 63;
+        gg_status es = enqueue(st, true);
+        if (es != GG_OK) return es;
+        GG_CK(cudaStreamSynchronize(st));
+        GG_CK(cudaEventElapsedTime(&ms, e->ev0, e->ev1));
+        e->last_ms += ms;
+        e->last_launches += launches;
+    }
     e->last_batches = nb;
 
     if (e->form == FORM_GRAPH && !within && *e->h_bad)
@@ -1084,6 +1177,7 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
         const unsigned long long *c = e->h_counts + (size_t)b * stride;
         const int run = e->h_levels_run[b];
         int last = 0;
+        // (sweep: a batch's own counts may be negative mod 2^64, their sums are not)
         for (int L = 0; L <= run && L <= cap_req; ++L) {
             R.reached += c[L];
             R.total += (uint64_t)L * c[L];

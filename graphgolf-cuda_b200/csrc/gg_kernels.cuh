@@ -653,29 +653,31 @@ static __device__ __noinline__ unsigned vpull_level(const BfsArgs &a, const int 
     return cnt;
 }
 
-// Dense visited-set pull level without own chunks on 32-chunk rows (a tile is one
-// row; tables without one-way entries): Y[v] = OR of the D neighbours' X rows, every
+// Dense visited-set pull level without own chunks on rows of 32 * parts chunks (a tile is
+// the part of one row; tables without one-way entries): Y[v] = OR of the D neighbours' X rows, every
 // chunk written, the row's flag and not-full words, and this thread's popcount of what
 // it wrote (the level's total, see BfsArgs::walk_asym).  The same result as
 // vpull_level with no_own, in a loop with nothing else in it: the generic tile function
 // measured 3-4 us slower a level on the 65536-row, 8-regular graph.  With `half`, the
 // first D/2 neighbours alone where they already fill the chunk.  Out of line: inlined,
-// it raised the level loop's spills.
-template <int D>
+// it raised the level loop's spills.  ONE: parts == 1 (the division cost 1-2 us a level).
+template <int D, bool ONE>
 static __device__ __noinline__ unsigned dense_rows32(const uint4 *X, uint4 *Y, const int32_t *adj,
-                                                     const unsigned v_base, const unsigned t_hi, uint32_t *fn,
-                                                     uint32_t *nfn, const bool half, unsigned *s_next) {
+                                                     const unsigned v_base, const unsigned parts, const unsigned t_hi,
+                                                     uint32_t *fn, uint32_t *nfn, const bool half, unsigned *s_next) {
     const unsigned lane = threadIdx.x & 31u;
     unsigned cnt = 0u;
     for (;;) {
-        unsigned v = 0u;
-        if (lane == 0) v = atomicAdd(s_next, 1u);
-        v = __shfl_sync(0xffffffffu, v, 0);
-        if (v >= t_hi) break;
+        unsigned t = 0u;
+        if (lane == 0) t = atomicAdd(s_next, 1u);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        if (t >= t_hi) break;
+        const unsigned v = ONE ? t : t / parts, at = ONE ? lane : (t - v * parts) * 32u + lane;
+        const unsigned w = ONE ? 32u : 32u * parts;
         const int32_t *row = adj + (size_t)(v - v_base) * D;
         unsigned tu[D];
 #pragma unroll
-        for (int i = 0; i < D; ++i) tu[i] = (unsigned)row[i] * 32u + lane;
+        for (int i = 0; i < D; ++i) tu[i] = (unsigned)row[i] * w + at;
         uint4 x[D];
         uint4 q;
         if (D >= 8 && half) {
@@ -699,13 +701,13 @@ static __device__ __noinline__ unsigned dense_rows32(const uint4 *X, uint4 *Y, c
 #pragma unroll
             for (int i = 1; i < D; ++i) or_into(q, x[i]);
         }
-        Y[(size_t)v * 32 + lane] = q;
+        Y[(size_t)t * 32 + lane] = q;
         cnt += u4popc(q);
         const unsigned fb = __ballot_sync(0xffffffffu, u4any(q));
         const unsigned nb = __ballot_sync(0xffffffffu, !u4full(q));
         if (lane == 0) {
-            fn[v] = fb;
-            nfn[v] = nb;
+            fn[t] = fb;
+            nfn[t] = nb;
         }
     }
     return cnt;
@@ -896,9 +898,11 @@ struct WalkIndexArgs {
     const int *bad;           // nonzero: the table failed its range check
     int *asym;                // set to 1 when some row u lacks v for an entry u of row v (nullptr: not checked)
     // walk_all_kernel only: the level-K visited rows of every batch and their flag words
-    uint4 *vall;              // [nb][rows * 32]
-    uint32_t *vall_fl;        // [nb][rows]
-    unsigned long long *counts;   // [nb][counts_stride]: levels 1..K added
+    // (nb counts 4096-source parts here, a multiple of `sub`; a batch is `sub` of them)
+    int sub;
+    uint4 *vall;              // [nb / sub][rows][sub][32]
+    uint32_t *vall_fl;        // [nb / sub][rows][sub]
+    unsigned long long *counts;   // [nb / sub][counts_stride]: levels 1..K added
     int counts_stride;
     const int *oneway;        // walk_check_kernel's flag (0: counts from the sources' side), or nullptr
 };
@@ -974,10 +978,12 @@ __device__ __forceinline__ void for_walk_ends(const WalkIndexArgs &a, const int 
 // ends from H2 or the adjacency rows), each classified as (key << 16) | payload with
 // key = batch * K + level - 1 and payload the source's place in its batch, or -1;
 // also the row's one-way check.  NV slots a lane.
+// (DD not a multiple of 4: the level-2 lists do not start at 16-byte boundaries; their
+// ends then come one by one, in the first component of each slot.)
 template <int D>
 struct RowEnds {
-    static constexpr int DD = D * D, Q = DD / 4;           // uint4 per level-2 list
-    static constexpr int U3 = D * Q, S3 = (U3 + 31) / 32;  // uint4 of the level-3 ends, per lane
+    static constexpr int DD = D * D, V = DD % 4 == 0 ? 4 : 1, Q = DD / V;   // slots per level-2 list, V ends each
+    static constexpr int U3 = D * Q, S3 = (U3 + 31) / 32;  // slots of the level-3 ends, per lane
     static constexpr int NV = 1 + 4 * ((Q + 31) / 32) + 4 * S3;
 };
 
@@ -1001,7 +1007,9 @@ __device__ __forceinline__ void row_ends_load(const WalkIndexArgs &a, const int 
     for (int s2 = 0; s2 < (Q + 31) / 32; ++s2) {
         const int i = s2 * 32 + (int)lane;
         r.q2[s2] = make_uint4(0u, 0u, 0u, 0u);
-        if (a.K >= 2 && i < Q)
+        if constexpr (RowEnds<D>::V == 1) {
+            if (a.K >= 2 && i < Q) r.q2[s2].x = (unsigned)__ldg(a.h2 + (size_t)v * DD + i);
+        } else if (a.K >= 2 && i < Q)
             r.q2[s2] = a.h2 ? __ldg(reinterpret_cast<const uint4 *>(a.h2 + (size_t)v * DD) + i)
                             : __ldg(reinterpret_cast<const uint4 *>(a.adj + (size_t)__ldg(arow + i / (D / 4)) * D) +
                                     i % (D / 4));
@@ -1010,16 +1018,18 @@ __device__ __forceinline__ void row_ends_load(const WalkIndexArgs &a, const int 
     for (int s3 = 0; s3 < S3; ++s3) {
         const int i = s3 * 32 + (int)lane;
         r.q3[s3] = make_uint4(0u, 0u, 0u, 0u);
-        if (a.K >= 3 && i < U3)
+        if constexpr (RowEnds<D>::V == 1) {
+            if (a.K >= 3 && i < U3) r.q3[s3].x = (unsigned)__ldg(a.h2 + (size_t)__ldg(arow + i / Q) * DD + i % Q);
+        } else if (a.K >= 3 && i < U3)
             r.q3[s3] = __ldg(reinterpret_cast<const uint4 *>(a.h2 + (size_t)__ldg(arow + i / Q) * DD) + i % Q);
     }
     if (a.asym) {
-        if (a.K >= 2) {
+        if (D % 4 == 0 && a.K >= 2) {
             // the level-2 lists are the neighbours' rows, D / 4 lanes per row
             bool f = (int)lane < Q && ((int)r.q2[0].x == v || (int)r.q2[0].y == v || (int)r.q2[0].z == v ||
                                        (int)r.q2[0].w == v);
             if constexpr (D / 4 == 2) f |= __shfl_xor_sync(0xffffffffu, f, 1) != 0;
-            if ((int)lane < Q && (int)lane % (D / 4) == 0 && !f) *a.asym = 1;
+            if ((int)lane < Q && (int)lane % (D >= 4 ? D / 4 : 1) == 0 && !f) *a.asym = 1;
         } else {
             row_oneway_check(a, v, lane, D);
         }
@@ -1045,17 +1055,17 @@ __device__ __forceinline__ void row_ends_classify(const WalkIndexArgs &a, const 
     for (int s2 = 0; s2 < (Q + 31) / 32; ++s2) {
         const bool ok = a.K >= 2 && s2 * 32 + (int)lane < Q;
         pk[n++] = ok ? classify((int32_t)r.q2[s2].x, 2) : -1;
-        pk[n++] = ok ? classify((int32_t)r.q2[s2].y, 2) : -1;
-        pk[n++] = ok ? classify((int32_t)r.q2[s2].z, 2) : -1;
-        pk[n++] = ok ? classify((int32_t)r.q2[s2].w, 2) : -1;
+        pk[n++] = ok && RowEnds<D>::V == 4 ? classify((int32_t)r.q2[s2].y, 2) : -1;
+        pk[n++] = ok && RowEnds<D>::V == 4 ? classify((int32_t)r.q2[s2].z, 2) : -1;
+        pk[n++] = ok && RowEnds<D>::V == 4 ? classify((int32_t)r.q2[s2].w, 2) : -1;
     }
 #pragma unroll
     for (int s3 = 0; s3 < S3; ++s3) {
         const bool ok = a.K >= 3 && s3 * 32 + (int)lane < U3;
         pk[n++] = ok ? classify((int32_t)r.q3[s3].x, 3) : -1;
-        pk[n++] = ok ? classify((int32_t)r.q3[s3].y, 3) : -1;
-        pk[n++] = ok ? classify((int32_t)r.q3[s3].z, 3) : -1;
-        pk[n++] = ok ? classify((int32_t)r.q3[s3].w, 3) : -1;
+        pk[n++] = ok && RowEnds<D>::V == 4 ? classify((int32_t)r.q3[s3].y, 3) : -1;
+        pk[n++] = ok && RowEnds<D>::V == 4 ? classify((int32_t)r.q3[s3].z, 3) : -1;
+        pk[n++] = ok && RowEnds<D>::V == 4 ? classify((int32_t)r.q3[s3].w, 3) : -1;
     }
 }
 
@@ -1105,7 +1115,7 @@ __device__ __forceinline__ void index_row_regs(const WalkIndexArgs &a, const int
     copy_row_out(a, v, lane, row, total);
 }
 
-// Walk pass of every batch at once (4096-source batches, D = 4 or 8, K <= 3): one warp
+// Walk pass of every batch at once (batches of a multiple of 4096 sources, K <= 3): one warp
 // per row loads the row's walk ends once (row_ends_load) and writes the row's
 // level-K visited row of every batch to vall[b] (padding, the diagonal and every
 // end of that batch), a flag word to vall_fl[b] and the level counts into counts[b].
@@ -1165,7 +1175,8 @@ static __global__ void walk_check_kernel(const int32_t *adj, const int rows, con
     }
 }
 
-template <int D, int K>
+// (ONE: batches of 4096, sub == 1; the divisions by sub cost 0.4 us a batch)
+template <int D, int K, bool ONE>
 __global__ void __launch_bounds__(kIndexBlock, 3) walk_all_kernel(const WalkIndexArgs a) {
     extern __shared__ __align__(16) unsigned char s_walk[];
     __shared__ unsigned long long s_cnt[kIndexMaxKeys];
@@ -1187,9 +1198,16 @@ __global__ void __launch_bounds__(kIndexBlock, 3) walk_all_kernel(const WalkInde
     uint32_t *buf = reinterpret_cast<uint32_t *>(mine);
     int *set = reinterpret_cast<int *>(mine + (mode == 2 ? kWalkAllWide : kWalkAllOrGroup) * 512);
     constexpr int Q = RowEnds<D>::Q, U3 = RowEnds<D>::U3, S3 = RowEnds<D>::S3, NV = RowEnds<D>::NV;
+    auto insert4 = [](int *T, const uint4 &q, const int bits) -> unsigned {   // the ends of a slot
+        unsigned n = set_insert(T, (int)q.x, bits);
+        if constexpr (RowEnds<D>::V == 4)
+            n += set_insert(T, (int)q.y, bits) + set_insert(T, (int)q.z, bits) + set_insert(T, (int)q.w, bits);
+        return n;
+    };
     RowEndsRaw<D> r;
     int pk[NV];
-    const size_t items = (size_t)a.rows * 32u;
+    const unsigned sub = ONE ? 1u : (unsigned)a.sub;               // 4096-source parts of a batch's row
+    const size_t items = (size_t)a.rows * 32u * sub;    // chunks of a batch
     const unsigned long long pad_all = (unsigned long long)nb * (unsigned long long)a.S - (unsigned long long)a.ns_total;
     for (int v = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); v < a.rows;
          v += (int)((gridDim.x * blockDim.x) >> 5)) {
@@ -1215,16 +1233,14 @@ __global__ void __launch_bounds__(kIndexBlock, 3) walk_all_kernel(const WalkInde
 #pragma unroll
                 for (int s2 = 0; s2 < (Q + 31) / 32; ++s2)
                     if (s2 * 32 + (int)lane < Q)
-                        n2 += set_insert(set, (int)r.q2[s2].x, set_bits) + set_insert(set, (int)r.q2[s2].y, set_bits) +
-                              set_insert(set, (int)r.q2[s2].z, set_bits) + set_insert(set, (int)r.q2[s2].w, set_bits);
+                        n2 += insert4(set, r.q2[s2], set_bits);
                 __syncwarp();
             }
             if (top >= 3) {
 #pragma unroll
                 for (int s3 = 0; s3 < S3; ++s3)
                     if (s3 * 32 + (int)lane < U3)
-                        n3 += set_insert(set, (int)r.q3[s3].x, set_bits) + set_insert(set, (int)r.q3[s3].y, set_bits) +
-                              set_insert(set, (int)r.q3[s3].z, set_bits) + set_insert(set, (int)r.q3[s3].w, set_bits);
+                        n3 += insert4(set, r.q3[s3], set_bits);
                 __syncwarp();
             }
         }
@@ -1246,9 +1262,10 @@ __global__ void __launch_bounds__(kIndexBlock, 3) walk_all_kernel(const WalkInde
                     }
                 }
             __syncwarp();
-            uint4 *out = a.vall + (size_t)g0 * items + (size_t)v * 32 + lane;
-            for (int bb = 0; bb < G; ++bb, out += items) {
+            for (int bb = 0; bb < G; ++bb) {
                 const int b = g0 + bb;
+                const unsigned bw = ONE ? (unsigned)b : (unsigned)b / sub, part = (unsigned)b - bw * sub;
+                const size_t tile = (size_t)v * sub + part;
                 const int ns = min(a.S, a.ns_total - b * a.S);
                 uint4 vv = ns < a.S ? pad_mask((int)lane, ns) : u4zero();
                 if (b == bd && (unsigned)(jj_d >> 7) == lane) {
@@ -1277,9 +1294,9 @@ __global__ void __launch_bounds__(kIndexBlock, 3) walk_all_kernel(const WalkInde
                     }
                     flag = u4any(andnot(vv, prev));
                 }
-                *out = vv;
+                a.vall[(size_t)bw * items + tile * 32u + lane] = vv;
                 const unsigned m = __ballot_sync(0xffffffffu, flag);
-                if (lane == 0) a.vall_fl[(size_t)b * a.rows + v] = m;
+                if (lane == 0) a.vall_fl[(size_t)bw * a.rows * sub + tile] = m;
             }
             __syncwarp();
         }
@@ -1303,7 +1320,7 @@ __global__ void __launch_bounds__(kIndexBlock, 3) walk_all_kernel(const WalkInde
     }
     __syncthreads();
     for (int k = (int)threadIdx.x; k < nkeys; k += (int)blockDim.x)
-        if (s_cnt[k]) atomicAdd(a.counts + (size_t)(k / K) * a.counts_stride + (k % K) + 1, s_cnt[k]);
+        if (s_cnt[k]) atomicAdd(a.counts + (size_t)(k / K / sub) * a.counts_stride + (k % K) + 1, s_cnt[k]);
 }
 
 template <int D>
@@ -1996,8 +2013,11 @@ __global__ void __launch_bounds__(kBlock, min_blocks_for(D)) bfs_batch_kernel(co
                 }
                 __syncthreads();
                 if (D > 0 && no_own && !nf_use && a.nC == 32)
-                    cnt = dense_rows32<(D > 0 ? D : 1)>(X, Y, adj, v_base, t_hi, odd ? a.fl1 : a.fl0,
-                                                        odd ? a.nf2 : a.nf, split, &s_next);
+                    cnt = dense_rows32<(D > 0 ? D : 1), true>(X, Y, adj, v_base, 1u, t_hi, odd ? a.fl1 : a.fl0,
+                                                              odd ? a.nf2 : a.nf, split, &s_next);
+                else if (D > 0 && no_own && !nf_use && a.nC % 32 == 0)
+                    cnt = dense_rows32<(D > 0 ? D : 1), false>(X, Y, adj, v_base, (unsigned)a.nC / 32u, t_hi,
+                                                               odd ? a.fl1 : a.fl0, odd ? a.nf2 : a.nf, split, &s_next);
                 else
                     cnt = vpull_level<D>(a, d, adj, v_base, t_lo, t_hi, X, Y,
                                          first ? S.fl_walk : (odd ? a.fl0 : a.fl1), odd ? a.fl1 : a.fl0,

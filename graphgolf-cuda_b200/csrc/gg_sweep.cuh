@@ -1,0 +1,294 @@
+// Levels after the walk of all batches, when every vertex is a source and the table has
+// no one-way entries: sweep_kernel<D>.  bfs_batch_kernel does the same job in general;
+// this one takes the plain case, where each level is a whole dense pull, and ends each
+// batch with last_rows.
+//
+// last_rows (one pass in place of the last two levels).  Distances are symmetric here,
+// so of the pairs the levels before L left over it looks only at those whose vertex is
+// in the source's batch or a later one, and counts the later ones twice: half of the
+// rows on average.  A row's chunk that level L does not fill is finished on the spot
+// from two steps away, V_{L+1}[v] = OR of V_{L-1}[w] over the walks v-u-w (the rows of
+// level L - 1 are all there and nothing overwrites them), so neither level writes rows
+// and no barrier lies between them.  All batches take it at the same level, the one
+// batch 0 finds (else pairs would be counted twice or not at all), and the counts add
+// up over the batches only: a batch's own may be off, or "negative", mod 2^64.
+//
+// Measured, whole evaluations: n = 65536, d = 8, 16 batches of three levels and last_rows,
+// 1936 -> 1645 us (a batch 120 -> 82: last_rows 8-13 us falling with the rows left, in
+// place of levels of 19 and 6 us with a barrier each; four barriers of 592 blocks and
+// their tails -> three of 148); n = 30011, d = 6, irregular, 772 -> 515 us (of which the
+// walk of all batches at degree 6, on batches of two 4096-source parts, 772 -> 590).
+// A level is bound by L2: 268 MB gathered in 22 us.
+//
+// When something does not fit -- a one-way entry, a thin level (flag words would be
+// better), the level cap, a pair further than L + 1 -- *redo is set and the host runs
+// bfs_batch_kernel instead.
+#pragma once
+#include "gg_kernels.cuh"
+
+namespace gg {
+
+constexpr int kSweepBlock = 1024;   // one block per SM: a grid barrier takes 148 arrivals, not 592
+
+struct SweepArgs {
+    const int32_t *adj;
+    const int *bad, *oneway;
+    const uint4 *vall;        // [nb][rows * nC]: level-K rows (walk_all_kernel)
+    uint4 *A, *B;             // [rows * nC] each: the levels after it in turn
+    Ctl *ctl;
+    unsigned expected;
+    long long wait_ns;
+    unsigned long long *counts;   // [nb][stride], levels 1..K from the walk, zeros above
+    unsigned long long *vtot;     // [nb][3], zeros
+    int stride;
+    int *levels_run;              // [nb], zeros
+    unsigned long long *batch_ns;
+    int *redo;
+    int rows, nC, nb, K, max_levels;
+    int thin_ppm;             // below this share of the pairs a feeding frontier is thin
+    int last_ppm;             // last_rows once fewer of the pairs than this are left
+    int adj_smem_rows;
+};
+
+// A batch's state in shared memory (thread 0 writes it between block barriers).
+struct SweepState {
+    unsigned long long reached, c_prev, pairs;
+    int last;                 // level at which every batch takes last_rows (0: none yet)
+    int act;                  // next step: 0 level, 1 last_rows, 2 batch done, 3 give up
+};
+
+// Adjacency row v of the table, the same in every lane.
+template <int D>
+__device__ __forceinline__ void sweep_row(const int32_t *adj, const unsigned v, unsigned (&u)[D]) {
+    if constexpr (D % 4 == 0) {
+        const int4 *p = reinterpret_cast<const int4 *>(adj + (size_t)v * D);
+#pragma unroll
+        for (int i = 0; i < D / 4; ++i) {
+            const int4 x = __ldg(p + i);
+            u[4 * i] = (unsigned)x.x; u[4 * i + 1] = (unsigned)x.y;
+            u[4 * i + 2] = (unsigned)x.z; u[4 * i + 3] = (unsigned)x.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < D; ++i) u[i] = (unsigned)__ldg(adj + (size_t)v * D + i);
+    }
+}
+
+// The pairs of chunk `at` of row v that level L (rows q so far) misses: how many, and
+// whether two steps from V_{L-1} reach them all.
+template <int D>
+static __device__ __noinline__ unsigned sweep_tail(const uint4 *X, const int32_t *adj, const unsigned v,
+                                                   const unsigned nC, const unsigned at, uint4 q, int *redo) {
+    const unsigned miss = 128u - u4popc(q);
+    for (int i = 0; i < D && !u4full(q); ++i) {
+        const unsigned u = (unsigned)__ldg(adj + (size_t)v * D + i);
+        unsigned w[D];
+        sweep_row<D>(adj, u, w);
+        uint4 x[D];
+#pragma unroll
+        for (int j = 0; j < D; ++j) x[j] = __ldcg(X + (w[j] * nC + at));
+#pragma unroll
+        for (int j = 0; j < D; ++j) or_into(q, x[j]);
+    }
+    if (!u4full(q)) *redo = 1;
+    return miss;
+}
+
+template <int D>
+static __device__ __noinline__ unsigned last_rows(const SweepArgs &a, const uint4 *X, const int b, const int L) {
+    constexpr int H = D >= 8 ? D / 2 : D;   // neighbours gathered first: half usually fill the chunk
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned warps = gridDim.x * (kSweepBlock / 32), gw = blockIdx.x * (kSweepBlock / 32) + (threadIdx.x >> 5);
+    const unsigned nC = (unsigned)a.nC, parts = nC / 32u, S = 128u * nC;
+    const unsigned v0 = (unsigned)b * S, t_end = (unsigned)a.rows * parts;
+    unsigned cnt = 0u;
+    constexpr int U = H <= 4 ? 2 : 1;       // tiles a round: at most 8 gathers in flight, as registers allow
+    for (unsigned t0 = v0 * parts + gw; t0 < t_end; t0 += (unsigned)U * warps) {
+        unsigned v[U], at[U], tu[U][D];
+        bool ok[U];
+        uint4 q[U], x[U][H];
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const unsigned t = t0 + (unsigned)k * warps;
+            ok[k] = t < t_end;
+            v[k] = ok[k] ? (parts == 1u ? t : t / parts) : v0;
+            at[k] = ok[k] ? (t - v[k] * parts) * 32u + lane : lane;
+            sweep_row<D>(a.adj, v[k], tu[k]);
+#pragma unroll
+            for (int i = 0; i < D; ++i) tu[k][i] = tu[k][i] * nC + at[k];
+        }
+#pragma unroll
+        for (int k = 0; k < U; ++k)
+#pragma unroll
+            for (int i = 0; i < H; ++i) x[k][i] = __ldcg(X + tu[k][i]);
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            q[k] = x[k][0];
+#pragma unroll
+            for (int i = 1; i < H; ++i) or_into(q[k], x[k][i]);
+            if constexpr (H < D)
+                if (!u4full(q[k])) {
+                    uint4 y[D - H];
+#pragma unroll
+                    for (int i = H; i < D; ++i) y[i - H] = __ldcg(X + tu[k][i]);
+#pragma unroll
+                    for (int i = H; i < D; ++i) or_into(q[k], y[i - H]);
+                }
+            if (ok[k] && !u4full(q[k])) {
+                const unsigned m = sweep_tail<D>(X, a.adj, v[k], nC, at[k], q[k], a.redo);
+                const unsigned bv = v[k] / S;
+                cnt += bv == (unsigned)b ? m : 2u * m;
+                // level L + 1 is not empty for either batch of these pairs
+                atomicMax(a.levels_run + b, L + 1);
+                atomicMax(a.levels_run + bv, L + 1);
+            }
+        }
+    }
+    return cnt;
+}
+
+// One dense level on the block's tiles [s_next, t_hi): Y[v] = OR of the neighbours' X
+// rows (without one-way entries V_{L-1}[v] lies within them for L >= 2), and this
+// thread's popcount of what it wrote.
+template <int D, bool ONE>
+static __device__ __noinline__ unsigned sweep_rows(const uint4 *X, uint4 *Y, const int32_t *adj, const unsigned v_base,
+                                                   const unsigned parts, const unsigned t_hi, unsigned *s_next) {
+    const unsigned lane = threadIdx.x & 31u;
+    unsigned cnt = 0u;
+    for (;;) {
+        unsigned t = 0u;
+        if (lane == 0) t = atomicAdd(s_next, 1u);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        if (t >= t_hi) break;
+        const unsigned v = ONE ? t : t / parts, at = ONE ? lane : (t - v * parts) * 32u + lane;
+        const unsigned w = ONE ? 32u : 32u * parts;
+        const int32_t *row = adj + (size_t)(v - v_base) * D;
+        unsigned tu[D];
+#pragma unroll
+        for (int i = 0; i < D; ++i) tu[i] = (unsigned)row[i] * w + at;
+        uint4 x[D];
+#pragma unroll
+        for (int i = 0; i < D; ++i) x[i] = __ldcg(X + tu[i]);
+        uint4 q = x[0];
+#pragma unroll
+        for (int i = 1; i < D; ++i) or_into(q, x[i]);
+        Y[(size_t)t * 32 + lane] = q;
+        cnt += u4popc(q);
+    }
+    return cnt;
+}
+
+// What comes next in batch b, whose levels below L are done (thread 0).
+__device__ __forceinline__ void sweep_next(const SweepArgs &a, SweepState &S, const int b, const int L) {
+    const unsigned long long left = S.pairs - S.reached;
+    if (left == 0ull) {
+        if (blockIdx.x == 0) atomicMax(a.levels_run + b, L - 1);
+        S.act = 2;
+        return;
+    }
+    if (b == 0 && S.last == 0 && L >= 2 && left * 1000000ull < S.pairs * (unsigned long long)a.last_ppm) S.last = L;
+    if (L == S.last) {
+        S.act = L + 1 <= a.max_levels ? 1 : 3;
+    } else {
+        const bool thin = S.c_prev * 1000000ull < S.pairs * (unsigned long long)a.thin_ppm;
+        S.act = thin || L > a.max_levels ? 3 : 0;
+    }
+}
+
+template <int D>
+__global__ void __launch_bounds__(kSweepBlock, 1) sweep_kernel(const __grid_constant__ SweepArgs a) {
+    extern __shared__ int32_t s_adj[];
+    __shared__ SweepState S;
+    __shared__ unsigned s_next;
+    __shared__ unsigned long long s_sum;
+    if (a.bad && *a.bad) return;   // uniform across the grid, as is the next
+    if (ld_acquire_i(a.oneway) != 0) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) *a.redo = 1;
+        return;
+    }
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned parts = (unsigned)a.nC / 32u, items = (unsigned)a.rows * (unsigned)a.nC;
+    const unsigned v_lo = (unsigned)((unsigned long long)a.rows * blockIdx.x / gridDim.x);
+    const unsigned v_hi = (unsigned)((unsigned long long)a.rows * (blockIdx.x + 1) / gridDim.x);
+    const unsigned t_lo = v_lo * parts, t_hi = v_hi * parts;
+    const bool keep = v_hi - v_lo <= (unsigned)a.adj_smem_rows;   // the block's rows of the table stay in shared memory
+    if (keep)
+        for (unsigned k = threadIdx.x; k < (v_hi - v_lo) * D; k += blockDim.x) s_adj[k] = __ldg(a.adj + (size_t)v_lo * D + k);
+    const int32_t *adj = keep ? s_adj : a.adj;
+    const unsigned v_base = keep ? v_lo : 0u;
+    unsigned epoch = 0u;
+    bool odd = false;              // which of A and B the next level writes
+    if (threadIdx.x == 0) S.last = 0;
+    for (int b = 0; b < a.nb; ++b) {
+        unsigned long long *counts = a.counts + (size_t)b * (size_t)a.stride;
+        const int ns = min(128 * a.nC, a.rows - b * 128 * a.nC);
+        const unsigned long long pad = (unsigned long long)a.rows * (unsigned long long)(128 * a.nC - ns);
+        int L = a.K + 1;
+        if (threadIdx.x == 0) {
+            if (blockIdx.x == 0) {
+                a.batch_ns[2 * b] = gtimer();
+                counts[0] = (unsigned long long)ns;
+            }
+            S.pairs = (unsigned long long)ns * (unsigned long long)a.rows;
+            S.reached = (unsigned long long)ns;
+            S.c_prev = 0ull;
+            int k = 1;
+            for (; k <= a.K && S.reached < S.pairs; ++k) {
+                S.c_prev = ld_relaxed_u64(counts + k);
+                S.reached += S.c_prev;
+            }
+            sweep_next(a, S, b, S.reached == S.pairs ? k : a.K + 1);
+        }
+        __syncthreads();
+        const uint4 *X = a.vall + (size_t)b * items;
+        for (; S.act == 0; ++L) {
+            uint4 *Y = odd ? a.B : a.A;
+            if (threadIdx.x == 0) { s_next = t_lo; s_sum = 0ull; }
+            __syncthreads();
+            const unsigned cnt = parts == 1u ? sweep_rows<D, true>(X, Y, adj, v_base, 1u, t_hi, &s_next)
+                                             : sweep_rows<D, false>(X, Y, adj, v_base, parts, t_hi, &s_next);
+            const unsigned wsum = __reduce_add_sync(0xffffffffu, cnt);
+            if (lane == 0) atomicAdd(&s_sum, (unsigned long long)wsum);
+            __syncthreads();
+            unsigned long long *vt = a.vtot + 3 * (size_t)b;
+            if (threadIdx.x == 0) {
+                atomicAdd(vt + L % 3, s_sum);
+                if (blockIdx.x == 0) vt[(L + 1) % 3] = 0ull;   // read last after level L - 2
+            }
+            unsigned long long total = 0ull;
+            if (!grid_sync_value(a.ctl, a.expected, a.wait_ns, L, epoch, vt + L % 3, total)) return;
+            if (threadIdx.x == 0) {
+                const unsigned long long cL = total - pad - S.reached;
+                if (blockIdx.x == 0) counts[L] = cL;
+                S.reached += cL;
+                S.c_prev = cL;
+                sweep_next(a, S, b, L + 1);
+            }
+            __syncthreads();
+            X = Y;
+            odd = !odd;
+        }
+        if (S.act == 3) {
+            if (blockIdx.x == 0 && threadIdx.x == 0) *a.redo = 1;
+            return;
+        }
+        if (S.act == 1) {
+            // No barrier before the next batch: its first level writes the other buffer,
+            // and the second one only after the barrier between them.
+            if (blockIdx.x == 0 && threadIdx.x == 0) {
+                atomicMax(a.levels_run + b, L);
+                atomicAdd(counts + L, S.pairs - S.reached);
+            }
+            const unsigned cnt = last_rows<D>(a, X, b, L);
+            const unsigned m = __reduce_add_sync(0xffffffffu, cnt);
+            if (lane == 0 && m) {
+                atomicAdd(counts + L, 0ull - (unsigned long long)m);
+                atomicAdd(counts + L + 1, (unsigned long long)m);
+            }
+        }
+        if (blockIdx.x == 0 && threadIdx.x == 0) a.batch_ns[2 * b + 1] = gtimer();
+        __syncthreads();   // S is rewritten for the next batch
+    }
+}
+
+}  // namespace gg

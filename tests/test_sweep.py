@@ -1,0 +1,89 @@
+"""The levels after the walk of all batches in their plain case (csrc/gg_sweep.cuh) and the
+walk itself at degrees 3, 4, 6 and 8 on batches of one or more 4096-source parts: every
+result field against the oracle and against the general level loop (GG_SWEEP=0)."""
+import numpy as np
+import pytest
+
+import graphgolf as G
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+KEYS = ("total", "reached", "pairs", "levels", "capped", "connected", "n_sources", "level_steps")
+
+
+def both(monkeypatch, n, d, batch, calls):
+    out = []
+    for sweep in ("0", "1"):
+        monkeypatch.setenv("GG_SWEEP", sweep)
+        e = G.cudaASPLgraph(n, d)
+        if batch:
+            e.set_batch_sources(batch)
+        out.append([c(e) for c in calls for _ in range(2)])
+        e.close()
+    for want, got in zip(*out):
+        assert all(got[k] == want[k] for k in KEYS)
+        assert np.array_equal(got["level_counts"], want["level_counts"])
+    return out[1][0]
+
+
+def full(adj, cap=40):
+    return lambda e: e.eval(adj, max_levels=cap, level_counts=True)
+
+
+def check_oracle(r, adj):
+    o = O.bfs_pull(adj, np.arange(len(adj)))
+    assert (r["total"], r["reached"], r["levels"]) == (o.total(), int(o.reached.sum()), o.levels)
+
+
+@pytest.mark.parametrize("n,d,batch", [(5000, 3, 4096), (4098, 8, 4096), (8192, 8, 4096), (8193, 8, 8192), (12290, 4, 4096),
+                                       (12289, 6, 8192), (20002, 8, 8192), (20002, 6, 12288), (30011, 6, 0)])
+def test_sweep_equals_the_level_loop(n, d, batch, monkeypatch):
+    adj = G.random_regular(n if n * d % 2 == 0 else n + 1, d, 7)
+    r = both(monkeypatch, len(adj), d, batch, [full(adj)])
+    if n <= 13000:
+        check_oracle(r, adj)
+
+
+@pytest.mark.parametrize("cap", [1, 3, 4, 5, 6, 7])
+def test_sweep_under_a_level_cap(cap, monkeypatch):
+    adj = G.random_regular(9000, 8, 2)
+    both(monkeypatch, 9000, 8, 4096, [full(adj, cap), full(adj)])
+
+
+@pytest.mark.parametrize("what", ["padded", "tail", "ring", "halves", "one-way", "alone", "close"])
+def test_sweep_gives_up_where_it_must(what, monkeypatch):
+    n, d = 9000, 8
+    adj = G.random_regular(n, d, 4)
+    if what == "padded":          # self-loops in place of edges
+        for v in range(0, n, 50):
+            u = int(adj[v, 3])
+            if u != v:
+                adj[u, np.nonzero(adj[u] == v)[0][0]] = u
+                adj[v, 3] = v
+    elif what == "tail":          # a path of 5 vertices hanging off a random graph
+        adj = np.concatenate([adj, np.arange(n, n + 5, dtype=np.int32)[:, None].repeat(d, 1)])
+        u = int(adj[0, 0])
+        adj[0, 0], adj[u, np.nonzero(adj[u] == 0)[0][0]] = n, u
+        adj[n, 0] = 0
+        for k in range(4):
+            adj[n + k, 1], adj[n + k + 1, 0] = n + k + 1, n + k
+        n += 5
+    elif what == "ring":          # thin frontiers throughout
+        adj = ((np.arange(n)[:, None] + np.array([-4, -3, -2, -1, 1, 2, 3, 4])) % n).astype(np.int32)
+    elif what == "halves":
+        half = G.random_regular(n // 2, d, 5)
+        adj = np.concatenate([half, half + n // 2]).astype(np.int32)
+    elif what == "one-way":
+        adj[17, 2] = (int(adj[17, 2]) + 11) % n
+    elif what == "alone":         # a vertex with no neighbour
+        for u in set(adj[8999].tolist()):
+            adj[u][adj[u] == 8999] = u
+        adj[8999] = 8999
+    else:                         # everything within the walk: no level left
+        n, d = 4160, 8
+        adj = G.random_regular(n, d, 4)
+    adj = np.ascontiguousarray(adj, dtype=np.int32)
+    r = both(monkeypatch, n, d, 4096, [full(adj, 1200)])
+    if what != "ring":
+        check_oracle(r, adj)
