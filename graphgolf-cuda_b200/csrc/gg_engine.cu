@@ -327,6 +327,68 @@ int walk_levels(gg_engine *e) {
     return K;
 }
 
+// Share of the pairs (ppm) below which a level's feeding frontier is left to the flag words.
+constexpr int kSweepThinPpm = 2000;
+
+// Degrees 3 to 8 walk four steps, 9 to 16 three: at most 4096 walk ends a row.
+constexpr int sweep_K(int d) { return d <= 8 ? 4 : 3; }
+struct SweepKernels { void *ball, *sweep; };
+template <int D = 3>
+SweepKernels sweep_for(int d) {
+    if constexpr (D > 16) {
+        return {nullptr, nullptr};
+    } else {
+        if (d == D) return {(void *)gg::ball_kernel<D, sweep_K(D)>, (void *)gg::sweep_kernel<D>};
+        return sweep_for<D + 1>(d);
+    }
+}
+
+// Pairs left (ppm) below which last_rows takes a level.  A share u of the pairs left
+// becomes about u^(d-1) with the level, and a row's 4096 pairs must then rarely (one row
+// in twenty) hold one that is still missing: those cost d^2 gathers, one after the other.
+int sweep_last_ppm(int d) { return (int)(1e6 * std::min(0.2, std::pow(1.2e-5, 1.0 / (d - 1)))); }
+
+// Room for the rows of every batch (walk_all_kernel, ball_kernel), grown as needed.
+bool vall_room(gg_engine *e, int nb) {
+    const size_t bytes = (size_t)nb * e->items * sizeof(uint4);
+    const size_t fbytes = (size_t)nb * ((e->items + 31) / 32) * sizeof(uint32_t);
+    if ((long long)(bytes >> 20) > e->walk_all_mb) return false;
+    if ((size_t)nb <= e->vall_batches) return true;
+    invalidate_graph(e);
+    cudaFree(e->d_vall); cudaFree(e->d_vall_fl);
+    e->d_vall = nullptr;
+    e->d_vall_fl = nullptr;
+    e->vall_batches = 0;
+    if (cudaMalloc(&e->d_vall, bytes) != cudaSuccess || cudaMalloc(&e->d_vall_fl, fbytes) != cudaSuccess) {
+        cudaFree(e->d_vall); cudaFree(e->d_vall_fl);
+        e->d_vall = nullptr;
+        e->d_vall_fl = nullptr;
+        (void)cudaGetLastError();
+        return false;
+    }
+    e->vall_batches = (size_t)nb;
+    return true;
+}
+
+// Shared memory of a ball_kernel block.
+size_t ball_smem(const gg_engine *e, int nb) {
+    return (size_t)(gg::kBallBlock / 32) * gg::ball_warp_bytes(e->d, sweep_K(e->d), nb * (e->nC / 32));
+}
+
+// Whether sweep_kernel can take evaluations of every vertex in order, by size: whole
+// 4096-source parts, two ball_kernel blocks an SM, and the walk's last level not thin on a
+// graph whose walks rarely meet (others find out at batch 0).
+bool sweep_fits(const gg_engine *e) {
+    if (!e->sweep || e->d < 3 || e->d > 16 || e->nC % 32 != 0 || (int)e->reps.size() != e->rows || e->d_inv ||
+        e->src_first != 0)
+        return false;
+    const int K = sweep_K(e->d), nb = (e->rows + e->batch_bits - 1) / e->batch_bits;
+    if (nb * K > gg::kBallCounts || 2 * (ball_smem(e, nb) + 4096) > (size_t)e->smem_optin) return false;
+    double last = e->d;
+    for (int k = 1; k < K; ++k) last *= e->d - 1;
+    return last * 1e6 >= (double)e->rows * kSweepThinPpm;
+}
+
 template <int D, bool ONE>
 void *walk_all_of(int K) {
     return K == 1 ? (void *)gg::walk_all_kernel<D, 1, ONE> : K == 2 ? (void *)gg::walk_all_kernel<D, 2, ONE>
@@ -342,24 +404,7 @@ void *walk_all_for(gg_engine *e, int K, int nb) {
     if (!e->walk_vpull || e->nC % 32 != 0 || K < 1 || K > 3 || nb * (e->nC / 32) * K > gg::kIndexMaxKeys) return nullptr;
     if (e->d != 3 && e->d != 4 && e->d != 6 && e->d != 8) return nullptr;
     if (K < 3 && e->d % 4 != 0) return nullptr;
-    const size_t bytes = (size_t)nb * e->items * sizeof(uint4);
-    const size_t fbytes = (size_t)nb * ((e->items + 31) / 32) * sizeof(uint32_t);
-    if ((long long)(bytes >> 20) > e->walk_all_mb) return nullptr;
-    if ((size_t)nb > e->vall_batches) {
-        invalidate_graph(e);
-        cudaFree(e->d_vall); cudaFree(e->d_vall_fl);
-        e->d_vall = nullptr;
-        e->d_vall_fl = nullptr;
-        e->vall_batches = 0;
-        if (cudaMalloc(&e->d_vall, bytes) != cudaSuccess || cudaMalloc(&e->d_vall_fl, fbytes) != cudaSuccess) {
-            cudaFree(e->d_vall); cudaFree(e->d_vall_fl);
-            e->d_vall = nullptr;
-            e->d_vall_fl = nullptr;
-            (void)cudaGetLastError();
-            return nullptr;
-        }
-        e->vall_batches = (size_t)nb;
-    }
+    if (!vall_room(e, nb)) return nullptr;
     void *k = nullptr;
     if (e->nC == 32)
         k = e->d == 8 ? walk_all_of<8, true>(K) : e->d == 4 ? walk_all_of<4, true>(K)
@@ -373,19 +418,6 @@ void *walk_all_for(gg_engine *e, int K, int nb) {
     }
     return k;
 }
-
-// Share of the pairs (ppm) below which a level's feeding frontier is left to the flag words.
-constexpr int kSweepThinPpm = 2000;
-
-void *sweep_for(int d) {
-    return d == 8 ? (void *)gg::sweep_kernel<8> : d == 6 ? (void *)gg::sweep_kernel<6>
-         : d == 4 ? (void *)gg::sweep_kernel<4> : (void *)gg::sweep_kernel<3>;
-}
-
-// Pairs left (ppm) below which last_rows takes a level.  A share u of the pairs left
-// becomes about u^(d-1) with the level, and a row's 4096 pairs must then rarely (one row
-// in twenty) hold one that is still missing: those cost d^2 gathers, one after the other.
-int sweep_last_ppm(int d) { return d == 8 ? 190000 : d == 6 ? 100000 : d == 4 ? 22000 : 3400; }
 
 void *index_kernel_for(int d) {
     switch (kernel_degree_slot(d)) {
@@ -471,7 +503,7 @@ gg_status plan(gg_engine *e, int want_bits) {
         e->walk_rpg = 32 / g;
         walk_bytes = (size_t)(gg::kBlock / 32) * gg::walk_smem_per_warp(e->nC);
     }
-    const size_t h2_need = e->walk_K >= 3 ? (size_t)e->rows * e->d * e->d : 0;
+    const size_t h2_need = e->walk_K >= 3 || sweep_fits(e) ? (size_t)e->rows * e->d * e->d : 0;
     if (h2_need != e->h2_elems) {
         cudaFree(e->d_h2);
         e->d_h2 = nullptr;
@@ -891,18 +923,17 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
     // (one level less where the walk of all batches then covers them: a level costs less
     // than a walk pass per batch)
     if (walk_K == 4 && e->walk_auto && walk_all_for(e, 3, nb)) walk_K = 3;
-    const int launches = 1 + ((long long)e->rows * e->d > 0 ? 1 : 0) + (walk_K > 0 ? 1 : 0) + (walk_K >= 3 ? 1 : 0);
+    const int launches_plain = 1 + ((long long)e->rows * e->d > 0 ? 1 : 0) + (walk_K > 0 ? 1 : 0) + (walk_K >= 3 ? 1 : 0);
     void *wall = walk_K > 0 ? walk_all_for(e, walk_K, nb) : nullptr;
-    // sweep_kernel: every vertex a source, in order, and the walk's last level not thin on
-    // a graph whose walks rarely meet (others find out at batch 0 and pay for the attempt,
-    // so one that gave up keeps to bfs_batch_kernel for a while)
-    bool sweep = e->sweep && wall && walk_K == 3 && !x && !want_ns && !extra && e->walk_third && e->walk_own_skip &&
-                 !e->d_inv && e->src_first == 0 && s0 == 0 && ns_all == e->rows &&
-                 (long long)e->d * (e->d - 1) * (e->d - 1) * 1000000ll >= (long long)e->rows * kSweepThinPpm;
+    // sweep_kernel.  A graph that it gave up on pays for the attempt and keeps to
+    // bfs_batch_kernel for a while.
+    bool sweep = !x && !wvc && !want_ns && !extra && s0 == 0 && ns_all == e->rows && sweep_fits(e) &&
+                 sweep_K(e->d) <= cap_req && e->h2_elems && vall_room(e, nb);
     if (sweep && e->sweep_wait > 0) {
         --e->sweep_wait;
         sweep = false;
     }
+    const int launches = sweep ? 4 : launches_plain;
 
     // Everything the GPU does for one evaluation, on `q`: status words zeroed,
     // table -> adjacency (checked), one cooperative launch for every source
@@ -914,7 +945,7 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
         // control block, range-check and symmetry words
         // (and, when a walk adds into them before any grid barrier, the levels run and the counts)
         GG_CK(cudaMemsetAsync(e->d_status, 0,
-                              walk_K > 0 ? e->off_counts + (size_t)nb * stride * sizeof(unsigned long long)
+                              sweep || walk_K > 0 ? e->off_counts + (size_t)nb * stride * sizeof(unsigned long long)
                                          : sizeof(Ctl) + 4 * sizeof(int), q));   // ctl, bad, asym, wasym, redo
         const long long n = (long long)e->rows * e->d;
         if (e->form == FORM_GRAPH && within) {
@@ -933,6 +964,71 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
         }
         if (want_ns)
             GG_CK(cudaMemsetAsync(e->d_level_ns, 0, lv * sizeof(unsigned long long), q));
+        if (sweep) {
+            const int K = sweep_K(e->d);
+            const SweepKernels k = sweep_for(e->d);
+            GG_CK(cudaMemsetAsync(e->d_vtot, 0, (size_t)nb * 3 * sizeof(unsigned long long), q));
+            // the level-2 lists, and with them (whole neighbour rows in a warp) the one-way check
+            const long long nh = n * e->d;
+            const int qd = e->d / 4;
+            const bool h2_checks = e->d % 4 == 0 && (qd & (qd - 1)) == 0 && (nh / 4) % 32 == 0;
+            gg::h2_kernel<<<(int)std::min<long long>((nh + 255) / 256, 8192), 256, 0, q>>>(
+                e->d_adj, e->d_h2, e->rows, e->d, e->form == FORM_GRAPH ? e->d_bad : nullptr,
+                h2_checks ? e->d_wasym : nullptr);
+            GG_CK(cudaGetLastError());
+            if (!h2_checks) {
+                gg::walk_check_kernel<<<(int)std::min<long long>((n + 255) / 256, 8192), 256, 0, q>>>(
+                    e->d_adj, e->rows, e->d, e->d_wasym, e->form == FORM_GRAPH ? e->d_bad : nullptr);
+                GG_CK(cudaGetLastError());
+            }
+            gg::BallArgs ba{};
+            ba.adj = e->d_adj;
+            ba.h2 = e->d_h2;
+            ba.bad = e->form == FORM_GRAPH ? e->d_bad : nullptr;
+            ba.oneway = e->d_wasym;
+            ba.vall = e->d_vall;
+            ba.counts = e->d_counts;
+            ba.stride = stride;
+            ba.rows = e->rows; ba.nC = e->nC; ba.nb = nb;
+            const size_t bsmem = ball_smem(e, nb);
+            int per_sm = 0;
+            GG_CK(cudaFuncSetAttribute(k.ball, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem));
+            GG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.ball, gg::kBallBlock, bsmem));
+            const int warps = gg::kBallBlock / 32;
+            const int bgrid = std::min((e->rows + warps - 1) / warps, e->sms * std::max(per_sm, 1));
+            void *bargs[] = {&ba};
+            GG_CK(cudaLaunchKernel(k.ball, dim3(bgrid), dim3(gg::kBallBlock), bargs, bsmem, q));
+            gg::SweepArgs sa{};
+            sa.adj = e->d_adj;
+            sa.bad = ba.bad;
+            sa.oneway = e->d_wasym;
+            sa.vall = e->d_vall;
+            sa.A = e->d_V;
+            sa.B = e->d_F0;
+            sa.ctl = e->d_ctl;
+            sa.expected = (unsigned)e->sms;
+            sa.wait_ns = e->wait_ns;
+            sa.counts = e->d_counts;
+            sa.vtot = e->d_vtot;
+            sa.stride = stride;
+            sa.levels_run = e->d_levels_run;
+            sa.batch_ns = e->d_batch_ns;
+            sa.redo = e->d_redo;
+            sa.rows = e->rows; sa.nC = e->nC; sa.nb = nb; sa.K = K;
+            sa.max_levels = cap_req;
+            sa.thin_ppm = kSweepThinPpm;
+            sa.last_ppm = sweep_last_ppm(e->d);
+            const int per = (e->rows + e->sms - 1) / e->sms;
+            const size_t ssmem = (size_t)per * e->d * sizeof(int32_t);
+            sa.adj_smem_rows = ssmem <= 32u << 10 ? per : 0;   // (no opt-in needed; 65536 rows of 8 take 14 KB)
+            void *sargs[] = {&sa};
+            GG_CK(cudaLaunchCooperativeKernel(k.sweep, dim3(e->sms), dim3(gg::kSweepBlock), sargs,
+                                              sa.adj_smem_rows ? ssmem : 0, q));
+            if (timed) GG_CK(cudaEventRecord(e->ev1, q));
+            GG_CK(cudaMemcpyAsync(e->h_status, e->d_status, e->off_counts + (size_t)nb * stride * 8,
+                                  cudaMemcpyDeviceToHost, q));
+            return GG_OK;
+        }
         if (walk_K > 0) {
             GG_CK(cudaMemsetAsync(e->d_vtot, 0, (size_t)nb * 3 * sizeof(unsigned long long), q));
             // the walk of all batches needs the table's one-way flag first; h2_kernel
@@ -994,38 +1090,6 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
                                                                               (long long)sms * std::max(per_sm, 1)));
             void *wargs[] = {&wi};
             GG_CK(cudaLaunchKernel(wk, dim3(wgrid), dim3(gg::kIndexBlock), wargs, wsmem, q));
-        }
-        if (sweep) {
-            gg::SweepArgs sa{};
-            sa.adj = e->d_adj;
-            sa.bad = e->form == FORM_GRAPH ? e->d_bad : nullptr;
-            sa.oneway = e->d_wasym;
-            sa.vall = e->d_vall;
-            sa.A = e->d_V;
-            sa.B = e->d_F0;
-            sa.ctl = e->d_ctl;
-            sa.expected = (unsigned)e->sms;
-            sa.wait_ns = e->wait_ns;
-            sa.counts = e->d_counts;
-            sa.vtot = e->d_vtot;
-            sa.stride = stride;
-            sa.levels_run = e->d_levels_run;
-            sa.batch_ns = e->d_batch_ns;
-            sa.redo = e->d_redo;
-            sa.rows = e->rows; sa.nC = e->nC; sa.nb = nb; sa.K = walk_K;
-            sa.max_levels = cap_req;
-            sa.thin_ppm = kSweepThinPpm;
-            sa.last_ppm = sweep_last_ppm(e->d);
-            const int per = (e->rows + e->sms - 1) / e->sms;
-            const size_t ssmem = (size_t)per * e->d * sizeof(int32_t);
-            sa.adj_smem_rows = ssmem <= 32u << 10 ? per : 0;   // (no opt-in needed; 65536 rows of 8 take 14 KB)
-            void *sargs[] = {&sa};
-            GG_CK(cudaLaunchCooperativeKernel(sweep_for(e->d), dim3(e->sms), dim3(gg::kSweepBlock), sargs,
-                                              sa.adj_smem_rows ? ssmem : 0, q));
-            if (timed) GG_CK(cudaEventRecord(e->ev1, q));
-            GG_CK(cudaMemcpyAsync(e->h_status, e->d_status, e->off_counts + (size_t)nb * stride * 8,
-                                  cudaMemcpyDeviceToHost, q));
-            return GG_OK;
         }
         BfsArgs a{};
         a.adj = within ? d_table_in : e->d_adj;
@@ -1153,7 +1217,7 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
         GG_CK(cudaStreamSynchronize(st));
         GG_CK(cudaEventElapsedTime(&ms, e->ev0, e->ev1));
         e->last_ms += ms;
-        e->last_launches += launches;
+        e->last_launches += launches_plain;
     }
     e->last_batches = nb;
 

@@ -28,12 +28,160 @@
 
 namespace gg {
 
+// ---------------------------------------------------------------------------
+// ball_kernel<D, K>: the rows V_K of every batch, one warp per row.  Row v is a bit string
+// over all vertices in shared memory (8 KB at 65536); the ends of v's walks of up to K
+// steps set their bits -- neighbours, the level-2 list of v, those of its neighbours
+// (level 3) and, K = 4, those of its level-2 ends other than v -- and the row goes out
+// once, each 4096-source part to its batch.  An end is new at its level when atomicOr
+// returns its bit clear; the last level's count is the row's popcount less the others'.
+//
+// Bound by the shared-memory atomics (d^K ends a row, random banks).
+// ---------------------------------------------------------------------------
+constexpr int kBallBlock = 256;
+constexpr int kBallCounts = 256;   // batches * K
+
+struct BallArgs {
+    const int32_t *adj, *h2;  // [rows][D], [rows][D * D]
+    const int *bad, *oneway;
+    uint4 *vall;              // [nb][rows][nC]
+    unsigned long long *counts;   // [nb][stride]: levels 1..K added
+    int stride;
+    int rows, nC, nb;
+};
+
+__host__ __device__ constexpr int ball_warp_bytes(int D, int K, int parts) {
+    return parts * 512 + (K == 4 ? D * D * 4 + 15 : D * 4 + 15) / 16 * 16;
+}
+
+template <int D, int K>
+__global__ void __launch_bounds__(kBallBlock, 3) ball_kernel(const __grid_constant__ BallArgs a) {
+    extern __shared__ __align__(16) unsigned char s_ball[];
+    __shared__ unsigned long long s_cnt[kBallCounts];
+    if ((a.bad && *a.bad) || ld_acquire_i(a.oneway) != 0) return;   // (one-way: sweep_kernel says so)
+    constexpr int Q = D * D, V = Q % 4 == 0 ? 4 : 1, SL = Q / V;    // a list: SL slots of V ends
+    constexpr int UN = V == 4 ? 4 : 8;                              // slots a lane has in flight
+    const unsigned lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
+    const int sub = a.nC / 32, parts = a.nb * sub;
+    for (int k = (int)threadIdx.x; k < a.nb * K; k += (int)blockDim.x) s_cnt[k] = 0ull;
+    uint4 *row4 = reinterpret_cast<uint4 *>(s_ball + (size_t)wib * ball_warp_bytes(D, K, parts));
+    unsigned *row = reinterpret_cast<unsigned *>(row4);
+    int *list = reinterpret_cast<int *>(row4 + parts * 32);
+    for (int p = 0; p < parts; ++p) row4[p * 32 + lane] = u4zero();
+    __syncthreads();
+    auto add = [&](const unsigned w) -> unsigned {   // 1 when w's bit was clear
+        const unsigned bit = 1u << (w & 31u);
+        return (atomicOr(row + (w >> 5), bit) & bit) == 0u;
+    };
+    auto put = [&](const unsigned w) { atomicOr(row + (w >> 5), 1u << (w & 31u)); };
+    // The ends in the level-2 lists of list[0 .. n): f on each.
+    auto lists = [&](const int n, auto &&f) {
+        const int slots = n * SL;
+        for (int i0 = (int)lane; i0 < slots; i0 += 32 * UN) {
+            if constexpr (V == 4) {
+                uint4 q[UN];
+#pragma unroll
+                for (int k = 0; k < UN; ++k) {
+                    const int i = i0 + 32 * k;
+                    if (i < slots) {
+                        const int j = i / SL;
+                        q[k] = __ldg(reinterpret_cast<const uint4 *>(a.h2 + (size_t)list[j] * Q) + (i - j * SL));
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < UN; ++k)
+                    if (i0 + 32 * k < slots) { f(q[k].x); f(q[k].y); f(q[k].z); f(q[k].w); }
+            } else {
+                unsigned q[UN];
+#pragma unroll
+                for (int k = 0; k < UN; ++k) {
+                    const int i = i0 + 32 * k;
+                    if (i < slots) {
+                        const int j = i / SL;
+                        q[k] = (unsigned)__ldg(a.h2 + (size_t)list[j] * Q + (i - j * SL));
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < UN; ++k)
+                    if (i0 + 32 * k < slots) f(q[k]);
+            }
+        }
+    };
+    const size_t items = (size_t)a.rows * (size_t)a.nC;
+    for (int v = (int)(blockIdx.x * (kBallBlock / 32) + wib); v < a.rows; v += (int)(gridDim.x * (kBallBlock / 32))) {
+        unsigned n1 = 0u, n2 = 0u, n3 = 0u, all = 0u;
+        int mine[(Q + 31) / 32];   // this lane's share of v's level-2 list
+#pragma unroll
+        for (int k = 0; k < (Q + 31) / 32; ++k) {
+            const int i = (int)lane + 32 * k;
+            mine[k] = i < Q ? __ldg(a.h2 + (size_t)v * Q + i) : v;
+        }
+        if (lane == 0) put((unsigned)v);
+        int u = v;
+        if (lane < (unsigned)D) {
+            u = __ldg(a.adj + (size_t)v * D + lane);
+            list[lane] = u;
+        }
+        __syncwarp();
+        if (lane < (unsigned)D) n1 = add((unsigned)u);
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < (Q + 31) / 32; ++k)
+            if (mine[k] != v) n2 += add((unsigned)mine[k]);
+        __syncwarp();
+        if constexpr (K == 4) {
+            lists(D, [&](const unsigned w) { n3 += add(w); });
+            __syncwarp();
+            // the level-2 ends other than v itself (its list is set)
+            int n = 0;
+#pragma unroll
+            for (int k = 0; k < (Q + 31) / 32; ++k) {
+                const unsigned m = __ballot_sync(0xffffffffu, mine[k] != v);
+                if (mine[k] != v) list[n + __popc(m & ((1u << lane) - 1u))] = mine[k];
+                n += __popc(m);
+            }
+            __syncwarp();
+            lists(n, put);
+        } else {
+            lists(D, put);
+        }
+        __syncwarp();
+        uint4 *out = a.vall + (size_t)v * a.nC + lane;
+        for (int p = 0, c = 0; p < parts; ++p) {
+            uint4 q = row4[p * 32 + lane];
+            row4[p * 32 + lane] = u4zero();
+            if (a.rows < (p + 1) * 4096) q = u4or(q, pad_mask((int)lane, a.rows - p * 4096));
+            all += u4popc(q);
+            __stcs(out + c * 32, q);
+            if (++c == sub) {
+                c = 0;
+                out += items;
+            }
+        }
+        n1 = __reduce_add_sync(0xffffffffu, n1);
+        n2 = __reduce_add_sync(0xffffffffu, n2);
+        if (K == 4) n3 = __reduce_add_sync(0xffffffffu, n3);
+        all = __reduce_add_sync(0xffffffffu, all) - (unsigned)(parts * 4096 - a.rows) - 1u - n1 - n2 - n3;
+        if (lane == 0) {
+            unsigned long long *c = s_cnt + v / (128 * a.nC) * K;
+            atomicAdd(c, (unsigned long long)n1);
+            atomicAdd(c + 1, (unsigned long long)n2);
+            if (K == 4) atomicAdd(c + 2, (unsigned long long)n3);
+            atomicAdd(c + K - 1, (unsigned long long)all);
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    for (int k = (int)threadIdx.x; k < a.nb * K; k += (int)blockDim.x)
+        if (s_cnt[k]) atomicAdd(a.counts + (size_t)(k / K) * a.stride + k % K + 1, s_cnt[k]);
+}
+
 constexpr int kSweepBlock = 1024;   // one block per SM: a grid barrier takes 148 arrivals, not 592
 
 struct SweepArgs {
     const int32_t *adj;
     const int *bad, *oneway;
-    const uint4 *vall;        // [nb][rows * nC]: level-K rows (walk_all_kernel)
+    const uint4 *vall;        // [nb][rows * nC]: level-K rows (ball_kernel)
     uint4 *A, *B;             // [rows * nC] each: the levels after it in turn
     Ctl *ctl;
     unsigned expected;

@@ -37,7 +37,9 @@ def check_oracle(r, adj):
 
 
 @pytest.mark.parametrize("n,d,batch", [(5000, 3, 4096), (4098, 8, 4096), (8192, 8, 4096), (8193, 8, 8192), (12290, 4, 4096),
-                                       (12289, 6, 8192), (20002, 8, 8192), (20002, 6, 12288), (30011, 6, 0)])
+                                       (12289, 6, 8192), (4097, 5, 4096), (9001, 7, 8192), (10001, 9, 4096),
+                                       (12001, 10, 4096), (9000, 11, 4096), (12300, 12, 12288), (8200, 13, 4096),
+                                       (13001, 14, 0), (12290, 15, 0), (14001, 16, 0), (20002, 8, 8192), (20002, 6, 12288), (30011, 6, 0)])
 def test_sweep_equals_the_level_loop(n, d, batch, monkeypatch):
     adj = G.random_regular(n if n * d % 2 == 0 else n + 1, d, 7)
     r = both(monkeypatch, len(adj), d, batch, [full(adj)])
@@ -80,7 +82,7 @@ def test_sweep_gives_up_where_it_must(what, monkeypatch):
         for u in set(adj[8999].tolist()):
             adj[u][adj[u] == 8999] = u
         adj[8999] = 8999
-    else:                         # everything within the walk: no level left
+    else:                         # one level after the walk, then the last
         n, d = 4160, 8
         adj = G.random_regular(n, d, 4)
     adj = np.ascontiguousarray(adj, dtype=np.int32)
