@@ -155,12 +155,15 @@ struct gg_engine {
     int *d_redo = nullptr, *h_redo = nullptr;   // sweep_kernel gave up: bfs_batch_kernel instead
     bool sweep = true;                   // sweep_kernel where it applies (GG_SWEEP, and no level mode asked for)
     int sweep_wait = 0;                  // evaluations until it is tried again
+    int sweep_nC = 0;                    // its chunks per row (0: never)
+    uint4 *d_swA = nullptr, *d_swB = nullptr;   // its level buffers, when wider than d_V
+    size_t sw_chunks = 0;                // chunks each of them holds
     int *d_wasym = nullptr;              // one-way flag of the table (walk_index_kernel)
     unsigned long long *d_vtot = nullptr;   // [nb][3] level totals (dense visited-set pull without own chunks)
     // walk_all_kernel output: the level-K rows of every batch and their flag words
     uint4 *d_vall = nullptr;
     uint32_t *d_vall_fl = nullptr;
-    size_t vall_batches = 0;             // batches d_vall holds
+    size_t vall_chunks = 0;              // chunks d_vall holds
     long long walk_all_mb = 4096;        // budget for d_vall (GG_WALK_ALL_MB; 0: per-batch walk passes)
     bool p_dirty = true;                 // push buffers must be zeroed before the next launch
     unsigned long long *d_counts = nullptr;
@@ -207,7 +210,10 @@ void free_batch_buffers(gg_engine *e) {
     cudaFree(e->d_vall); cudaFree(e->d_vall_fl);
     e->d_vall = nullptr;
     e->d_vall_fl = nullptr;
-    e->vall_batches = 0;
+    e->vall_chunks = 0;
+    cudaFree(e->d_swA); cudaFree(e->d_swB);
+    e->d_swA = e->d_swB = nullptr;
+    e->sw_chunks = 0;
     cudaFree(e->d_V); cudaFree(e->d_F0); cudaFree(e->d_F1);
     cudaFree(e->d_fl0); cudaFree(e->d_fl1);
     cudaFree(e->d_P0); cudaFree(e->d_P1); cudaFree(e->d_pf0); cudaFree(e->d_pf1);
@@ -327,7 +333,9 @@ int walk_levels(gg_engine *e) {
     return K;
 }
 
-// Share of the pairs (ppm) below which a level's feeding frontier is left to the flag words.
+// Share of the pairs (ppm) below which a level's feeding frontier is left to the flag words
+// of bfs_batch_kernel (n = 60000, d = 5, 0.5 % after the walk: 1561 us here, 3739 there; n =
+// 40000, d = 4, 0.27 %: 1023 / 1463).
 constexpr int kSweepThinPpm = 2000;
 
 // Degrees 3 to 8 walk four steps, 9 to 16 three: at most 4096 walk ends a row.
@@ -345,48 +353,95 @@ SweepKernels sweep_for(int d) {
 
 // Pairs left (ppm) below which last_rows takes a level.  A share u of the pairs left
 // becomes about u^(d-1) with the level, and a row's 4096 pairs must then rarely (one row
-// in twenty) hold one that is still missing: those cost d^2 gathers, one after the other.
+// in twenty) hold one that is still missing: those cost d^2 gathers.  Far from critical:
+// a random graph's share falls from above a half to below a tenth in one level.
 int sweep_last_ppm(int d) { return (int)(1e6 * std::min(0.2, std::pow(1.2e-5, 1.0 / (d - 1)))); }
 
 // Room for the rows of every batch (walk_all_kernel, ball_kernel), grown as needed.
-bool vall_room(gg_engine *e, int nb) {
-    const size_t bytes = (size_t)nb * e->items * sizeof(uint4);
-    const size_t fbytes = (size_t)nb * ((e->items + 31) / 32) * sizeof(uint32_t);
-    if ((long long)(bytes >> 20) > e->walk_all_mb) return false;
-    if ((size_t)nb <= e->vall_batches) return true;
+bool vall_room(gg_engine *e, size_t chunks) {
+    if ((long long)((chunks * sizeof(uint4)) >> 20) > e->walk_all_mb) return false;
+    if (chunks <= e->vall_chunks) return true;
     invalidate_graph(e);
     cudaFree(e->d_vall); cudaFree(e->d_vall_fl);
     e->d_vall = nullptr;
     e->d_vall_fl = nullptr;
-    e->vall_batches = 0;
-    if (cudaMalloc(&e->d_vall, bytes) != cudaSuccess || cudaMalloc(&e->d_vall_fl, fbytes) != cudaSuccess) {
+    e->vall_chunks = 0;
+    if (cudaMalloc(&e->d_vall, chunks * sizeof(uint4)) != cudaSuccess ||
+        cudaMalloc(&e->d_vall_fl, (chunks + 31) / 32 * sizeof(uint32_t)) != cudaSuccess) {
         cudaFree(e->d_vall); cudaFree(e->d_vall_fl);
         e->d_vall = nullptr;
         e->d_vall_fl = nullptr;
         (void)cudaGetLastError();
         return false;
     }
-    e->vall_batches = (size_t)nb;
+    e->vall_chunks = chunks;
     return true;
 }
 
-// Shared memory of a ball_kernel block.
-size_t ball_smem(const gg_engine *e, int nb) {
-    return (size_t)(gg::kBallBlock / 32) * gg::ball_warp_bytes(e->d, sweep_K(e->d), nb * (e->nC / 32));
+// sweep_kernel's level buffers: d_V and d_F0, or a wider pair of its own.
+bool sweep_room(gg_engine *e, int nb) {
+    const size_t chunks = (size_t)e->rows * e->sweep_nC;
+    if (!e->h2_elems || !vall_room(e, nb * chunks)) return false;
+    if (e->sweep_nC <= e->nC || chunks <= e->sw_chunks) return true;
+    invalidate_graph(e);
+    cudaFree(e->d_swA); cudaFree(e->d_swB);
+    e->d_swA = e->d_swB = nullptr;
+    e->sw_chunks = 0;
+    if (cudaMalloc(&e->d_swA, chunks * sizeof(uint4)) != cudaSuccess ||
+        cudaMalloc(&e->d_swB, chunks * sizeof(uint4)) != cudaSuccess) {
+        cudaFree(e->d_swA); cudaFree(e->d_swB);
+        e->d_swA = e->d_swB = nullptr;
+        (void)cudaGetLastError();
+        return false;
+    }
+    e->sw_chunks = chunks;
+    return true;
 }
 
-// Whether sweep_kernel can take evaluations of every vertex in order, by size: whole
-// 4096-source parts, two ball_kernel blocks an SM, and the walk's last level not thin on a
-// graph whose walks rarely meet (others find out at batch 0).
-bool sweep_fits(const gg_engine *e) {
-    if (!e->sweep || e->d < 3 || e->d > 16 || e->nC % 32 != 0 || (int)e->reps.size() != e->rows || e->d_inv ||
+int sweep_batches(const gg_engine *e) { return (e->rows + 128 * e->sweep_nC - 1) / (128 * e->sweep_nC); }
+
+// Shared memory of a ball_kernel block.
+size_t ball_smem(const gg_engine *e) {
+    return (size_t)(gg::kBallBlock / 32) *
+           gg::ball_warp_bytes(e->d, sweep_K(e->d), sweep_batches(e) * (e->sweep_nC / 32));
+}
+
+// sweep_kernel's chunks per row, or 0 where it never applies.  Every vertex a source, in
+// order; batches of whole 4096-source parts; two ball_kernel blocks an SM; and the walk's
+// last level not thin on a graph whose walks rarely meet (others find out at batch 0).
+// Its batches are as wide as keeps a level's rows within 64 MB, and even: half a level's
+// gathers then still hit L2, and there are fewer barriers and last_rows passes.  n = 65536,
+// d = 8: 4096 wide 1322 us, 8192 1225, 12288 1441; n = 50000, d = 6: 923, 893, 978;
+// n = 30012, d = 6: 4096 wide 452, 8192 408, 16384 386.
+int sweep_width(gg_engine *e, const bool chosen) {
+    if (!e->sweep || e->d < 3 || e->d > 16 || e->rows < 4096 || (int)e->reps.size() != e->rows || e->d_inv ||
         e->src_first != 0)
-        return false;
-    const int K = sweep_K(e->d), nb = (e->rows + e->batch_bits - 1) / e->batch_bits;
-    if (nb * K > gg::kBallCounts || 2 * (ball_smem(e, nb) + 4096) > (size_t)e->smem_optin) return false;
+        return 0;
+    const int parts = (e->rows + 4095) / 4096;
+    const int most = std::max(1, (int)((64ll << 20) / ((long long)e->rows * 512)));
+    const int nb = (parts + most - 1) / most;
+    e->sweep_nC = chosen ? e->nC : 32 * ((parts + nb - 1) / nb);
+    const int K = sweep_K(e->d);
+    if (e->sweep_nC % 32 != 0 || (long long)e->rows * e->sweep_nC >= (1ll << 31) || sweep_batches(e) * K > gg::kBallCounts ||
+        2 * (ball_smem(e) + 4096) > (size_t)e->smem_optin)
+        return 0;
     double last = e->d;
     for (int k = 1; k < K; ++k) last *= e->d - 1;
-    return last * 1e6 >= (double)e->rows * kSweepThinPpm;
+    return last * 1e6 >= (double)e->rows * kSweepThinPpm ? e->sweep_nC : 0;
+}
+
+// Whether an evaluation goes to sweep_kernel (asked once per evaluation).  A graph that it
+// gave up on has paid for the attempt, and its engine leaves it out for a while.
+bool sweep_turn(gg_engine *e, const gg_eval_opts *o) {
+    const int cap = (o && o->max_levels > 0) ? o->max_levels : std::max(e->rows, 1);
+    if (!e->sweep_nC || (o && (o->level_ns || o->want_wvc || o->src_begin || o->src_end)) || fault("barrier") ||
+        sweep_K(e->d) > cap)
+        return false;
+    if (e->sweep_wait > 0) {
+        --e->sweep_wait;
+        return false;
+    }
+    return sweep_room(e, sweep_batches(e));
 }
 
 template <int D, bool ONE>
@@ -404,7 +459,7 @@ void *walk_all_for(gg_engine *e, int K, int nb) {
     if (!e->walk_vpull || e->nC % 32 != 0 || K < 1 || K > 3 || nb * (e->nC / 32) * K > gg::kIndexMaxKeys) return nullptr;
     if (e->d != 3 && e->d != 4 && e->d != 6 && e->d != 8) return nullptr;
     if (K < 3 && e->d % 4 != 0) return nullptr;
-    if (!vall_room(e, nb)) return nullptr;
+    if (!vall_room(e, (size_t)nb * e->items)) return nullptr;
     void *k = nullptr;
     if (e->nC == 32)
         k = e->d == 8 ? walk_all_of<8, true>(K) : e->d == 4 ? walk_all_of<4, true>(K)
@@ -442,6 +497,7 @@ gg_status plan(gg_engine *e, int want_bits) {
     invalidate_graph(e);
     const int n_src = (int)e->reps.size();
     int bits;
+    bool chosen = true;   // the batch width was asked for, or tuned
     if (want_bits > 0) {
         bits = want_bits;
     } else {
@@ -454,6 +510,7 @@ gg_status plan(gg_engine *e, int want_bits) {
             e->bps_cap = tuned[1];
             e->walk_pref = tuned[2];
         } else {
+            chosen = false;
             // The widest batch whose three bitsets (3 * rows * bits / 8 bytes)
             // stay within 3/4 of the L2, so that the gathers hit L2 rather than
             // HBM; at least 4096 sources (one 512-byte row segment per vertex)
@@ -503,7 +560,8 @@ gg_status plan(gg_engine *e, int want_bits) {
         e->walk_rpg = 32 / g;
         walk_bytes = (size_t)(gg::kBlock / 32) * gg::walk_smem_per_warp(e->nC);
     }
-    const size_t h2_need = e->walk_K >= 3 || sweep_fits(e) ? (size_t)e->rows * e->d * e->d : 0;
+    e->sweep_nC = sweep_width(e, chosen);
+    const size_t h2_need = e->walk_K >= 3 || e->sweep_nC ? (size_t)e->rows * e->d * e->d : 0;
     if (h2_need != e->h2_elems) {
         cudaFree(e->d_h2);
         e->d_h2 = nullptr;
@@ -712,7 +770,9 @@ struct DirectPlan {
 // The word width that makes the fewest rounds of blocks cheapest, or none: the visited
 // sets of every width must fit a block's shared memory.  A random row of 4, 8 or 16 bytes
 // per lane costs about 3.5, 6.2 and 10.4 shared-memory cycles a warp.
-DirectPlan direct_plan(const gg_engine *e, int ns, bool wvc) {
+constexpr double kSweepUsPerChunk = 0.064e-3, kLoopUsPerChunk = 0.12e-3;
+
+DirectPlan direct_plan(const gg_engine *e, int ns, bool wvc, bool sweep) {
     DirectPlan best;
     if (!e->direct || e->rows < 1 || e->rows > 65535 || ns < 1) return best;
     const size_t budget = (size_t)e->smem_optin - 1024;
@@ -736,13 +796,16 @@ DirectPlan direct_plan(const gg_engine *e, int ns, bool wvc) {
     // 27000 and lifts of 20 to 4000 orbits).  A round of one-word groups takes 3.2 + 0.1 d
     // ns a row (a tenth more with the WVC masks), less certain for a single round; the level
     // loop 50 us and 0.12 ns a chunk of 128 sources.  Device times: n = 4096, d = 16: 25
-    // against 67 us; 16000, 6: 239 / 372; 20000, 8: 337 / 499; 24000, 6: 552 / 448; lifts of
-    // 6000 vertices, 500 orbits: 29 / 59, of 20000, 1000: 85 / 82, of 20000, 2000: 96 / 90.
+    // against 67 us; 16000, 6: 239 / 372; lifts of 6000 vertices, 500 orbits: 29 / 59, of
+    // 20000, 1000: 85 / 82, of 20000, 2000: 96 / 90.
+    // Against sweep_kernel, whose levels take half of that a chunk (whole calls, direct
+    // first): n = 8192, d = 4: 70 against 111 us, 8192, 16: 120 / 131, 9000, 7: 104 / 133,
+    // 10000, 8: 169 / 126, 10000, 5: 150 / 129, 12000, 4: 144 / 145, 16384, 6: 302 / 187.
     if (best.W) {
         const bool one = best.grid <= e->sms;
         const double direct_us = cost / 3.5 * e->rows * (3.2 + 0.1 * e->d) * 1e-3 * (wvc ? 1.1 : 1.0) * (one ? 1.12 : 1.0);
         const double chunks = (double)e->rows * ((ns + 127) / 128);
-        if (direct_us > 50.0 + 0.12e-3 * chunks) best.W = 0;
+        if (direct_us > 50.0 + (sweep ? kSweepUsPerChunk : kLoopUsPerChunk) * chunks) best.W = 0;
     }
     return best;
 }
@@ -862,7 +925,7 @@ gg_status direct_eval(gg_engine *e, const DirectPlan &p, const int32_t *table, c
 
 // Core evaluation with the table already on the device (d_table_in) on `st`.
 gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *o, gg_result *r,
-                   cudaStream_t st, const gg::EvalExtra *x = nullptr) {
+                   cudaStream_t st, const gg::EvalExtra *x = nullptr, int sweep_asked = -1) {
     const int n_src_all = x && x->inv ? x->ns : (int)e->reps.size();
     int s0 = 0, s1 = n_src_all;
     if (x && x->inv && (n_src_all < 1 || n_src_all > e->rows)) return fail(GG_BAD_ARG, "bad source list");
@@ -877,18 +940,20 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
     const bool wvc = o && o->want_wvc;
     const bool want_ns = o && o->level_ns;
     const int ns_all = s1 - s0;
+    bool sweep = !x && (sweep_asked < 0 ? sweep_turn(e, o) : sweep_asked != 0);
     if (!x && !want_ns && !fault("barrier")) {
-        const DirectPlan p = direct_plan(e, ns_all, wvc);
+        const DirectPlan p = direct_plan(e, ns_all, wvc, sweep);
         if (p.W) return direct_eval(e, p, d_table_in, nullptr, o, s0, ns_all, cap_req, r, st);
     }
-    const int nb = (ns_all + e->batch_bits - 1) / e->batch_bits;
+    const int nb_plain = (ns_all + e->batch_bits - 1) / e->batch_bits;
+    int nb = sweep ? sweep_batches(e) : nb_plain;
     const bool within = x && x->within;
     if (within && (!x->inv || wvc || x->planes || e->form != FORM_GRAPH)) return fail(GG_BAD_ARG, "pairs within the sources need a source list");
     // Row width.  A short source list fills one batch of narrower rows (1600 of 65536
     // sources: 13 chunks instead of 32).
     const int nC = within && nb == 1 ? (ns_all + 127) / 128 : e->nC;
     const uint32_t items = (uint32_t)((long long)e->rows * nC);
-    gg_status s = ensure_counters(e, cap_req, nb);
+    gg_status s = ensure_counters(e, cap_req, std::max(nb, nb_plain));
     if (s != GG_OK) return s;
     if (within && (size_t)nb * (cap_req + 1) > e->wcounts_n) {
         cudaFree(e->d_wcounts); cudaFreeHost(e->h_wcounts);
@@ -914,7 +979,7 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
     if (fault("launch")) return fail(GG_CUDA_ERROR, "injected launch failure");
     const unsigned extra = fault("barrier") ? 1u : 0u;
     const size_t lv = (size_t)cap_req + 1;
-    uint64_t d2h = e->off_counts + (size_t)nb * stride * sizeof(unsigned long long);
+    uint64_t d2h = e->off_counts + (size_t)std::max(nb, nb_plain) * stride * sizeof(unsigned long long);
     if (wvc) d2h += (size_t)nb * stride * sizeof(unsigned);
     if (want_ns) d2h += lv * sizeof(unsigned long long);
     // Walk pass for this evaluation: not with the WVC masks or the distance planes
@@ -922,17 +987,9 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
     int walk_K = (wvc || (x && (x->planes || within))) ? 0 : std::min(e->walk_K, cap_req);
     // (one level less where the walk of all batches then covers them: a level costs less
     // than a walk pass per batch)
-    if (walk_K == 4 && e->walk_auto && walk_all_for(e, 3, nb)) walk_K = 3;
+    if (walk_K == 4 && e->walk_auto && walk_all_for(e, 3, nb_plain)) walk_K = 3;
     const int launches_plain = 1 + ((long long)e->rows * e->d > 0 ? 1 : 0) + (walk_K > 0 ? 1 : 0) + (walk_K >= 3 ? 1 : 0);
-    void *wall = walk_K > 0 ? walk_all_for(e, walk_K, nb) : nullptr;
-    // sweep_kernel.  A graph that it gave up on pays for the attempt and keeps to
-    // bfs_batch_kernel for a while.
-    bool sweep = !x && !wvc && !want_ns && !extra && s0 == 0 && ns_all == e->rows && sweep_fits(e) &&
-                 sweep_K(e->d) <= cap_req && e->h2_elems && vall_room(e, nb);
-    if (sweep && e->sweep_wait > 0) {
-        --e->sweep_wait;
-        sweep = false;
-    }
+    void *wall = walk_K > 0 ? walk_all_for(e, walk_K, nb_plain) : nullptr;
     const int launches = sweep ? 4 : launches_plain;
 
     // Everything the GPU does for one evaluation, on `q`: status words zeroed,
@@ -989,8 +1046,8 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
             ba.vall = e->d_vall;
             ba.counts = e->d_counts;
             ba.stride = stride;
-            ba.rows = e->rows; ba.nC = e->nC; ba.nb = nb;
-            const size_t bsmem = ball_smem(e, nb);
+            ba.rows = e->rows; ba.nC = e->sweep_nC; ba.nb = nb;
+            const size_t bsmem = ball_smem(e);
             int per_sm = 0;
             GG_CK(cudaFuncSetAttribute(k.ball, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem));
             GG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.ball, gg::kBallBlock, bsmem));
@@ -1003,8 +1060,8 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
             sa.bad = ba.bad;
             sa.oneway = e->d_wasym;
             sa.vall = e->d_vall;
-            sa.A = e->d_V;
-            sa.B = e->d_F0;
+            sa.A = e->sweep_nC > e->nC ? e->d_swA : e->d_V;
+            sa.B = e->sweep_nC > e->nC ? e->d_swB : e->d_F0;
             sa.ctl = e->d_ctl;
             sa.expected = (unsigned)e->sms;
             sa.wait_ns = e->wait_ns;
@@ -1014,16 +1071,17 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
             sa.levels_run = e->d_levels_run;
             sa.batch_ns = e->d_batch_ns;
             sa.redo = e->d_redo;
-            sa.rows = e->rows; sa.nC = e->nC; sa.nb = nb; sa.K = K;
+            sa.rows = e->rows; sa.nC = e->sweep_nC; sa.nb = nb; sa.K = K;
             sa.max_levels = cap_req;
             sa.thin_ppm = kSweepThinPpm;
             sa.last_ppm = sweep_last_ppm(e->d);
             const int per = (e->rows + e->sms - 1) / e->sms;
             const size_t ssmem = (size_t)per * e->d * sizeof(int32_t);
-            sa.adj_smem_rows = ssmem <= 32u << 10 ? per : 0;   // (no opt-in needed; 65536 rows of 8 take 14 KB)
+            // two slices of the table a block: a level's and last_rows' (65536 rows of 8: 14 KB each)
+            sa.adj_smem_rows = 2 * ssmem <= 38u << 10 ? per : 0;
             void *sargs[] = {&sa};
             GG_CK(cudaLaunchCooperativeKernel(k.sweep, dim3(e->sms), dim3(gg::kSweepBlock), sargs,
-                                              sa.adj_smem_rows ? ssmem : 0, q));
+                                              sa.adj_smem_rows ? 2 * ssmem : 0, q));
             if (timed) GG_CK(cudaEventRecord(e->ev1, q));
             GG_CK(cudaMemcpyAsync(e->h_status, e->d_status, e->off_counts + (size_t)nb * stride * 8,
                                   cudaMemcpyDeviceToHost, q));
@@ -1212,6 +1270,17 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
     if (sweep && *e->h_redo && !*e->h_bad && !e->h_ctl->err) {
         sweep = false;
         e->sweep_wait = 63;
+        const DirectPlan p = direct_plan(e, ns_all, wvc, false);
+        if (p.W) {
+            const double first_ms = e->last_ms;
+            const int first_launches = e->last_launches;
+            e->p_dirty = false;
+            const gg_status ds = direct_eval(e, p, d_table_in, nullptr, o, s0, ns_all, cap_req, r, st);
+            e->last_ms += first_ms;
+            e->last_launches += first_launches;
+            return ds;
+        }
+        nb = nb_plain;
         gg_status es = enqueue(st, true);
         if (es != GG_OK) return es;
         GG_CK(cudaStreamSynchronize(st));
@@ -1350,9 +1419,11 @@ gg_status eval_host(gg_engine *e, const int32_t *table, const gg_eval_opts *o, g
     if (e->table_elems && !table) return fail(GG_BAD_ARG, "null table");
     GG_CK(cudaSetDevice(e->device));
     e->table_stale = false;
+    int sweep = -1;
     if (e->form == FORM_GRAPH && e->table_elems && !(o && (o->level_ns || o->src_begin || o->src_end || o->want_wvc)) &&
         !fault("barrier")) {
-        const DirectPlan p = direct_plan(e, (int)e->reps.size(), false);
+        sweep = sweep_turn(e, o);
+        const DirectPlan p = direct_plan(e, (int)e->reps.size(), false, sweep);
         if (p.W && p.adj_smem) return direct_host(e, p, table, o, r);
     }
     if (e->table_elems) {
@@ -1360,7 +1431,7 @@ gg_status eval_host(gg_engine *e, const int32_t *table, const gg_eval_opts *o, g
         GG_CK(cudaMemcpyAsync(e->d_table, e->h_table, e->table_elems * sizeof(int32_t),
                               cudaMemcpyHostToDevice, e->stream));
     }
-    gg_status s = run_eval(e, e->d_table, o, r, e->stream);
+    gg_status s = run_eval(e, e->d_table, o, r, e->stream, nullptr, sweep);
     e->last_h2d = e->table_elems * sizeof(int32_t);
     return s;
 }

@@ -13,12 +13,12 @@
 // batch 0 finds (else pairs would be counted twice or not at all), and the counts add
 // up over the batches only: a batch's own may be off, or "negative", mod 2^64.
 //
-// Measured, whole evaluations: n = 65536, d = 8, 16 batches of three levels and last_rows,
-// 1936 -> 1645 us (a batch 120 -> 82: last_rows 8-13 us falling with the rows left, in
-// place of levels of 19 and 6 us with a barrier each; four barriers of 592 blocks and
-// their tails -> three of 148); n = 30011, d = 6, irregular, 772 -> 515 us (of which the
-// walk of all batches at degree 6, on batches of two 4096-source parts, 772 -> 590).
-// A level is bound by L2: 268 MB gathered in 22 us.
+// Measured, whole calls: n = 65536, d = 8: 1925 us with bfs_batch_kernel, 1225 here; n =
+// 30011, d = 6, irregular: 766 / 390; n = 40000, d = 10: 1857 / 617; n = 16384, d = 6:
+// 302 / 187.  Of the 1225: ball_kernel 265, per 8192-source batch two levels of 45 (rows
+// from HBM) and 39 us and last_rows 27 falling to 7, the table's way to the device 100.
+// A level is bound by the gathers' way from L2: 537 MB in 39 us (ncu on 4096-source
+// batches: L2 at 46 %, warps waiting for loads), 148 blocks finishing within 2 us.
 //
 // When something does not fit -- a one-way entry, a thin level (flag words would be
 // better), the level cap, a pair further than L + 1 -- *redo is set and the host runs
@@ -198,10 +198,21 @@ struct SweepArgs {
     int adj_smem_rows;
 };
 
-// A batch's state in shared memory (thread 0 writes it between block barriers).
+// A block's state in shared memory (thread 0 writes it between block barriers), so that
+// the functions below keep the kernel's registers to their loops: with these as kernel
+// variables a value of sweep_rows' loop was spilled, and its levels took 46 us, not 39.
 struct SweepState {
     unsigned long long reached, c_prev, pairs;
     int last;                 // level at which every batch takes last_rows (0: none yet)
+    int half;                 // last_rows' H
+    const uint4 *X;           // rows the next level reads
+    uint4 *Y;                 // and writes
+    const int32_t *adj;       // the table, or the block's slice of it in shared memory,
+    unsigned v_base;          // which starts at this row
+    unsigned t_lo, t_hi;      // the block's tiles of a level
+    unsigned next;            // its next tile
+    unsigned long long sum;   // its level total
+    unsigned epoch;           // grid barriers passed
     int act;                  // next step: 0 level, 1 last_rows, 2 batch done, 3 give up
 };
 
@@ -222,90 +233,138 @@ __device__ __forceinline__ void sweep_row(const int32_t *adj, const unsigned v, 
     }
 }
 
-// The pairs of chunk `at` of row v that level L (rows q so far) misses: how many, and
-// whether two steps from V_{L-1} reach them all.
+// Up to 32 chunks (item = v * nC + place, one a lane) that some of their row's neighbours
+// left open: the other neighbours, and for the pairs that level L misses (counted twice
+// when the vertex is in a later batch) two steps from V_{L-1}.
 template <int D>
-static __device__ __noinline__ unsigned sweep_tail(const uint4 *X, const int32_t *adj, const unsigned v,
-                                                   const unsigned nC, const unsigned at, uint4 q, int *redo) {
+static __device__ __noinline__ unsigned finish_chunks(const SweepArgs &a, const SweepState &S, const int b, const int L,
+                                                      const unsigned *list, const unsigned n) {
+    const uint4 *X = S.X;
+    const unsigned lane = threadIdx.x & 31u, nC = (unsigned)a.nC;
+    if (lane >= n) return 0u;
+    const unsigned item = list[lane], v = item / nC, at = item - v * nC;
+    unsigned u[D];
+    sweep_row<D>(a.adj, v, u);
+    uint4 q = __ldcg(X + (u[0] * nC + at));
+#pragma unroll
+    for (int i = 1; i < D; ++i) or_into(q, __ldcg(X + (u[i] * nC + at)));
+    if (u4full(q)) return 0u;
     const unsigned miss = 128u - u4popc(q);
     for (int i = 0; i < D && !u4full(q); ++i) {
-        const unsigned u = (unsigned)__ldg(adj + (size_t)v * D + i);
         unsigned w[D];
-        sweep_row<D>(adj, u, w);
+        sweep_row<D>(a.adj, (unsigned)__ldg(a.adj + (size_t)v * D + i), w);
         uint4 x[D];
 #pragma unroll
         for (int j = 0; j < D; ++j) x[j] = __ldcg(X + (w[j] * nC + at));
 #pragma unroll
         for (int j = 0; j < D; ++j) or_into(q, x[j]);
     }
-    if (!u4full(q)) *redo = 1;
-    return miss;
+    if (!u4full(q)) *a.redo = 1;
+    const int bv = (int)(v / (128u * nC));
+    // level L + 1 is not empty for either batch of these pairs
+    atomicMax(a.levels_run + b, L + 1);
+    atomicMax(a.levels_run + bv, L + 1);
+    return bv == b ? miss : 2u * miss;
 }
 
-template <int D>
-static __device__ __noinline__ unsigned last_rows(const SweepArgs &a, const uint4 *X, const int b, const int L) {
-    constexpr int H = D >= 8 ? D / 2 : D;   // neighbours gathered first: half usually fill the chunk
+// The block's share of the rows from batch b on (its slice of the table to s_row first).  A tile takes the first H neighbours of its row, such that a chunk is
+// then rarely open; those go on a list of the warp's and are finished 32 at a time.  (At
+// once, a warp in three waited for a second round of gathers; and in line with the kernel,
+// as sweep_rows: as a call the loop's gathers were held back by the registers kept for the
+// caller.  All rows of n = 65536, d = 8 on an 8192-source batch: 31 -> 27 us.)
+template <int D, int H>
+__device__ __forceinline__ unsigned last_rows(const SweepArgs &a, SweepState &S, const int b, const int L,
+                                              int32_t *s_row, unsigned *list) {
+    constexpr int U = H <= 4 ? 8 / H : 1;   // tiles a round: up to 8 gathers in flight
+    const uint4 *X = S.X;
     const unsigned lane = threadIdx.x & 31u;
-    const unsigned warps = gridDim.x * (kSweepBlock / 32), gw = blockIdx.x * (kSweepBlock / 32) + (threadIdx.x >> 5);
-    const unsigned nC = (unsigned)a.nC, parts = nC / 32u, S = 128u * nC;
-    const unsigned v0 = (unsigned)b * S, t_end = (unsigned)a.rows * parts;
-    unsigned cnt = 0u;
-    constexpr int U = H <= 4 ? 2 : 1;       // tiles a round: at most 8 gathers in flight, as registers allow
-    for (unsigned t0 = v0 * parts + gw; t0 < t_end; t0 += (unsigned)U * warps) {
-        unsigned v[U], at[U], tu[U][D];
-        bool ok[U];
-        uint4 q[U], x[U][H];
+    const unsigned nC = (unsigned)a.nC, parts = nC / 32u;
+    const unsigned v0 = (unsigned)b * 128u * nC, left = (unsigned)a.rows - v0;
+    const unsigned r_lo = v0 + (unsigned)((unsigned long long)left * blockIdx.x / gridDim.x);
+    const unsigned r_hi = v0 + (unsigned)((unsigned long long)left * (blockIdx.x + 1) / gridDim.x);
+    const bool keep = r_hi - r_lo <= (unsigned)a.adj_smem_rows;
+    if (keep)
+        for (unsigned k = threadIdx.x; k < (r_hi - r_lo) * D; k += blockDim.x) s_row[k] = __ldg(a.adj + (size_t)r_lo * D + k);
+    const int32_t *adj = keep ? s_row : a.adj;
+    const unsigned v_base = keep ? r_lo : 0u, t_end = r_hi * parts;
+    if (threadIdx.x == 0) S.next = r_lo * parts;
+    __syncthreads();
+    unsigned cnt = 0u, open = 0u;
+    for (;;) {
+        unsigned t0 = 0u;
+        if (lane == 0) t0 = atomicAdd(&S.next, (unsigned)U);
+        t0 = __shfl_sync(0xffffffffu, t0, 0);
+        if (t0 >= t_end) break;
+        uint4 x[U][H];
 #pragma unroll
         for (int k = 0; k < U; ++k) {
-            const unsigned t = t0 + (unsigned)k * warps;
-            ok[k] = t < t_end;
-            v[k] = ok[k] ? (parts == 1u ? t : t / parts) : v0;
-            at[k] = ok[k] ? (t - v[k] * parts) * 32u + lane : lane;
-            sweep_row<D>(a.adj, v[k], tu[k]);
+            const unsigned t = min(t0 + (unsigned)k, t_end - 1u);
+            const unsigned v = parts == 1u ? t : t / parts, at = (t - v * parts) * 32u + lane;
+            const int32_t *row = adj + (size_t)(v - v_base) * D;
 #pragma unroll
-            for (int i = 0; i < D; ++i) tu[k][i] = tu[k][i] * nC + at[k];
+            for (int i = 0; i < H; ++i) x[k][i] = __ldcg(X + ((unsigned)row[i] * nC + at));
         }
 #pragma unroll
-        for (int k = 0; k < U; ++k)
-#pragma unroll
-            for (int i = 0; i < H; ++i) x[k][i] = __ldcg(X + tu[k][i]);
-#pragma unroll
         for (int k = 0; k < U; ++k) {
-            q[k] = x[k][0];
+            uint4 q = x[k][0];
 #pragma unroll
-            for (int i = 1; i < H; ++i) or_into(q[k], x[k][i]);
-            if constexpr (H < D)
-                if (!u4full(q[k])) {
-                    uint4 y[D - H];
-#pragma unroll
-                    for (int i = H; i < D; ++i) y[i - H] = __ldcg(X + tu[k][i]);
-#pragma unroll
-                    for (int i = H; i < D; ++i) or_into(q[k], y[i - H]);
-                }
-            if (ok[k] && !u4full(q[k])) {
-                const unsigned m = sweep_tail<D>(X, a.adj, v[k], nC, at[k], q[k], a.redo);
-                const unsigned bv = v[k] / S;
-                cnt += bv == (unsigned)b ? m : 2u * m;
-                // level L + 1 is not empty for either batch of these pairs
-                atomicMax(a.levels_run + b, L + 1);
-                atomicMax(a.levels_run + bv, L + 1);
+            for (int i = 1; i < H; ++i) or_into(q, x[k][i]);
+            const bool o = t0 + (unsigned)k < t_end && !u4full(q);
+            const unsigned m = __ballot_sync(0xffffffffu, o);
+            if (m == 0u) continue;
+            if (o) list[open + __popc(m & ((1u << lane) - 1u))] = (t0 + (unsigned)k) * 32u + lane;
+            open += __popc(m);
+            __syncwarp();
+            if (open >= 32u) {
+                open -= 32u;
+                cnt += finish_chunks<D>(a, S, b, L, list + open, 32u);
+                __syncwarp();
             }
         }
     }
+    cnt += finish_chunks<D>(a, S, b, L, list, open);
     return cnt;
 }
 
-// One dense level on the block's tiles [s_next, t_hi): Y[v] = OR of the neighbours' X
+// Neighbours a tile of last_rows takes, with a share u of the pairs left: a chunk of 128
+// stays open with 128 u^H, and costs D gathers of a 32-byte sector each when it does.
+__device__ __forceinline__ int last_half(const int D, const float u) {
+    const int hs[5] = {2, 3, 4, 6, 8};
+    float p = u;
+    int k = 1;
+    for (int i = 0; i < 5; ++i) {
+        if (hs[i] >= D) break;
+        for (; k < hs[i]; ++k) p *= u;
+        if (128.f * p < 0.03f) return hs[i];
+    }
+    return D <= 8 ? D : 8;
+}
+
+template <int D>
+__device__ __forceinline__ unsigned last_rows_of(const SweepArgs &a, SweepState &S, const int b, const int L,
+                                                 int32_t *s_row, unsigned *list) {
+    const int H = S.half;
+    if (H == 2) return last_rows<D, 2>(a, S, b, L, s_row, list);
+    if constexpr (D >= 3) if (H == 3) return last_rows<D, 3>(a, S, b, L, s_row, list);
+    if constexpr (D >= 4) if (H == 4) return last_rows<D, 4>(a, S, b, L, s_row, list);
+    if constexpr (D >= 6) if (H == 6) return last_rows<D, 6>(a, S, b, L, s_row, list);
+    return last_rows<D, (D < 8 ? D : 8)>(a, S, b, L, s_row, list);
+}
+
+// One dense level on the block's tiles [next, t_hi): Y[v] = OR of the neighbours' X
 // rows (without one-way entries V_{L-1}[v] lies within them for L >= 2), and this
 // thread's popcount of what it wrote.
 template <int D, bool ONE>
-static __device__ __noinline__ unsigned sweep_rows(const uint4 *X, uint4 *Y, const int32_t *adj, const unsigned v_base,
-                                                   const unsigned parts, const unsigned t_hi, unsigned *s_next) {
+__device__ __forceinline__ unsigned sweep_rows(SweepState &S, const unsigned parts) {
     const unsigned lane = threadIdx.x & 31u;
+    const uint4 *X = S.X;
+    uint4 *Y = S.Y;
+    const int32_t *adj = S.adj;
+    const unsigned v_base = S.v_base, t_hi = S.t_hi;
     unsigned cnt = 0u;
     for (;;) {
         unsigned t = 0u;
-        if (lane == 0) t = atomicAdd(s_next, 1u);
+        if (lane == 0) t = atomicAdd(&S.next, 1u);
         t = __shfl_sync(0xffffffffu, t, 0);
         if (t >= t_hi) break;
         const unsigned v = ONE ? t : t / parts, at = ONE ? lane : (t - v * parts) * 32u + lane;
@@ -327,6 +386,7 @@ static __device__ __noinline__ unsigned sweep_rows(const uint4 *X, uint4 *Y, con
 }
 
 // What comes next in batch b, whose levels below L are done (thread 0).
+template <int D>
 __device__ __forceinline__ void sweep_next(const SweepArgs &a, SweepState &S, const int b, const int L) {
     const unsigned long long left = S.pairs - S.reached;
     if (left == 0ull) {
@@ -337,6 +397,7 @@ __device__ __forceinline__ void sweep_next(const SweepArgs &a, SweepState &S, co
     if (b == 0 && S.last == 0 && L >= 2 && left * 1000000ull < S.pairs * (unsigned long long)a.last_ppm) S.last = L;
     if (L == S.last) {
         S.act = L + 1 <= a.max_levels ? 1 : 3;
+        S.half = last_half(D, (float)left / (float)S.pairs);
     } else {
         const bool thin = S.c_prev * 1000000ull < S.pairs * (unsigned long long)a.thin_ppm;
         S.act = thin || L > a.max_levels ? 3 : 0;
@@ -346,33 +407,34 @@ __device__ __forceinline__ void sweep_next(const SweepArgs &a, SweepState &S, co
 template <int D>
 __global__ void __launch_bounds__(kSweepBlock, 1) sweep_kernel(const __grid_constant__ SweepArgs a) {
     extern __shared__ int32_t s_adj[];
+    __shared__ unsigned s_open[kSweepBlock / 32][64];   // last_rows' lists (one array for all its instances)
     __shared__ SweepState S;
-    __shared__ unsigned s_next;
-    __shared__ unsigned long long s_sum;
     if (a.bad && *a.bad) return;   // uniform across the grid, as is the next
     if (ld_acquire_i(a.oneway) != 0) {
         if (blockIdx.x == 0 && threadIdx.x == 0) *a.redo = 1;
         return;
     }
-    const unsigned lane = threadIdx.x & 31u;
-    const unsigned parts = (unsigned)a.nC / 32u, items = (unsigned)a.rows * (unsigned)a.nC;
-    const unsigned v_lo = (unsigned)((unsigned long long)a.rows * blockIdx.x / gridDim.x);
-    const unsigned v_hi = (unsigned)((unsigned long long)a.rows * (blockIdx.x + 1) / gridDim.x);
-    const unsigned t_lo = v_lo * parts, t_hi = v_hi * parts;
-    const bool keep = v_hi - v_lo <= (unsigned)a.adj_smem_rows;   // the block's rows of the table stay in shared memory
-    if (keep)
-        for (unsigned k = threadIdx.x; k < (v_hi - v_lo) * D; k += blockDim.x) s_adj[k] = __ldg(a.adj + (size_t)v_lo * D + k);
-    const int32_t *adj = keep ? s_adj : a.adj;
-    const unsigned v_base = keep ? v_lo : 0u;
-    unsigned epoch = 0u;
-    bool odd = false;              // which of A and B the next level writes
-    if (threadIdx.x == 0) S.last = 0;
+    {
+        const unsigned v_lo = (unsigned)((unsigned long long)a.rows * blockIdx.x / gridDim.x);
+        const unsigned v_hi = (unsigned)((unsigned long long)a.rows * (blockIdx.x + 1) / gridDim.x);
+        const bool keep = v_hi - v_lo <= (unsigned)a.adj_smem_rows;   // the block's slice of the table
+        if (keep)
+            for (unsigned k = threadIdx.x; k < (v_hi - v_lo) * D; k += blockDim.x) s_adj[k] = __ldg(a.adj + (size_t)v_lo * D + k);
+        if (threadIdx.x == 0) {
+            S.adj = keep ? s_adj : a.adj;
+            S.v_base = keep ? v_lo : 0u;
+            S.t_lo = v_lo * ((unsigned)a.nC / 32u);
+            S.t_hi = v_hi * ((unsigned)a.nC / 32u);
+            S.last = 0;
+            S.epoch = 0u;
+            S.Y = a.A;
+        }
+    }
     for (int b = 0; b < a.nb; ++b) {
-        unsigned long long *counts = a.counts + (size_t)b * (size_t)a.stride;
-        const int ns = min(128 * a.nC, a.rows - b * 128 * a.nC);
-        const unsigned long long pad = (unsigned long long)a.rows * (unsigned long long)(128 * a.nC - ns);
         int L = a.K + 1;
         if (threadIdx.x == 0) {
+            const int ns = min(128 * a.nC, a.rows - b * 128 * a.nC);
+            unsigned long long *counts = a.counts + (size_t)b * (size_t)a.stride;
             if (blockIdx.x == 0) {
                 a.batch_ns[2 * b] = gtimer();
                 counts[0] = (unsigned long long)ns;
@@ -380,41 +442,46 @@ __global__ void __launch_bounds__(kSweepBlock, 1) sweep_kernel(const __grid_cons
             S.pairs = (unsigned long long)ns * (unsigned long long)a.rows;
             S.reached = (unsigned long long)ns;
             S.c_prev = 0ull;
+            S.X = a.vall + (size_t)b * ((size_t)a.rows * (size_t)a.nC);
             int k = 1;
             for (; k <= a.K && S.reached < S.pairs; ++k) {
                 S.c_prev = ld_relaxed_u64(counts + k);
                 S.reached += S.c_prev;
             }
-            sweep_next(a, S, b, S.reached == S.pairs ? k : a.K + 1);
+            sweep_next<D>(a, S, b, S.reached == S.pairs ? k : L);
+            S.next = S.t_lo;
+            S.sum = 0ull;
         }
         __syncthreads();
-        const uint4 *X = a.vall + (size_t)b * items;
         for (; S.act == 0; ++L) {
-            uint4 *Y = odd ? a.B : a.A;
-            if (threadIdx.x == 0) { s_next = t_lo; s_sum = 0ull; }
-            __syncthreads();
-            const unsigned cnt = parts == 1u ? sweep_rows<D, true>(X, Y, adj, v_base, 1u, t_hi, &s_next)
-                                             : sweep_rows<D, false>(X, Y, adj, v_base, parts, t_hi, &s_next);
+            const unsigned cnt = a.nC == 32 ? sweep_rows<D, true>(S, 1u) : sweep_rows<D, false>(S, (unsigned)a.nC / 32u);
             const unsigned wsum = __reduce_add_sync(0xffffffffu, cnt);
-            if (lane == 0) atomicAdd(&s_sum, (unsigned long long)wsum);
+            if ((threadIdx.x & 31u) == 0u) atomicAdd(&S.sum, (unsigned long long)wsum);
             __syncthreads();
             unsigned long long *vt = a.vtot + 3 * (size_t)b;
             if (threadIdx.x == 0) {
-                atomicAdd(vt + L % 3, s_sum);
+                atomicAdd(vt + L % 3, S.sum);
                 if (blockIdx.x == 0) vt[(L + 1) % 3] = 0ull;   // read last after level L - 2
             }
             unsigned long long total = 0ull;
+            unsigned epoch = S.epoch;
             if (!grid_sync_value(a.ctl, a.expected, a.wait_ns, L, epoch, vt + L % 3, total)) return;
             if (threadIdx.x == 0) {
+                // total bits of V_L less the padding and the pairs reached before
+                const int ns = min(128 * a.nC, a.rows - b * 128 * a.nC);
+                const unsigned long long pad = (unsigned long long)a.rows * (unsigned long long)(128 * a.nC - ns);
                 const unsigned long long cL = total - pad - S.reached;
-                if (blockIdx.x == 0) counts[L] = cL;
+                if (blockIdx.x == 0) a.counts[(size_t)b * (size_t)a.stride + L] = cL;
                 S.reached += cL;
                 S.c_prev = cL;
-                sweep_next(a, S, b, L + 1);
+                S.epoch = epoch;
+                S.X = S.Y;
+                S.Y = S.Y == a.A ? a.B : a.A;
+                S.next = S.t_lo;
+                S.sum = 0ull;
+                sweep_next<D>(a, S, b, L + 1);
             }
             __syncthreads();
-            X = Y;
-            odd = !odd;
         }
         if (S.act == 3) {
             if (blockIdx.x == 0 && threadIdx.x == 0) *a.redo = 1;
@@ -423,15 +490,16 @@ __global__ void __launch_bounds__(kSweepBlock, 1) sweep_kernel(const __grid_cons
         if (S.act == 1) {
             // No barrier before the next batch: its first level writes the other buffer,
             // and the second one only after the barrier between them.
+            unsigned long long *counts = a.counts + (size_t)b * (size_t)a.stride + L;
             if (blockIdx.x == 0 && threadIdx.x == 0) {
                 atomicMax(a.levels_run + b, L);
-                atomicAdd(counts + L, S.pairs - S.reached);
+                atomicAdd(counts, S.pairs - S.reached);
             }
-            const unsigned cnt = last_rows<D>(a, X, b, L);
+            const unsigned cnt = last_rows_of<D>(a, S, b, L, s_adj + (size_t)a.adj_smem_rows * D, s_open[threadIdx.x >> 5]);
             const unsigned m = __reduce_add_sync(0xffffffffu, cnt);
-            if (lane == 0 && m) {
-                atomicAdd(counts + L, 0ull - (unsigned long long)m);
-                atomicAdd(counts + L + 1, (unsigned long long)m);
+            if ((threadIdx.x & 31u) == 0u && m) {
+                atomicAdd(counts, 0ull - (unsigned long long)m);
+                atomicAdd(counts + 1, (unsigned long long)m);
             }
         }
         if (blockIdx.x == 0 && threadIdx.x == 0) a.batch_ns[2 * b + 1] = gtimer();
