@@ -156,6 +156,9 @@ struct gg_engine {
     bool sweep = true;                   // sweep_kernel where it applies (GG_SWEEP, and no level mode asked for)
     int sweep_wait = 0;                  // evaluations until it is tried again
     int sweep_nC = 0;                    // its chunks per row (0: never)
+    int sweep_K = 0;                     // levels before its dense ones
+    int sweep_ends = 1;                  // most new vertices of a source's level below that
+    bool sweep_list = false;             // the sources are a list (source_ball_kernel)
     uint4 *d_swA = nullptr, *d_swB = nullptr;   // its level buffers, when wider than d_V
     size_t sw_chunks = 0;                // chunks each of them holds
     int *d_wasym = nullptr;              // one-way flag of the table (walk_index_kernel)
@@ -340,13 +343,15 @@ constexpr int kSweepThinPpm = 2000;
 
 // Degrees 3 to 8 walk four steps, 9 to 16 three: at most 4096 walk ends a row.
 constexpr int sweep_K(int d) { return d <= 8 ? 4 : 3; }
-struct SweepKernels { void *ball, *sweep; };
+struct SweepKernels { void *ball, *source_ball, *wide, *narrow; };
 template <int D = 3>
 SweepKernels sweep_for(int d) {
     if constexpr (D > 16) {
-        return {nullptr, nullptr};
+        return {};
     } else {
-        if (d == D) return {(void *)gg::ball_kernel<D, sweep_K(D)>, (void *)gg::sweep_kernel<D>};
+        if (d == D)
+            return {(void *)gg::ball_kernel<D, sweep_K(D)>, (void *)gg::source_ball_kernel<D>,
+                    (void *)gg::sweep_kernel<D, true>, (void *)gg::sweep_kernel<D, false>};
         return sweep_for<D + 1>(d);
     }
 }
@@ -381,7 +386,7 @@ bool vall_room(gg_engine *e, size_t chunks) {
 // sweep_kernel's level buffers: d_V and d_F0, or a wider pair of its own.
 bool sweep_room(gg_engine *e, int nb) {
     const size_t chunks = (size_t)e->rows * e->sweep_nC;
-    if (!e->h2_elems || !vall_room(e, nb * chunks)) return false;
+    if ((!e->sweep_list && !e->h2_elems) || !vall_room(e, nb * chunks)) return false;
     if (e->sweep_nC <= e->nC || chunks <= e->sw_chunks) return true;
     invalidate_graph(e);
     cudaFree(e->d_swA); cudaFree(e->d_swB);
@@ -398,13 +403,15 @@ bool sweep_room(gg_engine *e, int nb) {
     return true;
 }
 
-int sweep_batches(const gg_engine *e) { return (e->rows + 128 * e->sweep_nC - 1) / (128 * e->sweep_nC); }
+int sweep_batches(const gg_engine *e) { return ((int)e->reps.size() + 128 * e->sweep_nC - 1) / (128 * e->sweep_nC); }
 
 // Shared memory of a ball_kernel block.
 size_t ball_smem(const gg_engine *e) {
     return (size_t)(gg::kBallBlock / 32) *
            gg::ball_warp_bytes(e->d, sweep_K(e->d), sweep_batches(e) * (e->sweep_nC / 32));
 }
+
+constexpr int kSrcBallWarps = gg::kSrcBallBlock / 32;
 
 // sweep_kernel's chunks per row, or 0 where it never applies.  Every vertex a source, in
 // order; batches of whole 4096-source parts; two ball_kernel blocks an SM; and the walk's
@@ -414,20 +421,44 @@ size_t ball_smem(const gg_engine *e) {
 // d = 8: 4096 wide 1322 us, 8192 1225, 12288 1441; n = 50000, d = 6: 923, 893, 978;
 // n = 30012, d = 6: 4096 wide 452, 8192 408, 16384 386.
 int sweep_width(gg_engine *e, const bool chosen) {
-    if (!e->sweep || e->d < 3 || e->d > 16 || e->rows < 4096 || (int)e->reps.size() != e->rows || e->d_inv ||
-        e->src_first != 0)
-        return 0;
-    const int parts = (e->rows + 4095) / 4096;
+    const int n_src = (int)e->reps.size();
+    const bool all = n_src == e->rows && !e->d_inv && e->src_first == 0;
+    e->sweep_list = !all;
+    if (!e->sweep || e->d < 3 || e->d > 16 || n_src < 1) return 0;
+    if (all ? e->rows < 4096 : (e->form == FORM_GRAPH || e->rows != e->N)) return 0;   // (rows past N: one-way)
+    const int parts = (n_src + 4095) / 4096;
     const int most = std::max(1, (int)((64ll << 20) / ((long long)e->rows * 512)));
     const int nb = (parts + most - 1) / most;
-    e->sweep_nC = chosen ? e->nC : 32 * ((parts + nb - 1) / nb);
-    const int K = sweep_K(e->d);
-    if (e->sweep_nC % 32 != 0 || (long long)e->rows * e->sweep_nC >= (1ll << 31) || sweep_batches(e) * K > gg::kBallCounts ||
-        2 * (ball_smem(e) + 4096) > (size_t)e->smem_optin)
-        return 0;
+    int nC = 32 * ((parts + nb - 1) / nb);
+    if (!all && n_src <= 2048)
+        for (nC = 1; 128 * nC < n_src;) nC *= 2;
+    e->sweep_nC = chosen ? e->nC : nC;
+    if (e->sweep_nC % 32 != 0 && (all || (e->sweep_nC & (e->sweep_nC - 1)) != 0 || e->sweep_nC > 16)) return 0;
+    if ((long long)e->rows * e->sweep_nC >= (1ll << 31)) return 0;
+    if (all) {
+        const int K = e->sweep_K = sweep_K(e->d);
+        if (sweep_batches(e) * K > gg::kBallCounts || 2 * (ball_smem(e) + 4096) > (size_t)e->smem_optin) return 0;
+        double last = e->d;
+        for (int k = 1; k < K; ++k) last *= e->d - 1;
+        return last * 1e6 >= (double)e->rows * kSweepThinPpm ? e->sweep_nC : 0;
+    }
+    // A list: another walked level as long as its reductions (41 a ns: 1024 sources, 32768
+    // rows, d = 12, three levels 44 us) cost no more than a dense level (4 us and 13 TB/s of
+    // gathers)
+    const double dense_ns = 4000.0 + (double)e->rows * e->d * n_src / 8.0 / 13000.0;
     double last = e->d;
-    for (int k = 1; k < K; ++k) last *= e->d - 1;
-    return last * 1e6 >= (double)e->rows * kSweepThinPpm ? e->sweep_nC : 0;
+    int K = 1;
+    e->sweep_ends = 1;
+    // (a one-way table's level may be d times the one before)
+    while (K + 1 < gg::kSrcBallLevels && e->sweep_ends * e->d <= gg::kSrcBallList &&
+           last * (e->d - 1) * n_src / 41.0 <= dense_ns) {
+        e->sweep_ends *= e->d;
+        last *= e->d - 1;
+        ++K;
+    }
+    e->sweep_K = K;
+    if (2 * (kSrcBallWarps * (size_t)gg::source_ball_warp_bytes(e->rows, e->sweep_ends) + 2048) > (size_t)e->smem_optin) return 0;
+    return e->sweep_nC;
 }
 
 // Whether an evaluation goes to sweep_kernel (asked once per evaluation).  A graph that it
@@ -435,7 +466,7 @@ int sweep_width(gg_engine *e, const bool chosen) {
 bool sweep_turn(gg_engine *e, const gg_eval_opts *o) {
     const int cap = (o && o->max_levels > 0) ? o->max_levels : std::max(e->rows, 1);
     if (!e->sweep_nC || (o && (o->level_ns || o->want_wvc || o->src_begin || o->src_end)) || fault("barrier") ||
-        sweep_K(e->d) > cap)
+        e->sweep_K > cap)
         return false;
     if (e->sweep_wait > 0) {
         --e->sweep_wait;
@@ -561,7 +592,7 @@ gg_status plan(gg_engine *e, int want_bits) {
         walk_bytes = (size_t)(gg::kBlock / 32) * gg::walk_smem_per_warp(e->nC);
     }
     e->sweep_nC = sweep_width(e, chosen);
-    const size_t h2_need = e->walk_K >= 3 || e->sweep_nC ? (size_t)e->rows * e->d * e->d : 0;
+    const size_t h2_need = e->walk_K >= 3 || (e->sweep_nC && !e->sweep_list) ? (size_t)e->rows * e->d * e->d : 0;
     if (h2_need != e->h2_elems) {
         cudaFree(e->d_h2);
         e->d_h2 = nullptr;
@@ -746,7 +777,7 @@ gg_status finish_create(gg_engine *e, gg_engine **out) {
 }
 
 // A lifted form's table (device memory) -> the pull adjacency d_adj.
-void launch_expand(gg_engine *e, const int32_t *d_table, cudaStream_t st) {
+void launch_expand(gg_engine *e, const int32_t *d_table, cudaStream_t st, const bool sweep = false) {
     const long long n = (long long)e->rows * e->d;
     ExpandArgs x{};
     x.table = d_table;
@@ -755,6 +786,12 @@ void launch_expand(gg_engine *e, const int32_t *d_table, cudaStream_t st) {
     x.rows = e->rows; x.d = e->d; x.N = e->N; x.M = e->M;
     x.Nx = e->dims[0]; x.Ny = e->dims[1]; x.Nz = e->dims[2];
     x.Mx = e->dims[3]; x.My = e->dims[4]; x.Mz = e->dims[5];
+    if (sweep && e->sweep_list) {
+        x.vall = e->d_vall;
+        x.chunks = (long long)sweep_batches(e) * e->rows * e->sweep_nC;
+        x.nC = e->sweep_nC;
+        x.ns_total = (int)e->reps.size();
+    }
     gg::expand_kernel<<<(int)std::min<long long>((n + 255) / 256, 8192), 256, 0, st>>>(x);
 }
 
@@ -990,7 +1027,7 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
     if (walk_K == 4 && e->walk_auto && walk_all_for(e, 3, nb_plain)) walk_K = 3;
     const int launches_plain = 1 + ((long long)e->rows * e->d > 0 ? 1 : 0) + (walk_K > 0 ? 1 : 0) + (walk_K >= 3 ? 1 : 0);
     void *wall = walk_K > 0 ? walk_all_for(e, walk_K, nb_plain) : nullptr;
-    const int launches = sweep ? 4 : launches_plain;
+    const int launches = sweep ? (e->sweep_list ? 3 : 4) : launches_plain;
 
     // Everything the GPU does for one evaluation, on `q`: status words zeroed,
     // table -> adjacency (checked), one cooperative launch for every source
@@ -1016,48 +1053,68 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
                 GG_CK(cudaGetLastError());
             }
         } else if (n > 0) {
-            launch_expand(e, d_table_in, q);
+            launch_expand(e, d_table_in, q, sweep);
             GG_CK(cudaGetLastError());
         }
         if (want_ns)
             GG_CK(cudaMemsetAsync(e->d_level_ns, 0, lv * sizeof(unsigned long long), q));
         if (sweep) {
-            const int K = sweep_K(e->d);
+            const int K = e->sweep_K;
             const SweepKernels k = sweep_for(e->d);
             GG_CK(cudaMemsetAsync(e->d_vtot, 0, (size_t)nb * 3 * sizeof(unsigned long long), q));
-            // the level-2 lists, and with them (whole neighbour rows in a warp) the one-way check
-            const long long nh = n * e->d;
-            const int qd = e->d / 4;
-            const bool h2_checks = e->d % 4 == 0 && (qd & (qd - 1)) == 0 && (nh / 4) % 32 == 0;
-            gg::h2_kernel<<<(int)std::min<long long>((nh + 255) / 256, 8192), 256, 0, q>>>(
-                e->d_adj, e->d_h2, e->rows, e->d, e->form == FORM_GRAPH ? e->d_bad : nullptr,
-                h2_checks ? e->d_wasym : nullptr);
-            GG_CK(cudaGetLastError());
-            if (!h2_checks) {
-                gg::walk_check_kernel<<<(int)std::min<long long>((n + 255) / 256, 8192), 256, 0, q>>>(
-                    e->d_adj, e->rows, e->d, e->d_wasym, e->form == FORM_GRAPH ? e->d_bad : nullptr);
+            if (e->sweep_list) {
+                gg::SourceBallArgs ba{};
+                ba.adj = e->d_adj;
+                ba.src = e->d_src;
+                ba.src_first = e->src_first;
+                ba.ns_total = ns_all;
+                ba.vall = reinterpret_cast<unsigned *>(e->d_vall);
+                ba.counts = e->d_counts;
+                ba.stride = stride;
+                ba.oneway = e->d_wasym;
+                ba.rows = e->rows; ba.nC = e->sweep_nC; ba.K = K;
+                ba.list = e->sweep_ends;
+                ba.ball_blocks = (ns_all + kSrcBallWarps - 1) / kSrcBallWarps;
+                const size_t bsmem = kSrcBallWarps * (size_t)gg::source_ball_warp_bytes(e->rows, e->sweep_ends);
+                GG_CK(cudaFuncSetAttribute(k.source_ball, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem));
+                const int check = (int)std::min<long long>((n + gg::kSrcBallBlock - 1) / gg::kSrcBallBlock, 16 * e->sms);
+                void *bargs[] = {&ba};
+                GG_CK(cudaLaunchKernel(k.source_ball, dim3(ba.ball_blocks + check), dim3(gg::kSrcBallBlock), bargs, bsmem, q));
+            } else {
+                // the level-2 lists, and with them (whole neighbour rows in a warp) the one-way check
+                const long long nh = n * e->d;
+                const int qd = e->d / 4;
+                const bool h2_checks = e->d % 4 == 0 && (qd & (qd - 1)) == 0 && (nh / 4) % 32 == 0;
+                gg::h2_kernel<<<(int)std::min<long long>((nh + 255) / 256, 8192), 256, 0, q>>>(
+                    e->d_adj, e->d_h2, e->rows, e->d, e->form == FORM_GRAPH ? e->d_bad : nullptr,
+                    h2_checks ? e->d_wasym : nullptr);
                 GG_CK(cudaGetLastError());
+                if (!h2_checks) {
+                    gg::walk_check_kernel<<<(int)std::min<long long>((n + 255) / 256, 8192), 256, 0, q>>>(
+                        e->d_adj, e->rows, e->d, e->d_wasym, e->form == FORM_GRAPH ? e->d_bad : nullptr);
+                    GG_CK(cudaGetLastError());
+                }
+                gg::BallArgs ba{};
+                ba.adj = e->d_adj;
+                ba.h2 = e->d_h2;
+                ba.bad = e->form == FORM_GRAPH ? e->d_bad : nullptr;
+                ba.oneway = e->d_wasym;
+                ba.vall = e->d_vall;
+                ba.counts = e->d_counts;
+                ba.stride = stride;
+                ba.rows = e->rows; ba.nC = e->sweep_nC; ba.nb = nb;
+                const size_t bsmem = ball_smem(e);
+                int per_sm = 0;
+                GG_CK(cudaFuncSetAttribute(k.ball, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem));
+                GG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.ball, gg::kBallBlock, bsmem));
+                const int warps = gg::kBallBlock / 32;
+                const int bgrid = std::min((e->rows + warps - 1) / warps, e->sms * std::max(per_sm, 1));
+                void *bargs[] = {&ba};
+                GG_CK(cudaLaunchKernel(k.ball, dim3(bgrid), dim3(gg::kBallBlock), bargs, bsmem, q));
             }
-            gg::BallArgs ba{};
-            ba.adj = e->d_adj;
-            ba.h2 = e->d_h2;
-            ba.bad = e->form == FORM_GRAPH ? e->d_bad : nullptr;
-            ba.oneway = e->d_wasym;
-            ba.vall = e->d_vall;
-            ba.counts = e->d_counts;
-            ba.stride = stride;
-            ba.rows = e->rows; ba.nC = e->sweep_nC; ba.nb = nb;
-            const size_t bsmem = ball_smem(e);
-            int per_sm = 0;
-            GG_CK(cudaFuncSetAttribute(k.ball, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem));
-            GG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.ball, gg::kBallBlock, bsmem));
-            const int warps = gg::kBallBlock / 32;
-            const int bgrid = std::min((e->rows + warps - 1) / warps, e->sms * std::max(per_sm, 1));
-            void *bargs[] = {&ba};
-            GG_CK(cudaLaunchKernel(k.ball, dim3(bgrid), dim3(gg::kBallBlock), bargs, bsmem, q));
             gg::SweepArgs sa{};
             sa.adj = e->d_adj;
-            sa.bad = ba.bad;
+            sa.bad = e->form == FORM_GRAPH ? e->d_bad : nullptr;
             sa.oneway = e->d_wasym;
             sa.vall = e->d_vall;
             sa.A = e->sweep_nC > e->nC ? e->d_swA : e->d_V;
@@ -1073,14 +1130,19 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
             sa.redo = e->d_redo;
             sa.rows = e->rows; sa.nC = e->sweep_nC; sa.nb = nb; sa.K = K;
             sa.max_levels = cap_req;
-            sa.thin_ppm = kSweepThinPpm;
+            sa.ns_total = ns_all;
+            sa.all = e->sweep_list ? 0 : 1;
+            while ((1 << sa.sh) < sa.nC) ++sa.sh;
+            sa.thin_ppm = e->sweep_list ? 0 : kSweepThinPpm;
             sa.last_ppm = sweep_last_ppm(e->d);
-            const int per = (e->rows + e->sms - 1) / e->sms;
+            const bool wide = sa.nC % 32 == 0;
+            const int rows_tile = wide ? 1 : 32 / sa.nC;
+            const int per = ((e->rows + rows_tile - 1) / rows_tile + e->sms - 1) / e->sms * rows_tile;
             const size_t ssmem = (size_t)per * e->d * sizeof(int32_t);
             // two slices of the table a block: a level's and last_rows' (65536 rows of 8: 14 KB each)
             sa.adj_smem_rows = 2 * ssmem <= 38u << 10 ? per : 0;
             void *sargs[] = {&sa};
-            GG_CK(cudaLaunchCooperativeKernel(k.sweep, dim3(e->sms), dim3(gg::kSweepBlock), sargs,
+            GG_CK(cudaLaunchCooperativeKernel(wide ? k.wide : k.narrow, dim3(e->sms), dim3(gg::kSweepBlock), sargs,
                                               sa.adj_smem_rows ? 2 * ssmem : 0, q));
             if (timed) GG_CK(cudaEventRecord(e->ev1, q));
             GG_CK(cudaMemcpyAsync(e->h_status, e->d_status, e->off_counts + (size_t)nb * stride * 8,

@@ -1,10 +1,11 @@
-// Levels after the walk of all batches, when every vertex is a source and the table has
-// no one-way entries: sweep_kernel<D>.  bfs_batch_kernel does the same job in general;
+// Balls of a few steps and the dense levels after them, when every vertex is a source (or,
+// for a lift, one vertex of each orbit) and the table has no one-way entries: ball_kernel
+// or source_ball_kernel, then sweep_kernel<D>.  bfs_batch_kernel does the same job in general;
 // this one takes the plain case, where each level is a whole dense pull, and ends each
 // batch with last_rows.
 //
-// last_rows (one pass in place of the last two levels).  Distances are symmetric here,
-// so of the pairs the levels before L left over it looks only at those whose vertex is
+// last_rows (one pass in place of the last two levels).  Distances are symmetric, so
+// with every vertex a source, of the pairs the levels before L left over it looks only at those whose vertex is
 // in the source's batch or a later one, and counts the later ones twice: half of the
 // rows on average.  A row's chunk that level L does not fill is finished on the spot
 // from two steps away, V_{L+1}[v] = OR of V_{L-1}[w] over the walks v-u-w (the rows of
@@ -176,6 +177,116 @@ __global__ void __launch_bounds__(kBallBlock, 3) ball_kernel(const __grid_consta
         if (s_cnt[k]) atomicAdd(a.counts + (size_t)(k / K) * a.stride + k % K + 1, s_cnt[k]);
 }
 
+// ---------------------------------------------------------------------------
+// source_ball_kernel<D>: the same rows for a list of sources (the orbits of a lift), from
+// the sources' side: one warp walks out from a source, level by level over the new
+// vertices, with a bit per vertex in shared memory, and sets its own bit in each vertex's
+// row by a reduction in L2.  The rows hold the padding beforehand (expand_kernel).  The
+// blocks after ball_blocks do the table's one-way check meanwhile (the lists are as long
+// as the levels need, so that those find room: 16 -> 11 us at 32768 rows of 8).
+// A lift's sources are few: from the rows' side all of them would walk.
+// Bound by the reductions (41 a ns) and, at two levels, by its round trips.  Whole calls,
+// bfs_batch_kernel first: cyclic lift of 1024 x 32, d = 12: 118 -> 104 us; 2-D lift of
+// 32768 vertices, 1024 orbits, d = 8: 120 -> 97; 60000 vertices, 2000 orbits, d = 4: 240 ->
+// 136; 60000, 4000, d = 12: 362 -> 209; 50000, 10000, d = 8: 422 -> 393.
+// ---------------------------------------------------------------------------
+constexpr int kSrcBallBlock = 128;
+constexpr int kSrcBallList = 1024;   // most new vertices of a level that a warp walks on from
+constexpr int kSrcBallLevels = 16;
+
+struct SourceBallArgs {
+    const int32_t *adj;       // [rows][D]
+    const int32_t *src;       // sources, or nullptr: src_first, src_first + 1, ...
+    int src_first, ns_total;
+    unsigned *vall;           // [nb][rows][nC] uint4
+    unsigned long long *counts;
+    int stride;
+    int *oneway;
+    int rows, nC, K;
+    int list;                 // most new vertices of a level below K: D^(K-1), one-way entries included
+    int ball_blocks;
+};
+
+__host__ __device__ constexpr int source_ball_warp_bytes(int rows, int list) {
+    return (rows + 127) / 128 * 16 + 2 * ((list + 3) / 4 * 4) * 4;
+}
+
+template <int D>
+__global__ void __launch_bounds__(kSrcBallBlock) source_ball_kernel(const __grid_constant__ SourceBallArgs a) {
+    extern __shared__ __align__(16) unsigned char s_ball[];
+    __shared__ unsigned s_cnt[kSrcBallLevels];
+    if ((int)blockIdx.x >= a.ball_blocks) {
+        const long long n = (long long)a.rows * D;
+        for (long long k = (long long)(blockIdx.x - a.ball_blocks) * blockDim.x + threadIdx.x; k < n;
+             k += (long long)(gridDim.x - a.ball_blocks) * blockDim.x) {
+            const int v = (int)(k / D);
+            const int32_t *ur = a.adj + (size_t)__ldg(a.adj + k) * D;
+            bool f = false;
+#pragma unroll
+            for (int j = 0; j < D; ++j) f |= __ldg(ur + j) == v;
+            if (!f) *a.oneway = 1;
+        }
+        return;
+    }
+    const unsigned lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
+    const int words4 = (a.rows + 127) / 128;
+    uint4 *set4 = reinterpret_cast<uint4 *>(s_ball + (size_t)wib * source_ball_warp_bytes(a.rows, a.list));
+    unsigned *set = reinterpret_cast<unsigned *>(set4);
+    int *lists = reinterpret_cast<int *>(set4 + words4);
+    const int S = 128 * a.nC, half = (a.list + 3) / 4 * 4;
+    const int j = (int)(blockIdx.x * (kSrcBallBlock / 32) + wib);   // (a batch's sources are whole blocks)
+    if (threadIdx.x < kSrcBallLevels) s_cnt[threadIdx.x] = 0u;
+    __syncthreads();
+    if (j < a.ns_total) {
+        for (int i = (int)lane; i < words4; i += 32) set4[i] = u4zero();
+        const int s = a.src ? __ldg(a.src + j) : a.src_first + j;
+        const int b = j / S, jj = j - b * S;
+        unsigned *col = a.vall + (size_t)b * a.rows * a.nC * 4 + (jj >> 5);
+        const unsigned mine = 1u << (jj & 31);
+        const size_t pitch = (size_t)a.nC * 4;
+        if (lane == 0) {
+            lists[0] = s;
+            atomicOr(col + (size_t)s * pitch, mine);
+        }
+        __syncwarp();
+        if (lane == 0) set[s >> 5] = 1u << (s & 31);
+        __syncwarp();
+        int n = 1;
+        for (int L = 1; L <= a.K && n > 0; ++L) {
+            const int *list = lists + ((L - 1) & 1) * half;
+            int *next = lists + (L & 1) * half;
+            const int total = n * D;
+            int nn = 0;
+            for (int i0 = 0; i0 < total; i0 += 32 * 8) {
+                unsigned w[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const int i = i0 + 32 * k + (int)lane;
+                    w[k] = i < total ? (unsigned)__ldg(a.adj + (size_t)list[i / D] * D + i % D) : 0u;
+                }
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    if (i0 + 32 * k >= total) break;
+                    const unsigned bit = 1u << (w[k] & 31u);
+                    const bool fresh = i0 + 32 * k + (int)lane < total && (atomicOr(set + (w[k] >> 5), bit) & bit) == 0u;
+                    if (fresh) atomicOr(col + w[k] * pitch, mine);
+                    const unsigned m = __ballot_sync(0xffffffffu, fresh);
+                    const int at = nn + __popc(m & ((1u << lane) - 1u));
+                    if (fresh && L < a.K && at < half) next[at] = (int)w[k];   // (never more: D^L at most)
+                    nn += __popc(m);
+                }
+            }
+            if (lane == 0) atomicAdd(s_cnt + L, (unsigned)nn);
+            n = min(nn, half);
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x >= 1u && (int)threadIdx.x <= a.K && s_cnt[threadIdx.x])
+        atomicAdd(a.counts + (size_t)((int)(blockIdx.x * (kSrcBallBlock / 32)) / S) * a.stride + threadIdx.x,
+                  (unsigned long long)s_cnt[threadIdx.x]);
+}
+
 constexpr int kSweepBlock = 1024;   // one block per SM: a grid barrier takes 148 arrivals, not 592
 
 struct SweepArgs {
@@ -193,6 +304,8 @@ struct SweepArgs {
     unsigned long long *batch_ns;
     int *redo;
     int rows, nC, nb, K, max_levels;
+    int ns_total, all;        // sources; 1: every vertex, in order (last_rows takes half of the rows)
+    int sh;                   // log2 of nC, when that is below 32
     int thin_ppm;             // below this share of the pairs a feeding frontier is thin
     int last_ppm;             // last_rows once fewer of the pairs than this are left
     int adj_smem_rows;
@@ -215,6 +328,46 @@ struct SweepState {
     unsigned epoch;           // grid barriers passed
     int act;                  // next step: 0 level, 1 last_rows, 2 batch done, 3 give up
 };
+
+// Row and chunk of a lane in tile t (32 chunks in a row).  Batches of whole 4096-source
+// parts (kOnePart: one): a part of one row; narrower ones (kNarrow): 32 / nC rows.  False:
+// past the last row.
+enum { kOnePart = 0, kParts = 1, kNarrow = 2 };
+template <int MODE>
+__device__ __forceinline__ bool tile_place(const SweepArgs &a, const unsigned t, const unsigned lane, unsigned &v, unsigned &at) {
+    if constexpr (MODE == kOnePart) {
+        v = t;
+        at = lane;
+    } else if constexpr (MODE == kParts) {
+        const unsigned parts = (unsigned)a.nC / 32u;
+        v = t / parts;
+        at = (t - v * parts) * 32u + lane;
+    } else {
+        const unsigned item = t * 32u + lane;
+        v = item >> a.sh;
+        at = item & ((1u << a.sh) - 1u);
+        if (v >= (unsigned)a.rows) {
+            v = (unsigned)a.rows - 1u;
+            return false;
+        }
+    }
+    return true;
+}
+
+// The block's share [lo, hi) of the tiles of the rows from v0 on, and the rows they lie in.
+template <bool WIDE>
+__device__ __forceinline__ void tile_share(const SweepArgs &a, const unsigned v0, unsigned &t_lo, unsigned &t_hi, unsigned &r_lo,
+                                           unsigned &r_hi) {
+    const unsigned step = WIDE ? (unsigned)a.nC / 32u : 1u;                     // tiles that stay together
+    const unsigned first = WIDE ? v0 : 0u;
+    const unsigned n = WIDE ? (unsigned)a.rows - v0 : ((unsigned)a.rows * (unsigned)a.nC + 31u) / 32u;
+    const unsigned lo = first + (unsigned)((unsigned long long)n * blockIdx.x / gridDim.x);
+    const unsigned hi = first + (unsigned)((unsigned long long)n * (blockIdx.x + 1) / gridDim.x);
+    t_lo = lo * step;
+    t_hi = hi * step;
+    r_lo = WIDE ? lo : lo * (32u >> a.sh);
+    r_hi = WIDE ? hi : min((unsigned)a.rows, hi * (32u >> a.sh));
+}
 
 // Adjacency row v of the table, the same in every lane.
 template <int D>
@@ -260,34 +413,35 @@ static __device__ __noinline__ unsigned finish_chunks(const SweepArgs &a, const 
         for (int j = 0; j < D; ++j) or_into(q, x[j]);
     }
     if (!u4full(q)) *a.redo = 1;
-    const int bv = (int)(v / (128u * nC));
-    // level L + 1 is not empty for either batch of these pairs
     atomicMax(a.levels_run + b, L + 1);
+    if (!a.all) return miss;
+    const int bv = (int)(v / (128u * nC));
+    // (level L + 1 is not empty for either batch of these pairs)
     atomicMax(a.levels_run + bv, L + 1);
     return bv == b ? miss : 2u * miss;
 }
 
-// The block's share of the rows from batch b on (its slice of the table to s_row first).  A tile takes the first H neighbours of its row, such that a chunk is
-// then rarely open; those go on a list of the warp's and are finished 32 at a time.  (At
+// The block's share of the rows from batch b on (its slice of the table to s_row first).
+// A tile takes the first H neighbours of its row, such that a chunk is then rarely open;
+// those go on a list of the warp's and are finished 32 at a time.  (At
 // once, a warp in three waited for a second round of gathers; and in line with the kernel,
 // as sweep_rows: as a call the loop's gathers were held back by the registers kept for the
 // caller.  All rows of n = 65536, d = 8 on an 8192-source batch: 31 -> 27 us.)
-template <int D, int H>
+template <int D, int H, bool WIDE>
 __device__ __forceinline__ unsigned last_rows(const SweepArgs &a, SweepState &S, const int b, const int L,
                                               int32_t *s_row, unsigned *list) {
     constexpr int U = H <= 4 ? 8 / H : 1;   // tiles a round: up to 8 gathers in flight
     const uint4 *X = S.X;
     const unsigned lane = threadIdx.x & 31u;
-    const unsigned nC = (unsigned)a.nC, parts = nC / 32u;
-    const unsigned v0 = (unsigned)b * 128u * nC, left = (unsigned)a.rows - v0;
-    const unsigned r_lo = v0 + (unsigned)((unsigned long long)left * blockIdx.x / gridDim.x);
-    const unsigned r_hi = v0 + (unsigned)((unsigned long long)left * (blockIdx.x + 1) / gridDim.x);
-    const bool keep = r_hi - r_lo <= (unsigned)a.adj_smem_rows;
+    const unsigned nC = (unsigned)a.nC;
+    unsigned t_lo, t_end, r_lo, r_hi;
+    tile_share<WIDE>(a, a.all ? (unsigned)b * 128u * nC : 0u, t_lo, t_end, r_lo, r_hi);
+    const bool keep = r_hi <= r_lo + (unsigned)a.adj_smem_rows;
     if (keep)
-        for (unsigned k = threadIdx.x; k < (r_hi - r_lo) * D; k += blockDim.x) s_row[k] = __ldg(a.adj + (size_t)r_lo * D + k);
+        for (unsigned k = threadIdx.x; r_lo < r_hi && k < (r_hi - r_lo) * D; k += blockDim.x) s_row[k] = __ldg(a.adj + (size_t)r_lo * D + k);
     const int32_t *adj = keep ? s_row : a.adj;
-    const unsigned v_base = keep ? r_lo : 0u, t_end = r_hi * parts;
-    if (threadIdx.x == 0) S.next = r_lo * parts;
+    const unsigned v_base = keep ? r_lo : 0u;
+    if (threadIdx.x == 0) S.next = t_lo;
     __syncthreads();
     unsigned cnt = 0u, open = 0u;
     for (;;) {
@@ -296,10 +450,11 @@ __device__ __forceinline__ unsigned last_rows(const SweepArgs &a, SweepState &S,
         t0 = __shfl_sync(0xffffffffu, t0, 0);
         if (t0 >= t_end) break;
         uint4 x[U][H];
+        bool in[U];
 #pragma unroll
         for (int k = 0; k < U; ++k) {
-            const unsigned t = min(t0 + (unsigned)k, t_end - 1u);
-            const unsigned v = parts == 1u ? t : t / parts, at = (t - v * parts) * 32u + lane;
+            unsigned v, at;
+            in[k] = tile_place<WIDE ? kParts : kNarrow>(a, min(t0 + (unsigned)k, t_end - 1u), lane, v, at);
             const int32_t *row = adj + (size_t)(v - v_base) * D;
 #pragma unroll
             for (int i = 0; i < H; ++i) x[k][i] = __ldcg(X + ((unsigned)row[i] * nC + at));
@@ -309,7 +464,7 @@ __device__ __forceinline__ unsigned last_rows(const SweepArgs &a, SweepState &S,
             uint4 q = x[k][0];
 #pragma unroll
             for (int i = 1; i < H; ++i) or_into(q, x[k][i]);
-            const bool o = t0 + (unsigned)k < t_end && !u4full(q);
+            const bool o = t0 + (unsigned)k < t_end && in[k] && !u4full(q);
             const unsigned m = __ballot_sync(0xffffffffu, o);
             if (m == 0u) continue;
             if (o) list[open + __popc(m & ((1u << lane) - 1u))] = (t0 + (unsigned)k) * 32u + lane;
@@ -340,22 +495,22 @@ __device__ __forceinline__ int last_half(const int D, const float u) {
     return D <= 8 ? D : 8;
 }
 
-template <int D>
+template <int D, bool WIDE>
 __device__ __forceinline__ unsigned last_rows_of(const SweepArgs &a, SweepState &S, const int b, const int L,
                                                  int32_t *s_row, unsigned *list) {
     const int H = S.half;
-    if (H == 2) return last_rows<D, 2>(a, S, b, L, s_row, list);
-    if constexpr (D >= 3) if (H == 3) return last_rows<D, 3>(a, S, b, L, s_row, list);
-    if constexpr (D >= 4) if (H == 4) return last_rows<D, 4>(a, S, b, L, s_row, list);
-    if constexpr (D >= 6) if (H == 6) return last_rows<D, 6>(a, S, b, L, s_row, list);
-    return last_rows<D, (D < 8 ? D : 8)>(a, S, b, L, s_row, list);
+    if (H == 2) return last_rows<D, 2, WIDE>(a, S, b, L, s_row, list);
+    if constexpr (D >= 3) if (H == 3) return last_rows<D, 3, WIDE>(a, S, b, L, s_row, list);
+    if constexpr (D >= 4) if (H == 4) return last_rows<D, 4, WIDE>(a, S, b, L, s_row, list);
+    if constexpr (D >= 6) if (H == 6) return last_rows<D, 6, WIDE>(a, S, b, L, s_row, list);
+    return last_rows<D, (D < 8 ? D : 8), WIDE>(a, S, b, L, s_row, list);
 }
 
 // One dense level on the block's tiles [next, t_hi): Y[v] = OR of the neighbours' X
 // rows (without one-way entries V_{L-1}[v] lies within them for L >= 2), and this
 // thread's popcount of what it wrote.
-template <int D, bool ONE>
-__device__ __forceinline__ unsigned sweep_rows(SweepState &S, const unsigned parts) {
+template <int D, int MODE>
+__device__ __forceinline__ unsigned sweep_rows(const SweepArgs &a, SweepState &S) {
     const unsigned lane = threadIdx.x & 31u;
     const uint4 *X = S.X;
     uint4 *Y = S.Y;
@@ -367,8 +522,9 @@ __device__ __forceinline__ unsigned sweep_rows(SweepState &S, const unsigned par
         if (lane == 0) t = atomicAdd(&S.next, 1u);
         t = __shfl_sync(0xffffffffu, t, 0);
         if (t >= t_hi) break;
-        const unsigned v = ONE ? t : t / parts, at = ONE ? lane : (t - v * parts) * 32u + lane;
-        const unsigned w = ONE ? 32u : 32u * parts;
+        unsigned v, at;
+        const bool in = tile_place<MODE>(a, t, lane, v, at);
+        const unsigned w = MODE == kOnePart ? 32u : (unsigned)a.nC;
         const int32_t *row = adj + (size_t)(v - v_base) * D;
         unsigned tu[D];
 #pragma unroll
@@ -379,8 +535,10 @@ __device__ __forceinline__ unsigned sweep_rows(SweepState &S, const unsigned par
         uint4 q = x[0];
 #pragma unroll
         for (int i = 1; i < D; ++i) or_into(q, x[i]);
-        Y[(size_t)t * 32 + lane] = q;
-        cnt += u4popc(q);
+        if (in) {
+            Y[(size_t)t * 32 + lane] = q;
+            cnt += u4popc(q);
+        }
     }
     return cnt;
 }
@@ -394,17 +552,17 @@ __device__ __forceinline__ void sweep_next(const SweepArgs &a, SweepState &S, co
         S.act = 2;
         return;
     }
-    if (b == 0 && S.last == 0 && L >= 2 && left * 1000000ull < S.pairs * (unsigned long long)a.last_ppm) S.last = L;
+    if ((b == 0 || !a.all) && S.last == 0 && L >= 2 && left * 1000000ull < S.pairs * (unsigned long long)a.last_ppm) S.last = L;
     if (L == S.last) {
         S.act = L + 1 <= a.max_levels ? 1 : 3;
         S.half = last_half(D, (float)left / (float)S.pairs);
     } else {
-        const bool thin = S.c_prev * 1000000ull < S.pairs * (unsigned long long)a.thin_ppm;
+        const bool thin = S.c_prev == 0ull || S.c_prev * 1000000ull < S.pairs * (unsigned long long)a.thin_ppm;
         S.act = thin || L > a.max_levels ? 3 : 0;
     }
 }
 
-template <int D>
+template <int D, bool WIDE>
 __global__ void __launch_bounds__(kSweepBlock, 1) sweep_kernel(const __grid_constant__ SweepArgs a) {
     extern __shared__ int32_t s_adj[];
     __shared__ unsigned s_open[kSweepBlock / 32][64];   // last_rows' lists (one array for all its instances)
@@ -415,16 +573,16 @@ __global__ void __launch_bounds__(kSweepBlock, 1) sweep_kernel(const __grid_cons
         return;
     }
     {
-        const unsigned v_lo = (unsigned)((unsigned long long)a.rows * blockIdx.x / gridDim.x);
-        const unsigned v_hi = (unsigned)((unsigned long long)a.rows * (blockIdx.x + 1) / gridDim.x);
-        const bool keep = v_hi - v_lo <= (unsigned)a.adj_smem_rows;   // the block's slice of the table
+        unsigned t_lo, t_hi, v_lo, v_hi;
+        tile_share<WIDE>(a, 0u, t_lo, t_hi, v_lo, v_hi);
+        const bool keep = v_hi <= v_lo + (unsigned)a.adj_smem_rows;   // the block's slice of the table
         if (keep)
-            for (unsigned k = threadIdx.x; k < (v_hi - v_lo) * D; k += blockDim.x) s_adj[k] = __ldg(a.adj + (size_t)v_lo * D + k);
+            for (unsigned k = threadIdx.x; v_lo < v_hi && k < (v_hi - v_lo) * D; k += blockDim.x) s_adj[k] = __ldg(a.adj + (size_t)v_lo * D + k);
         if (threadIdx.x == 0) {
             S.adj = keep ? s_adj : a.adj;
             S.v_base = keep ? v_lo : 0u;
-            S.t_lo = v_lo * ((unsigned)a.nC / 32u);
-            S.t_hi = v_hi * ((unsigned)a.nC / 32u);
+            S.t_lo = t_lo;
+            S.t_hi = t_hi;
             S.last = 0;
             S.epoch = 0u;
             S.Y = a.A;
@@ -433,7 +591,7 @@ __global__ void __launch_bounds__(kSweepBlock, 1) sweep_kernel(const __grid_cons
     for (int b = 0; b < a.nb; ++b) {
         int L = a.K + 1;
         if (threadIdx.x == 0) {
-            const int ns = min(128 * a.nC, a.rows - b * 128 * a.nC);
+            const int ns = min(128 * a.nC, a.ns_total - b * 128 * a.nC);
             unsigned long long *counts = a.counts + (size_t)b * (size_t)a.stride;
             if (blockIdx.x == 0) {
                 a.batch_ns[2 * b] = gtimer();
@@ -442,6 +600,7 @@ __global__ void __launch_bounds__(kSweepBlock, 1) sweep_kernel(const __grid_cons
             S.pairs = (unsigned long long)ns * (unsigned long long)a.rows;
             S.reached = (unsigned long long)ns;
             S.c_prev = 0ull;
+            if (!a.all) S.last = 0;
             S.X = a.vall + (size_t)b * ((size_t)a.rows * (size_t)a.nC);
             int k = 1;
             for (; k <= a.K && S.reached < S.pairs; ++k) {
@@ -454,7 +613,7 @@ __global__ void __launch_bounds__(kSweepBlock, 1) sweep_kernel(const __grid_cons
         }
         __syncthreads();
         for (; S.act == 0; ++L) {
-            const unsigned cnt = a.nC == 32 ? sweep_rows<D, true>(S, 1u) : sweep_rows<D, false>(S, (unsigned)a.nC / 32u);
+            const unsigned cnt = !WIDE ? sweep_rows<D, kNarrow>(a, S) : a.nC == 32 ? sweep_rows<D, kOnePart>(a, S) : sweep_rows<D, kParts>(a, S);
             const unsigned wsum = __reduce_add_sync(0xffffffffu, cnt);
             if ((threadIdx.x & 31u) == 0u) atomicAdd(&S.sum, (unsigned long long)wsum);
             __syncthreads();
@@ -468,7 +627,7 @@ __global__ void __launch_bounds__(kSweepBlock, 1) sweep_kernel(const __grid_cons
             if (!grid_sync_value(a.ctl, a.expected, a.wait_ns, L, epoch, vt + L % 3, total)) return;
             if (threadIdx.x == 0) {
                 // total bits of V_L less the padding and the pairs reached before
-                const int ns = min(128 * a.nC, a.rows - b * 128 * a.nC);
+                const int ns = min(128 * a.nC, a.ns_total - b * 128 * a.nC);
                 const unsigned long long pad = (unsigned long long)a.rows * (unsigned long long)(128 * a.nC - ns);
                 const unsigned long long cL = total - pad - S.reached;
                 if (blockIdx.x == 0) a.counts[(size_t)b * (size_t)a.stride + L] = cL;
@@ -495,7 +654,7 @@ __global__ void __launch_bounds__(kSweepBlock, 1) sweep_kernel(const __grid_cons
                 atomicMax(a.levels_run + b, L);
                 atomicAdd(counts, S.pairs - S.reached);
             }
-            const unsigned cnt = last_rows_of<D>(a, S, b, L, s_adj + (size_t)a.adj_smem_rows * D, s_open[threadIdx.x >> 5]);
+            const unsigned cnt = last_rows_of<D, WIDE>(a, S, b, L, s_adj + (size_t)a.adj_smem_rows * D, s_open[threadIdx.x >> 5]);
             const unsigned m = __reduce_add_sync(0xffffffffu, cnt);
             if ((threadIdx.x & 31u) == 0u && m) {
                 atomicAdd(counts, 0ull - (unsigned long long)m);

@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 import graphgolf as G
+import instances as I
 import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -90,3 +91,43 @@ def test_sweep_gives_up_where_it_must(what, monkeypatch):
     r = both(monkeypatch, n, d, 4096, [full(adj, 1200)])
     if what != "ring":
         check_oracle(r, adj)
+
+
+@pytest.mark.parametrize("form,args", [("part", (64, 40, 3)), ("part", (100, 30, 4)), ("part", (129, 17, 6)), ("part", (500, 12, 6)),
+                                       ("part", (700, 9, 5)), ("part", (1024, 32, 12)), ("part", (1500, 11, 7)), ("part", (2500, 5, 8)),
+                                       ("part", (4200, 3, 9)), ("part", (66, 500, 3)), ("piece", (16, 20, 4, 3, 8)),
+                                       ("piece", (30, 33, 2, 5, 10)), ("box", (8, 4, 6, 2, 3, 2, 6)), ("halves", ()), ("one-way", ()),
+                                       ("ring", ())])
+def test_source_list_equals_the_level_loop(form, args, monkeypatch):
+    if form == "piece":
+        a = G.piece_lift(*args, 1)
+        make, T = (lambda: G.cudaASPLpiece(*a[:4], args[-1])), a[4]
+    elif form == "box":
+        a = I.random_box(*args, 1)
+        make, T = (lambda: G.cudaASPLbox(*a[:6], args[-1])), a[6]
+    else:
+        if form == "part":
+            N, M, T = G.cyclic_lift(*args, 2)
+        elif form == "halves":            # even steps only: the two residues never meet
+            N, M, T = 8000, 8, np.array([[2, -2, 1000, -1000]] * 8, np.int32)
+        elif form == "ring":
+            N, M, T = 4000, 100, np.array([[1, -1, 2, -2]] * 100, np.int32)
+        else:
+            N, M, T = G.cyclic_lift(300, 11, 5, 3)
+            T = T.copy()
+            T[7, 2] += 1
+        make = lambda: G.cudaASPLconv(N, M, T.shape[1])
+    T = np.ascontiguousarray(T, dtype=np.int32)
+    monkeypatch.setenv("GG_DIRECT", "0")
+    out = []
+    for sweep in ("0", "1"):
+        monkeypatch.setenv("GG_SWEEP", sweep)
+        e = make()
+        out.append([e.eval(T, max_levels=cap, level_counts=True) for cap in (1100, 1100, 4)] + [e.diameterASPL(T)])
+        e.close()
+    for want, got in zip(*out):
+        if isinstance(want, tuple):
+            assert got == want
+        else:
+            assert all(got[k] == want[k] for k in KEYS)
+            assert np.array_equal(got["level_counts"], want["level_counts"])
