@@ -4,8 +4,9 @@
 // construction from its form and dimensions, the way the reference calculators
 // size theirs in their constructors (cudaASPLconv.cu:122-137,
 // cudaASPLgraph.cu:114-127).  An evaluation is:
-//   H2D of the packed table -> expand_kernel (lifted forms) -> one cooperative
-//   bfs_batch_kernel launch per source batch -> one D2H of the level counters
+//   H2D of the packed table -> expand_kernel (lifted forms) -> direct_kernel (small
+//   ones), balls and sweep_kernel (every vertex, or a lift's orbits), or the general
+//   bfs_batch_kernel over every source batch -> one D2H of the level counters
 //   -> exact host fold into gg_result -> the reference's return convention.
 // There is no per-level host round trip: the level loop, its termination test
 // and the connectivity test live on the device.
@@ -383,10 +384,13 @@ bool vall_room(gg_engine *e, size_t chunks) {
     return true;
 }
 
+// The rows of every batch for sweep_kernel: d_F1 where one batch fits it, else d_vall.
+bool sweep_in_f1(const gg_engine *e, int nb) { return nb == 1 && e->sweep_nC <= e->nC; }
+
 // sweep_kernel's level buffers: d_V and d_F0, or a wider pair of its own.
 bool sweep_room(gg_engine *e, int nb) {
     const size_t chunks = (size_t)e->rows * e->sweep_nC;
-    if ((!e->sweep_list && !e->h2_elems) || !vall_room(e, nb * chunks)) return false;
+    if ((!e->sweep_list && !e->h2_elems) || (!sweep_in_f1(e, nb) && !vall_room(e, nb * chunks))) return false;
     if (e->sweep_nC <= e->nC || chunks <= e->sw_chunks) return true;
     invalidate_graph(e);
     cudaFree(e->d_swA); cudaFree(e->d_swB);
@@ -787,7 +791,7 @@ void launch_expand(gg_engine *e, const int32_t *d_table, cudaStream_t st, const 
     x.Nx = e->dims[0]; x.Ny = e->dims[1]; x.Nz = e->dims[2];
     x.Mx = e->dims[3]; x.My = e->dims[4]; x.Mz = e->dims[5];
     if (sweep && e->sweep_list) {
-        x.vall = e->d_vall;
+        x.vall = sweep_in_f1(e, sweep_batches(e)) ? e->d_F1 : e->d_vall;
         x.chunks = (long long)sweep_batches(e) * e->rows * e->sweep_nC;
         x.nC = e->sweep_nC;
         x.ns_total = (int)e->reps.size();
@@ -1060,6 +1064,7 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
             GG_CK(cudaMemsetAsync(e->d_level_ns, 0, lv * sizeof(unsigned long long), q));
         if (sweep) {
             const int K = e->sweep_K;
+            uint4 *vall = sweep_in_f1(e, nb) ? e->d_F1 : e->d_vall;
             const SweepKernels k = sweep_for(e->d);
             GG_CK(cudaMemsetAsync(e->d_vtot, 0, (size_t)nb * 3 * sizeof(unsigned long long), q));
             if (e->sweep_list) {
@@ -1068,7 +1073,7 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
                 ba.src = e->d_src;
                 ba.src_first = e->src_first;
                 ba.ns_total = ns_all;
-                ba.vall = reinterpret_cast<unsigned *>(e->d_vall);
+                ba.vall = reinterpret_cast<unsigned *>(vall);
                 ba.counts = e->d_counts;
                 ba.stride = stride;
                 ba.oneway = e->d_wasym;
@@ -1099,7 +1104,7 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
                 ba.h2 = e->d_h2;
                 ba.bad = e->form == FORM_GRAPH ? e->d_bad : nullptr;
                 ba.oneway = e->d_wasym;
-                ba.vall = e->d_vall;
+                ba.vall = vall;
                 ba.counts = e->d_counts;
                 ba.stride = stride;
                 ba.rows = e->rows; ba.nC = e->sweep_nC; ba.nb = nb;
@@ -1116,7 +1121,7 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
             sa.adj = e->d_adj;
             sa.bad = e->form == FORM_GRAPH ? e->d_bad : nullptr;
             sa.oneway = e->d_wasym;
-            sa.vall = e->d_vall;
+            sa.vall = vall;
             sa.A = e->sweep_nC > e->nC ? e->d_swA : e->d_V;
             sa.B = e->sweep_nC > e->nC ? e->d_swB : e->d_F0;
             sa.ctl = e->d_ctl;
