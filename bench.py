@@ -66,7 +66,7 @@ WORKLOADS = {
     # geometric schedule 1e-3*ASPL -> 1e-6 over 1e5 steps, 32 exact scores per step
     "anneal_n4096_d8_time_to_target": dict(form="anneal", n=4096, d=8, seed=1, steps=100000),
     # one 2-opt move of a random 8-regular n=65536 graph per step, scored exactly by
-    # searching again only from the affected sources (gg_inc_eval)
+    # searching again only from the affected sources near the edit (gg_inc_eval)
     "incremental_n65536_d8": dict(form="incremental", n=65536, d=8, seed=1),
     # 256 shift / orbit 2-opt moves of a random cyclic lift (m=1024 orbits, g=32,
     # degree 12, N=32768) per step, all scored in one launch (gg_lift_eval)
@@ -489,7 +489,7 @@ def run_ours(args):
         l2 = {"gather_peak_gbs": gp, "gather_pass_ms": gms,
               "what": f"gg_gather_peak: {wl['N']} rows x ({wl['d']} random + 1 own) 512-byte row reads + "
                       "1 row write per pass, the access pattern of one dense BFS level of one source "
-                      "batch, arrays L2-resident",
+                      "batch, arrays L2-resident (levels_batch0_us: the general level loop, which per-level times ask for)",
               "levels_batch0_us": level_us,
               "dense_level_floor_us": floor_us,
               "dense_level_frac": (floor_us / statistics.median(dense)) if dense else None,
@@ -625,7 +625,7 @@ def bit_edges_per_eval(wl, r):
 
 def run_incremental(args):
     """One exact 2-opt move evaluation per step (gg_inc_eval: affected-source test
-    with the cached per-source sums, search from the affected sources).
+    with the cached per-source sums, search from the affected sources near the edit).
     The call is blocking and reads a count back halfway, so a step is timed by the
     host clock around the call (L2 flushed and the device idle before each step);
     that is also the end-to-end figure.  The full calculator call on the same moved

@@ -293,7 +293,8 @@ gg_status gg_inc_create(int n, int degree, int device, gg_inc **out);
 /* Make adj the current graph (full evaluation; r may be NULL). */
 gg_status gg_inc_set_graph(gg_inc *h, const int32_t *adj, gg_result *r);
 /* Exact counts of the current graph with move s applied (s->base is ignored);
- * *affected = sources searched again (may be NULL).  The current graph is kept. */
+ * *affected = sources the move can affect (may be NULL; only those near the edit are
+ * searched again).  The current graph is kept. */
 gg_status gg_inc_eval(gg_inc *h, const gg_swap *s, gg_cand_result *out, int *affected);
 /* Apply move s to the current graph (full evaluation; r may be NULL). */
 gg_status gg_inc_commit(gg_inc *h, const gg_swap *s, gg_result *r);
