@@ -8,7 +8,11 @@
 // there is to do (L2 round trips and a grid barrier).
 //
 // The first levels come from the sources' walk ends (a walk of length L from a source
-// sets its bit at the end) while those are few.
+// sets its bit at the end) while those are few.  A walk follows the table's rows from the
+// source, so its ends are what the source pulls from; they are the vertices that reach it,
+// too, when the table has no one-way entries.  The blocks check that between them (a share
+// of the rows each, d look-ups an entry) and the last one tells the host, which runs a
+// table that has some again without walks, every level a pass.
 //
 // The last block to finish writes the counters to host memory, clears them for the next
 // launch and stores the launch's number, which the host waits for: an evaluation is this
@@ -28,6 +32,7 @@ struct DirectCtl {
     unsigned done;       // blocks that finished
     int levels_run;      // last level executed by any block
     int bad;             // an adjacency entry outside [0, rows)
+    int oneway;          // the walk met a table with one-way entries: the counters are not its counts
     unsigned seq;        // host: the number of the launch that handed its counters over
 };
 
@@ -39,6 +44,11 @@ struct DirectArgs {
     int max_levels;
     const uint16_t *adj16;    // the same ids, checked by the caller (device or pinned host memory), or nullptr
     int adj_smem;             // the rows as 16-bit ids in shared memory (range-checked on the way from adj)
+    // The first levels by walks: rows to check for one-way entries (0: no walks, nothing to
+    // check): all of them, or, for a lift whose orbits translate onto one another, those of
+    // its sources (check_src: the list's vertices, else src_first ..)
+    int check;
+    int check_src;
     unsigned seq;             // number of this launch
     const int *bad_table;     // or set by a check kernel before; nullptr: checked already
     DirectCtl *ctl, *h_ctl;   // device (zero between launches), host
@@ -204,6 +214,21 @@ __global__ void __launch_bounds__(kDirectBlock, 1) direct_kernel(const DirectArg
     int L = 0, executed = 0;
     if (!any_bad) {
         for (int j = tid; j < ns; j += nthr) set_bit(vertex(j), j);
+        if (a.check) {
+            // the block's share of the one-way check: is v among the neighbours of its neighbour u?
+            auto entry = [&](const size_t at) { return smem ? (int)sadj[at] : __ldg(a.adj + at); };
+            const int lo = (int)((long long)a.check * blockIdx.x / gridDim.x);
+            const int hi = (int)((long long)a.check * (blockIdx.x + 1) / gridDim.x);
+            for (int k = tid; k < (hi - lo) * d; k += nthr) {
+                const int i = lo + k / d;
+                const int v = !a.check_src ? i : a.src ? __ldg(a.src + i) : a.src_first + i;
+                const size_t u = (size_t)entry((size_t)v * d + k % d) * d;
+                bool back = false;
+#pragma unroll 4
+                for (int l = 0; l < d; ++l) back |= entry(u + l) == v;
+                if (!back) a.ctl->oneway = 1;
+            }
+        }
         __syncthreads();
         const unsigned all = (unsigned)ns * (unsigned)rows;   // (rows < 2^16, ns <= 128)
         unsigned seen = (unsigned)ns;
@@ -235,7 +260,7 @@ __global__ void __launch_bounds__(kDirectBlock, 1) direct_kernel(const DirectArg
             done = c == 0u || seen == all || L >= a.max_levels;
         };
         L = 1;
-        for (unsigned ends = (unsigned)d; !done; ends *= (unsigned)d, ++L) {
+        for (unsigned ends = (unsigned)d; a.check && !done; ends *= (unsigned)d, ++L) {
             if ((unsigned long long)ends * (unsigned)ns > (unsigned long long)kDirectWalk * (unsigned)rows) break;
             // a thread takes a walk of L - 1 steps and its d ends (the ids of one row)
             unsigned cnt = 0u;
@@ -293,6 +318,7 @@ __global__ void __launch_bounds__(kDirectBlock, 1) direct_kernel(const DirectArg
     if (!s_last) return;
     __threadfence();
     const int run = ld_acquire_i(&a.ctl->levels_run), is_bad = ld_acquire_i(&a.ctl->bad);
+    const int is_oneway = ld_acquire_i(&a.ctl->oneway);
     for (int l = tid; l <= run; l += nthr) {
         a.h_counts[l] = l == 0 ? (unsigned long long)a.ns_total : __ldcg(a.counts + l);
         a.counts[l] = 0ull;
@@ -305,9 +331,11 @@ __global__ void __launch_bounds__(kDirectBlock, 1) direct_kernel(const DirectArg
     if (tid == 0) {
         a.h_ctl->levels_run = run;
         a.h_ctl->bad = is_bad;
+        a.h_ctl->oneway = is_oneway;
         a.ctl->done = 0u;
         a.ctl->levels_run = 0;
         a.ctl->bad = 0;
+        a.ctl->oneway = 0;
         a.batch_ns[1] = gtimer();
     }
     // everything above reaches the host before the launch's number does

@@ -199,6 +199,8 @@ struct gg_engine {
     unsigned char *d_dir = nullptr, *h_dir = nullptr;   // DirectCtl | counts[cap + 1] | masks[cap + 1]
     int dir_cap = 0;
     unsigned dir_seq = 0;                // launches of direct_kernel
+    int dir_wait = 0;                    // evaluations until it walks again (after a table with one-way entries)
+    int dir_orbits = 0;                  // sources whose rows hold one-way entries when any does (0: all rows do)
     uint16_t *d_pack = nullptr, *h_pack = nullptr;      // plain-graph table as 16-bit ids (on first use)
     bool table_stale = false;            // the last call's table went to h_pack, d_table is older
 
@@ -758,6 +760,14 @@ gg_status create_common(gg_engine *e) {
     e->sweep = e->direct && env_int("GG_SWEEP", 1) != 0;
     if (env_int("GG_DIRECT", 1) == 0) e->direct = false;
     e->direct_allowed = e->direct;
+    {
+        // a lift whose sizes are multiples of its orbit's: a row is its orbit's, translated
+        bool whole = e->form != FORM_GRAPH && e->rows == e->N;
+        if (e->form == FORM_PART) whole = whole && e->N % e->M == 0;
+        else
+            for (int j = 0; j < 3 && whole; ++j) whole = e->dims[j] % e->dims[3 + j] == 0;
+        e->dir_orbits = whole ? (int)e->reps.size() : 0;
+    }
     GG_CK(cudaDeviceGetAttribute(&e->sms, cudaDevAttrMultiProcessorCount, e->device));
     GG_CK(cudaDeviceGetAttribute(&e->smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, e->device));
     for (int W : {1, 2, 4})
@@ -812,6 +822,7 @@ struct DirectPlan {
 // sets of every width must fit a block's shared memory.  A random row of 4, 8 or 16 bytes
 // per lane costs about 3.5, 6.2 and 10.4 shared-memory cycles a warp.
 constexpr double kSweepUsPerChunk = 0.064e-3, kLoopUsPerChunk = 0.12e-3;
+constexpr int kDirectCheck = 32;   // look-ups of the one-way check, at most, a thread of direct_kernel
 
 DirectPlan direct_plan(const gg_engine *e, int ns, bool wvc, bool sweep) {
     DirectPlan best;
@@ -917,27 +928,42 @@ gg_status direct_eval(gg_engine *e, const DirectPlan &p, const int32_t *table, c
     a.masks = wvc ? reinterpret_cast<unsigned *>(e->d_dir + off) : nullptr;
     a.h_masks = reinterpret_cast<unsigned *>(e->h_dir + off);
     a.batch_ns = e->h_batch_ns;
-    a.seq = ++e->dir_seq;
-    if (a.seq == 0) a.seq = ++e->dir_seq;   // 0: none yet
+    // Walks, where the check for one-way entries is a small part of a pass (kDirectCheck
+    // look-ups a thread), and not for a while after a table that had some.
+    a.check = e->dir_orbits ? e->dir_orbits : e->rows;
+    a.check_src = e->dir_orbits > 0;
+    const long long looks = ((long long)a.check + p.grid - 1) / p.grid * e->d * e->d;
+    if (looks > (long long)kDirectCheck * p.block) a.check = 0;
+    else if (e->dir_wait > 0) { a.check = 0; --e->dir_wait; }
     void *k = direct_for(p.W);
-    void *args[] = {&a};
-    GG_CK(cudaLaunchKernel(k, dim3((unsigned)p.grid), dim3((unsigned)p.block), args, p.smem, st));
-    // The kernel's last block stores its number after the counters; a wait for the stream
-    // takes a few microseconds longer to come back.  Not there within a few milliseconds:
-    // wait for the stream (a long evaluation, or an error to report).
-    {
-        const volatile unsigned *seq = &a.h_ctl->seq;
-        const auto t0 = std::chrono::steady_clock::now();
-        unsigned it = 0;
-        while (*seq != a.seq) {
-            if ((++it & 1023u) == 0u && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(5)) {
-                GG_CK(cudaStreamSynchronize(st));
-                break;
+    e->last_ms = 0.0;
+    for (;;) {
+        a.seq = ++e->dir_seq;
+        if (a.seq == 0) a.seq = ++e->dir_seq;   // 0: none yet
+        void *args[] = {&a};
+        GG_CK(cudaLaunchKernel(k, dim3((unsigned)p.grid), dim3((unsigned)p.block), args, p.smem, st));
+        // The kernel's last block stores its number after the counters; a wait for the stream
+        // takes a few microseconds longer to come back.  Not there within a few milliseconds:
+        // wait for the stream (a long evaluation, or an error to report).
+        {
+            const volatile unsigned *seq = &a.h_ctl->seq;
+            const auto t0 = std::chrono::steady_clock::now();
+            unsigned it = 0;
+            while (*seq != a.seq) {
+                if ((++it & 1023u) == 0u && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(5)) {
+                    GG_CK(cudaStreamSynchronize(st));
+                    break;
+                }
             }
+            std::atomic_thread_fence(std::memory_order_acquire);
         }
-        std::atomic_thread_fence(std::memory_order_acquire);
+        e->last_ms += (double)(e->h_batch_ns[1] - e->h_batch_ns[0]) * 1e-6;
+        if (!a.check || !a.h_ctl->oneway || a.h_ctl->bad) break;
+        // one-way entries: what the walks found are not the sources' levels
+        a.check = 0;
+        e->dir_wait = 63;
+        ++launches;
     }
-    e->last_ms = (double)(e->h_batch_ns[1] - e->h_batch_ns[0]) * 1e-6;
     e->last_launches = launches;
     e->last_batches = 1;
     e->last_d2h = sizeof(gg::DirectCtl) + ((size_t)a.h_ctl->levels_run + 1) * (wvc ? 12 : 8);

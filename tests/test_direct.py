@@ -103,3 +103,67 @@ def test_direct_device_tables_of_any_alignment():
             got = e.eval_device(buf.data_ptr() + 4 * shift)
             assert all(got[k] == want[k] for k in KEYS)
         e.close()
+
+
+def one_way(n, d, seed, edits):
+    """A table of n rows whose entries do not come back: an arbitrary one, or (edits > 0) a
+    random regular graph's with a few entries replaced."""
+    rng = np.random.default_rng(seed)
+    if not edits:
+        return rng.integers(0, n, (n, d)).astype(np.int32)
+    adj = G.random_regular(n, d, seed).copy()
+    for v in rng.choice(n, edits, replace=False):
+        adj[v, rng.integers(d)] = (v + 1 + rng.integers(n - 1)) % n
+    return adj
+
+
+@pytest.mark.parametrize("n,d,edits", [(9, 2, 0), (31, 1, 0), (74, 4, 0), (552, 8, 1), (1236, 2, 0), (2667, 9, 0), (3001, 4, 3),
+                                       (4096, 16, 1), (9000, 8, 2), (20000, 6, 1)])
+def test_direct_tables_with_one_way_entries(n, d, edits):
+    adj = one_way(n + n * d % 2 * bool(edits), d, 11, edits)
+    n = len(adj)
+    o = O.bfs_pull(adj, np.arange(n))
+    e = G.cudaASPLgraph(n, d)
+    good = G.random_regular(n, d, 5) if n * d % 2 == 0 and n > d + 1 else None
+    for t in (adj, adj, good, adj):      # with walks and, after the first, without
+        if t is None:
+            continue
+        w = o if t is adj else O.bfs_pull(t, np.arange(n))
+        r = e.eval(t, level_counts=True, max_levels=w.levels + 3)
+        assert (r["total"], r["reached"], r["levels"]) == (w.total(), int(w.reached.sum()), w.levels)
+    part = O.bfs_pull(adj, np.arange(n // 3, n // 2 + 1))
+    e.close()
+    e = G.cudaASPLgraph(n, d)
+    r = e.eval(adj, src_range=(n // 3, n // 2 + 1))
+    assert (r["total"], r["reached"], r["levels"]) == (part.total(), int(part.reached.sum()), part.levels)
+    e.close()
+
+
+@pytest.mark.parametrize("form,args", [("part", (78, 2, 9)), ("part", (5, 1, 3)), ("part", (939, 6, 6)), ("part", (2, 39, 8)),
+                                       ("ragged", (71, 296, 12)), ("ragged", (3, 64, 4)), ("piece", (3, 13, 4, 1, 5)),
+                                       ("piece", (7, 17, 6, 3, 8)), ("box", (5, 5, 2, 4, 3, 2, 3)), ("one", (300, 11, 6))])
+def test_direct_lifts_with_one_way_entries(form, args):
+    rng = np.random.default_rng(5)
+    if form in ("part", "ragged", "one"):
+        M, g, d = args
+        N = g if form == "ragged" else M * g
+        T = rng.integers(-N, N, (M, d)).astype(np.int32)
+        if form == "one":                # one entry of a symmetric lift, in the last orbit
+            T = G.cyclic_lift(M, g, d, 3)[2].copy()
+            T[M - 1, 0] += 1
+        e, adj, src = G.cudaASPLconv(N, M, d), O.expand_part(N, M, T), np.arange(M)
+    else:
+        ax = 2 if form == "piece" else 3
+        m, k, d = args[:ax], args[ax:2 * ax], args[-1]
+        n = [x * y for x, y in zip(m, k)]
+        T = rng.integers(-9, 9, (int(np.prod(m)), d, ax)).astype(np.int32)
+        x = np.array(np.unravel_index(np.arange(int(np.prod(n))), n))
+        o = np.ravel_multi_index([x[j] % m[j] for j in range(ax)], m)
+        adj = np.ravel_multi_index([(x[j][:, None] + T[o][:, :, j]) % n[j] for j in range(ax)], n)
+        src = np.ravel_multi_index(list(np.array(np.unravel_index(np.arange(int(np.prod(m))), m))), n)
+        e = (G.cudaASPLpiece if ax == 2 else G.cudaASPLbox)(*n, *m, d)
+    w = O.bfs_pull(np.ascontiguousarray(adj, dtype=np.int32), src)
+    for wvc in (False, True, False):
+        r = e.eval(T, want_wvc=wvc)
+        assert (r["total"], r["reached"], r["levels"]) == (w.total(), int(w.reached.sum()), w.levels)
+    e.close()
