@@ -241,6 +241,9 @@ static __device__ __forceinline__ void level_pass(const uint4 *cur, uint4 *nxt, 
 // length L (d^L of them) get bit j, the ones not set before are its new pairs.  A pass
 // reads d + 2 rows of 16 bytes per vertex whatever is new; a walk end costs one atomic and
 // L dependent id loads, so the walk takes the levels with at most kWalkItems ends a row.
+// Walks leave a source along the table's rows, so their ends are the vertices that reach it
+// only in a graph without one-way entries: a near-source candidate is one (batch_select), a
+// full search need not be.
 //
 // batch_kernel and its three small launches, 2048 x (n=1024, d=6) + 512 x (n=3000, d=4)
 // candidates: 2243 us a call with every affected source searched (2020 us of it here), 720
@@ -362,7 +365,7 @@ __global__ void __launch_bounds__(kBatchBlock, 1) batch_kernel(const BatchArgs a
         int L = 1, last = 0;
         bool done = seen == all;
         // walk ends: levels 1, 2, .. while they are few (a pass visits every row)
-        if (!a.hist) {
+        if (!full) {
             for (unsigned ends = (unsigned)d; !done; ends *= (unsigned)d, ++L) {
                 if ((unsigned long long)ends * (unsigned)ns > (unsigned long long)kWalkItems * (unsigned)n) break;
                 // a thread takes a walk of L - 1 steps and its d ends (the ids of one row)

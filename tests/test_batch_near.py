@@ -117,3 +117,36 @@ def test_near_candidates_equal_the_oracle(name):
             r = O.bfs_pull(apply(s), np.arange(n))
             assert (int(got["total"]), int(got["reached"]), int(got["levels"]), bool(got["connected"])) == \
                 (r.total(), int(r.reached.sum()), r.levels, bool(r.connected)), (name, s)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,d", [(40, 3), (128, 4), (129, 2), (277, 5), (1226, 2), (1281, 4), (2475, 8)])
+def test_bases_with_one_way_entries_equal_the_oracle(n, d):
+    rng = np.random.default_rng(n)
+    adj = rng.integers(0, n, (n, d)).astype(np.int32)                  # few entries come back
+    near = G.random_regular(n + n * d % 2, d, 3)
+    near[5, 1 % d] = (near[5, 1 % d] + 9) % len(near)                   # one does not
+    b = G.Batch(0)
+    for t in (adj, near):
+        b.add_base(t)
+    for k, t in enumerate((adj, near)):
+        sw = [(k, -1, -1, -1, -1, 0)]
+        while len(sw) < 12:
+            x, y = rng.integers(len(t), size=2)
+            u, v = t[x, rng.integers(d)], t[y, rng.integers(d)]
+            if len({int(x), int(y), int(u), int(v)}) == 4:
+                sw.append((k, x, u, y, v, rng.integers(2)))
+        sw = np.array(sw, dtype=G.SWAP_DTYPE)
+        for s, got in zip(sw, b.eval(sw)):
+            c = t.copy()
+            if s["a"] >= 0:
+                p, q = (s["d"], s["c"]) if s["mode"] else (s["c"], s["d"])
+                back = (s["b"], s["a"]) if s["mode"] else (s["a"], s["b"])
+                for r, f, to in ((s["a"], s["b"], p), (s["b"], s["a"], q), (s["c"], s["d"], back[0]), (s["d"], s["c"], back[1])):
+                    j = np.nonzero(c[r] == f)[0]
+                    if len(j):
+                        c[r, j[0]] = to
+            o = O.bfs_pull(c, np.arange(len(c)))
+            assert (int(got["total"]), int(got["reached"]), int(got["levels"]), bool(got["connected"])) == \
+                (o.total(), int(o.reached.sum()), o.levels, bool(o.connected)), s
+    b.close()
