@@ -40,7 +40,7 @@ struct DirectArgs {
     const int32_t *adj;       // [rows][d]
     const int32_t *src;       // vertex of entry i of the source list, or nullptr: src_first + i
     int src_first, src_begin, ns_total;
-    int rows, d;
+    int rows, d;              // d >= 1
     int max_levels;
     const uint16_t *adj16;    // the same ids, checked by the caller (device or pinned host memory), or nullptr
     int adj_smem;             // the rows as 16-bit ids in shared memory (range-checked on the way from adj)

@@ -826,7 +826,7 @@ constexpr int kDirectCheck = 32;   // look-ups of the one-way check, at most, a 
 
 DirectPlan direct_plan(const gg_engine *e, int ns, bool wvc, bool sweep) {
     DirectPlan best;
-    if (!e->direct || e->rows < 1 || e->rows > 65535 || ns < 1) return best;
+    if (!e->direct || e->d < 1 || e->rows < 1 || e->rows > 65535 || ns < 1) return best;   // (d = 0: no walk ends)
     const size_t budget = (size_t)e->smem_optin - 1024;
     double cost = 1e300;
     for (int W : {1, 2, 4}) {

@@ -167,3 +167,18 @@ def test_direct_lifts_with_one_way_entries(form, args):
         r = e.eval(T, want_wvc=wvc)
         assert (r["total"], r["reached"], r["levels"]) == (w.total(), int(w.reached.sum()), w.levels)
     e.close()
+
+
+@pytest.mark.parametrize("rows", [1, 2, 33, 5000])
+def test_degree_zero_takes_the_level_loop(rows):
+    for make, table in ((lambda: G.cudaASPLgraph(rows, 0), np.zeros((rows, 0), np.int32)),
+                        (lambda: G.cudaASPLconv(2 * rows, rows, 0), np.zeros((rows, 0), np.int32)),
+                        (lambda: G.cudaASPLpiece(rows, 3, rows, 1, 0), np.zeros((rows, 0, 2), np.int32)),
+                        (lambda: G.cudaASPLbox(rows, 2, 2, rows, 1, 1, 0), np.zeros((rows, 0, 3), np.int32))):
+        e = make()
+        for _ in range(2):
+            r = e.eval(table)
+            one = r["pairs"] == r["n_sources"]        # a single vertex reaches all there is
+            assert (r["total"], r["reached"], r["levels"], r["connected"]) == (0, r["n_sources"], 0, int(one))
+            assert r["n_sources"] == rows
+        e.close()
