@@ -988,6 +988,7 @@ namespace {
 // and orbit ids, a distance row within a block's shared memory (at 64 KB three blocks a
 // SM), and 1 GiB of distance rows.  Without them (or the memory) candidates are searched.
 constexpr size_t kDeltaRowBytes = 24 * 1024;   // rows of a block, when one is smaller
+constexpr size_t kDeltaMostBytes = 64 * 1024;  // one row of the largest lift
 void delta_open(gg_lift *h) {
     const char *off = std::getenv("GG_LIFT_SEARCH");   // 1: search every candidate
     const size_t pitch = ((size_t)h->N + 15) / 16 * 16;
@@ -1002,7 +1003,8 @@ void delta_open(gg_lift *h) {
     h->unit_rows = (int)std::min<size_t>(gg::kDeltaRows, smem / pitch);
     int per_sm = 0;
     void *k = lift_delta_for(h->axes, h->dp, h->rw);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // (the limit belongs to the kernel, which handles of other sizes launch too)
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDeltaMostBytes);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kDeltaBlock, smem);
     h->delta_grid = per_sm * h->sms;
     if (e == cudaSuccess && per_sm < 1) e = cudaErrorInvalidConfiguration;

@@ -177,3 +177,27 @@ def test_single_moves_near_the_edit_equal_the_oracle(name):
         assert (got["total"], got["reached"], got["levels"], bool(got["connected"])) == \
             (r.total(), int(r.reached.sum()), r.levels, bool(r.connected)), (name, s)
     inc.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["part", "piece"])
+def test_lift_handles_of_different_sizes_take_turns(form, monkeypatch):
+    """The second handle's rows are shorter than the first one's; both use one kernel."""
+    monkeypatch.setenv("GG_LIFT_SEARCH", "0")
+    if form == "part":
+        lifts2 = [G.cyclic_lift(m, g, 12, 3) for m, g in ((512, 64), (250, 4))]
+        lifts2 = [((N, M), T, G.gen_lift_moves(N, M, T, 6, 4)) for N, M, T in lifts2]
+    else:
+        lifts2 = [G.piece_lift(*a, 8, 3) for a in ((16, 16, 16, 8), (8, 8, 4, 4))]
+        lifts2 = [(tuple(a[:4]), a[4], G.gen_piece_moves(*a, 6, 4)) for a in lifts2]
+    handles = []
+    for dims, T, _ in lifts2:
+        handles.append(handle(form, dims, T.shape[1]))
+        handles[-1].set_base(T)
+    truth = [[want(form, dims, G.apply_lift_edit(T, e)) for e in moves] for dims, T, moves in lifts2]
+    for _ in range(2):
+        for L, (_, _, moves), w in zip(handles, lifts2, truth):
+            got = L.eval(moves)
+            assert [(int(x["total"]), int(x["reached"]), int(x["levels"]), int(x["connected"])) for x in got] == w
+    for L in handles:
+        L.close()
