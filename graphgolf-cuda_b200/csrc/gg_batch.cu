@@ -50,6 +50,7 @@ namespace {
 
 constexpr int kBatchBlock = 1024;
 constexpr size_t kSmemBudget = 220 * 1024;
+constexpr size_t kSmemMost = kSmemBudget + 4 * 1024;   // with T's bits
 
 constexpr int kPlanes = 4;   // distance bit-planes: distances up to 15
 
@@ -735,7 +736,8 @@ gg_status refresh_plan(gg_batch *b) {
     }
     b->smem = smem;
     b->max_chunks = max_chunks;
-    GB_CK(cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // (the limit belongs to the kernel, which handles with other bases launch too)
+    GB_CK(cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMost));
     int per_sm = 0, sms = 0;
     GB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel, kBatchBlock, smem));
     GB_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device));

@@ -150,3 +150,20 @@ def test_bases_with_one_way_entries_equal_the_oracle(n, d):
             assert (int(got["total"]), int(got["reached"]), int(got["levels"]), bool(got["connected"])) == \
                 (o.total(), int(o.reached.sum()), o.levels, bool(o.connected)), s
     b.close()
+
+
+@pytest.mark.gpu
+def test_handles_with_bases_of_different_sizes_take_turns():
+    """The second handle's units are smaller than the first one's; both use one kernel."""
+    graphs = [G.random_regular(3000, 4, 1), G.random_regular(64, 3, 2)]
+    handles = []
+    for adj in graphs:
+        handles.append(G.Batch(0))
+        handles[-1].add_base(adj)
+    moves = [G.gen_swaps(adj, 0, 5, 3) for adj in graphs]
+    truth = [[O.bfs_pull(G.apply_swap(adj, s), np.arange(len(adj))).total() for s in sw] for adj, sw in zip(graphs, moves)]
+    for _ in range(2):
+        for b, sw, w in zip(handles, moves, truth):
+            assert [int(t) for t in b.eval(sw)["total"]] == w
+    for b in handles:
+        b.close()
