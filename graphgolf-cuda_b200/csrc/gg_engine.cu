@@ -160,6 +160,7 @@ struct gg_engine {
     int sweep_K = 0;                     // levels before its dense ones
     int sweep_ends = 1;                  // most new vertices of a source's level below that
     bool sweep_list = false;             // the sources are a list (source_ball_kernel)
+    bool ball_limits = false;            // the balls' kernels have their shared-memory limit
     uint4 *d_swA = nullptr, *d_swB = nullptr;   // its level buffers, when wider than d_V
     size_t sw_chunks = 0;                // chunks each of them holds
     int *d_wasym = nullptr;              // one-way flag of the table (walk_index_kernel)
@@ -389,10 +390,24 @@ bool vall_room(gg_engine *e, size_t chunks) {
 // The rows of every batch for sweep_kernel: d_F1 where one batch fits it, else d_vall.
 bool sweep_in_f1(const gg_engine *e, int nb) { return nb == 1 && e->sweep_nC <= e->nC; }
 
+// The shared-memory limit of the balls' kernels: the most sweep_width lets a block have (two
+// blocks an SM).  It belongs to the kernel, which engines of other sizes launch too, in
+// other threads perhaps: every engine sets the same, before its first use.
+bool ball_limits(gg_engine *e) {
+    if (e->ball_limits) return true;
+    const SweepKernels k = sweep_for(e->d);
+    if (cudaFuncSetAttribute(k.ball, cudaFuncAttributeMaxDynamicSharedMemorySize, e->smem_optin / 2) != cudaSuccess ||
+        cudaFuncSetAttribute(k.source_ball, cudaFuncAttributeMaxDynamicSharedMemorySize, e->smem_optin / 2) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return e->ball_limits = true;
+}
+
 // sweep_kernel's level buffers: d_V and d_F0, or a wider pair of its own.
 bool sweep_room(gg_engine *e, int nb) {
     const size_t chunks = (size_t)e->rows * e->sweep_nC;
-    if ((!e->sweep_list && !e->h2_elems) || (!sweep_in_f1(e, nb) && !vall_room(e, nb * chunks))) return false;
+    if (!ball_limits(e) || (!e->sweep_list && !e->h2_elems) || (!sweep_in_f1(e, nb) && !vall_room(e, nb * chunks))) return false;
     if (e->sweep_nC <= e->nC || chunks <= e->sw_chunks) return true;
     invalidate_graph(e);
     cudaFree(e->d_swA); cudaFree(e->d_swB);
@@ -1107,7 +1122,6 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
                 ba.list = e->sweep_ends;
                 ba.ball_blocks = (ns_all + kSrcBallWarps - 1) / kSrcBallWarps;
                 const size_t bsmem = kSrcBallWarps * (size_t)gg::source_ball_warp_bytes(e->rows, e->sweep_ends);
-                GG_CK(cudaFuncSetAttribute(k.source_ball, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem));
                 const int check = (int)std::min<long long>((n + gg::kSrcBallBlock - 1) / gg::kSrcBallBlock, 16 * e->sms);
                 void *bargs[] = {&ba};
                 GG_CK(cudaLaunchKernel(k.source_ball, dim3(ba.ball_blocks + check), dim3(gg::kSrcBallBlock), bargs, bsmem, q));
@@ -1136,7 +1150,6 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
                 ba.rows = e->rows; ba.nC = e->sweep_nC; ba.nb = nb;
                 const size_t bsmem = ball_smem(e);
                 int per_sm = 0;
-                GG_CK(cudaFuncSetAttribute(k.ball, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem));
                 GG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.ball, gg::kBallBlock, bsmem));
                 const int warps = gg::kBallBlock / 32;
                 const int bgrid = std::min((e->rows + warps - 1) / warps, e->sms * std::max(per_sm, 1));

@@ -131,3 +131,34 @@ def test_source_list_equals_the_level_loop(form, args, monkeypatch):
         else:
             assert all(got[k] == want[k] for k in KEYS)
             assert np.array_equal(got["level_counts"], want["level_counts"])
+
+
+def test_engines_of_different_sizes_in_two_threads(monkeypatch):
+    """Both engines launch the same kernels, each with shared memory for its own rows; a new
+    level cap makes each call prepare its launches anew."""
+    import threading
+    monkeypatch.setenv("GG_DIRECT", "0")
+    jobs, errors = [], []
+    for n in (9000, 40000):
+        adj = G.random_regular(n, 6, 1)
+        jobs.append((lambda adj=adj: G.cudaASPLgraph(len(adj), 6), adj))
+    for m, g in ((200, 12), (1024, 60)):
+        N, M, T = G.cyclic_lift(m, g, 6, 1)
+        jobs.append((lambda N=N, M=M: G.cudaASPLconv(N, M, 6), T))
+
+    def work(make, t):
+        try:
+            e = make()
+            seen = {(r["total"], r["reached"], r["levels"]) for r in (e.eval(t, max_levels=20 + k % 40) for k in range(120))}
+            e.close()
+            assert len(seen) == 1
+        except Exception as x:
+            errors.append(x)
+
+    for _ in range(2):
+        threads = [threading.Thread(target=work, args=j) for j in jobs]
+        for th in threads:
+            th.start()
+        for th in threads:
+            th.join()
+    assert not errors, errors
