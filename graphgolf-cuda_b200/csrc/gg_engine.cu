@@ -199,6 +199,7 @@ struct gg_engine {
     int32_t *d_src = nullptr;            // the source list, when not consecutive
     unsigned char *d_dir = nullptr, *h_dir = nullptr;   // DirectCtl | counts[cap + 1] | masks[cap + 1]
     int dir_cap = 0;
+    bool dir_dirty = true;               // d_dir's counters must be cleared before the next launch
     unsigned dir_seq = 0;                // launches of direct_kernel
     int dir_wait = 0;                    // evaluations until it walks again (after a table with one-way entries)
     int dir_orbits = 0;                  // sources whose rows hold one-way entries when any does (0: all rows do)
@@ -751,9 +752,10 @@ gg_status create_common(gg_engine *e) {
             inv[(size_t)v] = (int32_t)i;
         }
         GG_CK(cudaMalloc(&e->d_src, e->reps.size() * sizeof(int32_t)));
-        GG_CK(cudaMemcpy(e->d_src, e->reps.data(), e->reps.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+        GG_CK(cudaMemcpyAsync(e->d_src, e->reps.data(), e->reps.size() * sizeof(int32_t), cudaMemcpyHostToDevice, e->stream));
         GG_CK(cudaMalloc(&e->d_inv, inv.size() * sizeof(int32_t)));
-        GG_CK(cudaMemcpy(e->d_inv, inv.data(), inv.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+        GG_CK(cudaMemcpyAsync(e->d_inv, inv.data(), inv.size() * sizeof(int32_t), cudaMemcpyHostToDevice, e->stream));
+        GG_CK(cudaStreamSynchronize(e->stream));   // an evaluation may come on another stream
     }
     e->dense_w_ppm = env_int("GG_DENSE_W_PPM", e->dense_w_ppm);
     e->dense_r_ppm = env_int("GG_DENSE_R_PPM", e->dense_r_ppm);
@@ -887,9 +889,8 @@ gg_status ensure_direct(gg_engine *e, int cap) {
     GG_CK(cudaMalloc(&e->d_dir, bytes));
     GG_CK(cudaMallocHost(&e->h_dir, bytes));
     std::memset(e->h_dir, 0, 64);
-    GG_CK(cudaMemset(e->d_dir, 0, 64 + n * 8));
-    GG_CK(cudaMemset(e->d_dir + 64 + n * 8, 0xff, n * 4));
     e->dir_cap = cap;
+    e->dir_dirty = true;
     return GG_OK;
 }
 
@@ -952,7 +953,13 @@ gg_status direct_eval(gg_engine *e, const DirectPlan &p, const int32_t *table, c
     else if (e->dir_wait > 0) { a.check = 0; --e->dir_wait; }
     void *k = direct_for(p.W);
     e->last_ms = 0.0;
+    if (e->dir_dirty) {
+        const size_t c = 64 + ((size_t)e->dir_cap + 1) * 8;
+        GG_CK(cudaMemsetAsync(e->d_dir, 0, c, st));
+        GG_CK(cudaMemsetAsync(e->d_dir + c, 0xff, ((size_t)e->dir_cap + 1) * 4, st));
+    }
     for (;;) {
+        e->dir_dirty = true;   // until the launch has handed its counters over
         a.seq = ++e->dir_seq;
         if (a.seq == 0) a.seq = ++e->dir_seq;   // 0: none yet
         void *args[] = {&a};
@@ -967,11 +974,13 @@ gg_status direct_eval(gg_engine *e, const DirectPlan &p, const int32_t *table, c
             while (*seq != a.seq) {
                 if ((++it & 1023u) == 0u && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(5)) {
                     GG_CK(cudaStreamSynchronize(st));
+                    if (*seq != a.seq) return fail(GG_CUDA_ERROR, "direct_kernel ended without handing its counters over");
                     break;
                 }
             }
             std::atomic_thread_fence(std::memory_order_acquire);
         }
+        e->dir_dirty = false;
         e->last_ms += (double)(e->h_batch_ns[1] - e->h_batch_ns[0]) * 1e-6;
         if (!a.check || !a.h_ctl->oneway || a.h_ctl->bad) break;
         // one-way entries: what the walks found are not the sources' levels

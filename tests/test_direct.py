@@ -182,3 +182,26 @@ def test_degree_zero_takes_the_level_loop(rows):
             assert (r["total"], r["reached"], r["levels"], r["connected"]) == (0, r["n_sources"], 0, int(one))
             assert r["n_sources"] == rows
         e.close()
+
+
+def test_direct_while_the_default_stream_is_busy():
+    """A new engine's counters are cleared in the order of its own work: other work that waits
+    on the default stream neither delays nor follows it.  Also when a larger level cap makes
+    them anew, and on a caller's stream."""
+    import torch
+    adj = G.random_regular(600, 4, 3)
+    o = O.bfs_pull(adj, np.arange(600))
+    table = torch.from_numpy(adj).cuda()
+    other = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for _ in range(3):
+        torch.cuda._sleep(int(4e7))         # about 20 ms
+        e = G.cudaASPLgraph(600, 4)
+        torch.cuda._sleep(int(4e7))
+        for cap in (0, 300, 40000, 0):      # (0: 600 levels)
+            r = e.eval(adj, max_levels=cap)
+            assert (r["total"], r["reached"], r["levels"]) == (o.total(), int(o.reached.sum()), o.levels)
+            r = e.eval_device(table.data_ptr(), max_levels=2 * cap, stream=other.cuda_stream)
+            assert (r["total"], r["reached"], r["levels"]) == (o.total(), int(o.reached.sum()), o.levels)
+        e.close()
+        torch.cuda.synchronize()
