@@ -68,7 +68,9 @@ int env_int(const char *name, int dflt) {
 //   "barrier" -- the grid barrier waits for one block more than is launched, so
 //                its bounded wait runs out and the call returns GG_TIMEOUT;
 //   "alloc"   -- engine creation reports an allocation failure;
-//   "launch"  -- the BFS launch reports a CUDA error before anything is enqueued.
+//   "launch"  -- the BFS launch reports a CUDA error before anything is enqueued;
+//   "rows"    -- no memory for the rows of all batches (vall_room);
+//   "more_rows" -- no memory for more of them once there are some.
 // Nothing here faults, traps or hangs the GPU.
 bool fault(const char *what) {
     const char *s = std::getenv("GG_FAULT_INJECT");
@@ -372,11 +374,12 @@ bool vall_room(gg_engine *e, size_t chunks) {
     if ((long long)((chunks * sizeof(uint4)) >> 20) > e->walk_all_mb) return false;
     if (chunks <= e->vall_chunks) return true;
     invalidate_graph(e);
+    const bool had = e->vall_chunks > 0;
     cudaFree(e->d_vall); cudaFree(e->d_vall_fl);
     e->d_vall = nullptr;
     e->d_vall_fl = nullptr;
     e->vall_chunks = 0;
-    if (cudaMalloc(&e->d_vall, chunks * sizeof(uint4)) != cudaSuccess ||
+    if (fault("rows") || (had && fault("more_rows")) || cudaMalloc(&e->d_vall, chunks * sizeof(uint4)) != cudaSuccess ||
         cudaMalloc(&e->d_vall_fl, (chunks + 31) / 32 * sizeof(uint32_t)) != cudaSuccess) {
         cudaFree(e->d_vall); cudaFree(e->d_vall_fl);
         e->d_vall = nullptr;
@@ -1075,13 +1078,18 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
     if (want_ns) d2h += lv * sizeof(unsigned long long);
     // Walk pass for this evaluation: not with the WVC masks or the distance planes
     // (their per-level bookkeeping lives in the level loop), at most the level cap.
-    int walk_K = (wvc || (x && (x->planes || within))) ? 0 : std::min(e->walk_K, cap_req);
-    // (one level less where the walk of all batches then covers them: a level costs less
-    // than a walk pass per batch)
-    if (walk_K == 4 && e->walk_auto && walk_all_for(e, 3, nb_plain)) walk_K = 3;
-    const int launches_plain = 1 + ((long long)e->rows * e->d > 0 ? 1 : 0) + (walk_K > 0 ? 1 : 0) + (walk_K >= 3 ? 1 : 0);
-    void *wall = walk_K > 0 ? walk_all_for(e, walk_K, nb_plain) : nullptr;
-    const int launches = sweep ? (e->sweep_list ? 3 : 4) : launches_plain;
+    // Not with sweep_kernel either, whose rows are where the walk of all batches would put its.
+    int walk_K = 0, launches = e->sweep_list ? 3 : 4;
+    void *wall = nullptr;
+    auto plan_walk = [&] {
+        walk_K = (wvc || (x && (x->planes || within))) ? 0 : std::min(e->walk_K, cap_req);
+        // (one level less where the walk of all batches then covers them: a level costs less
+        // than a walk pass per batch)
+        if (walk_K == 4 && e->walk_auto && walk_all_for(e, 3, nb_plain)) walk_K = 3;
+        launches = 1 + ((long long)e->rows * e->d > 0 ? 1 : 0) + (walk_K > 0 ? 1 : 0) + (walk_K >= 3 ? 1 : 0);
+        wall = walk_K > 0 ? walk_all_for(e, walk_K, nb_plain) : nullptr;
+    };
+    if (!sweep) plan_walk();
 
     // Everything the GPU does for one evaluation, on `q`: status words zeroed,
     // table -> adjacency (checked), one cooperative launch for every source
@@ -1396,12 +1404,13 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
             return ds;
         }
         nb = nb_plain;
+        plan_walk();
         gg_status es = enqueue(st, true);
         if (es != GG_OK) return es;
         GG_CK(cudaStreamSynchronize(st));
         GG_CK(cudaEventElapsedTime(&ms, e->ev0, e->ev1));
         e->last_ms += ms;
-        e->last_launches += launches_plain;
+        e->last_launches += launches;
     }
     e->last_batches = nb;
 

@@ -162,3 +162,34 @@ def test_engines_of_different_sizes_in_two_threads(monkeypatch):
         for th in threads:
             th.join()
     assert not errors, errors
+
+
+@pytest.mark.parametrize("fault", ["rows", "more_rows"])
+@pytest.mark.parametrize("n,d,kind", [(10000, 4, "graph"), (17000, 6, "graph"), (20000, 8, "graph"), (12000, 8, "one-way"),
+                                      (20000, 6, "list"), (20000, 6, "one-way list")])
+def test_no_memory_for_the_rows_of_all_batches(n, d, kind, fault, monkeypatch):
+    """The allocation that fails (on the host's side) is the sweep's own, or a larger one that
+    only the general loop would need, when the sweep has its rows already."""
+    monkeypatch.setenv("GG_DIRECT", "0")
+    if kind.endswith("list"):
+        N, M, T = G.cyclic_lift(n // 2, 2, d, 3)
+        T = T.copy()
+        adj, src, make = None, np.arange(M), lambda: G.cudaASPLconv(N, M, d)
+    else:
+        T = G.random_regular(n, d, 3)
+        src, make = np.arange(n), lambda: G.cudaASPLgraph(n, d)
+    if kind.startswith("one-way"):
+        T[17, 2] += 1 if T[17, 2] + 1 < n else -1
+    adj = O.expand_part(N, M, T) if kind.endswith("list") else T
+    o = O.bfs_pull(adj, src)
+    e = make()
+    for inject in ("", fault, "", fault, fault):
+        monkeypatch.setenv("GG_FAULT_INJECT", inject)
+        r = e.eval(T)
+        assert (r["total"], r["reached"], r["levels"]) == (o.total(), int(o.reached.sum()), o.levels)
+    e.close()
+    monkeypatch.setenv("GG_FAULT_INJECT", fault)
+    e = make()
+    r = e.eval(T)
+    assert (r["total"], r["reached"], r["levels"]) == (o.total(), int(o.reached.sum()), o.levels)
+    e.close()
