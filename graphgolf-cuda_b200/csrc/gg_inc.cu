@@ -34,9 +34,9 @@ constexpr int kPlanes = 4;
 struct IncStatus {
     unsigned long long old_sum;   // distance sums of T (current graph)
     unsigned long long tt_sum;    // distances within T (current graph)
+    unsigned long long tops;      // pairs (T, any) at the current diameter (up to n^2)
     unsigned affected;            // affected sources
     unsigned count;               // |T|
-    unsigned tops;                // pairs (T, any) at the current diameter
     int found;                    // outside_at's answer
 };
 
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(128) inc_select(const IncArgs a) {
         }
         if (sum) atomicAdd(&a.st->old_sum, sum);
         tops = __reduce_add_sync(0xffffffffu, tops);
-        if (lane == 0 && tops) atomicAdd(&a.st->tops, tops);
+        if (lane == 0 && tops) atomicAdd(&a.st->tops, (unsigned long long)tops);
     }
     __syncthreads();
     // the places of the block's 1024 vertices, each warp the words of a quarter

@@ -201,3 +201,34 @@ def test_lift_handles_of_different_sizes_take_turns(form, monkeypatch):
             assert [(int(x["total"]), int(x["reached"]), int(x["levels"]), int(x["connected"])) for x in got] == w
     for L in handles:
         L.close()
+
+
+def twin_trees(b, depth):
+    """Two b-ary trees of the given depth with their roots joined, padded with self-loops:
+    b^(2 depth) pairs at the diameter 2 depth + 1 each way, all of them through one edge."""
+    size = (b ** (depth + 1) - 1) // (b - 1)
+    v = np.arange(size)
+    kids = v[:, None] * b + 1 + np.arange(b)
+    adj = np.concatenate([np.maximum((v - 1) // b, 0)[:, None], np.where(kids < size, kids, v[:, None])], axis=1)
+    adj = np.concatenate([adj, adj + size]).astype(np.int32)
+    adj[0, 0], adj[size, 0] = size, 0
+    return adj, size
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("b,depth", [(3, 4), (5, 7)])      # (5, 7): 1.2e10 pairs at the diameter
+def test_single_move_that_takes_all_pairs_at_the_diameter_apart(b, depth):
+    adj, size = twin_trees(b, depth)
+    n = len(adj)
+    inc = G.Incremental(n, b + 1)
+    assert inc.set_graph(adj)["levels"] == 2 * depth + 1
+    # the edge between the roots, and one between a child and a grandchild of the first
+    s = np.array([(0, 0, size, 1, b + 1, 0)], dtype=G.SWAP_DTYPE)[0]
+    got, _ = inc.eval(s)
+    inc.close()
+    left = size - (b ** (depth - 1) - 1) // (b - 1)             # less the grandchild's subtree
+    right = n - left
+    assert (got["levels"], got["connected"], got["reached"]) == (2 * depth, 0, left * left + right * right)
+    if n < 1000:
+        o = O.bfs_pull(G.apply_swap(adj, s), np.arange(n))
+        assert (got["total"], got["reached"], got["levels"]) == (o.total(), int(o.reached.sum()), o.levels)
