@@ -743,8 +743,8 @@ gg_status refresh_plan(gg_batch *b) {
     GB_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device));
     if (per_sm < 1) return bfail(GG_BAD_ARG, "batch task does not fit in shared memory");
     b->grid = per_sm * sms;
-    GB_CK(cudaMemcpy(b->d_bases, b->bases.data(), b->bases.size() * sizeof(BatchBase),
-                     cudaMemcpyHostToDevice));
+    GB_CK(cudaMemcpyAsync(b->d_bases, b->bases.data(), b->bases.size() * sizeof(BatchBase), cudaMemcpyHostToDevice, b->stream));
+    GB_CK(cudaStreamSynchronize(b->stream));   // a population may come on another stream
     drop_graph(b);
     return GG_OK;
 }
@@ -945,7 +945,8 @@ gg_status gg_batch_add_base(gg_batch *b, int n, int degree, const int32_t *adj, 
     GB_CK(cudaMalloc(&d, (size_t)n * degree * sizeof(int32_t)));
     cudaError_t me = cudaMalloc(&d16, b16);
     if (me != cudaSuccess) { cudaFree(d); GB_CK(me); }
-    GB_CK(cudaMemcpy(d, adj, (size_t)n * degree * sizeof(int32_t), cudaMemcpyHostToDevice));
+    // (on the stream that reads it: a copy on another one may still be under way)
+    GB_CK(cudaMemcpyAsync(d, adj, (size_t)n * degree * sizeof(int32_t), cudaMemcpyHostToDevice, b->stream));
     pack16_kernel<<<64, 256, 0, b->stream>>>(d, d16, n * degree, (int)(b16 / 2));
     GB_CK(cudaGetLastError());
     BatchBase B{};

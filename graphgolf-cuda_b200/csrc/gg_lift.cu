@@ -1133,7 +1133,9 @@ gg_status lift_open(int axes, const int n_in[3], const int m_in[3], int degree, 
                 for (int z = 0; z < h->m[2]; ++z)
                     inv[((size_t)x * ny + y) * nz + z] = (x * h->m[1] + y) * h->m[2] + z;
         e = cudaMalloc(&h->d_inv, inv.size() * sizeof(int32_t));
-        if (e == cudaSuccess) e = cudaMemcpy(h->d_inv, inv.data(), inv.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(h->d_inv, inv.data(), inv.size() * sizeof(int32_t), cudaMemcpyHostToDevice, h->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     }
     if (e != cudaSuccess)
         return fail(lfail(e == cudaErrorMemoryAllocation ? GG_OUT_OF_MEMORY : GG_CUDA_ERROR,

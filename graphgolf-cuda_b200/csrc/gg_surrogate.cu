@@ -915,8 +915,9 @@ gg_status gg_surrogate_create(int device, int n, int degree, int in_features, ui
             cudaSuccess ||
         s->bwd_per_sm < 1)
         return bad(sfail(GG_CUDA_ERROR, "fused backward cannot be resident"));
-    if (cudaMemcpy(s->params, p.data(), pb, cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemset(s->adam_m, 0, pb) != cudaSuccess || cudaMemset(s->adam_v, 0, pb) != cudaSuccess)
+    if (cudaMemcpyAsync(s->params, p.data(), pb, cudaMemcpyHostToDevice, s->st) != cudaSuccess ||
+        cudaMemsetAsync(s->adam_m, 0, pb, s->st) != cudaSuccess || cudaMemsetAsync(s->adam_v, 0, pb, s->st) != cudaSuccess ||
+        cudaStreamSynchronize(s->st) != cudaSuccess)
         return bad(sfail(GG_CUDA_ERROR, "surrogate initialisation failed"));
     *out = s;
     return GG_OK;
@@ -979,8 +980,9 @@ gg_status gg_surrogate_get_params(gg_surrogate *s, float *params) {
 gg_status gg_surrogate_set_params(gg_surrogate *s, const float *params) {
     if (!s || !params) return sfail(GG_BAD_ARG, "null argument");
     GS_CK(cudaSetDevice(s->device));
-    GS_CK(cudaMemcpy(s->params, params, (size_t)s->n_params * 4, cudaMemcpyHostToDevice));
+    GS_CK(cudaMemcpyAsync(s->params, params, (size_t)s->n_params * 4, cudaMemcpyHostToDevice, s->st));
     s->fwd_valid = false;
+    GS_CK(cudaStreamSynchronize(s->st));
     return GG_OK;
 }
 

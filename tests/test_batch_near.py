@@ -167,3 +167,26 @@ def test_handles_with_bases_of_different_sizes_take_turns():
             assert [int(t) for t in b.eval(sw)["total"]] == w
     for b in handles:
         b.close()
+
+
+@pytest.mark.gpu
+def test_bases_added_while_other_copies_are_under_way():
+    """A new base's rows are on the device before the kernel that packs them reads them, also
+    with the copy engine busy and memory that held other tables."""
+    import torch
+    n, d = 2536, 8
+    ring = ((np.arange(n)[:, None] + np.array([1, -1, 2, -2, 3, -3, 4, -4])) % n).astype(np.int32)
+    host = torch.empty(256 << 20, dtype=torch.uint8).pin_memory()
+    dev = torch.empty(256 << 20, dtype=torch.uint8, device="cuda")
+    side = torch.cuda.Stream()
+    base = np.array([(0, -1, -1, -1, -1, 0)], dtype=G.SWAP_DTYPE)
+    total = n * sum(-(-min(k, n - k) // 4) for k in range(1, n))
+    for k in range(12):
+        with torch.cuda.stream(side):
+            dev.copy_(host, non_blocking=True)          # about 5 ms
+        b = G.Batch(0)
+        b.add_base(ring)
+        got = b.eval(base)[0]
+        assert (int(got["total"]), int(got["reached"])) == (total, n * n)
+        b.close()
+    torch.cuda.synchronize()
