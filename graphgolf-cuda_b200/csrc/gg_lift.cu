@@ -34,19 +34,20 @@
 // round's counts, and the round ends when no candidate found a pair or every
 // candidate reached all M*N pairs.
 //
-// Moves by change (default, within the limits of delta_limits): the base's distance rows
-// are kept (one search of the base that also writes bit-planes, when the first
-// population after gg_lift_set_base comes), and a candidate is scored by following what
-// its edit changes in the rows near it (gg_delta.cuh): lift_select lists the rows,
-// lift_delta follows them.  Edits that leave the lift asymmetric, changes that outgrow
-// the lists or reach distances past kDeltaMax, bases that are asymmetric, disconnected or
-// of diameter above 15, and handles with an explicit group run the search above.
+// Moves by change (within the limits of delta_fits, where delta_pays says so): the base's
+// distance rows are kept (delta_base: one search of the base that also writes bit-planes),
+// and a candidate is scored by following what its edit changes in the rows near it
+// (gg_delta.cuh): lift_select lists the rows, lift_delta follows them.  Edits that leave
+// the lift asymmetric, changes that outgrow the lists or reach distances past kDeltaMax,
+// bases that are asymmetric, disconnected or of diameter above 15, and handles with an
+// explicit group run the search above.
 #include "gg.h"
 #include "gg_delta.cuh"
 #include "gg_internal.h"
 #include "gg_kernels.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <string>
@@ -897,8 +898,11 @@ struct gg_lift {
     bool base_set = false;
     float last_ms = 0.f;
     // moves by change
-    bool delta_on = false;                           // the lift is within the limits and the buffers are there
+    int delta_on = 0;                                // buffers: 0 not there yet, 1 there, -1 past the limits or no memory
+    bool delta_always = false;                       // whatever delta_pays says (GG_LIFT_SEARCH=0)
+    int delta_wait = 0;                              // evaluations until it is tried again
     int base_state = 0;                              // distances of the base: 0 not computed, 1 usable, -1 not usable
+    long long base_cands = 0;                        // candidates of this base that would have gone by change with them
     int rw = 0, pitch = 0, words = 0, unit_rows = 1, delta_grid = 0;
     unsigned char *d_arena = nullptr, *d_each = nullptr;   // what the pointers below lie in (d_each: per candidate)
     uint4 *d_planes = nullptr;                       // [4][N][cpc]
@@ -978,23 +982,48 @@ gg_status alloc_group(gg_lift *h, int groups) {
 
 }  // namespace
 
-extern "C" {
-
-}  // extern "C"
-
 namespace {
 
-// Buffers of the moves by change, where the lift is within their limits: 16-bit vertex
-// and orbit ids, a distance row within a block's shared memory (at 64 KB three blocks a
-// SM), and 1 GiB of distance rows.  Without them (or the memory) candidates are searched.
+// Moves by change: 16-bit vertex and orbit ids, a distance row within a block's shared
+// memory (at 64 KB three blocks a SM), and 1 GiB of distance rows.  The row of an edited
+// orbit loses one of its d subtrees, about N / d vertices and more when few others reach
+// them as soon, so a small degree outgrows the lists (kDeltaList + kDeltaSpill) in nearly
+// every candidate, which is then searched as well.  256 candidates, by change / searched:
+// m = 418, g = 23, d = 4: 2185 / 1274 us (87 % outgrew them), m = 512, g = 64, d = 8: 5653 /
+// 3188 (all); m = 546, g = 10, d = 4: 700 / 988 (6 %), m = 1024, g = 32, d = 12: 1779 / 6053
+// (0.4 %).
 constexpr size_t kDeltaRowBytes = 24 * 1024;   // rows of a block, when one is smaller
 constexpr size_t kDeltaMostBytes = 64 * 1024;  // one row of the largest lift
-void delta_open(gg_lift *h) {
-    const char *off = std::getenv("GG_LIFT_SEARCH");   // 1: search every candidate
+constexpr int kDeltaMostPerDegree = 3600;      // N / (d - 2): 2730 and 3277 for the last two, 4807 and 5461 for the first
+bool delta_fits(const gg_lift *h) {
     const size_t pitch = ((size_t)h->N + 15) / 16 * 16;
-    if ((off && std::atoi(off) != 0) || h->N > 65536 || h->M > 65535 || h->N / h->M > 65535 ||
-        pitch * h->M > (1ull << 30))
-        return;
+    return h->N <= 65536 && h->M <= 65535 && h->N / h->M <= 65535 && pitch * h->M <= (1ull << 30) &&
+           (h->delta_always || (long long)h->N <= (long long)kDeltaMostPerDegree * (h->d - 2));
+}
+
+// Whether a population of n goes by change.  Microseconds, fits over 35 lifts (N = 512 to
+// 32768, d = 4 to 12): a searched candidate takes `each`, one by change about a third of
+// that; by change a population takes `more` longer before its first candidate (its waves
+// are chains, longer at small degrees); the distances of a new base take 135 and three
+// searched candidates.  They are worth it once the candidates seen on the base would have
+// paid for them: 32 candidates on a new base are searched at m = 500, g = 12, d = 6 (148 us,
+// 314 by change) and go by change at m = 1024, g = 32, d = 12 (849 / 529); the lines lie
+// at 111 and 17 (both ways alike at about 165 and 14).
+bool delta_pays(gg_lift *h, const int n) {
+    if (h->delta_always) return true;
+    const double each = 1.2 + 9e-6 * (double)h->N * h->cpc * h->d, k = h->d - 2;
+    const double more = std::max(70.0, 0.11 * h->N / (k * std::sqrt(k)));
+    if (n < 2.0 + more / each) return false;
+    h->base_cands += n;
+    return h->base_state == 1 || (double)h->base_cands >= 2.0 + more / each + 4.3 + 193.0 / each;
+}
+
+// Buffers of the moves by change, for the first population that goes that way.  Without
+// them candidates are searched.
+bool delta_open(gg_lift *h) {
+    if (h->delta_on) return h->delta_on > 0;
+    h->delta_on = -1;
+    const size_t pitch = ((size_t)h->N + 15) / 16 * 16;
     h->pitch = (int)pitch;
     h->rw = (h->d + 2 + 7) / 8 * 8;
     h->dp = (h->d + 3) / 4 * 4;
@@ -1023,7 +1052,7 @@ void delta_open(gg_lift *h) {
     if (e == cudaSuccess) e = cudaMalloc(&h->d_arena, at);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
-        return;
+        return false;
     }
     h->d_planes = reinterpret_cast<uint4 *>(h->d_arena + o_planes);
     h->d_dist = h->d_arena + o_dist;
@@ -1032,7 +1061,8 @@ void delta_open(gg_lift *h) {
     h->d_ball = reinterpret_cast<uint32_t *>(h->d_arena + o_ball);
     h->d_spill = reinterpret_cast<uint32_t *>(h->d_arena + o_spill);
     h->d_ctr = reinterpret_cast<int *>(h->d_arena + o_ctr);
-    h->delta_on = true;
+    h->delta_on = 1;
+    return true;
 }
 
 // Per-candidate buffers of the moves by change; false: not enough memory.
@@ -1143,7 +1173,9 @@ gg_status lift_open(int axes, const int n_in[3], const int m_in[3], int degree, 
     // bitsets for the automatic group (a larger group set later reallocates)
     const gg_status s = alloc_group(h, h->g_auto);
     if (s != GG_OK) return fail(s);
-    delta_open(h);
+    const char *search = std::getenv("GG_LIFT_SEARCH");   // 1: search every candidate, 0: none that can go by change
+    h->delta_always = search && std::atoi(search) == 0;
+    if ((search && !h->delta_always) || !delta_fits(h)) h->delta_on = -1;
     *out = h;
     return GG_OK;
 }
@@ -1360,6 +1392,7 @@ gg_status gg_lift_set_base(gg_lift *h, const int32_t *table) {
     GL_CK(cudaStreamSynchronize(h->stream));
     h->base_set = true;
     h->base_state = 0;
+    h->base_cands = 0;
     return GG_OK;
 }
 
@@ -1449,21 +1482,23 @@ gg_status gg_lift_eval(gg_lift *h, int n_cand, const gg_lift_edit *edits, int ma
             }
         }
     }
-    // By change, once the base's distances are there; a first population of a few
-    // candidates is not worth computing them (a search of the base, about one candidate's).
-    std::vector<int> left;
-    const bool delta = h->delta_on && h->group == 0 && h->base_state >= 0 && (h->base_state == 1 || n_cand >= 4);
-    if (delta && delta_ensure(h, n_cand)) {
+    const bool can = h->delta_on >= 0 && h->group == 0 && h->base_state >= 0;
+    if (can && h->delta_wait > 0) {
+        --h->delta_wait;
+    } else if (can && delta_pays(h, n_cand) && delta_open(h) && delta_ensure(h, n_cand)) {
         if (h->base_state == 0) {
             const gg_lift_edit first = h->h_ed[0];
             s = delta_base(h);
             if (s != GG_OK) return s;
             h->h_ed[0] = first;
+            if (h->base_state < 0 && !h->delta_always) h->delta_wait = 63;   // (the next bases are often like it)
         }
         if (h->base_state == 1) {
+            std::vector<int> left;
             s = delta_eval(h, n_cand, max_levels, out, left);
             if (s != GG_OK || left.empty()) return s;
-            // the rest is searched
+            // the rest is searched (and the next populations whole, when that is a lot)
+            if (left.size() * 4 > (size_t)n_cand && !h->delta_always) h->delta_wait = 63;
             for (size_t i = 0; i < left.size(); ++i) h->h_ed[i] = h->h_ed[left[i]];
             std::vector<gg_cand_result> res(left.size());
             const float ms = h->last_ms;

@@ -6,6 +6,8 @@ counts.  GPU: forms (part, 2-D, 3-D torus), degrees with and without an unrolled
 copy and many, small and odd sizes, edits that do not keep the lift symmetric, level caps,
 and a new base table, against the oracle; single moves at group edges, with repeated edges
 and with few pairs at the diameter."""
+import time
+
 import numpy as np
 import pytest
 
@@ -130,6 +132,61 @@ def test_lift_moves_by_change_equal_the_oracle(name, monkeypatch):
         for e, got in zip(part, L.eval(part)):
             w = want(form, dims, G.apply_lift_edit(T2, e))
             assert (int(got["total"]), int(got["reached"]), int(got["levels"]), int(got["connected"])) == w
+    L.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", list(lifts()))
+def test_every_population_by_change_equals_the_oracle(name, monkeypatch):
+    """GG_LIFT_SEARCH=0: no population is too small, no change likely to outgrow the lists."""
+    monkeypatch.setenv("GG_LIFT_SEARCH", "0")
+    form, dims, T, gen = lifts()[name]
+    L = handle(form, dims, T.shape[1])
+    for k in range(2):
+        L.set_base(T)
+        for moves in (gen(1, k), gen(9, 5 + k)):
+            for e, got in zip(moves, L.eval(moves)):
+                assert (int(got["total"]), int(got["reached"]), int(got["levels"]), int(got["connected"])) == \
+                    want(form, dims, G.apply_lift_edit(T, e))
+        T = G.apply_lift_edit(T, moves[0])
+    L.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,g,d,n", [(130, 5, 6, 128), (200, 15, 4, 200)])
+def test_populations_before_and_after_the_base_is_followed_agree(m, g, d, n):
+    """The first populations of a base are searched, the later ones go by change."""
+    N, M, T = G.cyclic_lift(m, g, d, 2)
+    moves = G.gen_lift_moves(N, M, T, n, 3)
+    L = G.Lift(N, M, d)
+    L.set_base(T)
+    first = L.eval(moves)
+    assert all(L.eval(moves).tobytes() == first.tobytes() for _ in range(4))
+    for e, got in zip(moves[:6], first):
+        assert (int(got["total"]), int(got["reached"]), int(got["levels"]), int(got["connected"])) == \
+            want("part", (N, M), G.apply_lift_edit(T, e))
+    L.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,g,d,n", [(500, 12, 6, 32), (418, 23, 4, 256), (64, 8, 4, 8)])
+def test_population_on_a_new_base_takes_no_longer_than_its_search(m, g, d, n, monkeypatch):
+    """An annealer's step: a new base, then a population.  (Least of many, both in turn.)"""
+    N, M, T = G.cyclic_lift(m, g, d, 1)
+    moves = G.gen_lift_moves(N, M, T, n, 3)
+    monkeypatch.setenv("GG_LIFT_SEARCH", "1")
+    S = G.Lift(N, M, d)
+    monkeypatch.delenv("GG_LIFT_SEARCH")
+    L = G.Lift(N, M, d)
+    best = {S: 1e9, L: 1e9}
+    for _ in range(40):
+        for h in (S, L):
+            t = time.perf_counter()
+            h.set_base(T)
+            h.eval(moves)
+            best[h] = min(best[h], time.perf_counter() - t)
+    assert best[L] < 1.25 * best[S], best
+    S.close()
     L.close()
 
 
