@@ -813,7 +813,7 @@ gg_status base_pass(gg_batch *b, int id) {
         for (auto &pe : b->engines)
             if (pe.first == std::make_pair(B.n, B.d)) eng = pe.second;
         if (!eng) {
-            gg_status s = gg_graph_create(B.n, B.d, b->device, &eng);
+            gg_status s = gg::graph_engine(B.n, B.d, b->device, &eng);
             if (s != GG_OK) return s;
             b->engines.push_back({{B.n, B.d}, eng});
             GB_CK(cudaSetDevice(b->device));

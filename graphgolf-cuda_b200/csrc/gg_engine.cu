@@ -128,7 +128,6 @@ struct gg_engine {
     int walk_rpg = 1;                    // rows per walk group
     unsigned walk_smem_off = 0;          // byte offset of the walk buffers in dynamic smem
     int32_t *d_h2 = nullptr;             // [rows][d*d] level-2 walk ends (walk_K >= 3)
-    size_t h2_elems = 0;
     // walk index (walk_index_kernel): [rows][walk_cap] entries, [rows][walk_off_stride] bucket starts
     uint16_t *d_went = nullptr, *d_woff = nullptr;
     size_t went_elems = 0, woff_elems = 0;
@@ -149,13 +148,15 @@ struct gg_engine {
     size_t off_levels_run = 0, off_batch_ns = 0, off_counts = 0;
     int *d_bad = nullptr;                // the table failed its range check
     int *d_asym = nullptr;               // adjacency not symmetric: no push levels
-    uint4 *d_V = nullptr, *d_F0 = nullptr, *d_F1 = nullptr;
+    uint4 *d_V = nullptr, *d_F0 = nullptr, *d_F1 = nullptr;   // one allocation (rows_room)
+    unsigned char *d_loop = nullptr;     // the level loop's other buffers lie in it (loop_room)
     uint32_t *d_fl0 = nullptr, *d_fl1 = nullptr;
     uint4 *d_P0 = nullptr, *d_P1 = nullptr;     // push-level frontier, all zero between launches
     uint32_t *d_pf0 = nullptr, *d_pf1 = nullptr;
     uint32_t *d_nf = nullptr;            // not-full bit per visited chunk
     uint32_t *d_nf2 = nullptr;           // its second copy (visited-set pull levels alternate)
     int *d_redo = nullptr, *h_redo = nullptr;   // sweep_kernel gave up: bfs_batch_kernel instead
+    bool loop_only = false;              // every evaluation runs the level loop (graph_engine)
     bool sweep = true;                   // sweep_kernel where it applies (GG_SWEEP, and no level mode asked for)
     int sweep_wait = 0;                  // evaluations until it is tried again
     int sweep_nC = 0;                    // its chunks per row (0: never)
@@ -163,7 +164,7 @@ struct gg_engine {
     int sweep_ends = 1;                  // most new vertices of a source's level below that
     bool sweep_list = false;             // the sources are a list (source_ball_kernel)
     bool ball_limits = false;            // the balls' kernels have their shared-memory limit
-    uint4 *d_swA = nullptr, *d_swB = nullptr;   // its level buffers, when wider than d_V
+    uint4 *d_swA = nullptr, *d_swB = nullptr;   // its level buffers (one allocation), when wider than d_V
     size_t sw_chunks = 0;                // chunks each of them holds
     int *d_wasym = nullptr;              // one-way flag of the table (walk_index_kernel)
     unsigned long long *d_vtot = nullptr;   // [nb][3] level totals (dense visited-set pull without own chunks)
@@ -221,14 +222,11 @@ void free_batch_buffers(gg_engine *e) {
     e->d_vall = nullptr;
     e->d_vall_fl = nullptr;
     e->vall_chunks = 0;
-    cudaFree(e->d_swA); cudaFree(e->d_swB);
+    cudaFree(e->d_swA);
     e->d_swA = e->d_swB = nullptr;
     e->sw_chunks = 0;
-    cudaFree(e->d_V); cudaFree(e->d_F0); cudaFree(e->d_F1);
-    cudaFree(e->d_fl0); cudaFree(e->d_fl1);
-    cudaFree(e->d_P0); cudaFree(e->d_P1); cudaFree(e->d_pf0); cudaFree(e->d_pf1);
-    cudaFree(e->d_nf);
-    cudaFree(e->d_nf2);
+    cudaFree(e->d_V); cudaFree(e->d_loop);
+    e->d_loop = nullptr;
     e->d_nf = e->d_nf2 = nullptr;
     e->d_V = e->d_F0 = e->d_F1 = nullptr;
     e->d_fl0 = e->d_fl1 = nullptr;
@@ -408,22 +406,85 @@ bool ball_limits(gg_engine *e) {
     return e->ball_limits = true;
 }
 
-// sweep_kernel's level buffers: d_V and d_F0, or a wider pair of its own.
+// An engine is created with the buffers of what its evaluations go to and takes others when
+// one needs them: of direct_kernel, sweep_kernel and the level loop most engines only ever
+// run one.  Creation and first call, with all of the level loop's at once and the others on
+// the first call -> now: n = 9000, d = 4: 5.9 -> 3.7 ms; n = 30012, d = 6: 5.7 -> 4.7.
+
+// The level-2 lists.
+gg_status h2_room(gg_engine *e) {
+    if (e->d_h2) return GG_OK;
+    invalidate_graph(e);
+    GG_CK(cudaMalloc(&e->d_h2, (size_t)e->rows * e->d * e->d * sizeof(int32_t)));
+    return GG_OK;
+}
+
+// Three buffers of a batch's rows.
+gg_status rows_room(gg_engine *e) {
+    if (e->d_V) return GG_OK;
+    invalidate_graph(e);
+    const size_t n = ((size_t)e->items + 31) / 32 * 32;   // (512-byte boundaries)
+    GG_CK(cudaMalloc(&e->d_V, 3 * n * sizeof(uint4)));
+    e->d_F0 = e->d_V + n;
+    e->d_F1 = e->d_F0 + n;
+    return GG_OK;
+}
+
+// Everything the level loop (bfs_batch_kernel) needs for the present plan.
+gg_status loop_room(gg_engine *e) {
+    gg_status s = rows_room(e);
+    if (s == GG_OK && e->walk_K >= 3) s = h2_room(e);
+    if (s != GG_OK) return s;
+    if (!e->d_loop) {
+        const size_t n = ((size_t)e->items + 31) / 32 * 32, f = (n / 32 + 63) / 64 * 64;   // (256-byte boundaries)
+        invalidate_graph(e);
+        GG_CK(cudaMalloc(&e->d_loop, 2 * n * sizeof(uint4) + 6 * f * sizeof(uint32_t)));
+        e->d_P0 = reinterpret_cast<uint4 *>(e->d_loop);
+        e->d_P1 = e->d_P0 + n;
+        uint32_t *w = reinterpret_cast<uint32_t *>(e->d_P1 + n);
+        for (uint32_t **q : {&e->d_fl0, &e->d_fl1, &e->d_pf0, &e->d_pf1, &e->d_nf, &e->d_nf2}) {
+            *q = w;
+            w += f;
+        }
+        e->p_dirty = true;
+    }
+    const size_t went = (size_t)e->rows * e->walk_cap, woff = (size_t)e->rows * e->walk_off_stride;
+    if (went != e->went_elems || woff != e->woff_elems) {
+        invalidate_graph(e);
+        cudaFree(e->d_went);
+        cudaFree(e->d_woff);
+        e->d_went = e->d_woff = nullptr;
+        e->went_elems = e->woff_elems = 0;
+        if (went) {
+            GG_CK(cudaMalloc(&e->d_went, went * sizeof(uint16_t)));
+            GG_CK(cudaMalloc(&e->d_woff, woff * sizeof(uint16_t)));
+        }
+        e->went_elems = went;
+        e->woff_elems = woff;
+    }
+    return GG_OK;
+}
+
+// sweep_kernel's buffers: the level-2 lists or none, the rows of every batch, and two level
+// buffers -- d_V and d_F0, or a wider pair of its own.  False: no memory for them.
 bool sweep_room(gg_engine *e, int nb) {
     const size_t chunks = (size_t)e->rows * e->sweep_nC;
-    if (!ball_limits(e) || (!e->sweep_list && !e->h2_elems) || (!sweep_in_f1(e, nb) && !vall_room(e, nb * chunks))) return false;
-    if (e->sweep_nC <= e->nC || chunks <= e->sw_chunks) return true;
-    invalidate_graph(e);
-    cudaFree(e->d_swA); cudaFree(e->d_swB);
-    e->d_swA = e->d_swB = nullptr;
-    e->sw_chunks = 0;
-    if (cudaMalloc(&e->d_swA, chunks * sizeof(uint4)) != cudaSuccess ||
-        cudaMalloc(&e->d_swB, chunks * sizeof(uint4)) != cudaSuccess) {
-        cudaFree(e->d_swA); cudaFree(e->d_swB);
-        e->d_swA = e->d_swB = nullptr;
+    if (!ball_limits(e)) return false;
+    if ((!e->sweep_list && h2_room(e) != GG_OK) || (e->sweep_nC <= e->nC && rows_room(e) != GG_OK)) {
         (void)cudaGetLastError();
         return false;
     }
+    if (!sweep_in_f1(e, nb) && !vall_room(e, nb * chunks)) return false;
+    if (e->sweep_nC <= e->nC || chunks <= e->sw_chunks) return true;
+    invalidate_graph(e);
+    cudaFree(e->d_swA);
+    e->d_swA = e->d_swB = nullptr;
+    e->sw_chunks = 0;
+    if (cudaMalloc(&e->d_swA, 2 * chunks * sizeof(uint4)) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    e->d_swB = e->d_swA + chunks;
     e->sw_chunks = chunks;
     return true;
 }
@@ -486,8 +547,9 @@ int sweep_width(gg_engine *e, const bool chosen) {
     return e->sweep_nC;
 }
 
-// Whether an evaluation goes to sweep_kernel (asked once per evaluation).  A graph that it
-// gave up on has paid for the attempt, and its engine leaves it out for a while.
+// Whether an evaluation goes to sweep_kernel (asked once per evaluation), if direct_kernel
+// does not take it and sweep_room has the memory.  A graph that it gave up on has paid for
+// the attempt, and its engine leaves it out for a while.
 bool sweep_turn(gg_engine *e, const gg_eval_opts *o) {
     const int cap = (o && o->max_levels > 0) ? o->max_levels : std::max(e->rows, 1);
     if (!e->sweep_nC || (o && (o->level_ns || o->want_wvc || o->src_begin || o->src_end)) || fault("barrier") ||
@@ -497,7 +559,7 @@ bool sweep_turn(gg_engine *e, const gg_eval_opts *o) {
         --e->sweep_wait;
         return false;
     }
-    return sweep_room(e, sweep_batches(e));
+    return true;
 }
 
 template <int D, bool ONE>
@@ -591,20 +653,6 @@ gg_status plan(gg_engine *e, int want_bits) {
         e->batch_bits = bits;
         e->nC = bits / 128;
         e->items = (uint32_t)items;
-        const size_t vbytes = (size_t)items * sizeof(uint4);
-        const size_t fwords = (size_t)((items + 31) / 32);
-        GG_CK(cudaMalloc(&e->d_V, vbytes));
-        GG_CK(cudaMalloc(&e->d_F0, vbytes));
-        GG_CK(cudaMalloc(&e->d_F1, vbytes));
-        GG_CK(cudaMalloc(&e->d_fl0, fwords * 4));
-        GG_CK(cudaMalloc(&e->d_fl1, fwords * 4));
-        GG_CK(cudaMalloc(&e->d_P0, vbytes));
-        GG_CK(cudaMalloc(&e->d_P1, vbytes));
-        GG_CK(cudaMalloc(&e->d_pf0, fwords * 4));
-        GG_CK(cudaMalloc(&e->d_pf1, fwords * 4));
-        GG_CK(cudaMalloc(&e->d_nf, fwords * 4));
-        GG_CK(cudaMalloc(&e->d_nf2, fwords * 4));
-        e->p_dirty = true;
     }
     // Walk pass: levels 1..K of each batch from the walk ends of every row.
     e->walk_K = walk_levels(e);
@@ -617,33 +665,10 @@ gg_status plan(gg_engine *e, int want_bits) {
         walk_bytes = (size_t)(gg::kBlock / 32) * gg::walk_smem_per_warp(e->nC);
     }
     e->sweep_nC = sweep_width(e, chosen);
-    const size_t h2_need = e->walk_K >= 3 || (e->sweep_nC && !e->sweep_list) ? (size_t)e->rows * e->d * e->d : 0;
-    if (h2_need != e->h2_elems) {
-        cudaFree(e->d_h2);
-        e->d_h2 = nullptr;
-        e->h2_elems = 0;
-        if (h2_need) {
-            GG_CK(cudaMalloc(&e->d_h2, h2_need * sizeof(int32_t)));
-            e->h2_elems = h2_need;
-        }
-    }
     // row stride of the index: the walk ends, rounded up to a multiple of 8 (rows start
     // 16-byte aligned: the index kernel writes them 16 bytes at a time)
     e->walk_cap = e->walk_K ? (int)((walk_cap_for(e->d, e->walk_K) + 7) & ~7ll) : 0;
     e->walk_off_stride = e->walk_K ? (int)(((long long)e->reps.size() + bits - 1) / bits) * e->walk_K + 1 : 0;
-    const size_t went_need = (size_t)e->rows * e->walk_cap, woff_need = (size_t)e->rows * e->walk_off_stride;
-    if (went_need != e->went_elems || woff_need != e->woff_elems) {
-        cudaFree(e->d_went);
-        cudaFree(e->d_woff);
-        e->d_went = e->d_woff = nullptr;
-        e->went_elems = e->woff_elems = 0;
-        if (went_need) {
-            GG_CK(cudaMalloc(&e->d_went, went_need * sizeof(uint16_t)));
-            GG_CK(cudaMalloc(&e->d_woff, woff_need * sizeof(uint16_t)));
-            e->went_elems = went_need;
-            e->woff_elems = woff_need;
-        }
-    }
     int per_sm = 0, sms = 0;
     GG_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device));
     GG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel_for(e->d), gg::kBlock, walk_bytes));
@@ -718,6 +743,59 @@ gg_status ensure_counters(gg_engine *e, int cap, int nb) {
 
 void *direct_for(int W) {
     return W == 1 ? (void *)gg::direct_kernel<1> : W == 2 ? (void *)gg::direct_kernel<2> : (void *)gg::direct_kernel<4>;
+}
+
+// ---- small graphs: direct_kernel -------------------------------------------------
+
+struct DirectPlan {
+    int W = 0;            // 32-source words a vertex (0: not for this evaluation)
+    bool adj_smem = false;
+    size_t smem = 0;
+    int grid = 0, block = 0;
+};
+
+constexpr double kSweepUsPerChunk = 0.064e-3, kLoopUsPerChunk = 0.12e-3;
+constexpr int kDirectCheck = 32;   // look-ups of the one-way check, at most, a thread of direct_kernel
+
+// The word width that makes the fewest rounds of blocks cheapest, or none: the visited
+// sets of every width must fit a block's shared memory.  A random row of 4, 8 or 16 bytes
+// per lane costs about 3.5, 6.2 and 10.4 shared-memory cycles a warp.
+DirectPlan direct_plan(const gg_engine *e, int ns, bool wvc, bool sweep) {
+    DirectPlan best;
+    if (!e->direct || e->d < 1 || e->rows < 1 || e->rows > 65535 || ns < 1) return best;   // (d = 0: no walk ends)
+    const size_t budget = (size_t)e->smem_optin - 1024;
+    double cost = 1e300;
+    for (int W : {1, 2, 4}) {
+        const size_t set = ((size_t)e->rows * W + 3) / 4 * 16, adj = ((size_t)e->rows * e->d * 2 + 15) / 16 * 16;
+        if (2 * set > budget) continue;
+        const int grid = (ns + 32 * W - 1) / (32 * W);
+        const bool in_smem = 2 * set + adj <= budget;
+        const size_t smem = 2 * set + (in_smem ? adj : 0);
+        const int block = e->rows >= 1024 ? gg::kDirectBlock : std::max(128, (e->rows + 31) / 32 * 32);
+        const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(1024 / block, budget / std::max<size_t>(smem + 1024, 1)));
+        const double rounds = std::ceil((double)grid / (e->sms * per_sm));
+        const double c = rounds * (W == 1 ? 3.5 : W == 2 ? 6.2 : 10.4) * per_sm;
+        if (c < cost && (rounds == 1 || e->rows <= 20480)) {
+            cost = c;
+            best = DirectPlan{W, in_smem, smem, grid, block};
+        }
+    }
+    // Against bfs_batch_kernel: microseconds of the two (fits of both sides over n = 64 to
+    // 27000 and lifts of 20 to 4000 orbits).  A round of one-word groups takes 3.2 + 0.1 d
+    // ns a row (a tenth more with the WVC masks), less certain for a single round; the level
+    // loop 50 us and 0.12 ns a chunk of 128 sources.  Device times: n = 4096, d = 16: 25
+    // against 67 us; 16000, 6: 239 / 372; lifts of 6000 vertices, 500 orbits: 29 / 59, of
+    // 20000, 1000: 85 / 82, of 20000, 2000: 96 / 90.
+    // Against sweep_kernel, whose levels take half of that a chunk (whole calls, direct
+    // first): n = 8192, d = 4: 70 against 111 us, 8192, 16: 120 / 131, 9000, 7: 104 / 133,
+    // 10000, 8: 169 / 126, 10000, 5: 150 / 129, 12000, 4: 144 / 145, 16384, 6: 302 / 187.
+    if (best.W) {
+        const bool one = best.grid <= e->sms;
+        const double direct_us = cost / 3.5 * e->rows * (3.2 + 0.1 * e->d) * 1e-3 * (wvc ? 1.1 : 1.0) * (one ? 1.12 : 1.0);
+        const double chunks = (double)e->rows * ((ns + 127) / 128);
+        if (direct_us > 50.0 + (sweep ? kSweepUsPerChunk : kLoopUsPerChunk) * chunks) best.W = 0;
+    }
+    return best;
 }
 
 gg_status create_common(gg_engine *e) {
@@ -795,6 +873,11 @@ gg_status create_common(gg_engine *e) {
     const int wait_ms = env_int("GG_WAIT_LIMIT_MS", 10000);
     e->wait_ns = (long long)std::max(wait_ms, 1) * 1000000ll;
     gg_status s = plan(e, 0);
+    // the buffers of a whole evaluation
+    const bool sweep = e->sweep_nC > 0;
+    if (s == GG_OK && (e->loop_only || !direct_plan(e, (int)e->reps.size(), false, sweep).W) &&
+        (e->loop_only || !sweep || !sweep_room(e, sweep_batches(e))))
+        s = loop_room(e);
     if (s != GG_OK) return s;
     return ensure_counters(e, 128, 1);
 }
@@ -808,6 +891,20 @@ gg_status finish_create(gg_engine *e, gg_engine **out) {
     }
     *out = e;
     return GG_OK;
+}
+
+gg_status graph_create(int N, int degree_max, int device, bool loop_only, gg_engine **out) {
+    if (!out) return fail(GG_BAD_ARG, "null out");
+    *out = nullptr;
+    if (N < 1 || degree_max < 0) return fail(GG_BAD_ARG, "need N >= 1, degree_max >= 0");
+    gg_engine *e = new gg_engine();
+    e->loop_only = loop_only;
+    e->form = FORM_GRAPH; e->device = device;
+    e->N = N; e->M = N; e->d = degree_max; e->rows = N; e->scale = 1;
+    e->table_elems = (size_t)N * degree_max;
+    e->reps.resize(N);
+    for (int i = 0; i < N; ++i) e->reps[i] = i;
+    return finish_create(e, out);
 }
 
 // A lifted form's table (device memory) -> the pull adjacency d_adj.
@@ -827,59 +924,6 @@ void launch_expand(gg_engine *e, const int32_t *d_table, cudaStream_t st, const 
         x.ns_total = (int)e->reps.size();
     }
     gg::expand_kernel<<<(int)std::min<long long>((n + 255) / 256, 8192), 256, 0, st>>>(x);
-}
-
-// ---- small graphs: direct_kernel -------------------------------------------------
-
-struct DirectPlan {
-    int W = 0;            // 32-source words a vertex (0: not for this evaluation)
-    bool adj_smem = false;
-    size_t smem = 0;
-    int grid = 0, block = 0;
-};
-
-// The word width that makes the fewest rounds of blocks cheapest, or none: the visited
-// sets of every width must fit a block's shared memory.  A random row of 4, 8 or 16 bytes
-// per lane costs about 3.5, 6.2 and 10.4 shared-memory cycles a warp.
-constexpr double kSweepUsPerChunk = 0.064e-3, kLoopUsPerChunk = 0.12e-3;
-constexpr int kDirectCheck = 32;   // look-ups of the one-way check, at most, a thread of direct_kernel
-
-DirectPlan direct_plan(const gg_engine *e, int ns, bool wvc, bool sweep) {
-    DirectPlan best;
-    if (!e->direct || e->d < 1 || e->rows < 1 || e->rows > 65535 || ns < 1) return best;   // (d = 0: no walk ends)
-    const size_t budget = (size_t)e->smem_optin - 1024;
-    double cost = 1e300;
-    for (int W : {1, 2, 4}) {
-        const size_t set = ((size_t)e->rows * W + 3) / 4 * 16, adj = ((size_t)e->rows * e->d * 2 + 15) / 16 * 16;
-        if (2 * set > budget) continue;
-        const int grid = (ns + 32 * W - 1) / (32 * W);
-        const bool in_smem = 2 * set + adj <= budget;
-        const size_t smem = 2 * set + (in_smem ? adj : 0);
-        const int block = e->rows >= 1024 ? gg::kDirectBlock : std::max(128, (e->rows + 31) / 32 * 32);
-        const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(1024 / block, budget / std::max<size_t>(smem + 1024, 1)));
-        const double rounds = std::ceil((double)grid / (e->sms * per_sm));
-        const double c = rounds * (W == 1 ? 3.5 : W == 2 ? 6.2 : 10.4) * per_sm;
-        if (c < cost && (rounds == 1 || e->rows <= 20480)) {
-            cost = c;
-            best = DirectPlan{W, in_smem, smem, grid, block};
-        }
-    }
-    // Against bfs_batch_kernel: microseconds of the two (fits of both sides over n = 64 to
-    // 27000 and lifts of 20 to 4000 orbits).  A round of one-word groups takes 3.2 + 0.1 d
-    // ns a row (a tenth more with the WVC masks), less certain for a single round; the level
-    // loop 50 us and 0.12 ns a chunk of 128 sources.  Device times: n = 4096, d = 16: 25
-    // against 67 us; 16000, 6: 239 / 372; lifts of 6000 vertices, 500 orbits: 29 / 59, of
-    // 20000, 1000: 85 / 82, of 20000, 2000: 96 / 90.
-    // Against sweep_kernel, whose levels take half of that a chunk (whole calls, direct
-    // first): n = 8192, d = 4: 70 against 111 us, 8192, 16: 120 / 131, 9000, 7: 104 / 133,
-    // 10000, 8: 169 / 126, 10000, 5: 150 / 129, 12000, 4: 144 / 145, 16384, 6: 302 / 187.
-    if (best.W) {
-        const bool one = best.grid <= e->sms;
-        const double direct_us = cost / 3.5 * e->rows * (3.2 + 0.1 * e->d) * 1e-3 * (wvc ? 1.1 : 1.0) * (one ? 1.12 : 1.0);
-        const double chunks = (double)e->rows * ((ns + 127) / 128);
-        if (direct_us > 50.0 + (sweep ? kSweepUsPerChunk : kLoopUsPerChunk) * chunks) best.W = 0;
-    }
-    return best;
 }
 
 gg_status ensure_direct(gg_engine *e, int cap) {
@@ -1036,7 +1080,11 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
     const int ns_all = s1 - s0;
     bool sweep = !x && (sweep_asked < 0 ? sweep_turn(e, o) : sweep_asked != 0);
     if (!x && !want_ns && !fault("barrier")) {
-        const DirectPlan p = direct_plan(e, ns_all, wvc, sweep);
+        DirectPlan p = direct_plan(e, ns_all, wvc, sweep);
+        if (!p.W && sweep && !sweep_room(e, sweep_batches(e))) {
+            sweep = false;
+            p = direct_plan(e, ns_all, wvc, false);
+        }
         if (p.W) return direct_eval(e, p, d_table_in, nullptr, o, s0, ns_all, cap_req, r, st);
     }
     const int nb_plain = (ns_all + e->batch_bits - 1) / e->batch_bits;
@@ -1060,16 +1108,6 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
     const int stride = cap_req + 1;      // counts of batch b at [b * stride, (b + 1) * stride)
 
     (void)cudaGetLastError();  // launch checks below must not see an earlier, unrelated error
-    if (e->p_dirty) {
-        // New buffers, or a launch that stopped early: the push buffers are
-        // zero again only after these four writes.
-        const size_t vbytes = (size_t)e->items * sizeof(uint4), fbytes = (size_t)((e->items + 31) / 32) * 4;
-        GG_CK(cudaMemsetAsync(e->d_P0, 0, vbytes, st));
-        GG_CK(cudaMemsetAsync(e->d_P1, 0, vbytes, st));
-        GG_CK(cudaMemsetAsync(e->d_pf0, 0, fbytes, st));
-        GG_CK(cudaMemsetAsync(e->d_pf1, 0, fbytes, st));
-        e->p_dirty = false;
-    }
     if (fault("launch")) return fail(GG_CUDA_ERROR, "injected launch failure");
     const unsigned extra = fault("barrier") ? 1u : 0u;
     const size_t lv = (size_t)cap_req + 1;
@@ -1081,15 +1119,32 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
     // Not with sweep_kernel either, whose rows are where the walk of all batches would put its.
     int walk_K = 0, launches = e->sweep_list ? 3 : 4;
     void *wall = nullptr;
-    auto plan_walk = [&] {
+    // What the level loop needs before it is enqueued or replayed.
+    auto loop_ready = [&]() -> gg_status {
+        gg_status ls = loop_room(e);
+        if (ls != GG_OK) return ls;
+        if (e->p_dirty) {
+            // New buffers, or a launch that stopped early: the push buffers are
+            // zero again only after these four writes.
+            const size_t vbytes = (size_t)e->items * sizeof(uint4), fbytes = (size_t)((e->items + 31) / 32) * 4;
+            GG_CK(cudaMemsetAsync(e->d_P0, 0, vbytes, st));
+            GG_CK(cudaMemsetAsync(e->d_P1, 0, vbytes, st));
+            GG_CK(cudaMemsetAsync(e->d_pf0, 0, fbytes, st));
+            GG_CK(cudaMemsetAsync(e->d_pf1, 0, fbytes, st));
+        }
+        e->p_dirty = true;  // until the launch is known to have finished cleanly
         walk_K = (wvc || (x && (x->planes || within))) ? 0 : std::min(e->walk_K, cap_req);
         // (one level less where the walk of all batches then covers them: a level costs less
         // than a walk pass per batch)
         if (walk_K == 4 && e->walk_auto && walk_all_for(e, 3, nb_plain)) walk_K = 3;
         launches = 1 + ((long long)e->rows * e->d > 0 ? 1 : 0) + (walk_K > 0 ? 1 : 0) + (walk_K >= 3 ? 1 : 0);
         wall = walk_K > 0 ? walk_all_for(e, walk_K, nb_plain) : nullptr;
+        return GG_OK;
     };
-    if (!sweep) plan_walk();
+    if (!sweep) {
+        s = loop_ready();
+        if (s != GG_OK) return s;
+    }
 
     // Everything the GPU does for one evaluation, on `q`: status words zeroed,
     // table -> adjacency (checked), one cooperative launch for every source
@@ -1352,7 +1407,6 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
     // the outputs asked for, reallocated buffers -- captures a new graph.
     const EvalKey key{d_table_in, e->d_status, e->d_V, x ? (const void *)x->inv : nullptr,
                       x ? (const void *)x->planes : nullptr, s0, ns_all, cap_req, wvc, want_ns, sweep};
-    e->p_dirty = true;  // until the launch is known to have finished cleanly
     bool replayed = false;
     if (e->use_graph && !extra && !(x && x->no_graph)) {
         if (!e->graph_exec || !(key == e->graph_key)) {
@@ -1397,15 +1451,14 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
         if (p.W) {
             const double first_ms = e->last_ms;
             const int first_launches = e->last_launches;
-            e->p_dirty = false;
             const gg_status ds = direct_eval(e, p, d_table_in, nullptr, o, s0, ns_all, cap_req, r, st);
             e->last_ms += first_ms;
             e->last_launches += first_launches;
             return ds;
         }
         nb = nb_plain;
-        plan_walk();
-        gg_status es = enqueue(st, true);
+        gg_status es = loop_ready();
+        if (es == GG_OK) es = enqueue(st, true);
         if (es != GG_OK) return es;
         GG_CK(cudaStreamSynchronize(st));
         GG_CK(cudaEventElapsedTime(&ms, e->ev0, e->ev1));
@@ -1419,7 +1472,7 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
     if (e->h_ctl->err)
         return fail(GG_TIMEOUT, "grid barrier wait exceeded its limit at level " +
                                     std::to_string(e->h_ctl->err_level));
-    e->p_dirty = false;
+    if (!sweep) e->p_dirty = false;
 
     // Exact fold of the per-batch level counters.
     gg_result R{};
@@ -1598,6 +1651,8 @@ gg_status engine_eval(gg_engine *e, const int32_t *d_table, const gg_eval_opts *
     GG_CK(cudaSetDevice(e->device));
     return run_eval(e, d_table, o, r, st ? st : e->stream, x);
 }
+gg_status graph_engine(int n, int d, int device, gg_engine **out) { return graph_create(n, d, device, true, out); }
+
 int engine_plane_cols(const gg_engine *e) {
     const int n_src = (int)e->reps.size();
     return ((n_src + e->batch_bits - 1) / e->batch_bits) * e->nC;
@@ -1623,16 +1678,7 @@ const char *gg_status_str(gg_status s) {
 const char *gg_last_error(void) { return g_err.c_str(); }
 
 gg_status gg_graph_create(int N, int degree_max, int device, gg_engine **out) {
-    if (!out) return fail(GG_BAD_ARG, "null out");
-    *out = nullptr;
-    if (N < 1 || degree_max < 0) return fail(GG_BAD_ARG, "need N >= 1, degree_max >= 0");
-    gg_engine *e = new gg_engine();
-    e->form = FORM_GRAPH; e->device = device;
-    e->N = N; e->M = N; e->d = degree_max; e->rows = N; e->scale = 1;
-    e->table_elems = (size_t)N * degree_max;
-    e->reps.resize(N);
-    for (int i = 0; i < N; ++i) e->reps[i] = i;
-    return finish_create(e, out);
+    return graph_create(N, degree_max, device, false, out);
 }
 
 gg_status gg_conv_create(int N, int M, int degree, int device, gg_engine **out) {
@@ -1754,7 +1800,8 @@ gg_status gg_set_batch_sources(gg_engine *e, int sources) {
     GG_CK(cudaSetDevice(e->device));
     GG_CK(cudaStreamSynchronize(e->stream));
     e->direct = sources == 0 && e->direct_allowed;   // an explicit width runs the batches it asks for
-    return plan(e, sources);
+    const gg_status s = plan(e, sources);
+    return s == GG_OK ? loop_room(e) : s;
 }
 
 gg_status gg_autotune(gg_engine *e, const int32_t *table, int trials, int *best_sources, double *best_ms) {
@@ -1813,6 +1860,7 @@ gg_status gg_autotune(gg_engine *e, const int32_t *table, int trials, int *best_
                 e->bps_cap = bps;
                 e->walk_pref = walk;
                 gg_status s = plan(e, w);
+                if (s == GG_OK) s = loop_room(e);
                 if (s == GG_OUT_OF_MEMORY) { (void)cudaGetLastError(); break; }  // too wide for this device
                 if (s != GG_OK) return s;
                 if (walk == -1) auto_walks = e->walk_K > 0;

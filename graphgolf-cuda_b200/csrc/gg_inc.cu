@@ -308,7 +308,7 @@ gg_status gg_inc_create(int n, int degree, int device, gg_inc **out) {
     *out = nullptr;
     gg_inc *h = new gg_inc();
     h->n = n; h->d = degree; h->device = device;
-    gg_status s = gg_graph_create(n, degree, device, &h->eng);
+    gg_status s = gg::graph_engine(n, degree, device, &h->eng);
     if (s != GG_OK) { inc_free(h); return s; }
     if (cudaSetDevice(device) != cudaSuccess) { inc_free(h); return ifail(GG_NO_DEVICE, "cudaSetDevice failed"); }
     h->cols = (unsigned)gg::engine_plane_cols(h->eng);

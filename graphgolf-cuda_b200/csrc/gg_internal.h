@@ -30,6 +30,9 @@ __attribute__((visibility("hidden"))) std::string tune_key(int device, const cha
 __attribute__((visibility("hidden"))) bool tune_get(const std::string &key, std::vector<int> *vals);
 __attribute__((visibility("hidden"))) void tune_put(const std::string &key, const std::vector<int> &vals);
 
+// gg_graph_create for an engine that only engine_eval runs, with options that need the level loop.
+__attribute__((visibility("hidden"))) gg_status graph_engine(int n, int d, int device, gg_engine **out);
+
 // One evaluation of `e` on the device table `d_table` (on stream `st`, blocking),
 // with the extra options `x` (nullptr: none).
 __attribute__((visibility("hidden"))) gg_status engine_eval(gg_engine *e, const int32_t *d_table,

@@ -205,3 +205,29 @@ def test_direct_while_the_default_stream_is_busy():
             assert (r["total"], r["reached"], r["levels"]) == (o.total(), int(o.reached.sum()), o.levels)
         e.close()
         torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("n,d", [(5000, 6), (9000, 4), (12000, 8)])
+def test_an_engine_takes_the_memory_of_what_it_runs(n, d):
+    """Created and called once: the rows of all batches, the level loop's buffers and the
+    level-2 lists only where the call needs them (bytes of the whole engine)."""
+    import torch
+    adj = G.random_regular(n, d, 1)
+    G.cudaASPLgraph(n, d).calc(adj)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    e = G.cudaASPLgraph(n, d)
+    e.calc(adj)
+    used = before - torch.cuda.mem_get_info()[0]
+    rows = n * ((n + 4095) // 4096) * 512                    # of every source, once
+    assert used <= (3 * rows if n > 10000 else 0) + n * d * d * 4 + (8 << 20), used
+    # and what it runs after that: a range of the sources, a graph with one-way entries
+    half = [e.eval(adj, src_range=r) for r in ((0, 3000), (3000, n))]
+    assert sum(r["total"] for r in half) == e.calc(adj)[1]
+    odd = adj.copy()
+    odd[7, 1] = (odd[7, 1] + 1) % n
+    for t in (odd, adj):
+        o = O.bfs_pull(t, np.arange(n))
+        r = e.eval(t)
+        assert (r["total"], r["reached"], r["levels"]) == (o.total(), int(o.reached.sum()), o.levels)
+    e.close()
