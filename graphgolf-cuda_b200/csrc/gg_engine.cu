@@ -160,6 +160,7 @@ struct gg_engine {
     bool sweep = true;                   // sweep_kernel where it applies (GG_SWEEP, and no level mode asked for)
     int sweep_wait = 0;                  // evaluations until it is tried again
     int sweep_nC = 0;                    // its chunks per row (0: never)
+    bool width_asked = false;            // ... are those of the batch width asked for (gg_set_batch_sources)
     int sweep_K = 0;                     // levels before its dense ones
     int sweep_ends = 1;                  // most new vertices of a source's level below that
     bool sweep_list = false;             // the sources are a list (source_ball_kernel)
@@ -506,7 +507,7 @@ constexpr int kSrcBallWarps = gg::kSrcBallBlock / 32;
 // gathers then still hit L2, and there are fewer barriers and last_rows passes.  n = 65536,
 // d = 8: 4096 wide 1322 us, 8192 1225, 12288 1441; n = 50000, d = 6: 923, 893, 978;
 // n = 30012, d = 6: 4096 wide 452, 8192 408, 16384 386.
-int sweep_width(gg_engine *e, const bool chosen) {
+int sweep_width(gg_engine *e) {
     const int n_src = (int)e->reps.size();
     const bool all = n_src == e->rows && !e->d_inv && e->src_first == 0;
     e->sweep_list = !all;
@@ -518,7 +519,7 @@ int sweep_width(gg_engine *e, const bool chosen) {
     int nC = 32 * ((parts + nb - 1) / nb);
     if (!all && n_src <= 2048)
         for (nC = 1; 128 * nC < n_src;) nC *= 2;
-    e->sweep_nC = chosen ? e->nC : nC;
+    e->sweep_nC = e->width_asked ? e->nC : nC;
     if (e->sweep_nC % 32 != 0 && (all || (e->sweep_nC & (e->sweep_nC - 1)) != 0 || e->sweep_nC > 16)) return 0;
     if ((long long)e->rows * e->sweep_nC >= (1ll << 31)) return 0;
     if (all) {
@@ -615,7 +616,6 @@ gg_status plan(gg_engine *e, int want_bits) {
     invalidate_graph(e);
     const int n_src = (int)e->reps.size();
     int bits;
-    bool chosen = true;   // the batch width was asked for, or tuned
     if (want_bits > 0) {
         bits = want_bits;
     } else {
@@ -628,7 +628,6 @@ gg_status plan(gg_engine *e, int want_bits) {
             e->bps_cap = tuned[1];
             e->walk_pref = tuned[2];
         } else {
-            chosen = false;
             // The widest batch whose three bitsets (3 * rows * bits / 8 bytes)
             // stay within 3/4 of the L2, so that the gathers hit L2 rather than
             // HBM; at least 4096 sources (one 512-byte row segment per vertex)
@@ -664,7 +663,7 @@ gg_status plan(gg_engine *e, int want_bits) {
         e->walk_rpg = 32 / g;
         walk_bytes = (size_t)(gg::kBlock / 32) * gg::walk_smem_per_warp(e->nC);
     }
-    e->sweep_nC = sweep_width(e, chosen);
+    e->sweep_nC = sweep_width(e);
     // row stride of the index: the walk ends, rounded up to a multiple of 8 (rows start
     // 16-byte aligned: the index kernel writes them 16 bytes at a time)
     e->walk_cap = e->walk_K ? (int)((walk_cap_for(e->d, e->walk_K) + 7) & ~7ll) : 0;
@@ -1800,6 +1799,7 @@ gg_status gg_set_batch_sources(gg_engine *e, int sources) {
     GG_CK(cudaSetDevice(e->device));
     GG_CK(cudaStreamSynchronize(e->stream));
     e->direct = sources == 0 && e->direct_allowed;   // an explicit width runs the batches it asks for
+    e->width_asked = sources > 0;
     const gg_status s = plan(e, sources);
     return s == GG_OK ? loop_room(e) : s;
 }
@@ -1811,10 +1811,10 @@ gg_status gg_autotune(gg_engine *e, const int32_t *table, int trials, int *best_
     const int n_src = (int)e->reps.size();
     struct Planned {   // the shapes timed here are bfs_batch_kernel's
         gg_engine *e;
-        bool was;
-        ~Planned() { e->direct = was; }
-    } planned{e, e->direct};
-    e->direct = false;
+        bool direct, sweep;
+        ~Planned() { e->direct = direct; e->sweep = sweep; }
+    } planned{e, e->direct, e->sweep};
+    e->direct = e->sweep = e->width_asked = false;
     // the L2-resident width the default plan picks, and its neighbours
     int base = 0, max_bps = 0;
     {
@@ -1879,6 +1879,7 @@ gg_status gg_autotune(gg_engine *e, const int32_t *table, int trials, int *best_
     if (!best) return fail(GG_OUT_OF_MEMORY, "no batch width fits");
     e->bps_cap = best_bps;
     e->walk_pref = best_walk;
+    e->sweep = planned.sweep;
     gg_status s = plan(e, best);
     if (s != GG_OK) return s;
     gg::tune_put(engine_tune_key(e), {best, best_bps, best_walk});

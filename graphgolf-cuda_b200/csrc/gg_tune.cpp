@@ -123,9 +123,9 @@ std::string tune_key(int device, const char *what, const std::vector<long long> 
             names[device] = gpu;
         }
     }
-    // the format version also retires entries tuned for earlier kernels (v2: the
-    // level kernel at 4 resident blocks a SM, the walk of all batches in one launch)
-    std::string k = "v2|" + gpu + "|" + what;
+    // the format version also retires entries tuned for earlier kernels (v3: the walk of
+    // all batches at degrees 3 and 6 too, near sources in the batch kernel)
+    std::string k = "v3|" + gpu + "|" + what;
     for (long long d : dims) k += "|" + std::to_string(d);
     return k;
 }

@@ -146,7 +146,9 @@ gg_status gg_set_batch_sources(gg_engine *e, int sources);
  * the walk pass (automatic depth, or off) -- keeps the fastest in this engine's
  * plan and records it in the tuning cache (see gg_set_tune_cache) for engines of the
  * same form, size, degree and source count on the same kind of GPU, in this process
- * and later ones.  best_sources / best_ms may be NULL. */
+ * and later ones.  The shapes, and best_ms, are the general level loop's: evaluations
+ * that a kernel of their own takes (small graphs, every vertex a source, lifts) choose
+ * theirs by themselves.  best_sources / best_ms may be NULL. */
 gg_status gg_autotune(gg_engine *e, const int32_t *table, int trials, int *best_sources,
                       double *best_ms);
 /* The engine's current plan: sources per batch, resident blocks per SM, levels the

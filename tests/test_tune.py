@@ -81,3 +81,32 @@ def test_batch_and_lift_tuning_persist(tmp_path):
         assert other == {"chunk": chunk, "group": grp}
     finally:
         G.set_tune_cache(os.environ.get("GG_TUNE_CACHE"))
+
+
+def test_tuned_width_leaves_the_sweep_its_own(tmp_path):
+    """gg_autotune times the level loop; a graph that sweep_kernel takes runs batches of that
+    kernel's own width before and after, in the tuned engine and in later processes."""
+    cache = str(tmp_path / "tune.tsv")
+    G.set_tune_cache(cache)
+    keys = ("total", "reached", "levels", "batches")
+    try:
+        adj = G.random_regular(20484, 6, 3)
+        e = G.cudaASPLgraph(20484, 6, 0)
+        want = e.eval(adj)
+        e.autotune(adj, trials=1)
+        got = e.eval(adj)
+        assert all(got[k] == want[k] for k in keys)
+        part = e.eval(adj, src_range=(0, 20483))     # (the level loop's, at the tuned shape)
+        assert (part["levels"], part["reached"]) == (want["levels"], 20483 * 20484)
+        e.set_batch_sources(4096)                    # asked for: the sweep's too
+        assert e.eval(adj)["batches"] == 6
+    finally:
+        G.set_tune_cache(os.environ.get("GG_TUNE_CACHE"))
+    key = next(r.split("\t")[0] for r in open(cache) if "|graph|" in r and "|20484|" in r)
+    for width in (4096, 8192):
+        with open(cache, "w") as f:
+            f.write("%s\t%d 0 -1\n" % (key, width))
+        other = second_process(
+            "adj = G.random_regular(20484, 6, 3)\ne = G.cudaASPLgraph(20484, 6, 0)\nr = e.eval(adj)\n"
+            "print(json.dumps({'plan': e.plan()[0], **{k: int(r[k]) for k in %r}}))" % (keys,), cache)
+        assert other == {"plan": width, **{k: int(want[k]) for k in keys}}
