@@ -756,6 +756,15 @@ struct DirectPlan {
 constexpr double kSweepUsPerChunk = 0.064e-3, kLoopUsPerChunk = 0.12e-3;
 constexpr int kDirectCheck = 32;   // look-ups of the one-way check, at most, a thread of direct_kernel
 
+// Rows that an evaluation checks for one-way entries, to take its first levels from walks
+// then, or 0: where the check is not a small part of a pass, and for a while after a table
+// that had some.
+int direct_check(const gg_engine *e, int grid, int block) {
+    const int rows = e->dir_orbits ? e->dir_orbits : e->rows;
+    const long long looks = ((long long)rows + grid - 1) / grid * e->d * e->d;
+    return e->dir_wait > 0 || looks > (long long)kDirectCheck * block ? 0 : rows;
+}
+
 // The word width that makes the fewest rounds of blocks cheapest, or none: the visited
 // sets of every width must fit a block's shared memory.  A random row of 4, 8 or 16 bytes
 // per lane costs about 3.5, 6.2 and 10.4 shared-memory cycles a warp.
@@ -788,10 +797,17 @@ DirectPlan direct_plan(const gg_engine *e, int ns, bool wvc, bool sweep) {
     // Against sweep_kernel, whose levels take half of that a chunk (whole calls, direct
     // first): n = 8192, d = 4: 70 against 111 us, 8192, 16: 120 / 131, 9000, 7: 104 / 133,
     // 10000, 8: 169 / 126, 10000, 5: 150 / 129, 12000, 4: 144 / 145, 16384, 6: 302 / 187.
+    // Degrees without a loop of their own cost more where no walk shortens the search (tables
+    // with one-way entries, whole calls against bfs_batch_kernel: 16000, 10: 536 / 454; 20000,
+    // 10: 828 / 567; 14000, 13: 443 / 392; 10000, 9: 250 / 276; 9000, 16: 174 / 241), and above 20
+    // they need their rows in shared memory (4096, 24: 89 / 116; 9000, 24: 344 / 301; 3000, 40,
+    // 120 KB short of room: 159 / 109), few of them (1000, 64: 136 / 107; 1000, 40: 59 / 88).
     if (best.W) {
         const bool one = best.grid <= e->sms;
-        const double direct_us = cost / 3.5 * e->rows * (3.2 + 0.1 * e->d) * 1e-3 * (wvc ? 1.1 : 1.0) * (one ? 1.12 : 1.0);
+        double direct_us = cost / 3.5 * e->rows * (3.2 + 0.1 * e->d) * 1e-3 * (wvc ? 1.1 : 1.0) * (one ? 1.12 : 1.0);
+        if (e->d >= 9 && e->d != 12 && !direct_check(e, best.grid, best.block)) direct_us *= std::min(1.3, 1.0 + 0.06 * (e->d - 7));
         const double chunks = (double)e->rows * ((ns + 127) / 128);
+        if (e->d > 20 && (!best.adj_smem || (e->d > 48 && (long long)e->rows * e->d > 50000))) best.W = 0;
         if (direct_us > 50.0 + (sweep ? kSweepUsPerChunk : kLoopUsPerChunk) * chunks) best.W = 0;
     }
     return best;
@@ -990,13 +1006,9 @@ gg_status direct_eval(gg_engine *e, const DirectPlan &p, const int32_t *table, c
     a.masks = wvc ? reinterpret_cast<unsigned *>(e->d_dir + off) : nullptr;
     a.h_masks = reinterpret_cast<unsigned *>(e->h_dir + off);
     a.batch_ns = e->h_batch_ns;
-    // Walks, where the check for one-way entries is a small part of a pass (kDirectCheck
-    // look-ups a thread), and not for a while after a table that had some.
-    a.check = e->dir_orbits ? e->dir_orbits : e->rows;
+    a.check = direct_check(e, p.grid, p.block);
     a.check_src = e->dir_orbits > 0;
-    const long long looks = ((long long)a.check + p.grid - 1) / p.grid * e->d * e->d;
-    if (looks > (long long)kDirectCheck * p.block) a.check = 0;
-    else if (e->dir_wait > 0) { a.check = 0; --e->dir_wait; }
+    if (e->dir_wait > 0) --e->dir_wait;
     void *k = direct_for(p.W);
     e->last_ms = 0.0;
     if (e->dir_dirty) {
@@ -1085,6 +1097,7 @@ gg_status run_eval(gg_engine *e, const int32_t *d_table_in, const gg_eval_opts *
             p = direct_plan(e, ns_all, wvc, false);
         }
         if (p.W) return direct_eval(e, p, d_table_in, nullptr, o, s0, ns_all, cap_req, r, st);
+        if (e->dir_wait > 0) --e->dir_wait;
     }
     const int nb_plain = (ns_all + e->batch_bits - 1) / e->batch_bits;
     int nb = sweep ? sweep_batches(e) : nb_plain;

@@ -231,3 +231,29 @@ def test_an_engine_takes_the_memory_of_what_it_runs(n, d):
         r = e.eval(t)
         assert (r["total"], r["reached"], r["levels"]) == (o.total(), int(o.reached.sum()), o.levels)
     e.close()
+
+
+@pytest.mark.parametrize("n,d,oneway", [(3000, 40, 0), (9000, 24, 0), (1000, 64, 0), (20000, 10, 1), (14000, 13, 1)])
+def test_calls_take_no_longer_than_the_level_loop(n, d, oneway, monkeypatch):
+    """High degrees, and tables whose first levels no walk takes.  (Least of many, in turn.)"""
+    import time
+    q = -(-d // 12)
+    t = np.ascontiguousarray(np.concatenate([G.random_regular(n, (d + k) // q, k) for k in range(q)], axis=1))
+    if oneway:
+        t[5, 0] = (t[5, 0] + 1) % n
+    monkeypatch.setenv("GG_DIRECT", "0")
+    monkeypatch.setenv("GG_SWEEP", "0")
+    loop = G.cudaASPLgraph(n, d)
+    monkeypatch.delenv("GG_DIRECT")
+    monkeypatch.delenv("GG_SWEEP")
+    e = G.cudaASPLgraph(n, d)
+    best, seen = {loop: 1e9, e: 1e9}, set()
+    for _ in range(30):
+        for h in (loop, e):
+            t0 = time.perf_counter()
+            seen.add(h.calc(t))
+            best[h] = min(best[h], time.perf_counter() - t0)
+    assert len(seen) == 1
+    assert best[e] < 1.2 * best[loop], best
+    loop.close()
+    e.close()
