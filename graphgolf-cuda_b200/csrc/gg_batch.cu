@@ -26,9 +26,10 @@
 // 221 of 4096 (d = 8) on average, against 406, 1859 and 1116 affected ones.
 // The diameter is the larger of the largest new distance from T and the largest old
 // distance between vertices outside T.  Bases that are not symmetric, not connected or of
-// diameter above 15, candidates whose removed edges the base does not hold (or not
-// equally often at both ends) and the histogram pass search every source;
-// GG_BATCH_FULL=1 makes every candidate do so.
+// diameter above 15, small bases and populations (kIncMinN, worth_near), candidates whose
+// removed edges the base does not hold (or not equally often at both ends) and the histogram
+// pass search every source.  GG_BATCH_FULL=1 makes every candidate do so, 0 none of the
+// small ones.
 //
 // batch_select finds each candidate's sources and cuts them into work units; the units
 // come off one counter, and the candidate and base counts are read from device memory, so
@@ -72,6 +73,7 @@ struct BatchBase {
     int levels;
     int radius;           // floor((levels - 1) / 2)
     int valid;            // symmetric, connected, diameter <= 15
+    int few_near;         // near sources even where a population's full searches fill no wave of blocks
 };
 
 // How a candidate is scored.
@@ -121,6 +123,7 @@ struct BatchArgs {
     int tbits_stride;
     Unit *units;
     int force_full;       // every candidate searches every source
+    int wave;             // blocks of batch_kernel that run at once
 };
 
 __device__ __forceinline__ uint4 z4() { return make_uint4(0u, 0u, 0u, 0u); }
@@ -547,6 +550,7 @@ __global__ void __launch_bounds__(128) batch_select(const BatchArgs a, const int
         const int f = i == 0 ? sr.f[0] : i == 1 ? sr.f[1] : i == 2 ? sr.f[2] : sr.f[3];
         const int t = i == 0 ? sr.t[0] : i == 1 ? sr.t[1] : i == 2 ? sr.t[2] : sr.t[3];
         int mode = a.force_full || !B.valid ? kFull : (sw.a < 0 ? kBase : kNear);
+        if (mode == kNear && !B.few_near && (long long)n_cand * B.chunks <= a.wave) mode = kFull;
         if (mode == kNear) {
             // both ends list each removed edge equally often (the edited graph is symmetric)
             int c[4] = {0, 0, 0, 0};
@@ -676,6 +680,7 @@ struct gg_batch {
     double last_ms = 0.0;
     // near-source mode
     bool full_only = false;                // GG_BATCH_FULL=1: every candidate searches every source
+    bool near_always = false;              // GG_BATCH_FULL=0: near sources also where they do not pay
     std::vector<uint4 *> base_planes;      // per base: [kPlanes][n][cols]
     std::vector<unsigned *> base_stats;    // per base: rowsum[n], ecc[n], top[n]
     std::vector<std::pair<std::pair<int, int>, gg_engine *>> engines;  // per (n, degree): base passes
@@ -788,6 +793,7 @@ gg_status enqueue(gg_batch *b, const gg_swap *cands, gg_cand_result *out, cudaSt
     a.tbits = b->d_tbits; a.tbits_stride = b->tbits_stride;
     a.units = b->d_units;
     a.force_full = b->full_only || hist;   // the histogram pass searches every source of its one candidate
+    a.wave = b->near_always ? 0 : b->grid;
     batch_reset<<<64, 256, 0, st>>>(a);
     const unsigned long long blocks = (unsigned long long)b->cap * ((b->list_stride + 1023) / 1024);
     batch_select<<<(int)std::min<unsigned long long>(blocks, 148ull * 16), 128, 0, st>>>(a, b->list_stride);
@@ -798,6 +804,23 @@ gg_status enqueue(gg_batch *b, const gg_swap *cands, gg_cand_result *out, cudaSt
 }
 
 constexpr int kIncMaxN = 16384;   // larger bases search every source (planes of 4 n^2/8 bytes)
+// ... and smaller ones than this, whose T is most of them: populations of 1 to 2048, near /
+// full: n = 256, d = 4: 60 to 223 us / 48 to 184; n = 64, d = 3: 60 to 207 / 48 to 163 (n = 300, d = 6:
+// 60 to 213 / 51 to 213; and no base pass: set_base and 32 moves 165 / 72).
+constexpr int kIncMinN = 257;
+
+// Whether T is so small that a unit of it is worth finding even where the full searches of
+// a population run side by side (each then costs one unit's time, and batch_select 12 us):
+// rows at most a quarter as wide, of a base of more than 512 vertices.  32 moves, near /
+// full: n = 1000, d = 6: 62 / 73 us, d = 3: 110 / 75; n = 1500, d = 4: 97 / 77; n = 512, d = 3: 75 / 62;
+// n = 700, d = 12: 60 / 73.  T is put at 0.8 of four balls of the radius in the tree.
+bool worth_near(const BatchBase &B) {
+    double ball = 1.0, ring = B.d;
+    for (int k = 1; k <= B.radius && ball < B.n; ++k, ring *= B.d - 1) ball += ring;
+    int l = 0;
+    while (l < B.log_nc && (128 << l) < 0.8 * 4.0 * std::min<double>(ball, B.n)) ++l;
+    return B.n > 512 && l + 2 <= B.log_nc;
+}
 
 // The base pass of base `id` (near-source mode): the single-graph engine
 // evaluates the base with its distance planes (at most 16 levels), then every
@@ -808,7 +831,7 @@ gg_status base_pass(gg_batch *b, int id) {
     BatchBase &B = b->bases[id];
     const cudaStream_t st = b->stream;
     B.valid = 0;
-    if (!b->full_only && B.n <= kIncMaxN) {
+    if (!b->full_only && (B.n >= kIncMinN || b->near_always) && B.n <= kIncMaxN) {
         gg_engine *eng = nullptr;
         for (auto &pe : b->engines)
             if (pe.first == std::make_pair(B.n, B.d)) eng = pe.second;
@@ -859,6 +882,7 @@ gg_status base_pass(gg_batch *b, int id) {
             B.planes = b->base_planes[id];
             B.rowsum = b->base_stats[id];
             B.ecc = b->base_stats[id] + B.n;
+            B.few_near = worth_near(B);
         }
     }
     GB_CK(cudaMemcpyAsync(b->d_bases + id, &B, sizeof(BatchBase), cudaMemcpyHostToDevice, st));
@@ -927,6 +951,7 @@ gg_status gg_batch_create(int device, gg_batch **out) {
     std::memset(b->h_ctl, 0, sizeof(BatchCtl));
     const char *f = std::getenv("GG_BATCH_FULL");
     b->full_only = f && std::atoi(f) != 0;
+    b->near_always = f && !b->full_only;
     *out = b;
     return GG_OK;
 }
@@ -991,6 +1016,7 @@ gg_status gg_batch_set_chunk(gg_batch *b, int base_id, int sources) {
     if (!log_nc_fits(B.n, B.d, l)) return bfail(GG_BAD_ARG, "chunk does not fit in shared memory");
     B.log_nc = l;
     B.chunks = (B.n + (128 << l) - 1) / (128 << l);
+    B.few_near = worth_near(B);
     GB_CK(cudaSetDevice(b->device));
     return refresh_plan(b);
 }

@@ -190,3 +190,34 @@ def test_bases_added_while_other_copies_are_under_way():
         assert (int(got["total"]), int(got["reached"])) == (total, n * n)
         b.close()
     torch.cuda.synchronize()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", [k for k in bases()])
+def test_every_candidate_near_equals_the_oracle(name, monkeypatch):
+    """GG_BATCH_FULL=0: near sources also where a population is small."""
+    monkeypatch.setenv("GG_BATCH_FULL", "0")
+    test_near_candidates_equal_the_oracle(name)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,d,count", [(64, 3, 32), (256, 4, 2048), (1000, 3, 32), (1500, 4, 8)])
+def test_small_populations_take_no_longer_than_their_full_search(n, d, count, monkeypatch):
+    """Populations and steps of an annealer (least of many, both in turn)."""
+    import time
+    adj = G.random_regular(n, d, 1)
+    sw = G.gen_swaps(adj, 0, count, 5)
+    monkeypatch.setenv("GG_BATCH_FULL", "1")
+    full = G.Batch(0)
+    monkeypatch.delenv("GG_BATCH_FULL")
+    b = G.Batch(0)
+    for h in (full, b):
+        assert h.add_base(adj) == 0
+    best = {full: 1e9, b: 1e9}
+    for _ in range(60):
+        for h in (full, b):
+            t = time.perf_counter()
+            h.eval(sw)
+            best[h] = min(best[h], time.perf_counter() - t)
+    assert b.eval(sw).tobytes() == full.eval(sw).tobytes()
+    assert best[b] < 1.12 * best[full], best
