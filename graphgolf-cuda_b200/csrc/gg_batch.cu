@@ -503,6 +503,8 @@ __global__ void __launch_bounds__(128) batch_finalize(const BatchArgs a) {
 // point gets candidates the host never saw): base registered, endpoints inside the
 // base, distinct, mode 0 or 1.  One bad candidate sets ctl->bad, and the kernels
 // after this one return before reading a base or a row through it.
+// With force_full it makes the work units, too (a histogram pass is 3 to 8 us longer with a
+// launch of batch_select for them).
 __global__ void batch_reset(const BatchArgs a) {
     const int n_cand = a.ctl->n_cand;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_cand; i += gridDim.x * blockDim.x) {
@@ -519,6 +521,11 @@ __global__ void batch_reset(const BatchArgs a) {
         if (!ok) {
             atomicExch(&a.ctl->bad, 1);
             atomicMin(&a.ctl->bad_index, i);
+        } else if (a.force_full) {
+            const BatchBase &B = a.bases[sw.base];
+            const int S = 128 << B.log_nc, u0 = atomicAdd(&a.ctl->n_units, B.chunks);
+            a.cs[i].mode = kFull;
+            for (int k = 0; k < B.chunks; ++k) a.units[u0 + k] = Unit{i, k * S, min(S, B.n - k * S), B.log_nc};
         }
     }
 }
@@ -549,7 +556,7 @@ __global__ void __launch_bounds__(128) batch_select(const BatchArgs a, const int
         const int r = i == 0 ? sr.r[0] : i == 1 ? sr.r[1] : i == 2 ? sr.r[2] : sr.r[3];
         const int f = i == 0 ? sr.f[0] : i == 1 ? sr.f[1] : i == 2 ? sr.f[2] : sr.f[3];
         const int t = i == 0 ? sr.t[0] : i == 1 ? sr.t[1] : i == 2 ? sr.t[2] : sr.t[3];
-        int mode = a.force_full || !B.valid ? kFull : (sw.a < 0 ? kBase : kNear);
+        int mode = !B.valid ? kFull : (sw.a < 0 ? kBase : kNear);
         if (mode == kNear && !B.few_near && (long long)n_cand * B.chunks <= a.wave) mode = kFull;
         if (mode == kNear) {
             // both ends list each removed edge equally often (the edited graph is symmetric)
@@ -781,8 +788,8 @@ gg_status ensure_cap(gg_batch *b, int n) {
     return GG_OK;
 }
 
-// Enqueue reset -> select -> batch kernel -> finalize on `st` for candidates `cands`,
-// results `out`; the candidate count comes from d_ctl.
+// Enqueue reset -> select (unless every candidate is searched in full) -> batch kernel ->
+// finalize on `st` for candidates `cands`, results `out`; the candidate count comes from d_ctl.
 gg_status enqueue(gg_batch *b, const gg_swap *cands, gg_cand_result *out, cudaStream_t st,
                   unsigned *hist = nullptr, int hist_k = 0) {
     BatchArgs a{};
@@ -796,7 +803,7 @@ gg_status enqueue(gg_batch *b, const gg_swap *cands, gg_cand_result *out, cudaSt
     a.wave = b->near_always ? 0 : b->grid;
     batch_reset<<<64, 256, 0, st>>>(a);
     const unsigned long long blocks = (unsigned long long)b->cap * ((b->list_stride + 1023) / 1024);
-    batch_select<<<(int)std::min<unsigned long long>(blocks, 148ull * 16), 128, 0, st>>>(a, b->list_stride);
+    if (!a.force_full) batch_select<<<(int)std::min<unsigned long long>(blocks, 148ull * 16), 128, 0, st>>>(a, b->list_stride);
     batch_kernel<<<b->grid, kBatchBlock, b->smem, st>>>(a);
     batch_finalize<<<(int)std::min((b->cap + 3) / 4, 148 * 8), 128, 0, st>>>(a);
     GB_CK(cudaGetLastError());
