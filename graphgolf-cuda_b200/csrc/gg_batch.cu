@@ -687,6 +687,7 @@ struct gg_batch {
     double last_ms = 0.0;
     // near-source mode
     bool full_only = false;                // GG_BATCH_FULL=1: every candidate searches every source
+    bool any_near = false;                 // some base is valid (batch_select is launched)
     bool near_always = false;              // GG_BATCH_FULL=0: near sources also where they do not pay
     std::vector<uint4 *> base_planes;      // per base: [kPlanes][n][cols]
     std::vector<unsigned *> base_stats;    // per base: rowsum[n], ecc[n], top[n]
@@ -799,7 +800,7 @@ gg_status enqueue(gg_batch *b, const gg_swap *cands, gg_cand_result *out, cudaSt
     a.lists = b->d_lists; a.list_stride = b->list_stride;
     a.tbits = b->d_tbits; a.tbits_stride = b->tbits_stride;
     a.units = b->d_units;
-    a.force_full = b->full_only || hist;   // the histogram pass searches every source of its one candidate
+    a.force_full = !b->any_near || hist;   // the histogram pass searches every source of its one candidate
     a.wave = b->near_always ? 0 : b->grid;
     batch_reset<<<64, 256, 0, st>>>(a);
     const unsigned long long blocks = (unsigned long long)b->cap * ((b->list_stride + 1023) / 1024);
@@ -894,6 +895,10 @@ gg_status base_pass(gg_batch *b, int id) {
     }
     GB_CK(cudaMemcpyAsync(b->d_bases + id, &B, sizeof(BatchBase), cudaMemcpyHostToDevice, st));
     GB_CK(cudaStreamSynchronize(st));
+    bool any = false;
+    for (auto &x : b->bases) any |= x.valid != 0;
+    if (any != b->any_near) drop_graph(b);
+    b->any_near = any;
     return GG_OK;
 }
 
