@@ -608,26 +608,25 @@ __device__ __forceinline__ unsigned skip_group(const unsigned tiles, const bool 
 // One visited-set pull level over the block's tiles [s_next, t_hi) (s_next set by the
 // caller); returns this thread's count of new pairs (no_own: of the pairs in the
 // rows it wrote, padding included; every chunk is then written).  nf_use (the skip-full stage,
-// with nfc written whole by the level before): a warp takes a group of tiles, passes over
+// with nfc written whole by the level before): a warp takes s_next[1] tiles, passes over
 // those whose chunks are all full, and runs the others LAZY.
 template <int D>
 static __device__ __noinline__ unsigned vpull_level(const BfsArgs &a, const int d, const int32_t *adj,
-                                                    const unsigned v_base, const unsigned t_lo, const unsigned t_hi,
+                                                    const unsigned v_base, const unsigned t_hi,
                                                     const uint4 *X, uint4 *Y, const uint32_t *fc, uint32_t *fn,
                                                     const uint32_t *nfc, uint32_t *nfn, const bool dense, const bool wr_all,
                                                     const bool skip_full, const bool split, const bool nf_use,
-                                                    const bool nf_many, const bool no_own, unsigned *s_next) {
+                                                    const bool no_own, unsigned *s_next) {
     const unsigned lane = threadIdx.x & 31u;
     unsigned cnt = 0u;
     if (nf_use) {
-        const unsigned group = skip_group(t_hi - t_lo, nf_many);
         for (;;) {
             unsigned tile0 = 0;
-            if (lane == 0) tile0 = atomicAdd(s_next, group);
+            if (lane == 0) tile0 = atomicAdd(s_next, s_next[1]);
             tile0 = __shfl_sync(0xffffffffu, tile0, 0);
             if (tile0 >= t_hi) break;
             const unsigned my = tile0 + lane;
-            const bool in = lane < group && my < t_hi;
+            const bool in = lane < s_next[1] && my < t_hi;
             const unsigned w = in ? __ldcg(nfc + my) : 0u;
             if (in && w == 0u) {
                 fn[my] = 0u;
@@ -1851,7 +1850,7 @@ __global__ void __launch_bounds__(kBlock, min_blocks_for(D)) bfs_batch_kernel(co
     const unsigned items = a.items, ntiles = (items + 31u) >> 5;
     __shared__ unsigned long long s_sum[kBlock / 32];
     __shared__ unsigned s_and[2][kBlock / 32];
-    __shared__ unsigned s_next;
+    __shared__ unsigned s_next[2];   // the block's next tile; tiles a warp takes at once (skip-full stage)
     __shared__ LoopState S;
     if (a.bad && *a.bad) return;  // uniform across the grid: no block reaches a barrier
     unsigned epoch = 0u;          // grid barriers passed
@@ -1976,7 +1975,13 @@ __global__ void __launch_bounds__(kBlock, min_blocks_for(D)) bfs_batch_kernel(co
                                c_prev * 1000000ull >= pairs * (unsigned long long)a.dense_r_ppm;
             const bool skip_full = S.reached * 1000000ull >= pairs * (unsigned long long)a.full_skip_ppm;
             const bool nf_use = !push && skip_full && S.nf_valid;
-            const bool nf_many = (pairs - S.reached) * 4ull > ntiles;
+            // (kLate: counted where it is used.  The kernel is at its 64 registers, and which of its
+            // values spill in the loops before decides 5 to 10 % of a level there; 2500 sources x
+            // 1000000 rows, here / there: d = 4: 1988 / 1855 us, d = 6: 2029 / 2138.  The group in
+            // shared memory for vpull_level, not among its arguments: d = 8: 2525 -> 2386, d = 12: 2220
+            // -> 2400)
+            constexpr bool kLate = D == 4;
+            const bool nf_many = !kLate && (pairs - S.reached) * 4ull > ntiles;
             const bool split = dense && S.reached * 1000000ull >= pairs * (unsigned long long)a.split_ppm;
             const bool write_all =
                 !nf_use && c_prev * 1000000ull >= pairs * (unsigned long long)a.dense_w_ppm;
@@ -2008,22 +2013,23 @@ __global__ void __launch_bounds__(kBlock, min_blocks_for(D)) bfs_batch_kernel(co
                 const uint4 *X = first ? S.Pv : (even ? S.Qv : R);
                 uint4 *Y = first ? S.Qv : (even ? R : S.Qv);
                 if (threadIdx.x == 0) {
-                    s_next = t_lo;
+                    s_next[0] = t_lo;
+                    s_next[1] = skip_group(t_hi - t_lo, kLate ? (pairs - S.reached) * 4ull > ntiles : nf_many);
                     if (L == a.walk_K + 2) S.r_on = r_on;
                 }
                 __syncthreads();
                 if (D > 0 && no_own && !nf_use && a.nC == 32)
                     cnt = dense_rows32<(D > 0 ? D : 1), true>(X, Y, adj, v_base, 1u, t_hi, odd ? a.fl1 : a.fl0,
-                                                              odd ? a.nf2 : a.nf, split, &s_next);
+                                                              odd ? a.nf2 : a.nf, split, s_next);
                 else if (D > 0 && no_own && !nf_use && a.nC % 32 == 0)
                     cnt = dense_rows32<(D > 0 ? D : 1), false>(X, Y, adj, v_base, (unsigned)a.nC / 32u, t_hi,
-                                                               odd ? a.fl1 : a.fl0, odd ? a.nf2 : a.nf, split, &s_next);
+                                                               odd ? a.fl1 : a.fl0, odd ? a.nf2 : a.nf, split, s_next);
                 else
-                    cnt = vpull_level<D>(a, d, adj, v_base, t_lo, t_hi, X, Y,
+                    cnt = vpull_level<D>(a, d, adj, v_base, t_hi, X, Y,
                                          first ? S.fl_walk : (odd ? a.fl0 : a.fl1), odd ? a.fl1 : a.fl0,
                                          odd ? a.nf : a.nf2, odd ? a.nf2 : a.nf, dense,
-                                         first || (L == a.walk_K + 2 && r_on), skip_full, split, nf_use, nf_many, no_own,
-                                         &s_next);
+                                         first || (L == a.walk_K + 2 && r_on), skip_full, split, nf_use, no_own,
+                                         s_next);
             } else {
                 const uint4 *Fc = in_p >= 0 ? (in_p ? a.P1 : a.P0) : (odd ? a.F0 : a.F1);
                 const uint32_t *fc = in_p >= 0 ? (in_p ? a.pf1 : a.pf0) : (odd ? a.fl0 : a.fl1);
@@ -2031,16 +2037,16 @@ __global__ void __launch_bounds__(kBlock, min_blocks_for(D)) bfs_batch_kernel(co
                 uint32_t *fn = odd ? a.fl1 : a.fl0;
                 // Balanced contiguous tile range per block; the block's warps pull
                 // tiles from it through a shared-memory counter.
-                if (threadIdx.x == 0) s_next = t_lo;
+                if (threadIdx.x == 0) s_next[0] = t_lo;
                 __syncthreads();
                 if (nf_use) {
                     // Skip-full stage: a warp takes a group of tiles, reads their not-full
                     // words in one load, clears the frontier flags of the full ones
                     // and works only on the others.
-                    const unsigned group = skip_group(t_hi - t_lo, nf_many);
+                    const unsigned group = skip_group(t_hi - t_lo, kLate ? (pairs - S.reached) * 4ull > ntiles : nf_many);
                     for (;;) {
                         unsigned tile0 = 0;
-                        if (lane == 0) tile0 = atomicAdd(&s_next, group);
+                        if (lane == 0) tile0 = atomicAdd(s_next, group);
                         tile0 = __shfl_sync(0xffffffffu, tile0, 0);
                         if (tile0 >= t_hi) break;
                         const unsigned my = tile0 + lane;
@@ -2056,7 +2062,7 @@ __global__ void __launch_bounds__(kBlock, min_blocks_for(D)) bfs_batch_kernel(co
                 } else {
                     for (;;) {
                         unsigned tile0 = 0;
-                        if (lane == 0) tile0 = atomicAdd(&s_next, (unsigned)kGrab);
+                        if (lane == 0) tile0 = atomicAdd(s_next, (unsigned)kGrab);
                         tile0 = __shfl_sync(0xffffffffu, tile0, 0);
                         if (tile0 >= t_hi) break;
                         level_tiles<D, kGrab, MODE>(a, d, adj, v_base, tile0, t_hi, Fc, Fn, fc, fn, dense,
