@@ -898,7 +898,7 @@ struct gg_lift {
     bool base_set = false;
     float last_ms = 0.f;
     // moves by change
-    int delta_on = 0;                                // buffers: 0 not there yet, 1 there, -1 past the limits or no memory
+    bool delta_on = false;                           // the lift is within the limits and the buffers are there
     bool delta_always = false;                       // whatever delta_pays says (GG_LIFT_SEARCH=0)
     int delta_wait = 0;                              // evaluations until it is tried again
     int base_state = 0;                              // distances of the base: 0 not computed, 1 usable, -1 not usable
@@ -1018,11 +1018,8 @@ bool delta_pays(gg_lift *h, const int n) {
     return h->base_state == 1 || (double)h->base_cands >= 2.0 + more / each + 4.3 + 193.0 / each;
 }
 
-// Buffers of the moves by change, for the first population that goes that way.  Without
-// them candidates are searched.
-bool delta_open(gg_lift *h) {
-    if (h->delta_on) return h->delta_on > 0;
-    h->delta_on = -1;
+// Buffers of the moves by change.  Without them candidates are searched.
+void delta_open(gg_lift *h) {
     const size_t pitch = ((size_t)h->N + 15) / 16 * 16;
     h->pitch = (int)pitch;
     h->rw = (h->d + 2 + 7) / 8 * 8;
@@ -1052,7 +1049,7 @@ bool delta_open(gg_lift *h) {
     if (e == cudaSuccess) e = cudaMalloc(&h->d_arena, at);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
-        return false;
+        return;
     }
     h->d_planes = reinterpret_cast<uint4 *>(h->d_arena + o_planes);
     h->d_dist = h->d_arena + o_dist;
@@ -1061,8 +1058,7 @@ bool delta_open(gg_lift *h) {
     h->d_ball = reinterpret_cast<uint32_t *>(h->d_arena + o_ball);
     h->d_spill = reinterpret_cast<uint32_t *>(h->d_arena + o_spill);
     h->d_ctr = reinterpret_cast<int *>(h->d_arena + o_ctr);
-    h->delta_on = 1;
-    return true;
+    h->delta_on = true;
 }
 
 // Per-candidate buffers of the moves by change; false: not enough memory.
@@ -1175,7 +1171,7 @@ gg_status lift_open(int axes, const int n_in[3], const int m_in[3], int degree, 
     if (s != GG_OK) return fail(s);
     const char *search = std::getenv("GG_LIFT_SEARCH");   // 1: search every candidate, 0: none that can go by change
     h->delta_always = search && std::atoi(search) == 0;
-    if ((search && !h->delta_always) || !delta_fits(h)) h->delta_on = -1;
+    if (!(search && !h->delta_always) && delta_fits(h)) delta_open(h);
     *out = h;
     return GG_OK;
 }
@@ -1482,10 +1478,10 @@ gg_status gg_lift_eval(gg_lift *h, int n_cand, const gg_lift_edit *edits, int ma
             }
         }
     }
-    const bool can = h->delta_on >= 0 && h->group == 0 && h->base_state >= 0;
+    const bool can = h->delta_on && h->group == 0 && h->base_state >= 0;
     if (can && h->delta_wait > 0) {
         --h->delta_wait;
-    } else if (can && delta_pays(h, n_cand) && delta_open(h) && delta_ensure(h, n_cand)) {
+    } else if (can && delta_pays(h, n_cand) && delta_ensure(h, n_cand)) {
         if (h->base_state == 0) {
             const gg_lift_edit first = h->h_ed[0];
             s = delta_base(h);
