@@ -987,18 +987,19 @@ namespace {
 // Moves by change: 16-bit vertex and orbit ids, a distance row within a block's shared
 // memory (at 64 KB three blocks a SM), and 1 GiB of distance rows.  The row of an edited
 // orbit loses one of its d subtrees, about N / d vertices and more when few others reach
-// them as soon, so a small degree outgrows the lists (kDeltaList + kDeltaSpill) in nearly
-// every candidate, which is then searched as well.  256 candidates, by change / searched:
-// m = 418, g = 23, d = 4: 2185 / 1274 us (87 % outgrew them), m = 512, g = 64, d = 8: 5653 /
-// 3188 (all); m = 546, g = 10, d = 4: 700 / 988 (6 %), m = 1024, g = 32, d = 12: 1779 / 6053
-// (0.4 %).
+// them as soon; past a size that outgrows the lists (kDeltaList + kDeltaSpill) in nearly every
+// candidate, which is then searched as well.  128 candidates, N / (d - 2), by change / searched:
+// m = 1000, g = 18, d = 6, 4500: 2739 / 1918 us (125 of 128 searched); m = 1022, g = 22, d = 7, 4497:
+// 3884 / 2976; m = 1022, g = 32, d = 10, 4088: 1563 / 3048 (14); m = 1000, g = 24, d = 8, 4000: 1216 /
+// 2300 (7); m = 1022, g = 48, d = 12, 4906: 2248 / 4708 (17), g = 52, 5314: 6634 / 4993.  (Which side of
+// the line a lift near it falls turns on its diameter, too: gg_lift_eval looks.)
 constexpr size_t kDeltaRowBytes = 24 * 1024;   // rows of a block, when one is smaller
 constexpr size_t kDeltaMostBytes = 64 * 1024;  // one row of the largest lift
-constexpr int kDeltaMostPerDegree = 3600;      // N / (d - 2): 2730 and 3277 for the last two, 4807 and 5461 for the first
+constexpr int delta_most(int d) { return (d >= 12 ? 5000 : 4300) * (d - 2); }   // vertices
 bool delta_fits(const gg_lift *h) {
     const size_t pitch = ((size_t)h->N + 15) / 16 * 16;
     return h->N <= 65536 && h->M <= 65535 && h->N / h->M <= 65535 && pitch * h->M <= (1ull << 30) &&
-           (h->delta_always || (long long)h->N <= (long long)kDeltaMostPerDegree * (h->d - 2));
+           (h->delta_always || h->N <= delta_most(std::min(h->d, 64)));
 }
 
 // Whether a population of n goes by change.  Microseconds, fits over 35 lifts (N = 512 to
@@ -1493,13 +1494,17 @@ gg_status gg_lift_eval(gg_lift *h, int n_cand, const gg_lift_edit *edits, int ma
             std::vector<int> left;
             s = delta_eval(h, n_cand, max_levels, out, left);
             if (s != GG_OK || left.empty()) return s;
-            // the rest is searched (and the next populations whole, when that is a lot)
-            if (left.size() * 4 > (size_t)n_cand && !h->delta_always) h->delta_wait = 63;
+            // the rest is searched
             for (size_t i = 0; i < left.size(); ++i) h->h_ed[i] = h->h_ed[left[i]];
             std::vector<gg_cand_result> res(left.size());
             const float ms = h->last_ms;
             s = lift_search(h, (int)left.size(), max_levels, res.data());
             if (s != GG_OK) return s;
+            // (a search: 80 us and a time a candidate; when they are an eighth or more and all of
+            // them would have taken less, the next populations are searched)
+            const float each = std::max(h->last_ms - 0.08f, 0.f) / (float)left.size();
+            if (left.size() * 8 > (size_t)n_cand && ms + h->last_ms > 0.08f + each * (float)n_cand && !h->delta_always)
+                h->delta_wait = 63;
             h->last_ms += ms;
             for (size_t i = 0; i < left.size(); ++i) out[left[i]] = res[i];
             return GG_OK;
