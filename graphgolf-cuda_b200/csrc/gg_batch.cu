@@ -7,7 +7,7 @@
 // with both visited bitsets resident in shared memory:
 //     next[v][c] = cur[v][c] | (OR_{u in adj[v]} cur[u][c])        (all rows, one level)
 // i.e. the level step of cudaASPLconv.cu:35-56 with the reduction of :59-99
-// folded into per-thread popcounts and one __syncthreads_or per level.  The grid
+// folded into per-thread popcounts, a shared sum and one block barrier per level.  The grid
 // barrier of the single-graph path is not needed: a task never leaves its CTA.
 //
 // Near sources (default): per base, one pass of the single-graph engine also writes the

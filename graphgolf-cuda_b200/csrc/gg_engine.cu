@@ -573,7 +573,9 @@ void *walk_all_of(int K) {
 // batch): visited-set pull levels, batches of a multiple of 4096 sources, degree 3, 4, 6
 // or 8, K <= 3 (with the level-2 table, or 16-byte rows), and the level-K rows of all nb
 // batches within the GG_WALK_ALL_MB budget.  Grows d_vall as needed (a failed allocation
-// falls back to the per-batch pass).
+// falls back to the per-batch pass).  Only where the level loop runs a graph at all: after
+// sweep_kernel gave up, source ranges, per-level times (one-way n = 30011, d = 6, degree 6
+// walked for all batches: 784 -> 680 us).
 void *walk_all_for(gg_engine *e, int K, int nb) {
     if (!e->walk_vpull || e->nC % 32 != 0 || K < 1 || K > 3 || nb * (e->nC / 32) * K > gg::kIndexMaxKeys) return nullptr;
     if (e->d != 3 && e->d != 4 && e->d != 6 && e->d != 8) return nullptr;
