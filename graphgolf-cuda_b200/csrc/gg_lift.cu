@@ -1002,21 +1002,24 @@ bool delta_fits(const gg_lift *h) {
            (h->delta_always || h->N <= delta_most(std::min(h->d, 64)));
 }
 
-// Whether a population of n goes by change.  Microseconds, fits over 35 lifts (N = 512 to
-// 32768, d = 4 to 12): a searched candidate takes `each`, one by change about a third of
-// that; by change a population takes `more` longer before its first candidate (its waves
-// are chains, longer at small degrees); the distances of a new base take 135 and three
-// searched candidates.  They are worth it once the candidates seen on the base would have
-// paid for them: 32 candidates on a new base are searched at m = 500, g = 12, d = 6 (148 us,
-// 314 by change) and go by change at m = 1024, g = 32, d = 12 (849 / 529); the lines lie
-// at 111 and 17 (both ways alike at about 165 and 14).
+// Whether a population of n goes by change.  Microseconds, fits over 90 lifts (N = 268 to
+// 31062, d = 4 to 12): a searched candidate takes `each`, one by change about a third of that; by
+// change a population takes `more` longer before its first candidate (its waves are chains,
+// longer at small degrees and with many copies edited at once); the distances of a new base
+// take 135 and three searched candidates.  They are worth it once the candidates seen on the
+// base would have paid for them: 32 candidates on a new base are searched at m = 500, g = 12, d
+// = 6 (148 us, 314 by change) and go by change at m = 1024, g = 32, d = 12 (849 / 529).  Where
+// both ways take as long, by this and measured: m = 992, g = 12, d = 6: 38 and 50 candidates;
+// 752, 19, 7: 45, 47; 584, 6, 11: 98, 86; 558, 5, 6: 111, 126; 956, 32, 12: 21, 13; with the
+// distances there 12, 10; 17, 12; 17, 8 at most; 20, 15; 7, 8 at most.
 bool delta_pays(gg_lift *h, const int n) {
     if (h->delta_always) return true;
-    const double each = 1.2 + 9e-6 * (double)h->N * h->cpc * h->d, k = h->d - 2;
-    const double more = std::max(70.0, 0.11 * h->N / (k * std::sqrt(k)));
-    if (n < 2.0 + more / each) return false;
+    const double each = 1.0 + 88e-6 * (double)h->N * h->cpc, k = h->d - 2;
+    const double more = 40.0 + 0.012 * std::max(h->N / h->M - 4, 0) * h->N / (k * k);
+    const double next = 1.5 + more / each;
+    if (n < next) return false;
     h->base_cands += n;
-    return h->base_state == 1 || (double)h->base_cands >= 2.0 + more / each + 4.3 + 193.0 / each;
+    return h->base_state == 1 || (double)h->base_cands >= next + 4.0 + 190.0 / each;
 }
 
 // Buffers of the moves by change.  Without them candidates are searched.
