@@ -807,7 +807,7 @@ DirectPlan direct_plan(const gg_engine *e, int ns, bool wvc, bool sweep) {
     if (best.W) {
         const bool one = best.grid <= e->sms;
         double direct_us = cost / 3.5 * e->rows * (3.2 + 0.1 * e->d) * 1e-3 * (wvc ? 1.1 : 1.0) * (one ? 1.12 : 1.0);
-        if (e->d >= 9 && e->d != 12 && !direct_check(e, best.grid, best.block)) direct_us *= std::min(1.3, 1.0 + 0.06 * (e->d - 7));
+        if (!sweep && e->d >= 9 && e->d != 12 && !direct_check(e, best.grid, best.block)) direct_us *= std::min(1.3, 1.0 + 0.06 * (e->d - 7));
         const double chunks = (double)e->rows * ((ns + 127) / 128);
         if (e->d > 20 && (!best.adj_smem || (e->d > 48 && (long long)e->rows * e->d > 50000))) best.W = 0;
         if (direct_us > 50.0 + (sweep ? kSweepUsPerChunk : kLoopUsPerChunk) * chunks) best.W = 0;
